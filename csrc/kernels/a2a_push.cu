@@ -19,37 +19,81 @@ namespace fastb {
 
 namespace {
 
-__device__ __forceinline__ void copy_bytes(unsigned char* __restrict__ dst, const unsigned char* __restrict__ src, long long bytes) {
+// n 16-byte chunks, both sides aligned: U of them in flight per thread.
+template <int U>
+__device__ __forceinline__ void copy_aligned(int4* __restrict__ d, const int4* __restrict__ s, long long n) {
   const int tid = threadIdx.x, nt = blockDim.x;
-  if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | static_cast<uintptr_t>(bytes)) & 15u) == 0) {
-    const int4* s = reinterpret_cast<const int4*>(src);
-    int4* d = reinterpret_cast<int4*>(dst);
-    const long long n = bytes >> 4;
-    constexpr int U = 8;
-    long long i = tid;
-    for (; i + static_cast<long long>(U - 1) * nt < n; i += static_cast<long long>(U) * nt) {
-      int4 v[U];
+  for (long long i = tid; i < n; i += static_cast<long long>(U) * nt) {
+    int4 v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = __ldcg(s + i + static_cast<long long>(u) * nt);
+    for (int u = 0; u < U; ++u)
+      if (i + static_cast<long long>(u) * nt < n) v[u] = __ldcg(s + i + static_cast<long long>(u) * nt);
 #pragma unroll
-      for (int u = 0; u < U; ++u) __stcg(d + i + static_cast<long long>(u) * nt, v[u]);
+    for (int u = 0; u < U; ++u)
+      if (i + static_cast<long long>(u) * nt < n) __stcg(d + i + static_cast<long long>(u) * nt, v[u]);
+  }
+}
+
+// n 16-byte chunks to an aligned d from a source that starts 4 Q + r bytes (not 0) past the aligned s: chunk i is cut out
+// of the aligned source words i and i + 1. Every word is loaded once, by the lane that owns chunk i, and handed to
+// the lane before it by a shuffle (only the Q + 1 registers of it that the cut reaches into); both sides stay 16-byte
+// accesses. Word n is read too: it holds the last 4 Q + r bytes, so no read leaves a 16-byte block of the source.
+// Reads go to L2: a staged source may still be growing behind the piece, and a line of it must not linger in L1.
+template <int Q, int U>
+__device__ __forceinline__ void copy_shifted(uint4* __restrict__ d, const uint4* __restrict__ s, int r, long long n) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (warp >= nw) return;  // a last warp that is not full has no partners for the shuffles
+  for (long long base = static_cast<long long>(warp) * (32 * U); base < n; base += static_cast<long long>(nw) * (32 * U)) {
+    uint4 v[U], edge = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = base + 32 * u + lane;
+      v[u] = i <= n ? __ldcg(s + i) : make_uint4(0, 0, 0, 0);
     }
-    for (; i < n; i += nt) __stcg(d + i, __ldcg(s + i));
-    return;
+    if (lane == 0 && base + 32 * U <= n) edge = __ldcg(s + base + 32 * U);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint4 follow = u + 1 < U ? v[u + 1 < U ? u + 1 : 0] : edge;   // lane 0's word of the next 32 chunks is lane 31's neighbour
+      uint32_t w[8] = {v[u].x, v[u].y, v[u].z, v[u].w, 0u, 0u, 0u, 0u};
+      const uint32_t give[4] = {lane == 0 ? follow.x : v[u].x, lane == 0 ? follow.y : v[u].y, lane == 0 ? follow.z : v[u].z, lane == 0 ? follow.w : v[u].w};
+#pragma unroll
+      for (int k = 0; k <= Q; ++k) w[4 + k] = __shfl_sync(0xffffffffu, give[k], (lane + 1) & 31);
+      const long long i = base + 32 * u + lane;
+      if (i < n)
+        __stcg(d + i, make_uint4(__funnelshift_r(w[Q], w[Q + 1], 8 * r), __funnelshift_r(w[Q + 1], w[Q + 2], 8 * r),
+                                 __funnelshift_r(w[Q + 2], w[Q + 3], 8 * r), __funnelshift_r(w[Q + 3], w[Q + 4], 8 * r)));
+    }
   }
-  // Unaligned ends: bytes until dst is 16-aligned, then 16-byte stores if src happens to agree,
-  // else a plain byte loop (correct for any offsets; only tiny or odd-sized pieces land here).
-  if ((reinterpret_cast<uintptr_t>(dst) & 15u) == (reinterpret_cast<uintptr_t>(src) & 15u) && bytes >= 32) {
-    const long long head = (16 - (reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u;
-    const long long body = (bytes - head) & ~15ll;
-    for (long long i = tid; i < head; i += nt) dst[i] = src[i];
-    const int4* s = reinterpret_cast<const int4*>(src + head);
-    int4* d = reinterpret_cast<int4*>(dst + head);
-    for (long long i = tid; i < (body >> 4); i += nt) __stcg(d + i, __ldcg(s + i));
-    for (long long i = head + body + tid; i < bytes; i += nt) dst[i] = src[i];
-    return;
+}
+
+// Any offsets and sizes: bytes until the destination is 16-byte aligned, 16-byte stores, bytes for what is left. Segments
+// of odd element counts (2-byte units) put most pieces at different offsets inside 16 bytes on the two sides: copied
+// byte by byte they moved 0.17 TB/s.
+// THREADS: the block size that the registers are budgeted for; the bytes in flight per SM are the same either way.
+template <int THREADS>
+__device__ __forceinline__ void copy_bytes(unsigned char* __restrict__ dst, const unsigned char* __restrict__ src, long long bytes) {
+  constexpr int kAligned = THREADS > 512 ? 4 : 8, kShifted = THREADS > 512 ? 2 : 4;
+  const int tid = threadIdx.x;
+  const long long head = min(static_cast<long long>((16 - (reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u), bytes);
+  const long long n = (bytes - head) >> 4, done = head + (n << 4);
+  if (n > 0) {
+    const unsigned char* from = src + head;
+    const int off = static_cast<int>(reinterpret_cast<uintptr_t>(from) & 15u);
+    if (off == 0) {
+      copy_aligned<kAligned>(reinterpret_cast<int4*>(dst + head), reinterpret_cast<const int4*>(from), n);
+    } else {
+      uint4* d = reinterpret_cast<uint4*>(dst + head);
+      const uint4* s = reinterpret_cast<const uint4*>(from - off);
+      switch (off >> 2) {
+        case 0: copy_shifted<0, kShifted>(d, s, off & 3, n); break;
+        case 1: copy_shifted<1, kShifted>(d, s, off & 3, n); break;
+        case 2: copy_shifted<2, kShifted>(d, s, off & 3, n); break;
+        default: copy_shifted<3, kShifted>(d, s, off & 3, n); break;
+      }
+    }
   }
-  for (long long i = tid; i < bytes; i += nt) dst[i] = src[i];
+  if (tid < head) dst[tid] = src[tid];
+  if (tid < bytes - done) dst[done + tid] = src[done + tid];
 }
 
 // ---- bulk-copy variant of copy_bytes ---------------------------------------------------------------
@@ -118,6 +162,7 @@ __device__ __forceinline__ int phase_of(const A2AWork& w) {
   return w.wait_kind == 2 ? 2 : 3;
 }
 
+template <int THREADS>
 __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
   __shared__ int s_ok;
   // Bytes this CTA has stored into each peer's OUTPUT and not yet announced. Output arrivals are
@@ -159,8 +204,20 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
     st_release_sys(peer_sig + kSigReadyOff + a.rank, a.epoch);
   }
   bool alive = true;
-  for (int it = blockIdx.x; it < a.n_items && alive; it += gridDim.x) {
-    const A2AWork w = a.items[it];
+  // Items whose bytes are only announced at the end are walked in slices, so that the last round of the CTAs is a small
+  // one: 15 rounds of 1 MiB items for 14.2 rounds of work cost 5 %. (8 x 256 MiB on one GPU: 742 us whole, 687 us in
+  // 128 KiB slices, 707 us in 64 KiB ones, whose item reads are no longer hidden.) Staged data keeps whole items: one
+  // barrier and one release each.
+  const int n_slices = a.n_items * a.split;
+  for (int slice = blockIdx.x; slice < n_slices && alive; slice += gridDim.x) {
+    const int it = slice / a.split, part = slice % a.split;
+    A2AWork w = a.items[it];
+    if (a.split > 1) {
+      const long long step = w.signal_kind == 3 ? a.slice_bytes : w.bytes;
+      const long long begin = part * step;
+      if (begin >= w.bytes) continue;
+      w.src_off += begin; w.dst_off += begin; w.bytes = min(step, w.bytes - begin);
+    }
     // Every thread evaluates the same condition (shared memory is only written by thread 0 between
     // barriers), so the barriers below are taken by all threads or by none.
     const bool must_wait = !s_peer_ready[w.dst_rank] || w.wait_kind != 0;
@@ -190,7 +247,7 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
         if (bulk_ok && w.signal_kind != 3) bulk_drain();  // a forwarder waits for this piece: its stores must have landed before the counter moves
       }
     } else {
-      copy_bytes(dst_ptr, src_ptr, w.bytes);
+      copy_bytes<THREADS>(dst_ptr, src_ptr, w.bytes);
     }
     if (w.signal_kind == 3) {
       // Output bytes are announced once, after the whole list (one barrier below covers them all).
@@ -239,8 +296,28 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
   }
 }
 
-__global__ void __launch_bounds__(1024) a2a_push_kernel(const A2ARankArgs a) { run_rank(a); }
-__global__ void __launch_bounds__(1024) a2a_push_group_kernel(const A2ARankArgs* __restrict__ all) { run_rank(all[blockIdx.y]); }
+// THREADS: the block size that the registers are budgeted for. At 1024 the copy loops spill; blocks of up to 512 threads
+// (the default) get the variant that does not.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) a2a_push_kernel(const A2ARankArgs a) { run_rank<THREADS>(a); }
+// Every rank's arguments travel in the launch itself (no upload, so nothing for the host to wait for). The parameter block
+// is sized for 8 or for all kSigMaxWorld ranks: a launch copies the whole block.
+template <int N>
+struct A2AGroupArgs { A2ARankArgs rank[N]; };
+template <int N, int THREADS>
+__global__ void __launch_bounds__(THREADS) a2a_push_group_kernel(const __grid_constant__ A2AGroupArgs<N> all) { run_rank<THREADS>(all.rank[blockIdx.y]); }
+
+template <int N>
+cudaError_t launch_group(const A2ARankArgs* ranks, int n, int ctas, int threads, cudaStream_t stream) {
+  A2AGroupArgs<N> args;
+  std::copy(ranks, ranks + n, args.rank);
+  void* params[] = {&args};
+  // All virtual ranks wait on one another, so they must be co-resident: cooperative launch.
+  void* kern = threads <= 512 ? reinterpret_cast<void*>(a2a_push_group_kernel<N, 512>) : reinterpret_cast<void*>(a2a_push_group_kernel<N, 1024>);
+  cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(ctas, n), dim3(threads), params, 0, stream);
+  if (e == cudaSuccess) note_launch();
+  return e;
+}
 
 __global__ void wait_probe_kernel(const unsigned long long* flag, unsigned long long want, DeviceStatus* st, unsigned long long timeout_ns) {
   if (threadIdx.x == 0) wait_ge_bounded(flag, want, st, kSiteTest, 0, timeout_ns);
@@ -252,42 +329,40 @@ namespace { std::atomic<unsigned long long> g_launches{0}; }
 unsigned long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 void note_launch(int n) { g_launches.fetch_add(static_cast<unsigned long long>(n), std::memory_order_relaxed); }
 
-cudaError_t launch_a2a_push(const A2ARankArgs* host_args, const A2ARankArgs* device_args, int virtual_ranks, int ctas, int threads,
-                            cudaStream_t stream, bool needs_coresidency) {
-  if (ctas < 1 || threads < 32 || threads > 1024 || virtual_ranks < 1) return cudaErrorInvalidValue;
-  if (device_args == nullptr) {
-    if (host_args == nullptr || virtual_ranks != 1) return cudaErrorInvalidValue;
-    const int smem = host_args->bulk ? kBulkSmemBytes : 0;
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(a2a_push_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-    }
-    // The grid never exceeds what one GPU can hold at once. A plan with waiting work items (two-tier plans: forwarders
-    // wait for balance / rail arrivals that peers push, while peers' forwarders wait for what this rank pushes) is
-    // launched cooperatively: the driver then starts it only when the whole grid can be resident, so a waiting CTA
-    // can never keep a pushing one of the same launch off the GPU.
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, a2a_push_kernel, threads, smem);
+cudaError_t launch_a2a_push_group(const A2ARankArgs* ranks, int n, int ctas, int threads, cudaStream_t stream) {
+  if (ctas < 1 || threads < 32 || threads > 1024 || n < 1 || n > kSigMaxWorld || ranks == nullptr) return cudaErrorInvalidValue;
+  return n <= 8 ? launch_group<8>(ranks, n, ctas, threads, stream) : launch_group<kSigMaxWorld>(ranks, n, ctas, threads, stream);
+}
+
+cudaError_t launch_a2a_push(const A2ARankArgs& host_args, int ctas, int threads, cudaStream_t stream, bool needs_coresidency) {
+  if (ctas < 1 || threads < 32 || threads > 1024) return cudaErrorInvalidValue;
+  const int smem = host_args.bulk ? kBulkSmemBytes : 0;
+  auto* kern = threads <= 512 ? a2a_push_kernel<512> : a2a_push_kernel<1024>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-    ctas = std::min(ctas, sms * per_sm);
-    if (needs_coresidency) {
-      A2ARankArgs args = *host_args;
-      void* params[] = {&args};
-      e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(a2a_push_kernel), dim3(ctas), dim3(threads), params, smem, stream);
-      if (e == cudaSuccess) note_launch();
-      return e;
-    }
-    a2a_push_kernel<<<ctas, threads, smem, stream>>>(*host_args);
-    note_launch();
-    return cudaGetLastError();
   }
-  // All virtual ranks wait on one another, so they must be co-resident: cooperative launch.
-  void* params[] = {const_cast<A2ARankArgs**>(&device_args)};
+  // The grid never exceeds what one GPU can hold at once. A plan with waiting work items (two-tier plans: forwarders
+  // wait for balance / rail arrivals that peers push, while peers' forwarders wait for what this rank pushes) is
+  // launched cooperatively: the driver then starts it only when the whole grid can be resident, so a waiting CTA
+  // can never keep a pushing one of the same launch off the GPU.
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+  ctas = std::min(ctas, sms * per_sm);
+  if (needs_coresidency) {
+    A2ARankArgs args = host_args;
+    void* params[] = {&args};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kern), dim3(ctas), dim3(threads), params, smem, stream);
+    if (e == cudaSuccess) note_launch();
+    return e;
+  }
+  kern<<<ctas, threads, smem, stream>>>(host_args);
   note_launch();
-  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(a2a_push_group_kernel), dim3(ctas, virtual_ranks), dim3(threads), params, 0, stream);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_wait_probe(const unsigned long long* flag, unsigned long long want, DeviceStatus* status,

@@ -38,6 +38,8 @@ constexpr int kSigWords = kSigTicketOff + 2;
 struct A2ARankArgs {
   const A2AWork* items;
   int n_items, rank, world, num_stages;
+  int split;                             // slices of slice_bytes that an item is worked off in (>= 1), see run_rank
+  long long slice_bytes;
   void* const* peer_table;               // [world] slab bases (device array)
   const unsigned char* src_base[4];      // local bases of input / output / balance / rail
   long long dst_heap_off[4];             // slab offsets of the same four buffers on every rank
@@ -58,13 +60,11 @@ struct A2ARankArgs {
 };
 constexpr int kPhaseStampWords = 10;
 
-// device_args == nullptr: one real rank, `host_args` is passed by value. Otherwise one cooperative
-// launch with gridDim.y = virtual_ranks runs every rank of an in-process group (single-GPU
-// emulation); `device_args` points to an array of virtual_ranks structs in device memory.
-// needs_coresidency (real ranks): the work list has items that wait for other items of the same launch; the kernel is
-// then launched cooperatively so that its whole grid is resident at once.
-cudaError_t launch_a2a_push(const A2ARankArgs* host_args, const A2ARankArgs* device_args, int virtual_ranks, int ctas,
-                            int threads, cudaStream_t stream, bool needs_coresidency = false);
+// One rank on this GPU. needs_coresidency: the work list has items that wait for other items of the same launch; the
+// kernel is then launched cooperatively so that its whole grid is resident at once.
+cudaError_t launch_a2a_push(const A2ARankArgs& args, int ctas, int threads, cudaStream_t stream, bool needs_coresidency = false);
+// Every rank of an in-process group (single-GPU emulation) as one cooperative launch with gridDim.y = n; n <= kSigMaxWorld.
+cudaError_t launch_a2a_push_group(const A2ARankArgs* ranks, int n, int ctas, int threads, cudaStream_t stream);
 
 // Waits (bounded) on a flag nothing sets; used to test the timeout path without any peer.
 cudaError_t launch_wait_probe(const unsigned long long* flag, unsigned long long want, DeviceStatus* status,

@@ -6,6 +6,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <memory>
 
 #include "py_types.h"
@@ -23,10 +24,12 @@ struct A2AProgramPy {
   int n_items = 0, num_stages = 0;
   bool has_waits = false;  // some item waits for bytes another item of a peer's (or this) launch forwards
   unsigned long long expect_output = 0, expect_balance = 0;
-  int64_t total_bytes = 0;
+  int64_t total_bytes = 0, largest_item = 0;
+  int64_t input_bytes = 0, output_bytes = 0;  // what the rank's input and output hold (checked by the group launch)
 
   // items: int64[k, 10] as produced by Plan.lower(); expect_rail: list of bytes per stage.
-  A2AProgramPy(torch::Tensor items, std::vector<int64_t> expect_rail, int64_t exp_out, int64_t exp_bal, int device) {
+  A2AProgramPy(torch::Tensor items, std::vector<int64_t> expect_rail, int64_t exp_out, int64_t exp_bal, int device,
+               int64_t in_bytes, int64_t out_bytes) : input_bytes(in_bytes), output_bytes(out_bytes) {
     TORCH_CHECK(items.dim() == 2 && items.size(1) == 10 && items.dtype() == torch::kInt64 && items.is_cpu(), "items must be CPU int64[k, 10]");
     TORCH_CHECK(static_cast<int>(expect_rail.size()) <= kSigMaxStages, "too many stages for the signal block");
     n_items = static_cast<int>(items.size(0));
@@ -43,6 +46,7 @@ struct A2AProgramPy {
       w[i].wait_kind = static_cast<unsigned char>(q[6]); w[i].signal_kind = static_cast<unsigned char>(q[7]);
       w[i].stage = static_cast<int>(q[8]); w[i].wait_stage = static_cast<int>(q[9]); w[i].pad_ = 0;
       total_bytes += q[2];
+      largest_item = std::max(largest_item, q[2]);
       if (q[6] != 0) has_waits = true;
     }
     auto dev = torch::Device(torch::kCUDA, device);
@@ -57,6 +61,9 @@ struct A2AProgramPy {
     A2ARankArgs a{};
     a.items = reinterpret_cast<const A2AWork*>(items_dev.data_ptr());
     a.n_items = n_items; a.rank = heap.h->rank(); a.world = heap.h->world(); a.num_stages = num_stages;
+    // Slices of 128 KiB (two passes of the copy loop: 512 threads x 8 x 16 bytes each), at most 16 per item.
+    a.slice_bytes = std::max<int64_t>(128 << 10, (largest_item / 16 + 0xFFFF) & ~int64_t{0xFFFF});
+    a.split = static_cast<int>(std::max<int64_t>(1, (largest_item + a.slice_bytes - 1) / a.slice_bytes));
     a.peer_table = heap.h->device_peer_table();
     for (int i = 0; i < 4; ++i) { a.src_base[i] = reinterpret_cast<const unsigned char*>(src_ptrs[i]); a.dst_heap_off[i] = dst_offs[i]; }
     a.sig_heap_off = sig_off; a.epoch = epoch; a.expect_output = expect_output; a.expect_balance = expect_balance;
@@ -72,21 +79,38 @@ void a2a_launch(const A2AProgramPy& p, const HeapPy& heap, std::array<int64_t, 4
   TORCH_CHECK(heap.h->world() <= kSigMaxWorld, "world larger than the signal block supports");
   A2ARankArgs a = p.args(heap, src_ptrs, dst_offs, sig_off, epoch, st, timeout_ns, stamps_ptr);
   a.bulk = bulk ? 1 : 0;
-  cuda_check(launch_a2a_push(&a, nullptr, 1, ctas, threads, cur_stream(), p.has_waits), "a2a_push launch");
+  cuda_check(launch_a2a_push(a, ctas, threads, cur_stream(), p.has_waits), "a2a_push launch");
 }
 
-// One cooperative launch that runs every virtual rank of an in-process group.
-void a2a_launch_group(std::vector<const A2AProgramPy*> progs, std::vector<const HeapPy*> heaps,
-                      std::vector<std::array<int64_t, 4>> src_ptrs, std::array<int64_t, 4> dst_offs, int64_t sig_off, uint64_t epoch,
-                      std::vector<const StatusPy*> sts, uint64_t timeout_ns, int ctas, int threads) {
-  const int n = static_cast<int>(progs.size());
-  TORCH_CHECK(n >= 1 && static_cast<int>(heaps.size()) == n && static_cast<int>(src_ptrs.size()) == n && static_cast<int>(sts.size()) == n, "one entry per virtual rank");
-  std::vector<A2ARankArgs> host(n);
-  for (int r = 0; r < n; ++r) host[r] = progs[r]->args(*heaps[r], src_ptrs[r], dst_offs, sig_off, epoch, *sts[r], timeout_ns);
-  auto dev = torch::empty({static_cast<int64_t>(n * sizeof(A2ARankArgs))}, torch::TensorOptions().dtype(torch::kUInt8).device(torch::kCUDA, heaps[0]->device));
-  cuda_check(cudaMemcpyAsync(dev.data_ptr(), host.data(), n * sizeof(A2ARankArgs), cudaMemcpyHostToDevice, cur_stream()), "upload group args");
-  cuda_check(launch_a2a_push(nullptr, reinterpret_cast<const A2ARankArgs*>(dev.data_ptr()), n, ctas, threads, cur_stream()), "a2a_push group launch");
-  cuda_check(cudaStreamSynchronize(cur_stream()), "a2a_push group sync");  // args buffer must outlive the launch
+// One cooperative launch that runs every virtual rank of an in-process group. Outputs lie in the ranks' heaps at one common
+// offset (else nothing is launched and the answer is false: the caller stages them); the checks of sizes are made here, so
+// that a small collective is not paid for in interpreter time. stage_offs: heap offsets of the balance and rail areas.
+bool a2a_launch_group(const std::vector<const A2AProgramPy*>& progs, const std::vector<const HeapPy*>& heaps, const std::vector<torch::Tensor>& outs,
+                      const std::vector<torch::Tensor>& ins, std::array<int64_t, 2> stage_offs, int64_t sig_off, uint64_t epoch,
+                      const std::vector<const StatusPy*>& sts, uint64_t timeout_ns, int ctas, int threads) {
+  const size_t n = progs.size();
+  TORCH_CHECK(n >= 1 && n <= static_cast<size_t>(kSigMaxWorld) && heaps.size() == n && outs.size() == n && ins.size() == n && sts.size() == n,
+              "one entry per virtual rank");
+  std::array<int64_t, 4> dst{0, 0, stage_offs[0], stage_offs[1]};
+  std::array<A2ARankArgs, kSigMaxWorld> host;
+  int most = 1;
+  for (size_t r = 0; r < n; ++r) {
+    const int64_t base = reinterpret_cast<int64_t>(heaps[r]->h->local_base());
+    const int64_t out = reinterpret_cast<int64_t>(outs[r].data_ptr()), out_bytes = static_cast<int64_t>(outs[r].nbytes());
+    if (out < base || out + out_bytes > base + static_cast<int64_t>(heaps[r]->h->bytes())) return false;
+    if (r == 0) dst[1] = out - base;
+    if (static_cast<int64_t>(ins[r].nbytes()) < progs[r]->input_bytes) throw py::value_error("input smaller than the schedule needs");
+    if (out_bytes < progs[r]->output_bytes) throw py::value_error("output smaller than the schedule needs");
+    if (out - base != dst[1]) throw std::runtime_error("virtual ranks disagree on symmetric offsets; allocate in the same order on every rank");
+    most = std::max(most, progs[r]->n_items);
+  }
+  for (size_t r = 0; r < n; ++r) {
+    const int64_t base = reinterpret_cast<int64_t>(heaps[r]->h->local_base());
+    host[r] = progs[r]->args(*heaps[r], {reinterpret_cast<int64_t>(ins[r].data_ptr()), 0, base + dst[2], base + dst[3]}, dst, sig_off, epoch, *sts[r], timeout_ns);
+  }
+  // A rank with a handful of work items needs a handful of CTAs (every launched CTA takes a turn at the exit counter).
+  cuda_check(launch_a2a_push_group(host.data(), static_cast<int>(n), std::min(ctas, most), threads, cur_stream()), "a2a_push group launch");
+  return true;
 }
 
 }  // namespace
@@ -134,7 +158,8 @@ PYBIND11_MODULE(_C, m) {
       .def("ptr", [](const StatusPy& s) { return reinterpret_cast<int64_t>(s.d); });
 
   py::class_<A2AProgramPy>(m, "A2AProgram")
-      .def(py::init<torch::Tensor, std::vector<int64_t>, int64_t, int64_t, int>())
+      .def(py::init<torch::Tensor, std::vector<int64_t>, int64_t, int64_t, int, int64_t, int64_t>(), py::arg("items"), py::arg("expect_rail"),
+           py::arg("expect_output"), py::arg("expect_balance"), py::arg("device"), py::arg("input_bytes") = 0, py::arg("output_bytes") = 0)
       .def_readonly("n_items", &A2AProgramPy::n_items)
       .def_readonly("num_stages", &A2AProgramPy::num_stages)
       .def_readonly("has_waits", &A2AProgramPy::has_waits)

@@ -218,7 +218,8 @@ class Communicator:
                 raise RuntimeError(f"scheduler produced an invalid plan: {err}")
             low = plan.lower(self.rank, unit_bytes, chunk_bytes, rail_segment_bytes, MAX_RAIL_COUNTERS)
             prog = self._C.A2AProgram(torch.from_numpy(low["items"]), [int(x) for x in low["expect_rail_bytes"]],
-                                      int(low["expect_output_bytes"]), int(low["expect_balance_bytes"]), self.device.index)
+                                      int(low["expect_output_bytes"]), int(low["expect_balance_bytes"]), self.device.index,
+                                      int(low["input_bytes"]), int(low["output_bytes"]))
             s = Schedule(plan, unit_bytes, prog, low, self.rank)
             if CONFIG.log and self.rank == 0 and plan.only_rank < 0:
                 nv = sched.nvlink_model(900.0, 2.0)
@@ -231,13 +232,16 @@ class Communicator:
         return s
 
     # ---- execution --------------------------------------------------------------------------------
-    def _launch_args(self, s: Schedule, output: torch.Tensor, input: torch.Tensor, staging: Optional[dict] = None):
+    def _require_usable(self) -> None:
         if self.heap is None:
             raise RuntimeError("communicator is closed")
         if self.broken:
             raise RuntimeError("communicator saw a failed collective; call reset() on every rank first")
         if self.liveness is not None:
             self.liveness.require_alive(self.liveness_max_age_s)
+
+    def _launch_args(self, s: Schedule, output: torch.Tensor, input: torch.Tensor, staging: Optional[dict] = None):
+        self._require_usable()
         if input.numel() * input.element_size() < s.input_bytes:
             raise ValueError("input smaller than the schedule needs")
         if output.numel() * output.element_size() < s.output_bytes:
@@ -418,29 +422,30 @@ class LocalGroup:
         self.comms = [Communicator(heap_bytes=heap_bytes, topo=topo, device=device, timeout_s=timeout_s, ctas=ctas, threads=threads,
                                    _heap=h, _rank=r, _world=world) for r, h in enumerate(heaps)]
         self.world, self.ctas, self.threads = world, ctas, threads
+        self._heaps, self._statuses = heaps, [c.status for c in self.comms]
 
     def schedule(self, matrix, **kw) -> List[Schedule]:
         return [c.schedule(matrix, **kw) for c in self.comms]
 
     def all_to_all_v(self, outputs, inputs, scheds) -> None:
-        srcs, cbs = [], []
-        dst0 = None
-        for c, o, i, s in zip(self.comms, outputs, inputs, scheds):
-            src, dst, cb = c._launch_args(s, o, i)
-            if dst0 is None:
-                dst0 = dst
-            elif dst != dst0:
-                raise RuntimeError("virtual ranks disagree on symmetric offsets; allocate in the same order on every rank")
-            srcs.append(src)
-            cbs.append(cb)
-        c0 = self.comms[0]
-        for c in self.comms:
+        comms = self.comms
+        need = scheds[0].max_bytes
+        for c in comms:
+            c._require_usable()
+            bal, rail = c._stage("balance", need["balance"]), c._stage("rail", need["rail"])  # the same offsets on every rank
             c.epoch += 1
-        self._C.a2a_launch_group([s.program for s in scheds], [c.heap for c in self.comms], srcs, dst0, c0.sig_off, c0.epoch,
-                                 [c.status for c in self.comms], c0.timeout_ns, self.ctas, self.threads)
-        for o, cb, s in zip(outputs, cbs, scheds):
-            if cb is not None:
-                o.view(torch.uint8).reshape(-1)[: s.output_bytes].copy_(cb[: s.output_bytes])
+        c0 = comms[0]
+        progs, ins = [s.program for s in scheds], list(inputs)
+        args = ((bal, rail), c0.sig_off, c0.epoch, self._statuses, c0.timeout_ns, self.ctas, self.threads)
+        if self._C.a2a_launch_group(progs, self._heaps, list(outputs), ins, *args):
+            return
+        recv = [c.heap.tensor(c._stage("recv", need["output"]), [need["output"]], torch.uint8) for c in comms]  # library-owned, copied out afterwards
+        for o, s in zip(outputs, scheds):
+            if o.numel() * o.element_size() < s.output_bytes:
+                raise ValueError("output smaller than the schedule needs")
+        self._C.a2a_launch_group(progs, self._heaps, recv, ins, *args)
+        for o, t, s in zip(outputs, recv, scheds):
+            o.view(torch.uint8).reshape(-1)[: s.output_bytes].copy_(t[: s.output_bytes])
 
     def check(self) -> None:
         for c in self.comms:

@@ -84,6 +84,32 @@ def test_unaligned_byte_units():
         assert np.array_equal(d_out[r][: host_out[r].size].cpu().numpy(), host_out[r])
 
 
+@pytest.mark.parametrize("unit_bytes,threads", [(1, 256), (2, 512), (3, 96), (8, 100)])
+def test_odd_segments_bit_exact(unit_bytes, threads):
+    """Segments of every size around the 16-byte words and the 2 KiB a warp cuts per pass, starting on any address on both
+    sides: all sixteen relative offsets, last words, a block whose last warp is not full."""
+    from fast_b200.parallel import LocalGroup
+
+    n = 3
+    grp = LocalGroup(n, heap_bytes=16 << 20, ctas=2, threads=threads)
+    for seed, m in enumerate([[[0, 1, 15], [17, 31, 33], [47, 2, 5]], [[2047, 2049, 2065], [4097, 13, 100001], [65537, 40009, 7]],
+                              [[1, 2063, 3], [2064, 0, 2081], [8191, 9999, 16385]]]):
+        m = np.array(m, dtype=np.int64)
+        ss = grp.schedule(m, unit_bytes=unit_bytes, kind=PlanKind.FANOUT if seed else PlanKind.STAGED)
+        rng = np.random.default_rng(seed)
+        ins = [rng.integers(0, 256, int(m[r].sum()) * unit_bytes, dtype=np.uint8) for r in range(n)]
+        mx = ss[0].max_bytes["output"] + 64
+        d_in = [torch.from_numpy(np.concatenate([np.zeros(r, np.uint8), x])).cuda()[r:] for r, x in enumerate(ins)]   # odd input addresses
+        d_out = [c.alloc(mx, torch.uint8).fill_(0xEE) for c in grp.comms]
+        grp.all_to_all_v([o[:-16] for o in d_out], d_in, ss)
+        grp.check()
+        host_out = [np.zeros(int(m[:, r].sum()) * unit_bytes, np.uint8) for r in range(n)]
+        ss[0].plan.execute_on_host(unit_bytes, ins, host_out)
+        for r in range(n):
+            got = d_out[r].cpu().numpy()
+            assert np.array_equal(got[: host_out[r].size], host_out[r]) and (got[host_out[r].size:] == 0xEE).all()
+
+
 def test_bounded_wait_reports_timeout():
     """A wait on a flag nobody sets must end by itself and leave a readable status."""
     from fast_b200 import runtime
