@@ -25,11 +25,10 @@ struct A2AProgramPy {
   bool has_waits = false;  // some item waits for bytes another item of a peer's (or this) launch forwards
   unsigned long long expect_output = 0, expect_balance = 0;
   int64_t total_bytes = 0, largest_item = 0;
-  int64_t input_bytes = 0, output_bytes = 0;  // what the rank's input and output hold (checked by the group launch)
+  int64_t input_bytes = 0, output_bytes = 0;  // what the rank's input and output hold (set by the owner, checked by the group launch)
 
   // items: int64[k, 10] as produced by Plan.lower(); expect_rail: list of bytes per stage.
-  A2AProgramPy(torch::Tensor items, std::vector<int64_t> expect_rail, int64_t exp_out, int64_t exp_bal, int device,
-               int64_t in_bytes, int64_t out_bytes) : input_bytes(in_bytes), output_bytes(out_bytes) {
+  A2AProgramPy(torch::Tensor items, std::vector<int64_t> expect_rail, int64_t exp_out, int64_t exp_bal, int device) {
     TORCH_CHECK(items.dim() == 2 && items.size(1) == 10 && items.dtype() == torch::kInt64 && items.is_cpu(), "items must be CPU int64[k, 10]");
     TORCH_CHECK(static_cast<int>(expect_rail.size()) <= kSigMaxStages, "too many stages for the signal block");
     n_items = static_cast<int>(items.size(0));
@@ -158,8 +157,9 @@ PYBIND11_MODULE(_C, m) {
       .def("ptr", [](const StatusPy& s) { return reinterpret_cast<int64_t>(s.d); });
 
   py::class_<A2AProgramPy>(m, "A2AProgram")
-      .def(py::init<torch::Tensor, std::vector<int64_t>, int64_t, int64_t, int, int64_t, int64_t>(), py::arg("items"), py::arg("expect_rail"),
-           py::arg("expect_output"), py::arg("expect_balance"), py::arg("device"), py::arg("input_bytes") = 0, py::arg("output_bytes") = 0)
+      .def(py::init<torch::Tensor, std::vector<int64_t>, int64_t, int64_t, int>())
+      .def_readwrite("input_bytes", &A2AProgramPy::input_bytes)
+      .def_readwrite("output_bytes", &A2AProgramPy::output_bytes)
       .def_readonly("n_items", &A2AProgramPy::n_items)
       .def_readonly("num_stages", &A2AProgramPy::num_stages)
       .def_readonly("has_waits", &A2AProgramPy::has_waits)

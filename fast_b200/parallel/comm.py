@@ -218,8 +218,8 @@ class Communicator:
                 raise RuntimeError(f"scheduler produced an invalid plan: {err}")
             low = plan.lower(self.rank, unit_bytes, chunk_bytes, rail_segment_bytes, MAX_RAIL_COUNTERS)
             prog = self._C.A2AProgram(torch.from_numpy(low["items"]), [int(x) for x in low["expect_rail_bytes"]],
-                                      int(low["expect_output_bytes"]), int(low["expect_balance_bytes"]), self.device.index,
-                                      int(low["input_bytes"]), int(low["output_bytes"]))
+                                      int(low["expect_output_bytes"]), int(low["expect_balance_bytes"]), self.device.index)
+            prog.input_bytes, prog.output_bytes = int(low["input_bytes"]), int(low["output_bytes"])
             s = Schedule(plan, unit_bytes, prog, low, self.rank)
             if CONFIG.log and self.rank == 0 and plan.only_rank < 0:
                 nv = sched.nvlink_model(900.0, 2.0)
