@@ -48,8 +48,9 @@ class _MoEFunction(torch.autograd.Function):
 def _experts_backward(eng, grad_out, rs, weights, w13, w2, w2_param):
     """Backward of dispatch -> experts -> combine through the engine. Returns (grad_x, grad_weights, dW13,
     dW2 or None); dW2 is None when an attached optimizer applied W2's update inside the pass."""
-    if not hasattr(eng, "_dw13") or eng._dw13.shape != w13.shape:
-        eng._dw13, eng._dw2 = torch.empty_like(w13), torch.empty_like(w2)
+    # New tensors each time, held by nobody else when they are returned: autograd then keeps them as the parameters' .grad.
+    # Buffers that the engine kept were cloned instead (a pass over all expert gradients: 0.9 ms for 8 x 4096 x 14336).
+    dw13, dw2 = torch.empty_like(w13), torch.empty_like(w2)
     opt = getattr(eng, "optimizer_in_backward", None)
     early = opt is not None and opt.owns(w2_param)
     after = None
@@ -64,14 +65,14 @@ def _experts_backward(eng, grad_out, rs, weights, w13, w2, w2_param):
             ev = torch.cuda.Event()
             ev.record(main)
             eng._opt_stream.wait_event(ev)
-            opt.step_param(w2_param, eng._dw2, stream=eng._opt_stream, early=True)
+            opt.step_param(w2_param, dw2, stream=eng._opt_stream, early=True)
 
-    gx, gw = eng.backward(grad_out.contiguous(), rs, weights, w13, w2, eng._dw13, eng._dw2, after_dw2=after)
+    gx, gw = eng.backward(grad_out.contiguous(), rs, weights, w13, w2, dw13, dw2, after_dw2=after)
     if early:
         done = torch.cuda.Event()
         done.record(eng._opt_stream)
         torch.cuda.current_stream().wait_event(done)  # the next kernels on this stream may read W2 / reuse dW2
-    return gx, gw, eng._dw13, (None if early else eng._dw2)
+    return gx, gw, dw13, (None if early else dw2)
 
 
 class _NormRouteMoEFunction(torch.autograd.Function):
