@@ -10,7 +10,7 @@
 // GEMM, top-k, gather, softmax and their backward kernels with the activations re-read each time.
 // Limits: num_experts <= 32 (one logit per lane), hidden % 256 == 0, and the gate matrix (forward)
 // or the gate matrix plus the fp32 gradient accumulators (backward) must fit in shared memory.
-#include "api.h"
+#include "route_rank.cuh"
 
 namespace fastb {
 
@@ -70,30 +70,13 @@ __global__ void __launch_bounds__(kGateThreads) norm_gate_route_kernel(const Nor
     if (raw != raw) raw = -INFINITY;  // NaN counts as -inf: the selection stays total
     float sel = lane < E ? raw + (a.bias ? a.bias[lane] : 0.0f) : -INFINITY;
     if (sel != sel) sel = -INFINITY;
-    float mx = raw;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    bool taken = lane >= E;
-    float wsum = 0.0f, my_w = 0.0f;
-    int my_e = -1;
-    for (int j = 0; j < K; ++j) {
-      float best = taken ? -INFINITY : sel;
-      int best_e = taken ? 0x7fffffff : lane;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-        if (oe != 0x7fffffff && (best_e == 0x7fffffff || ob > best || (ob == best && oe < best_e))) { best = ob; best_e = oe; }
-      }
-      if (lane == best_e) taken = true;
-      const float r = __shfl_sync(0xffffffffu, raw, best_e & 31);
-      const float pw = r > -INFINITY ? __expf(r - mx) : 0.0f;
-      wsum += pw;
-      if (lane == j) { my_w = pw; my_e = best_e; }
-    }
+    int my_e;
+    float my_w;
+    const float sel1[1] = {sel}, raw1[1] = {lane < E ? raw : -INFINITY};
+    route::warp_topk<1>(sel1, raw1, E, K, my_e, my_w);
     if (lane < K) {
       a.topk_idx[static_cast<long long>(t) * K + lane] = my_e;
-      a.topk_w[static_cast<long long>(t) * K + lane] = wsum > 0.0f ? my_w / wsum : 0.0f;
+      a.topk_w[static_cast<long long>(t) * K + lane] = my_w;
       s_eid[lt * K + lane] = my_e;
     }
   };
@@ -148,16 +131,8 @@ __global__ void __launch_bounds__(kGateThreads) norm_gate_route_kernel(const Nor
     if (vb) finish(ltb, accb);
   }
   __syncthreads();
-  const int n = kTokensPerBlock * K;
-  for (int e = threadIdx.x; e < E; e += kGateThreads) {
-    int c = 0;
-    for (int i = 0; i < n; ++i)
-      if (s_eid[i] == e) {
-        a.slot_in_block[static_cast<long long>(t0) * K + i] = c;
-        ++c;
-      }
-    a.block_cnt[static_cast<long long>(blockIdx.x) * E + e] = c;
-  }
+  route::block_stable_ranks(s_eid, reinterpret_cast<unsigned short*>(s_eid + kTokensPerBlock * K), E, K, a.slot_in_block + static_cast<long long>(t0) * K,
+                            a.block_cnt + static_cast<long long>(blockIdx.x) * E);
 }
 
 // Dynamic shared memory: gate [E][H] bf16, norm weight [H] bf16, then fp32 accumulators d_gate [E][H], d_nw [H].
@@ -295,7 +270,7 @@ __global__ void __launch_bounds__(kGateBwdThreads) norm_gate_bwd_kernel(const No
 
 size_t norm_gate_smem_bytes(int E, int H, int K, bool backward) {
   const size_t base = (static_cast<size_t>(E) + 1) * H * 2;
-  return backward ? base + (static_cast<size_t>(E) + 1) * H * 4 : base + sizeof(int) * kTokensPerBlock * K;
+  return backward ? base + (static_cast<size_t>(E) + 1) * H * 4 : base + route::rank_smem_bytes(E, K);
 }
 
 cudaError_t launch_norm_gate_route(const NormGateArgs& a, cudaStream_t stream) {

@@ -6,21 +6,22 @@
 //                  group offsets for the grouped GEMM and cumulative arrival targets.
 // The reference has no router; its counterpart of the count exchange is the host-side workload
 // broadcast (nvidia/alltoall_nvshmem.cpp:452-472), which this replaces with ~1 KB of NVLink stores.
-#include "api.h"
+#include "route_rank.cuh"
 
 namespace fastb {
 
 namespace {
 
 constexpr int kTokensPerBlock = kRouteTokensPerBlock;
-constexpr int kRouteThreads = 256;
+constexpr int kRouteThreads = 1024;
 
-// One warp per token at a time. E <= 256 (8 values per lane).
+// One warp per token at a time. E <= 256 (8 values per lane). 32 warps: a block owns 128 tokens whatever T is, so at small T
+// the warps of one block are all the parallelism there is.
 template <int MAX_PER_LANE>
 __global__ void __launch_bounds__(kRouteThreads) route_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E,
                                                                    int K, int* __restrict__ topk_idx, float* __restrict__ topk_w,
                                                                    int* __restrict__ slot_in_block, int* __restrict__ block_cnt) {
-  extern __shared__ int s_eid[];  // [kTokensPerBlock * K]
+  extern __shared__ int s_eid[];  // [kTokensPerBlock * K], then the counts of block_stable_ranks
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kRouteThreads / 32;
   const int t0 = blockIdx.x * kTokensPerBlock;
   const int nt = min(kTokensPerBlock, T - t0);
@@ -30,71 +31,32 @@ __global__ void __launch_bounds__(kRouteThreads) route_topk_kernel(const float* 
       for (int j = lane; j < K; j += 32) s_eid[lt * K + j] = -1;
       continue;
     }
+    // Selection uses logits + bias; the weights are the softmax of the raw logits over the
+    // chosen experts (renormalised), which for bias == 0 is Mixtral's softmax-over-top-k.
     float sel[MAX_PER_LANE], raw[MAX_PER_LANE];
-    unsigned taken = 0u;  // bit i: candidate lane + 32 i is chosen already, or past the last expert
-    float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < MAX_PER_LANE; ++i) {
       const int e = lane + 32 * i;
-      // NaN logits count as -inf: the selection below stays total and the weights stay finite.
+      // NaN logits count as -inf: the selection stays total and the weights stay finite.
       float r = e < E ? logits[static_cast<long long>(t) * E + e] : -INFINITY;
       if (r != r) r = -INFINITY;
       float s = e < E ? r + (bias ? bias[e] : 0.0f) : -INFINITY;
       if (s != s) s = -INFINITY;
       raw[i] = r;
       sel[i] = s;
-      if (e >= E) taken |= 1u << i;
-      mx = fmaxf(mx, r);
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    // Selection uses logits + bias; the weights are the softmax of the raw logits over the
-    // chosen experts (renormalised), which for bias == 0 is Mixtral's softmax-over-top-k.
-    // A token with fewer than K selectable values (-inf / NaN rows, masked experts) still gets K
-    // distinct expert ids in range: the lowest unchosen ids, with weight 0.
-    float wsum = 0.0f;
-    float my_w = 0.0f;
-    int my_e = -1;
-    for (int j = 0; j < K; ++j) {
-      float best = -INFINITY;
-      int best_e = 0x7fffffff;
-#pragma unroll
-      for (int i = 0; i < MAX_PER_LANE; ++i)
-        if (!((taken >> i) & 1u) && (best_e == 0x7fffffff || sel[i] > best)) { best = sel[i]; best_e = lane + 32 * i; }
-#pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-        if (oe != 0x7fffffff && (best_e == 0x7fffffff || ob > best || (ob == best && oe < best_e))) { best = ob; best_e = oe; }
-      }
-      float r = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < MAX_PER_LANE; ++i)
-        if (lane + 32 * i == best_e) { r = raw[i]; taken |= 1u << i; }
-      r = __shfl_sync(0xffffffffu, r, best_e & 31);
-      const float p = r > -INFINITY ? __expf(r - mx) : 0.0f;
-      wsum += p;
-      if (lane == j) { my_w = p; my_e = best_e; }
-    }
+    int my_e;
+    float my_w;
+    route::warp_topk<MAX_PER_LANE>(sel, raw, E, K, my_e, my_w);
     if (lane < K) {
       topk_idx[static_cast<long long>(t) * K + lane] = my_e;
-      topk_w[static_cast<long long>(t) * K + lane] = wsum > 0.0f ? my_w / wsum : 0.0f;
+      topk_w[static_cast<long long>(t) * K + lane] = my_w;
       s_eid[lt * K + lane] = my_e;
     }
   }
   __syncthreads();
-  // Stable rank of every entry among the entries of the same expert in this block: thread e walks
-  // the block's entries in (token, slot) order.
-  const int n = kTokensPerBlock * K;
-  for (int e = threadIdx.x; e < E; e += kRouteThreads) {
-    int c = 0;
-    for (int i = 0; i < n; ++i)
-      if (s_eid[i] == e) {
-        slot_in_block[static_cast<long long>(t0) * K + i] = c;
-        ++c;
-      }
-    block_cnt[static_cast<long long>(blockIdx.x) * E + e] = c;
-  }
+  route::block_stable_ranks(s_eid, reinterpret_cast<unsigned short*>(s_eid + kTokensPerBlock * K), E, K, slot_in_block + static_cast<long long>(t0) * K,
+                            block_cnt + static_cast<long long>(blockIdx.x) * E);
 }
 
 // Single CTA. Thread e owns expert e (E <= 1024).
@@ -250,13 +212,20 @@ cudaError_t launch_route_topk(const float* logits, const float* bias, int T, int
   if (E < 1 || E > 256 || K < 1 || K > 32 || K > E) return cudaErrorInvalidValue;
   const int blocks = (T + kTokensPerBlock - 1) / kTokensPerBlock;
   if (blocks == 0) return cudaSuccess;
-  const size_t smem = sizeof(int) * kTokensPerBlock * K;
-  if (E <= 32) route_topk_kernel<1><<<blocks, kRouteThreads, smem, stream>>>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt);
-  else if (E <= 64) route_topk_kernel<2><<<blocks, kRouteThreads, smem, stream>>>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt);
-  else if (E <= 128) route_topk_kernel<4><<<blocks, kRouteThreads, smem, stream>>>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt);
-  else route_topk_kernel<8><<<blocks, kRouteThreads, smem, stream>>>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt);
-  note_launch();
-  return cudaGetLastError();
+  const size_t smem = route::rank_smem_bytes(E, K);
+  auto go = [&](auto kern) {
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      if (e != cudaSuccess) return e;
+    }
+    kern<<<blocks, kRouteThreads, smem, stream>>>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt);
+    note_launch();
+    return cudaGetLastError();
+  };
+  if (E <= 32) return go(route_topk_kernel<1>);
+  if (E <= 64) return go(route_topk_kernel<2>);
+  if (E <= 128) return go(route_topk_kernel<4>);
+  return go(route_topk_kernel<8>);
 }
 
 cudaError_t launch_splits_scan(const SplitsArgs& a, cudaStream_t stream) {
