@@ -104,7 +104,8 @@ struct GemmArgs {
   // CTA-pair kernel, forward only: operand A is e4m3 (map_a: u8 matrix, boxes {64,128}, no swizzle) with one fp32 scale per
   // 128 elements of a row in a_scales [rows, red_len / 128]; null = bf16 operand.
   const float* a_scales;
-  const int* group_rows;   // optional [num_groups]: real rows of each group; the e4m3 feed turns rows past them into zeros
+  const int* group_rows;   // optional [num_groups]: real rows of each group; the e4m3 feed turns rows past them into zeros, wgrad reduces
+                           // over them up to a multiple of 64
   int gate_tile_rows;      // 0: gate_counter / gate_target are indexed by group; > 0: by (row of the grouped matrix) / gate_tile_rows
   int gate_slots;          // entries of gate_counter / gate_target (indices are clamped to the last one)
 };
@@ -121,6 +122,39 @@ cudaError_t launch_grouped_gemm(GemmMode mode, GemmEpilogue epi, const CUtensorM
 // SwiGLU backward map_c2 is the saved gate|up matrix, which the epilogue TMA-loads.
 cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c,
                                      const CUtensorMap* map_c2, const GemmArgs& args, int ctas, cudaStream_t stream);
+
+// Weights as operand A, tokens as operand B (grouped_gemm_tokens.cu): forward and dgrad on CTA pairs, tiles of 256 features by
+// up to 256 tokens, the last wave cut into shares of the reduction.
+constexpr int kTokPartialFloats = 128 * 256;   // fp32 sums of one CTA's part of a tile
+constexpr int tok_counters(int ctas) { return 2 * ctas; }                                  // arrival counters a launch needs
+constexpr long long tok_partial_floats(int ctas) { return 2ll * ctas * kTokPartialFloats; }  // two partial tiles per CTA
+struct TokGemmMaps {   // bf16, 128-byte swizzle; boxes {inner, outer}
+  const CUtensorMap* w;      // forward store {64,128}; forward SwiGLU 5-D {64,16,2,4,1} over [tile][16-row group][gate|up][16][K]; dgrad {64,64}
+  const CUtensorMap *x128, *x32, *x16;   // tokens: {64,128}, {64,32}, {64,16}
+  const CUtensorMap* c;      // output {64,32}
+  const CUtensorMap* c2;     // gate|up: written by the SwiGLU forward (keep_gate_up), read by the SwiGLU backward {64,32}; else null
+};
+struct TokGemmArgs {
+  const int* group_off;      // [num_groups + 1] first rows, multiples of 256 (device)
+  const int* group_rows;     // [num_groups] real rows, or null: all rows up to the next group
+  int num_groups;
+  int m_tiles;               // 256-feature tiles of the output's columns (SwiGLU forward: of gate|up)
+  int red_blocks;            // 64-wide blocks of the reduction
+  int w_rows_per_group;      // rows of a group's slice in w's matrix (forward: features, dgrad: reduction)
+  int band_tiles;            // token tiles of a raster band
+  int granule;               // tile widths are multiples of this (32 or 64); rows up to a multiple of it are written
+  int keep_gate_up;
+  float* partials;           // tok_partial_floats(ctas)
+  unsigned int* counters;    // num_counters >= tok_counters(ctas), zero before the launch and after it
+  unsigned int* counters_next;   // num_counters; cleared by the launch
+  int num_counters;
+  DeviceStatus* status;
+  unsigned long long timeout_ns;
+  const unsigned long long* gate_counter;   // arrival gate as in GemmArgs
+  const unsigned long long* gate_target;
+  int gate_tile_rows, gate_slots;
+};
+cudaError_t launch_grouped_gemm_tokens(GemmMode mode, GemmEpilogue epi, const TokGemmMaps& maps, const TokGemmArgs& args, int ctas, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------
 // MoE routing / dispatch / combine
@@ -163,7 +197,8 @@ cudaError_t launch_splits_scan(const SplitsArgs& a, cudaStream_t stream);
 // Entries whose expert id is outside [0, E) are skipped and reported in `status` (kSiteExpertId).
 cudaError_t launch_build_send_list(const int* topk_idx, const int* slot_in_block, const int* block_base, const int* send_pos, int T, int K, int E,
                                    int* list, DeviceStatus* status, cudaStream_t stream);
-cudaError_t launch_zero_pad_rows(void* buf, long long row_bytes, const int* group_off, const int* group_rows, int groups, cudaStream_t stream);
+// Zeroes the rows from each group's real end to the next multiple of `align` inside the group (0: to the group's padded end).
+cudaError_t launch_zero_pad_rows(void* buf, long long row_bytes, const int* group_off, const int* group_rows, int groups, int align, cudaStream_t stream);
 
 // Router front end in one pass (moe_gate.cu): RMSNorm, router logits, top-k, softmax-over-top-k weights and the
 // per-block histogram / ranks of route_topk. num_experts <= 32, H % 256 == 0, (num_experts + 1) * H * 2 bytes of

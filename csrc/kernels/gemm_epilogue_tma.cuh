@@ -6,11 +6,7 @@
 // buffer laid out with the 128-byte swizzle (16-byte chunk j of row r sits at chunk j ^ (r & 7)),
 // which is free of bank conflicts for this access pattern, and one elected thread hands the
 // buffer to the TMA unit (cp.async.bulk.tensor store, bulk-group completion). Two buffers form a
-// ring, so that converting chunk n overlaps the store of chunk n - 1. The fused SwiGLU backward
-// also reads its saved gate|up tile through TMA loads into the same two buffers and transforms
-// it in place.
-//
-// All TMA loads here are plain loads of this GPU's own memory.
+// ring, so that converting chunk n overlaps the store of chunk n - 1.
 #pragma once
 #include "gemm_common.cuh"
 
@@ -110,64 +106,6 @@ __device__ __forceinline__ void epilogue_swiglu_tma(EpiRing& ring, const CUtenso
     ring.release(map_act, act_col0 + c * kEpiChunkCols, row0);
   }
   if (map_gu != nullptr) epilogue_store_tma(ring, map_gu, gu_col0, row0, r, t_row, false);
-}
-
-// SwiGLU backward fused into the dgrad that produces d(act): the tile's 256 accumulator columns
-// are d(act) of 256 consecutive features = two blocks of 128; block b sits in the gate|up layout
-// at columns [256 b, 256 b + 128) (gate) and [256 b + 128, 256 b + 256) (up) of the tile's
-// 512-column span that starts at gu_col0. Per chunk of 64 features the saved gate and up tiles
-// are TMA-loaded into the two staging buffers, every thread turns its own row into d(gate) and
-// d(up) in place, and both buffers are stored to map_dgu at the same coordinates.
-// `load_bar` is an mbarrier (count 1) of this CTA; `load_phase` carries its parity across calls.
-// Returns false if the wait for a load gave up.
-__device__ __forceinline__ bool epilogue_swiglu_bwd_tma(EpiRing& ring, const CUtensorMap* map_dgu, const CUtensorMap* map_gu, int gu_col0, int row0,
-                                                        int r, uint32_t t_row, uint64_t* load_bar, uint32_t& load_phase, volatile int* abort_flag,
-                                                        DeviceStatus* st, unsigned long long timeout_ns) {
-  uint8_t* gbuf = ring.base;
-  uint8_t* ubuf = ring.base + kEpiBufBytes;
-#pragma unroll 1
-  for (int c = 0; c < BN / kEpiChunkCols; ++c) {
-    const int col = gu_col0 + (c >> 1) * 256 + (c & 1) * kEpiChunkCols;
-    if (ring.issuer) {
-      bulk_wait_read<0>();  // the previous chunk's stores have read both buffers
-      ptx::mbar_arrive_expect_tx(load_bar, 2 * kEpiBufBytes);
-      ptx::tma_load_2d(gbuf, map_gu, col, row0, load_bar);
-      ptx::tma_load_2d(ubuf, map_gu, col + 128, row0, load_bar);
-    }
-    uint32_t d[2][32];
-    ptx::tmem_ld_32x32(t_row + c * kEpiChunkCols, d[0]);
-    ptx::tmem_ld_32x32(t_row + c * kEpiChunkCols + 32, d[1]);
-    if (!ptx::mbar_wait_bounded(load_bar, load_phase, abort_flag, st, 500, timeout_ns)) { ptx::tmem_wait_ld(); return false; }
-    load_phase ^= 1u;
-    ptx::tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint4* gp = chunk_ptr(gbuf, r, j);
-      uint4* up = chunk_ptr(ubuf, r, j);
-      float g[8], u[8], og[8], ou[8];
-      unpack8_bf16(*gp, g);
-      unpack8_bf16(*up, u);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        // d(act) is rounded to bf16 first, as the unfused path stores it before the element-wise kernel
-        const float da = __bfloat162float(__float2bfloat16_rn(__uint_as_float(d[j >> 2][(j & 3) * 8 + i])));
-        const float s = 1.0f / (1.0f + __expf(-g[i]));
-        const float sl = g[i] * s;
-        ou[i] = da * sl;
-        og[i] = da * u[i] * (s + sl * (1.0f - s));
-      }
-      *gp = make_uint4(pack_bf16(og[0], og[1]), pack_bf16(og[2], og[3]), pack_bf16(og[4], og[5]), pack_bf16(og[6], og[7]));
-      *up = make_uint4(pack_bf16(ou[0], ou[1]), pack_bf16(ou[2], ou[3]), pack_bf16(ou[4], ou[5]), pack_bf16(ou[6], ou[7]));
-    }
-    ptx::fence_proxy_async_smem();
-    epi_bar();
-    if (ring.issuer) {
-      tma_store_2d(map_dgu, gbuf, col, row0);
-      tma_store_2d(map_dgu, ubuf, col + 128, row0);
-      bulk_commit();
-    }
-  }
-  return true;
 }
 
 }  // namespace gemm

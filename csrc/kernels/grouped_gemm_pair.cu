@@ -1,4 +1,6 @@
-// Grouped bf16 GEMM on CTA pairs: tcgen05.mma.cta_group::2 over a 256 x 256 tile.
+// Grouped GEMM on CTA pairs with the grouped rows as operand A: tcgen05.mma.cta_group::2 over a 256 x 256 tile. It serves the
+// weight gradients (bf16, the group is the reduction) and the forward contraction from e4m3 rows; forward and dgrad of
+// bf16 rows take the tokens as operand B (grouped_gemm_tokens.cu).
 //
 // Two CTAs of a cluster share one output tile. CTA r of the pair loads its 128 rows of A and its
 // 128 columns of B (half of each operand, plain TMA loads, no multicast), the leader (cluster
@@ -12,8 +14,7 @@
 //   empty[s]     each CTA: released by the leader's commit, multicast to both CTAs.
 //   acc_full[a]  each CTA: leader's commit after the last k step, multicast to both.
 //   acc_empty[a] leader only: 8 arrivals (4 epilogue warps of each CTA; the peer's arrive remotely).
-//   epi_load     each CTA: bytes of the saved gate|up tiles the fused SwiGLU-backward epilogue loads.
-// Same modes, arrival gate and bounded waits as the one-CTA kernel; group offsets must be multiples
+// Same arrival gate and bounded waits as the one-CTA kernel; group offsets must be multiples
 // of 256. The epilogues leave through a two-buffer shared-memory ring and TMA stores
 // (gemm_epilogue_tma.cuh): output matrices are described by tensor maps of 64 x 128 boxes.
 #include <cuda_fp8.h>
@@ -49,7 +50,7 @@ constexpr int kCvtWarps = 4;
 constexpr int kThreadsFp8 = kThreads + 32 * kCvtWarps;
 
 struct __align__(8) SmemCtl {
-  uint64_t full[kStages], empty[kStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load, q_full[kQStages], q_empty[kQStages];
+  uint64_t full[kStages], empty[kStages], acc_full[kAccStages], acc_empty[kAccStages], q_full[kQStages], q_empty[kQStages];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -74,14 +75,14 @@ __device__ __forceinline__ uint32_t bf16_pair_of(float x) {  // x is bf16-repres
 }
 
 // TMA_EPI: outputs leave through the shared-memory ring and TMA stores; otherwise every epilogue
-// thread writes (and, for the fused SwiGLU backward, reads) its own row in global memory.
+// thread writes its own row in global memory.
 // A_FP8 (forward only): map_a describes e4m3 bytes (boxes of 64 bytes x 128 rows, no swizzle) and
 // p.a_scales their 1x128 scales; see kStagesFp8 above.
 template <GemmMode MODE, GemmEpilogue EPI, bool TMA_EPI, bool A_FP8>
 __global__ void __launch_bounds__(A_FP8 ? kThreadsFp8 : kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                          const __grid_constant__ CUtensorMap map_c2, const GemmArgs p) {
-  static_assert(!A_FP8 || MODE == GemmMode::kForward, "the e4m3 operand feeds the forward contraction only");
+  static_assert(A_FP8 ? MODE == GemmMode::kForward && TMA_EPI : MODE == GemmMode::kWgrad && EPI == GemmEpilogue::kStore, "e4m3 forward or bf16 weight gradient");
   constexpr int NS = A_FP8 ? kStagesFp8 : kStages;  // operand stages in use
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -99,7 +100,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     // each CTA's converter warp when the A tile is written by them instead of by TMA.
     for (int s = 0; s < NS; ++s) { mbar_init(&ctl->full[s], A_FP8 ? 1 + 2 : 1); mbar_init(&ctl->empty[s], 1); }
     for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * kEpiWarps); }
-    mbar_init(&ctl->epi_load, 1);
     for (int q = 0; q < kQStages; ++q) { mbar_init(&ctl->q_full[q], 1); mbar_init(&ctl->q_empty[q], 1); }
     ctl->abort_flag = 0;
     mbar_fence_init();
@@ -117,7 +117,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   volatile int* abort_flag = &ctl->abort_flag;
 
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  TileWalker<TILE_M> walk{p.group_off, p.num_groups, p.tiles_n, p.fixed_m_tiles, p.red_len, MODE == GemmMode::kWgrad, p.band_rows};
+  TileWalker<TILE_M> walk{p.group_off, p.num_groups, p.tiles_n, p.fixed_m_tiles, p.red_len, MODE == GemmMode::kWgrad, p.band_rows, MODE == GemmMode::kWgrad ? p.group_rows : nullptr};
   TileCoord tc;
 
   if (warp == 0) {
@@ -156,22 +156,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             continue;
           }
           if (leader) mbar_arrive_expect_tx(&ctl->full[s], 2 * kStageBytes);
-          if (MODE == GemmMode::kForward) {
-            tma_load_2d_pair(sa, &map_a, kb * BK, tc.row0 + m0, full_leader);
-            tma_load_2d_pair(sb, &map_b, kb * BK, tc.g * p.b_rows_per_group + n0, full_leader);
-          } else if (MODE == GemmMode::kDgrad) {
-            tma_load_2d_pair(sa, &map_a, kb * BK, tc.row0 + m0, full_leader);
 #pragma unroll
-            for (int j = 0; j < PN / 64; ++j)
-              tma_load_2d_pair(sb + j * (BK * 128), &map_b, n0 + j * 64, tc.g * p.b_rows_per_group + kb * BK, full_leader);
-          } else {
+          for (int j = 0; j < PM / 64; ++j)
+            tma_load_2d_pair(sa + j * (BK * 128), &map_a, m0 + j * 64, tc.row0 + kb * BK, full_leader);
 #pragma unroll
-            for (int j = 0; j < PM / 64; ++j)
-              tma_load_2d_pair(sa + j * (BK * 128), &map_a, m0 + j * 64, tc.row0 + kb * BK, full_leader);
-#pragma unroll
-            for (int j = 0; j < PN / 64; ++j)
-              tma_load_2d_pair(sb + j * (BK * 128), &map_b, n0 + j * 64, tc.row0 + kb * BK, full_leader);
-          }
+          for (int j = 0; j < PN / 64; ++j)
+            tma_load_2d_pair(sb + j * (BK * 128), &map_b, n0 + j * 64, tc.row0 + kb * BK, full_leader);
         }
       }
     }
@@ -275,7 +265,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;  // my accumulator row inside this CTA's half
     EpiRing ring{epi_stage, threadIdx.x == 64, 0u};
-    uint32_t acc_it = 0, load_phase = 0;
+    uint32_t acc_it = 0;
     bool ok = true;
     for (int tile = pair; ok && walk.locate(tile, tc); tile += pairs) {
       const int a = acc_it % kAccStages;
@@ -290,20 +280,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int c_row0 = (MODE == GemmMode::kWgrad ? tc.g * p.c_rows_per_group : tc.row0) + tc.m_idx * TILE_M + static_cast<int>(cta) * PM;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * BN;
       if (!TMA_EPI) {
-        const long long c_row = static_cast<long long>(c_row0) + r;
-        if (EPI == GemmEpilogue::kStore) {
-          epilogue_store_row(p.c + c_row * p.ldc + static_cast<long long>(tc.n_idx) * BN, t_row, empty_reduction);
-        } else if (EPI == GemmEpilogue::kSwiGLUBwd) {
-          epilogue_swiglu_bwd_row(p.c + c_row * p.ldc + static_cast<long long>(tc.n_idx) * (2 * BN),
-                                  p.c2 + c_row * p.ldc2 + static_cast<long long>(tc.n_idx) * (2 * BN), t_row);
-        } else {
-          epilogue_swiglu_row(p.c + c_row * p.ldc + static_cast<long long>(tc.n_idx) * (BN / 2),
-                              p.c2 ? p.c2 + c_row * p.ldc2 + static_cast<long long>(tc.n_idx) * BN : nullptr, t_row);
-        }
+        epilogue_store_row(p.c + (static_cast<long long>(c_row0) + r) * p.ldc + static_cast<long long>(tc.n_idx) * BN, t_row, empty_reduction);
       } else if (EPI == GemmEpilogue::kStore) {
         epilogue_store_tma(ring, &map_c, tc.n_idx * BN, c_row0, r, t_row, empty_reduction);
-      } else if (EPI == GemmEpilogue::kSwiGLUBwd) {
-        ok = epilogue_swiglu_bwd_tma(ring, &map_c, &map_c2, tc.n_idx * (2 * BN), c_row0, r, t_row, &ctl->epi_load, load_phase, abort_flag, p.status, p.timeout_ns);
       } else {
         epilogue_swiglu_tma(ring, &map_c, tc.n_idx * (BN / 2), p.c2 ? &map_c2 : nullptr, tc.n_idx * BN, c_row0, r, t_row);
       }
@@ -342,13 +321,6 @@ cudaError_t launch_kernel(Kernel kern, int threads, int smem, const CUtensorMap&
   return e;
 }
 
-template <GemmMode MODE, GemmEpilogue EPI>
-cudaError_t launch_one(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const CUtensorMap& c2, const GemmArgs& args, int ctas,
-                       cudaStream_t stream) {
-  if (args.direct_epilogue) return launch_kernel(grouped_gemm_pair_kernel<MODE, EPI, false, false>, kThreads, kSmemBytes, a, b, c, c2, args, ctas, stream);
-  return launch_kernel(grouped_gemm_pair_kernel<MODE, EPI, true, false>, kThreads, kSmemBytes, a, b, c, c2, args, ctas, stream);
-}
-
 }  // namespace
 
 cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c,
@@ -363,19 +335,10 @@ cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUte
       return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kForward, GemmEpilogue::kSwiGLU, true, true>, kThreadsFp8, kSmemBytesFp8, map_a, map_b, map_c, c2, args, ctas, stream);
     return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kForward, GemmEpilogue::kStore, true, true>, kThreadsFp8, kSmemBytesFp8, map_a, map_b, map_c, c2, args, ctas, stream);
   }
-  if (epi == GemmEpilogue::kSwiGLU) {
-    if (mode != GemmMode::kForward) return cudaErrorInvalidValue;
-    return launch_one<GemmMode::kForward, GemmEpilogue::kSwiGLU>(map_a, map_b, map_c, c2, args, ctas, stream);
-  }
-  if (epi == GemmEpilogue::kSwiGLUBwd) {
-    if (mode != GemmMode::kDgrad || args.c2 == nullptr) return cudaErrorInvalidValue;
-    return launch_one<GemmMode::kDgrad, GemmEpilogue::kSwiGLUBwd>(map_a, map_b, map_c, c2, args, ctas, stream);
-  }
-  switch (mode) {
-    case GemmMode::kForward: return launch_one<GemmMode::kForward, GemmEpilogue::kStore>(map_a, map_b, map_c, c2, args, ctas, stream);
-    case GemmMode::kDgrad: return launch_one<GemmMode::kDgrad, GemmEpilogue::kStore>(map_a, map_b, map_c, c2, args, ctas, stream);
-    default: return launch_one<GemmMode::kWgrad, GemmEpilogue::kStore>(map_a, map_b, map_c, c2, args, ctas, stream);
-  }
+  if (mode != GemmMode::kWgrad || epi != GemmEpilogue::kStore) return cudaErrorInvalidValue;
+  if (args.direct_epilogue)
+    return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, false, false>, kThreads, kSmemBytes, map_a, map_b, map_c, c2, args, ctas, stream);
+  return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, true, false>, kThreads, kSmemBytes, map_a, map_b, map_c, c2, args, ctas, stream);
 }
 
 }  // namespace fastb

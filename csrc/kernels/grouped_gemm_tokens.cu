@@ -1,0 +1,491 @@
+// Grouped bf16 GEMM with the weights as operand A and the tokens as operand B: out[token, feature] is computed as
+// W x X^T tile by tile, 256 features (M) by up to 256 tokens (N), on CTA pairs (tcgen05.mma.cta_group::2).
+//
+//   kForward : out[rows of g, N]  = x[rows of g, K]  * W_g[N, K]^T     (A K-major)      store, or SwiGLU of gate and up
+//   kDgrad   : out[rows of g, K]  = dy[rows of g, N] * W_g[N, K]       (A MN-major)     store, or SwiGLU backward
+//
+// Why the tokens are N. A tile of M = 256 costs the same whatever is in it, and an expert's tokens rarely fill a multiple
+// of 256: 625 tokens took three 256-row tiles, 23 % of the work on padding; a decode step of one token did
+// the work of 256. N is free in steps of 16, so a tile is as wide as the tokens it holds (in steps of 32, the rows of a
+// TMA store). The second loss was the last wave: 32 weight tiles of the down projection on 74 pairs, or 384 on 74, leave
+// half of a wave idle; what does not fill whole waves is cut into equal shares of the reduction (TokSplit), whose fp32
+// partial sums are exchanged through L2.
+// What bounds it: up to about 200 tokens per expert the weights' bytes (HBM), above that the tensor pipe.
+// Measured before (tokens as M, 256-row tiles) and after, us, both forward projections of 8 experts of 4096 x 14336: 1 token
+// 179 -> 137, 64 tokens 521 -> 465 (2.8 GB of weights: 6.1 TB/s), 625 tokens per expert 1518 -> 1321; at full 256-token
+// tiles equal within 2 %.
+//
+// Each CTA of a pair loads its 128 features of A and its half of the tokens of B; the leader issues one M = 256 MMA per 16-wide
+// k step; a CTA's accumulator is [128 features (TMEM lanes)] x [n tokens (columns)], the transpose of what is stored. The
+// epilogue reads it in 16 x 256-bit fragments (a thread holds pairs of tokens of a feature), packs the pairs to bf16 and
+// lets stmatrix.trans write [token][64 features] boxes in shared memory, which leave by TMA stores of 64 x 32; the saved
+// gate|up tiles of the SwiGLU backward come in by TMA loads and ldmatrix.trans. Shared memory is what the epilogue must spare:
+// the operand tiles' way in and out takes 128 bytes a cycle already, all that there is. Written value by value (2-byte
+// stores, half-filled wavefronts) the same epilogue slowed the SwiGLU backward from 743 to 896 us.
+// SwiGLU wants gate and up of a feature in one thread: the A tile is fetched through a 5-D tensor map as [16 gate rows | 16 up
+// rows] x 4, so that the two 16-lane halves of a warp's fragments are gate and up of the same features.
+//
+// Barriers as in grouped_gemm_pair.cu. Every wait is bounded. No load is multicast.
+#include "gemm_epilogue_tma.cuh"
+#include "token_walker.h"
+
+namespace fastb {
+
+namespace {
+
+using namespace ptx;
+using namespace gemm;
+
+constexpr int kPairM = 256, kHalfM = 128;
+constexpr int kStages = 6;
+constexpr int kAccStages = 2;
+constexpr int kTmemCols = 512;
+constexpr int kABytes = kHalfM * BK * 2;          // 16 KiB
+constexpr int kBBytes = kTokTileN / 2 * BK * 2;   // 16 KiB: half of the widest tile's tokens
+constexpr int kStageBytes = kABytes + kBBytes;
+constexpr int kThreads = 192;
+constexpr int kStepTokens = 32;                   // tokens per epilogue step = rows of a TMA store
+constexpr int kBox = kStepTokens * 128;           // 4 KiB: 32 tokens x 64 features
+constexpr int kPrefix = 256;                      // entries of the tile-count prefix (several groups each when there are more)
+
+struct __align__(8) TokCtl {
+  uint64_t full[kStages], empty[kStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load[2];
+  uint32_t tmem_base;
+  int abort_flag, last_arrived, widest, share_weights;
+  int base[kPrefix + 1];                          // tiles of the groups before entry i
+};
+__host__ __device__ constexpr int epi_boxes(GemmEpilogue e) { return e == GemmEpilogue::kStore ? 2 : e == GemmEpilogue::kSwiGLU ? 3 : 4; }
+__host__ __device__ constexpr int smem_bytes(GemmEpilogue e) { return kStages * kStageBytes + 2 * epi_boxes(e) * kBox + 1024 + static_cast<int>(sizeof(TokCtl)); }
+static_assert(smem_bytes(GemmEpilogue::kSwiGLUBwd) <= 227 * 1024, "dynamic shared memory of one CTA on sm_100a");
+static_assert(kAccStages * kTokTileN <= kTmemCols, "two accumulators of 256 columns");
+static_assert(kTokPartialFloats == kHalfM * kTokTileN, "a partial is one CTA's accumulator");
+
+// Rows of group q that are worked on: the real ones, up to a multiple of the granule.
+__device__ __forceinline__ int tok_rows(const TokGemmArgs& p, int q) {
+  return p.group_rows ? ceil_to(p.group_rows[q], p.granule) : p.group_off[q + 1] - p.group_off[q];
+}
+
+// Tiles in order, group by group; `locate` wants non-decreasing tile numbers.
+struct TokTiles {
+  const TokGemmArgs& p;
+  const int* base;
+  int per_entry, entry = 0, g = 0, g_base = 0;
+  __device__ __forceinline__ int rows_of(int q) const { return tok_rows(p, q); }
+  struct Tile { int g, m, row0, n; };             // first row of the tile in the grouped matrix, rows = columns of the MMA
+  __device__ __forceinline__ Tile locate(int tile) {
+    if (tile >= base[entry + 1]) {
+      while (tile >= base[entry + 1]) ++entry;
+      g = entry * per_entry; g_base = base[entry];
+    }
+    int rows = rows_of(g);
+    while (tile >= g_base + tok_tiles(rows) * p.m_tiles) { g_base += tok_tiles(rows) * p.m_tiles; rows = rows_of(++g); }
+    const TokPlace at = tok_place(tile - g_base, p.m_tiles, tok_tiles(rows), p.band_tiles);
+    const int per = tok_tile_size(rows), t0 = at.t * per;
+    return Tile{g, at.m, p.group_off[g] + t0, min(per, rows - t0)};
+  }
+};
+
+__device__ __forceinline__ void tma_load_5d_pair(void* smem_dst, const CUtensorMap* map, int x0, int x1, int x2, int x3, int x4, uint32_t bar_cluster_addr) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(x4)
+      : "memory");
+}
+
+// 16 lanes x 32 columns of fp32: thread T gets, for the 8-column block j, r[4 j + {0, 1}] = lane T / 4, columns 8 j + 2 (T % 4)
+// + {0, 1}, and r[4 j + {2, 3}] = the same columns of lane T / 4 + 8.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+        "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four 8 x 8 bf16 matrices; thread i names row i % 8 of matrix i / 8. Transposed: register m of thread T holds rows 2 (T % 4) +
+// {0, 1} of column T / 4 of matrix m.
+__device__ __forceinline__ void stmatrix_trans(uint32_t smem, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_trans(uint32_t smem, uint32_t (&v)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(smem) : "memory");
+}
+// Row address of this thread for 16 tokens from 16 jj on (matrices: features 0-7 and 8-15 of the first 8 tokens, then of the other 8)
+// at feature chunk `chunk` (8 features each) of a swizzled box of [32 tokens][64 features].
+__device__ __forceinline__ uint32_t box_row(uint32_t box, int lane, int jj, int chunk) {
+  const int t = jj * 16 + ((lane >> 4) << 3) + (lane & 7), ch = chunk + ((lane >> 3) & 1);
+  return box + t * 128 + ((ch ^ (t & 7)) << 4);
+}
+__device__ __forceinline__ float as_f(uint32_t x) { return __uint_as_float(x); }
+
+template <GemmMode MODE, GemmEpilogue EPI>
+__global__ void __launch_bounds__(kThreads, 1)
+grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x128, const __grid_constant__ CUtensorMap map_x32,
+                           const __grid_constant__ CUtensorMap map_x16, const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2,
+                           const TokGemmArgs p) {
+  constexpr bool A_MN = MODE == GemmMode::kDgrad;
+  constexpr int kRing = epi_boxes(EPI) * kBox;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* ring = tiles + kStages * kStageBytes;
+  TokCtl* ctl = reinterpret_cast<TokCtl*>(ring + 2 * kRing);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cta = static_cast<int>(cluster_cta_rank());  // 0 = leader
+  const bool leader = cta == 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
+    for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * 4); mbar_init(&ctl->epi_load[a], 1); }
+    ctl->abort_flag = 0;
+    mbar_fence_init();
+    prefetch_tmap(&map_w);
+    prefetch_tmap(&map_x128);
+    prefetch_tmap(&map_x32);
+    prefetch_tmap(&map_x16);
+    prefetch_tmap(&map_c);
+    if (EPI != GemmEpilogue::kStore) prefetch_tmap(&map_c2);
+  }
+  if (warp == 1) { tmem_alloc_pair(&ctl->tmem_base, kTmemCols); tmem_relinquish_pair(); }
+  const int per_entry = div_up(p.num_groups, kPrefix);
+  if (warp == 2) {
+    // Prefix sums of the tile counts over the groups, the widest tile, and whether any group has several token tiles.
+    int run = 0, widest = 0, most = 0;
+    const int entries = div_up(p.num_groups, per_entry);
+    for (int e0 = 0; e0 < entries; e0 += 32) {
+      int mine = 0;
+      for (int q = (e0 + lane) * per_entry; q < min((e0 + lane + 1) * per_entry, p.num_groups); ++q) {
+        const int rows = tok_rows(p, q);
+        mine += tok_tiles(rows) * p.m_tiles;
+        widest = max(widest, tok_tile_size(rows));
+        most = max(most, tok_tiles(rows));
+      }
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+      if (e0 + lane < entries) ctl->base[e0 + lane + 1] = run + incl;
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    widest = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(widest)));
+    most = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(most)));
+    if (lane == 0) { ctl->base[0] = 0; ctl->widest = widest; ctl->share_weights = most > 1; }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers exist before anything arrives on them remotely
+  tc_fence_after_sync();
+  const uint32_t tmem_base = ctl->tmem_base;
+  volatile int* abort_flag = &ctl->abort_flag;
+
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const TokSplit split = TokSplit::make(ctl->base[div_up(p.num_groups, per_entry)], p.red_blocks, pairs, ctl->widest, ctl->share_weights != 0);
+  TokSegments segs(split, pair);
+  TokTiles walk{p, ctl->base, per_entry};
+  TokSegment sg;
+  // The other arrival counters are cleared for the next launch; this launch's are back at zero once all parts have arrived.
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < p.num_counters; i += blockDim.x) p.counters_next[i] = 0u;
+
+  if (warp == 0) {
+    // ---------------- TMA producer (both CTAs, each for its own halves) ----------------
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      int gated = -1;
+      while (ok && segs.next(sg)) {
+        const TokTiles::Tile tc = walk.locate(sg.tile);
+        if (p.gate_counter != nullptr) {
+          // Arrival gate: per group, or (gate_tile_rows > 0) per tile of that many rows of the grouped matrix that this one touches.
+          const int lo = p.gate_tile_rows > 0 ? tc.row0 / p.gate_tile_rows : tc.g, hi = p.gate_tile_rows > 0 ? (tc.row0 + tc.n - 1) / p.gate_tile_rows : tc.g;
+          for (int q = lo; ok && q <= hi; ++q) {
+            const int slot = min(q, p.gate_slots - 1);
+            if (slot == gated) continue;
+            if (!(ok = wait_ge_bounded(p.gate_counter + slot, p.gate_target[slot], p.status, kSiteRailArrive, slot, p.timeout_ns))) { *abort_flag = 1; break; }
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            gated = slot;
+          }
+          if (!ok) break;
+        }
+        const int half = tc.n >> 1, x_row = tc.row0 + cta * half;
+        const int n32 = half == 128 ? 0 : half >> 5, n16 = half == 128 ? 0 : (half >> 4) & 1;
+        const uint32_t bytes = 2u * (kABytes + static_cast<uint32_t>(half) * 128u);
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+          if (!(ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1, abort_flag, p.status, 100 + s, p.timeout_ns))) break;
+          uint8_t* sa = tiles + s * kStageBytes;
+          uint8_t* sb = sa + kABytes;
+          const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
+          if (leader) mbar_arrive_expect_tx(&ctl->full[s], bytes);
+          if (A_MN) {
+#pragma unroll
+            for (int j = 0; j < kHalfM / 64; ++j)
+              tma_load_2d_pair(sa + j * (BK * 128), &map_w, tc.m * kPairM + cta * kHalfM + j * 64, tc.g * p.w_rows_per_group + kb * BK, full_leader);
+          } else if (EPI == GemmEpilogue::kSwiGLU) {
+            tma_load_5d_pair(sa, &map_w, kb * BK, 0, 0, cta * 4, tc.g * p.m_tiles + tc.m, full_leader);
+          } else {
+            tma_load_2d_pair(sa, &map_w, kb * BK, tc.g * p.w_rows_per_group + tc.m * kPairM + cta * kHalfM, full_leader);
+          }
+          if (half == 128) tma_load_2d_pair(sb, &map_x128, kb * BK, x_row, full_leader);
+          for (int j = 0; j < n32; ++j) tma_load_2d_pair(sb + j * 4096, &map_x32, kb * BK, x_row + 32 * j, full_leader);
+          if (n16) tma_load_2d_pair(sb + n32 * 4096, &map_x16, kb * BK, x_row + 32 * n32, full_leader);
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (leader CTA only) ----------------
+    if (leader && elect_one()) {
+      int s = 0;
+      uint32_t ph = 0, acc_it = 0;
+      bool ok = true;
+      while (ok && segs.next(sg)) {
+        const TokTiles::Tile tc = walk.locate(sg.tile);
+        const uint32_t idesc = make_idesc_bf16(kPairM, tc.n, A_MN, false);
+        const int a = acc_it % kAccStages;
+        const uint32_t aph = (acc_it / kAccStages) & 1;
+        ++acc_it;
+        if (!(ok = mbar_wait_bounded(&ctl->acc_empty[a], aph ^ 1, abort_flag, p.status, 200 + a, p.timeout_ns))) break;
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + a * kTokTileN;
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+          if (!(ok = mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.status, 300 + s, p.timeout_ns))) break;
+          tc_fence_after_sync();
+          const uint32_t sa = smem_u32(tiles + s * kStageBytes), sb = sa + kABytes;
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint64_t da = A_MN ? make_smem_desc(sa + k * 2048, BK * 128, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
+            const uint64_t db = make_smem_desc(sb + k * 32, 16, 1024);
+            mma_bf16_ss_pair(d_tmem, da, db, idesc, (kb != sg.kb0 || k != 0) ? 1u : 0u);
+          }
+          mma_commit_pair(&ctl->empty[s], 0x3);
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+        if (ok) mma_commit_pair(&ctl->acc_full[a], 0x3);
+      }
+    }
+  } else {
+    // ---------------- epilogue (both CTAs, each for its 128 features) ----------------
+    const int quarter = warp & 3;
+    const int et = threadIdx.x - 64;              // 0..127 among the epilogue threads
+    const bool issuer = threadIdx.x == 64;
+    uint32_t acc_it = 0, ring_n = 0, load_ph = 0u;   // load_ph: one parity bit per half of the ring
+    bool ok = true;
+    while (ok && segs.next(sg)) {
+      const TokTiles::Tile tc = walk.locate(sg.tile);
+      const int a = acc_it % kAccStages;
+      const uint32_t aph = (acc_it / kAccStages) & 1;
+      ++acc_it;
+      const int steps = tc.n / kStepTokens;
+      const int gu_col = tc.m * (2 * kPairM) + cta * kPairM;   // SwiGLU backward: my 128 features' gate columns; up 128 further
+      auto load_gu = [&](int st) {                             // issuer only
+        uint8_t* b = ring + (st & 1) * kRing;
+        mbar_arrive_expect_tx(&ctl->epi_load[st & 1], 4 * kBox);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tma_load_2d(b + q * kBox, &map_c2, gu_col + q * 64, tc.row0 + st * kStepTokens, &ctl->epi_load[st & 1]);
+      };
+      if (EPI == GemmEpilogue::kSwiGLUBwd && issuer && sg.parts == 1) {   // the saved tiles arrive while the MMAs still run
+        bulk_wait_read<0>();
+        load_gu(0);
+        if (steps > 1) load_gu(1);
+      }
+      if (!(ok = mbar_wait_bounded(&ctl->acc_full[a], aph, abort_flag, p.status, 400 + a, p.timeout_ns))) break;
+      tc_fence_after_sync();
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kTokTileN;
+      auto release_acc = [&]() {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->acc_empty[a]), 0));
+      };
+      const float4* parts_at[2] = {nullptr, nullptr};          // my values of the first and of the second part
+      const size_t part_step = static_cast<size_t>(sg.pair_step) * kTokPartialFloats;   // from there on, in float4s: four partials per pair
+      if (sg.parts > 1) {
+        // Part of a tile: leave my sums (values in the order in which the same thread of another CTA holds them), and go on only
+        // if all other parts are there already.
+        float4* out = reinterpret_cast<float4*>(p.partials + (static_cast<size_t>(pair * 2 + (sg.part == 0 ? 1 : 0)) * 2 + cta) * kTokPartialFloats) + et;
+        for (int st = 0; st < steps; ++st) {
+          uint32_t r[32];
+          tmem_ld_16x32(t_row + st * kStepTokens, r);
+          tmem_ld_16x32(t_row + (16u << 16) + st * kStepTokens, r + 16);
+          tmem_wait_ld();
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            __stcg(out + static_cast<size_t>(st * 8 + q) * kHalfM, make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3])));
+        }
+        release_acc();
+        __threadfence();
+        epi_bar();
+        if (issuer) ctl->last_arrived = atomicInc(p.counters + (sg.tile - split.whole_tiles) * 2 + cta, static_cast<unsigned>(sg.parts - 1)) == static_cast<unsigned>(sg.parts - 1);
+        epi_bar();
+        if (!ctl->last_arrived) continue;
+        __threadfence();
+        const float* base = p.partials + static_cast<size_t>(cta) * kTokPartialFloats;
+        parts_at[0] = reinterpret_cast<const float4*>(base + static_cast<size_t>(sg.first_pair * 2 + 1) * 2 * kTokPartialFloats) + et;
+        parts_at[1] = reinterpret_cast<const float4*>(base + static_cast<size_t>((sg.first_pair + sg.pair_step) * 2) * 2 * kTokPartialFloats) + et;
+        if (EPI == GemmEpilogue::kSwiGLUBwd && issuer) {
+          bulk_wait_read<0>();
+          load_gu(0);
+          if (steps > 1) load_gu(1);
+        }
+      }
+      // 32 tokens of my features (r[0..15]: lanes 0-15 of the warp, r[16..31]: lanes 16-31): from tensor memory, or the parts in
+      // the order of the reduction.
+      auto load_acc = [&](int st, uint32_t (&r)[32]) {
+        if (sg.parts == 1) {
+          tmem_ld_16x32(t_row + st * kStepTokens, r);
+          tmem_ld_16x32(t_row + (16u << 16) + st * kStepTokens, r + 16);
+          tmem_wait_ld();
+          return;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float4 v = __ldcg(parts_at[0] + static_cast<size_t>(st * 8 + q) * kHalfM);
+          r[4 * q] = __float_as_uint(v.x); r[4 * q + 1] = __float_as_uint(v.y); r[4 * q + 2] = __float_as_uint(v.z); r[4 * q + 3] = __float_as_uint(v.w);
+        }
+        const float4* more = parts_at[1];
+        for (int j = 1; j < sg.parts; ++j, more += part_step) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float4 v = __ldcg(more + static_cast<size_t>(st * 8 + q) * kHalfM);
+            r[4 * q] = __float_as_uint(as_f(r[4 * q]) + v.x); r[4 * q + 1] = __float_as_uint(as_f(r[4 * q + 1]) + v.y);
+            r[4 * q + 2] = __float_as_uint(as_f(r[4 * q + 2]) + v.z); r[4 * q + 3] = __float_as_uint(as_f(r[4 * q + 3]) + v.w);
+          }
+        }
+      };
+      // 16 features x 32 tokens (16 values a thread) -> bf16 -> a box, at feature chunk `chunk`.
+      auto put = [&](uint32_t box, int chunk, const uint32_t* v) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const uint32_t* q = v + 8 * jj;
+          stmatrix_trans(box_row(box, lane, jj, chunk), pack_bf16(as_f(q[0]), as_f(q[1])), pack_bf16(as_f(q[2]), as_f(q[3])), pack_bf16(as_f(q[4]), as_f(q[5])),
+                         pack_bf16(as_f(q[6]), as_f(q[7])));
+        }
+      };
+      for (int st = 0; st < steps; ++st) {
+        uint32_t r[32];
+        load_acc(st, r);
+        const int y = tc.row0 + st * kStepTokens;
+        if (EPI == GemmEpilogue::kSwiGLUBwd) {
+          uint8_t* b = ring + (st & 1) * kRing;
+          if (!(ok = mbar_wait_bounded(&ctl->epi_load[st & 1], (load_ph >> (st & 1)) & 1u, abort_flag, p.status, 500, p.timeout_ns))) break;
+          load_ph ^= 1u << (st & 1);
+          const uint32_t gb = smem_u32(b + (quarter >> 1) * kBox), ub = gb + 2 * kBox;
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              const int chunk = (quarter & 1) * 4 + h * 2;
+              const uint32_t ga = box_row(gb, lane, jj, chunk), ua = box_row(ub, lane, jj, chunk);
+              uint32_t gv[4], uv[4];
+              ldmatrix_trans(ga, gv);
+              ldmatrix_trans(ua, uv);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const float2 g2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv[q])), u2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&uv[q]));
+                float dg[2], du[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  const float g = i ? g2.y : g2.x, u = i ? u2.y : u2.x;
+                  // d(act) is rounded to bf16 first, as the unfused path stores it before the element-wise kernel
+                  const float da = __bfloat162float(__float2bfloat16_rn(as_f(r[16 * h + 8 * jj + 2 * q + i])));
+                  const float sgm = 1.0f / (1.0f + __expf(-g));
+                  const float sl = g * sgm;
+                  du[i] = da * sl;
+                  dg[i] = da * u * (sgm + sl * (1.0f - sgm));
+                }
+                gv[q] = pack_bf16(dg[0], dg[1]);
+                uv[q] = pack_bf16(du[0], du[1]);
+              }
+              stmatrix_trans(ga, gv[0], gv[1], gv[2], gv[3]);
+              stmatrix_trans(ua, uv[0], uv[1], uv[2], uv[3]);
+            }
+          fence_proxy_async_smem();
+          epi_bar();
+          if (issuer) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tma_store_2d(&map_c, b + q * kBox, gu_col + q * 64, y);
+            bulk_commit();
+            if (st + 2 < steps) { bulk_wait_read<0>(); load_gu(st + 2); }
+          }
+        } else {
+          uint8_t* b = ring + (ring_n & 1u) * kRing;
+          if (issuer) bulk_wait_read<1>();   // the stores that read this half of the ring two steps ago are done with it
+          epi_bar();
+          const uint32_t sb = smem_u32(b);
+          if (EPI == GemmEpilogue::kStore) {
+            put(sb + (quarter >> 1) * kBox, (quarter & 1) * 4, r);
+            put(sb + (quarter >> 1) * kBox, (quarter & 1) * 4 + 2, r + 16);
+          } else {  // r[0..15]: gate, r[16..31]: up of features 16 quarter ..
+            if (p.keep_gate_up) {
+              put(sb + kBox, quarter * 2, r);
+              put(sb + 2 * kBox, quarter * 2, r + 16);
+            }
+            uint32_t act[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) act[i] = __float_as_uint(silu(as_f(r[i])) * as_f(r[16 + i]));
+            put(sb, quarter * 2, act);
+          }
+          fence_proxy_async_smem();
+          epi_bar();
+          if (issuer) {
+            if (EPI == GemmEpilogue::kStore) {
+              const int x = tc.m * kPairM + cta * kHalfM;
+              tma_store_2d(&map_c, b, x, y);
+              tma_store_2d(&map_c, b + kBox, x + 64, y);
+            } else {
+              tma_store_2d(&map_c, b, tc.m * kHalfM + cta * 64, y);
+              if (p.keep_gate_up) {
+                tma_store_2d(&map_c2, b + kBox, tc.m * kPairM + cta * 64, y);
+                tma_store_2d(&map_c2, b + 2 * kBox, tc.m * kPairM + kHalfM + cta * 64, y);
+              }
+            }
+            bulk_commit();
+          }
+          ++ring_n;
+        }
+      }
+      if (!ok) break;
+      if (sg.parts == 1) release_acc();
+    }
+    if (issuer) bulk_wait_all();  // every bulk store of this CTA has landed before anything is torn down
+  }
+  // ---------------- teardown: nobody frees tensor memory while the pair still uses it ----------------
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) { tc_fence_after_sync(); tmem_dealloc_pair(tmem_base, kTmemCols); }
+}
+
+template <GemmMode MODE, GemmEpilogue EPI>
+cudaError_t launch(const TokGemmMaps& m, const TokGemmArgs& args, int ctas, cudaStream_t stream) {
+  auto kern = grouped_gemm_tokens_kernel<MODE, EPI>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(EPI));
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas & ~1);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem_bytes(EPI);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, kern, *m.w, *m.x128, *m.x32, *m.x16, *m.c, m.c2 ? *m.c2 : *m.c, args);
+  if (e == cudaSuccess) note_launch();
+  return e;
+}
+
+}  // namespace
+
+cudaError_t launch_grouped_gemm_tokens(GemmMode mode, GemmEpilogue epi, const TokGemmMaps& maps, const TokGemmArgs& args, int ctas, cudaStream_t stream) {
+  if (ctas < 2 || args.num_groups < 1 || args.m_tiles < 1 || args.red_blocks < 1 || args.band_tiles < 1) return cudaErrorInvalidValue;
+  if ((args.granule != 32 && args.granule != 64) || args.partials == nullptr || args.counters == nullptr || args.counters_next == nullptr) return cudaErrorInvalidValue;
+  if (args.num_counters < tok_counters(ctas)) return cudaErrorInvalidValue;
+  if (mode == GemmMode::kForward && epi == GemmEpilogue::kStore) return launch<GemmMode::kForward, GemmEpilogue::kStore>(maps, args, ctas, stream);
+  if (mode == GemmMode::kForward && epi == GemmEpilogue::kSwiGLU && (args.keep_gate_up != 0) == (maps.c2 != nullptr))
+    return launch<GemmMode::kForward, GemmEpilogue::kSwiGLU>(maps, args, ctas, stream);
+  if (mode == GemmMode::kDgrad && epi == GemmEpilogue::kStore) return launch<GemmMode::kDgrad, GemmEpilogue::kStore>(maps, args, ctas, stream);
+  if (mode == GemmMode::kDgrad && epi == GemmEpilogue::kSwiGLUBwd && maps.c2 != nullptr) return launch<GemmMode::kDgrad, GemmEpilogue::kSwiGLUBwd>(maps, args, ctas, stream);
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace fastb

@@ -194,12 +194,13 @@ __global__ void build_send_list_kernel(const int* __restrict__ topk_idx, const i
   list[send_pos[e] + block_base[static_cast<long long>(t / kTokensPerBlock) * E + e] + slot_in_block[tj]] = static_cast<int>(tj);
 }
 
-// Zeroes the rows between each group's real end and its padded end.
-__global__ void zero_pad_rows_kernel(unsigned char* buf, long long row_bytes, const int* __restrict__ group_off, const int* __restrict__ group_rows, int groups) {
+// Zeroes the rows between each group's real end and its padded end, or the next multiple of `align` rows.
+__global__ void zero_pad_rows_kernel(unsigned char* buf, long long row_bytes, const int* __restrict__ group_off, const int* __restrict__ group_rows, int groups, int align) {
   const int g = blockIdx.y;
   if (g >= groups) return;
   const long long begin = (static_cast<long long>(group_off[g]) + group_rows[g]) * row_bytes;
-  const long long end = static_cast<long long>(group_off[g + 1]) * row_bytes;
+  const long long last = align > 0 ? static_cast<long long>(group_off[g]) + (group_rows[g] + align - 1) / align * align : group_off[g + 1];
+  const long long end = last * row_bytes;
   uint4* p = reinterpret_cast<uint4*>(buf + begin);
   const long long n = (end - begin) / 16;
   for (long long i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += static_cast<long long>(gridDim.x) * blockDim.x) p[i] = make_uint4(0, 0, 0, 0);
@@ -249,10 +250,10 @@ cudaError_t launch_build_send_list(const int* topk_idx, const int* slot_in_block
   return cudaGetLastError();
 }
 
-cudaError_t launch_zero_pad_rows(void* buf, long long row_bytes, const int* group_off, const int* group_rows, int groups, cudaStream_t stream) {
-  if (row_bytes % 16) return cudaErrorInvalidValue;
+cudaError_t launch_zero_pad_rows(void* buf, long long row_bytes, const int* group_off, const int* group_rows, int groups, int align, cudaStream_t stream) {
+  if (row_bytes % 16 || align < 0) return cudaErrorInvalidValue;
   if (groups == 0) return cudaSuccess;
-  zero_pad_rows_kernel<<<dim3(8, groups), 256, 0, stream>>>(static_cast<unsigned char*>(buf), row_bytes, group_off, group_rows, groups);
+  zero_pad_rows_kernel<<<dim3(8, groups), 256, 0, stream>>>(static_cast<unsigned char*>(buf), row_bytes, group_off, group_rows, groups, align);
   note_launch();
   return cudaGetLastError();
 }

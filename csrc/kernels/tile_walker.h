@@ -29,6 +29,7 @@ constexpr int kDefaultBandRows = 4096;
 template <int TILE_M>
 struct TileWalker {
   const int* off; int G, tiles_n, fixed_m, red_len; bool wgrad; int band_rows;
+  const int* rows = nullptr;  // wgrad, optional: real rows per group; the reduction stops at the block that holds the last of them
   int g = 0, base = 0;
   FASTB_HD bool locate(int tile, TileCoord& c) {
     while (g < G) {
@@ -42,7 +43,7 @@ struct TileWalker {
         const int band = local / (kBand * tiles_n), rem = local % (kBand * tiles_n);
         const int m0 = band * kBand, left = mt - m0, cur = kBand < left ? kBand : left;
         c.g = g; c.n_idx = rem / cur; c.m_idx = m0 + rem % cur; c.row0 = r0;
-        c.red_blocks = wgrad ? (r1 - r0) / kWalkBK : red_len / kWalkBK;
+        c.red_blocks = !wgrad ? red_len / kWalkBK : rows ? (rows[g] + kWalkBK - 1) / kWalkBK : (r1 - r0) / kWalkBK;
         return true;
       }
       base += cnt; ++g;

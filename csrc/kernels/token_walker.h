@@ -1,0 +1,115 @@
+// Work split of the grouped GEMM whose N dimension is the tokens (grouped_gemm_tokens.cu): which tiles there are, in which
+// order, and which part of the reduction of which tile a CTA pair does. Plain arithmetic, usable from host code too.
+#pragma once
+
+#if defined(__CUDACC__)
+#define FASTB_HD __host__ __device__
+#else
+#define FASTB_HD
+#endif
+
+namespace fastb {
+namespace gemm {
+
+constexpr int kTokTileN = 256;      // most tokens of one tile
+
+FASTB_HD constexpr int ceil_to(int x, int q) { return (x + q - 1) / q * q; }
+FASTB_HD constexpr int div_up(int a, int b) { return (a + b - 1) / b; }
+
+// Token tiles of a group whose tokens are taken up to `rows` (real rows rounded up to the granule, a multiple of 32): as few
+// as hold them, all but the last of one width, in multiples of 32. 640 tokens are 3 tiles of 224, 224 and 192 instead of
+// 256, 256 and 128: tiles that run side by side then advance at one pace and keep sharing operand panels.
+FASTB_HD inline int tok_tiles(int rows) { return div_up(rows, kTokTileN); }
+FASTB_HD inline int tok_tile_size(int rows) {
+  const int t = tok_tiles(rows);
+  return t > 0 ? ceil_to(div_up(rows, t), 32) : 0;
+}
+
+// How `tiles` tiles of kb_tile reduction blocks are spread over `pairs` CTA pairs. Whole tiles go round robin; where the last
+// wave would be partly idle, its tiles are cut along the reduction. A pair that does a part of a tile leaves fp32 partial
+// sums, and the pair that arrives last adds them up. Two ways of cutting:
+//   stream (no two tiles share weights, i.e. every group fits one token tile): the last full wave and the rest are one sequence
+//       of reduction blocks, cut into equal shares wherever the cut falls. Every pair then works equally long. The weights are
+//       read once whatever the order, and the tokens stay in L2.
+//   parts  (tiles share weights): the rest is cut into as many equal parts as there are pairs for it, part by part: pairs that
+//       run side by side stay at the same depth of the reduction and share operand panels in L2. Cut as a stream, a
+//       reduction of 28672 over 4096 tokens fell from 1.5 to 1.2 PFLOP/s: each pair fetched panels of its own.
+// A cut pays when the blocks that the last wave would leave idle exceed what the exchange costs: about 2 blocks plus one per 16
+// tokens of the tile, i.e. its fp32 sums written and read once at an SM's share of L2.
+struct TokSplit {
+  int pairs, kb_tile;
+  int whole_tiles;     // tiles done whole, tile i by pair i % pairs
+  int cut_tiles;       // tiles from whole_tiles on, done in parts
+  int shares;          // stream: pairs that take a share; parts: parts per tile
+  bool stream;
+  FASTB_HD static TokSplit make(int tiles, int kb_tile, int pairs, int widest_n, bool share_weights) {
+    TokSplit s{pairs, kb_tile, tiles, 0, 1, !share_weights};
+    const int rest = tiles % pairs, cost = 2 + widest_n / 16;
+    if (rest == 0 || kb_tile < 2) return s;
+    if (share_weights) {
+      int n = pairs / rest < kb_tile / 4 ? pairs / rest : kb_tile / 4;
+      n = n < 8 ? n : 8;
+      if (n < 2 || kb_tile - div_up(kb_tile, n) <= cost) return s;
+      s.whole_tiles = tiles - rest; s.cut_tiles = rest; s.shares = n;
+      return s;
+    }
+    const long long idle = static_cast<long long>(pairs - rest) * kb_tile / pairs;   // blocks per pair that a last wave leaves idle
+    if (idle <= cost) return s;
+    const int full = tiles / pairs;
+    s.whole_tiles = full > 1 ? (full - 1) * pairs : 0;
+    s.cut_tiles = tiles - s.whole_tiles;
+    const long long units = static_cast<long long>(s.cut_tiles) * kb_tile;
+    s.shares = units / 4 < pairs ? static_cast<int>(units / 4 > 0 ? units / 4 : 1) : pairs;  // a share is at least four blocks
+    return s;
+  }
+  FASTB_HD long long cut_units() const { return static_cast<long long>(cut_tiles) * kb_tile; }
+  FASTB_HD int share_begin(int p) const { return static_cast<int>(cut_units() * p / shares); }
+  // The pair whose share holds unit u: the largest p with share_begin(p) <= u.
+  FASTB_HD int share_of(int u) const { return static_cast<int>(((static_cast<long long>(u) + 1) * shares - 1) / cut_units()); }
+};
+
+// One pair's segments in order: tile, first block, end block, number of parts of the tile, my part, and the pairs that do the
+// parts: first_pair + j * pair_step for part j.
+struct TokSegment { int tile, kb0, kb1, parts, part, first_pair, pair_step; };
+struct TokSegments {
+  TokSplit s;
+  int pair, next_whole, u, u_end;
+  FASTB_HD TokSegments(const TokSplit& split, int pair_) : s(split), pair(pair_), next_whole(pair_), u(0), u_end(0) {
+    if (s.cut_tiles == 0) return;
+    if (!s.stream) u_end = pair < s.cut_tiles * s.shares ? 1 : 0;
+    else if (pair < s.shares) { u = s.share_begin(pair); u_end = s.share_begin(pair + 1); }
+  }
+  FASTB_HD bool next(TokSegment& g) {
+    if (next_whole < s.whole_tiles) {
+      g = TokSegment{next_whole, 0, s.kb_tile, 1, 0, pair, 1};
+      next_whole += s.pairs;
+      return true;
+    }
+    if (u >= u_end) return false;
+    if (!s.stream) {
+      const int t = pair % s.cut_tiles, j = pair / s.cut_tiles;
+      g = TokSegment{s.whole_tiles + t, static_cast<int>(static_cast<long long>(s.kb_tile) * j / s.shares), static_cast<int>(static_cast<long long>(s.kb_tile) * (j + 1) / s.shares),
+                     s.shares, j, t, s.cut_tiles};
+      u = u_end;
+      return true;
+    }
+    const int t = u / s.kb_tile, kb0 = u - t * s.kb_tile;
+    const int left = s.kb_tile - kb0, kb1 = kb0 + (u_end - u < left ? u_end - u : left);
+    const int lo = s.share_of(t * s.kb_tile), hi = s.share_of((t + 1) * s.kb_tile - 1);
+    g = TokSegment{s.whole_tiles + t, kb0, kb1, hi - lo + 1, pair - lo, lo, 1};
+    u += kb1 - kb0;
+    return true;
+  }
+};
+
+// Place of tile `local` inside its group: bands of `band` token tiles, token tiles fastest inside a band, so that the
+// tiles that run together cover a squarish patch and share their operand panels in L2.
+struct TokPlace { int m, t; };
+FASTB_HD inline TokPlace tok_place(int local, int m_tiles, int t_tiles, int band_tiles) {
+  const int per_band = band_tiles * m_tiles, band = local / per_band, rem = local - band * per_band;
+  const int t0 = band * band_tiles, left = t_tiles - t0, cur = left < band_tiles ? left : band_tiles;
+  return TokPlace{rem / cur, t0 + rem % cur};
+}
+
+}  // namespace gemm
+}  // namespace fastb

@@ -67,6 +67,100 @@ struct TensorMap2D {
   }
 };
 
+CUtensorMap bf16_map(int rank, int64_t ptr, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+  TORCH_CHECK(ptr % 16 == 0, "tensor map base must be 16-byte aligned");
+  for (int i = 0; i + 1 < rank; ++i) TORCH_CHECK(strides[i] % 16 == 0, "tensor map strides must be multiples of 16 bytes");
+  alignas(64) CUtensorMap m;
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, reinterpret_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  TORCH_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", static_cast<int>(r));
+  return m;
+}
+CUtensorMap bf16_map_2d(const torch::Tensor& t, int box_rows) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 2 && t.stride(1) == 1, "expected a CUDA bf16 matrix with contiguous rows");
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(t.size(1)), static_cast<cuuint64_t>(t.size(0))}, strides[1] = {static_cast<cuuint64_t>(t.stride(0)) * 2};
+  const cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
+  return bf16_map(2, reinterpret_cast<int64_t>(t.data_ptr()), dims, strides, box);
+}
+
+// One contraction on fixed buffers (weights, tokens, outputs): everything about the launch of grouped_gemm_tokens that does not
+// change from call to call, the tensor maps above all.
+struct TokGemmPlan {
+  alignas(64) CUtensorMap w, x128, x32, x16, c, c2;
+  GemmMode mode;
+  GemmEpilogue epi;
+  bool has_c2;
+  int device;
+  int64_t groups;
+  TokGemmArgs a{};
+
+  // weights [G, N, K]; forward: tokens [R, K] -> out [R, N] (SwiGLU [R, N / 2]); dgrad: tokens [R, N] -> out [R, K] (SwiGLU backward [R, 2 K]).
+  TokGemmPlan(int mode_, int epi_, torch::Tensor weights, torch::Tensor tokens, torch::Tensor out, c10::optional<torch::Tensor> gate_up, int granule, int band_rows)
+      : mode(static_cast<GemmMode>(mode_)), epi(static_cast<GemmEpilogue>(epi_)), has_c2(gate_up.has_value()) {
+    TORCH_CHECK(weights.is_cuda() && weights.scalar_type() == torch::kBFloat16 && weights.dim() == 3 && weights.is_contiguous(), "weights: contiguous CUDA bf16 [G, N, K]");
+    const int64_t G = weights.size(0), N = weights.size(1), K = weights.size(2);
+    const bool fwd = mode == GemmMode::kForward;
+    const int64_t feats = fwd ? N : K, red = fwd ? K : N, cols = epi == GemmEpilogue::kSwiGLU ? N / 2 : epi == GemmEpilogue::kSwiGLUBwd ? 2 * K : feats;
+    TORCH_CHECK(mode != GemmMode::kWgrad && feats % 256 == 0 && red % 64 == 0, "grouped_gemm_tokens: features must be a multiple of 256, the reduction of 64");
+    TORCH_CHECK(tokens.dim() == 2 && tokens.size(1) == red && out.dim() == 2 && out.size(1) == cols && out.size(0) == tokens.size(0), "grouped_gemm_tokens: shapes");
+    TORCH_CHECK(!has_c2 || (gate_up->size(0) == tokens.size(0) && gate_up->size(1) == (fwd ? N : 2 * K)), "grouped_gemm_tokens: gate|up shape");
+    device = weights.get_device();
+    groups = G;
+    const int64_t wp = reinterpret_cast<int64_t>(weights.data_ptr());
+    if (fwd && epi == GemmEpilogue::kSwiGLU) {
+      // [G * N / 256 tiles][8 groups of 16 features][gate, up][16][K], fetched as four groups with both halves
+      const cuuint64_t k = static_cast<cuuint64_t>(K), dims[5] = {k, 16, 2, 8, static_cast<cuuint64_t>(G * N / 256)}, strides[4] = {2 * k, 256 * k, 32 * k, 512 * k};
+      const cuuint32_t box[5] = {64, 16, 2, 4, 1};
+      w = bf16_map(5, wp, dims, strides, box);
+    } else {
+      w = bf16_map_2d(weights.view({G * N, K}), fwd ? 128 : 64);
+    }
+    x128 = bf16_map_2d(tokens, 128); x32 = bf16_map_2d(tokens, 32); x16 = bf16_map_2d(tokens, 16);
+    c = bf16_map_2d(out, 32);
+    if (has_c2) c2 = bf16_map_2d(*gate_up, 32);
+    a.num_groups = static_cast<int>(G);
+    a.m_tiles = static_cast<int>(feats / 256); a.red_blocks = static_cast<int>(red / 64); a.w_rows_per_group = static_cast<int>(N);
+    a.band_tiles = std::max(1, (band_rows > 0 ? band_rows : 4096) / 256);
+    a.granule = granule; a.keep_gate_up = fwd && has_c2 ? 1 : 0;
+  }
+
+  // counters: int32 [2, >= tok_counters(ctas)], kept by the caller, parity alternating from launch to launch; none = cleared for this launch.
+  void run(torch::Tensor group_off, c10::optional<torch::Tensor> group_rows, int64_t status_ptr, uint64_t timeout_ns, int ctas, int64_t gate_counter_ptr,
+           c10::optional<torch::Tensor> gate_target, int gate_tile_rows, c10::optional<torch::Tensor> counters, int parity) const {
+    TORCH_CHECK(group_off.is_cuda() && group_off.dtype() == torch::kInt32 && group_off.is_contiguous() && group_off.numel() == groups + 1, "group_off: cuda int32[G+1]");
+    TokGemmArgs g = a;
+    g.group_off = group_off.data_ptr<int>();
+    if (group_rows.has_value()) {
+      want(*group_rows, torch::kInt32, "group_rows");
+      TORCH_CHECK(group_rows->numel() >= groups, "group_rows: int32 [G]");
+      g.group_rows = group_rows->data_ptr<int>();
+    }
+    g.status = reinterpret_cast<DeviceStatus*>(status_ptr);
+    g.timeout_ns = timeout_ns;
+    if (gate_counter_ptr != 0) {
+      TORCH_CHECK(gate_target.has_value() && gate_target->is_cuda() && gate_target->scalar_type() == torch::kInt64 &&
+                  gate_target->numel() >= (gate_tile_rows > 0 ? 1 : groups), "gate_target: cuda int64[G], or one entry per tile with gate_tile_rows");
+      g.gate_slots = static_cast<int>(gate_target->numel());
+      g.gate_counter = reinterpret_cast<const unsigned long long*>(gate_counter_ptr);
+      g.gate_target = reinterpret_cast<const unsigned long long*>(gate_target->data_ptr());
+      g.gate_tile_rows = gate_tile_rows;
+    }
+    ctas &= ~1;
+    const auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, device);
+    auto partials = torch::empty({tok_partial_floats(ctas)}, i32.dtype(torch::kFloat32));  // stream-ordered, as the launch is
+    torch::Tensor cnt = counters.has_value() ? *counters : torch::zeros({2, tok_counters(ctas)}, i32);
+    TORCH_CHECK(cnt.dim() == 2 && cnt.size(0) == 2 && cnt.is_contiguous() && cnt.scalar_type() == torch::kInt32, "counters: int32 [2, n]");
+    unsigned int* base = reinterpret_cast<unsigned int*>(cnt.data_ptr<int>());
+    g.partials = partials.data_ptr<float>();
+    g.num_counters = static_cast<int>(cnt.size(1));
+    g.counters = base + (parity & 1) * g.num_counters;
+    g.counters_next = base + (~parity & 1) * g.num_counters;
+    const TokGemmMaps maps{&w, &x128, &x32, &x16, &c, has_c2 ? &c2 : nullptr};
+    cu_check(launch_grouped_gemm_tokens(mode, epi, maps, g, ctas, stream_now()), "grouped_gemm_tokens launch");
+  }
+};
+
 void grouped_gemm(int mode, int epilogue, const TensorMap2D& a, const TensorMap2D& b, torch::Tensor group_off, int tiles_n, int fixed_m_tiles,
                   int red_len, int b_rows_per_group, int c_rows_per_group, torch::Tensor c, c10::optional<torch::Tensor> c2, int64_t status_ptr,
                   uint64_t timeout_ns, int ctas, int64_t gate_counter_ptr, c10::optional<torch::Tensor> gate_target, bool pair, int band_rows,
@@ -159,10 +253,10 @@ void splits_scan(const HeapPy& heap, int64_t counts_off, int64_t flags_off, uint
   cu_check(launch_splits_scan(a, stream_now()), "splits_scan");
 }
 
-void zero_pad_rows(torch::Tensor buf, torch::Tensor group_off, torch::Tensor group_rows) {
+void zero_pad_rows(torch::Tensor buf, torch::Tensor group_off, torch::Tensor group_rows, int align) {
   TORCH_CHECK(buf.is_cuda() && buf.dim() == 2 && buf.is_contiguous(), "buf: contiguous CUDA matrix");
   cu_check(launch_zero_pad_rows(buf.data_ptr(), buf.size(1) * buf.element_size(), group_off.data_ptr<int>(), group_rows.data_ptr<int>(),
-                                static_cast<int>(group_rows.numel()), stream_now()), "zero_pad_rows");
+                                static_cast<int>(group_rows.numel()), align, stream_now()), "zero_pad_rows");
 }
 
 void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, c10::optional<torch::Tensor> row_scale, torch::Tensor slot_in_block,
@@ -210,6 +304,11 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
 
 void bind_moe(py::module_& m) {
   py::class_<TensorMap2D>(m, "TensorMap2D").def(py::init<int64_t, int64_t, int64_t, int64_t, int, int>()).def_static("bytes", &TensorMap2D::bytes);
+  py::class_<TokGemmPlan>(m, "TokGemmPlan")
+      .def(py::init<int, int, torch::Tensor, torch::Tensor, torch::Tensor, c10::optional<torch::Tensor>, int, int>())
+      .def("run", &TokGemmPlan::run, py::arg("group_off"), py::arg("group_rows"), py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"),
+           py::arg("gate_counter_ptr") = 0, py::arg("gate_target") = py::none(), py::arg("gate_tile_rows") = 0, py::arg("counters") = py::none(), py::arg("parity") = 0);
+  m.attr("TOK_COUNTERS_PER_CTA") = tok_counters(1);
   m.def("grouped_gemm", &grouped_gemm, py::arg("mode"), py::arg("epilogue"), py::arg("a"), py::arg("b"), py::arg("group_off"), py::arg("tiles_n"),
         py::arg("fixed_m_tiles"), py::arg("red_len"), py::arg("b_rows_per_group"), py::arg("c_rows_per_group"), py::arg("c"), py::arg("c2"),
         py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"), py::arg("gate_counter_ptr"), py::arg("gate_target"), py::arg("pair"),
@@ -222,7 +321,7 @@ void bind_moe(py::module_& m) {
         py::arg("send_base"), py::arg("send_cnt"), py::arg("group_off"), py::arg("group_rows"), py::arg("arrive_target"), py::arg("traffic"),
         py::arg("num_channels"), py::arg("row_align"), py::arg("cap_rows"), py::arg("status"), py::arg("timeout_ns"), py::arg("send_pos"),
         py::arg("epoch_dev_ptr"), py::arg("tile_target") = py::none(), py::arg("tile_rows") = 0);
-  m.def("zero_pad_rows", &zero_pad_rows);
+  m.def("zero_pad_rows", &zero_pad_rows, py::arg("buf"), py::arg("group_off"), py::arg("group_rows"), py::arg("align") = 0);
   m.def("build_send_list", [](torch::Tensor topk_idx, torch::Tensor slot_in_block, torch::Tensor block_base, torch::Tensor send_pos, torch::Tensor list, const StatusPy& st) {
     want(topk_idx, torch::kInt32, "topk_idx"); want(send_pos, torch::kInt32, "send_pos"); want(list, torch::kInt32, "list");
     TORCH_CHECK(list.numel() >= topk_idx.numel(), "build_send_list: list too short");

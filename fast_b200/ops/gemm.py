@@ -20,7 +20,7 @@ _BM, _BN, _BK = 128, 256, 64
 USE_PAIR = CONFIG.gemm != "one"
 # Rows of a raster band (see csrc/kernels/gemm_common.cuh); 0 = kernel default.
 BAND_ROWS = CONFIG.band_rows
-# CTA-pair kernel: True = epilogue threads write global memory row by row; False = staged tiles + TMA stores.
+# CTA-pair weight gradients: True = epilogue threads write global memory row by row; False = staged tiles + TMA stores.
 DIRECT_EPILOGUE = False
 
 
@@ -89,9 +89,40 @@ def _tmap_bytes(t: torch.Tensor, box_rows: int):
     return m
 
 
+class TokScratch:
+    """Arrival counters of the token-major kernel's partial tiles, kept by a caller that launches it again and again on one
+    stream (an engine): one half serves a launch, which clears the other half for the next. Without it a launch clears its own."""
+
+    def __init__(self, device):
+        self.ctas = torch.cuda.get_device_properties(device).multi_processor_count
+        self.counters = torch.zeros(2, self.ctas * runtime.ext().TOK_COUNTERS_PER_CTA, dtype=torch.int32, device=device)
+        self.parity = 0
+
+
+_plans: dict = {}
+
+
+def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
+             granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch]) -> None:
+    key = (mode, epi, granule, BAND_ROWS, w.data_ptr(), w.shape, x.data_ptr(), x.shape, x.stride(0), out.data_ptr(), out.stride(0), gu.data_ptr() if gu is not None else 0)
+    plan = _plans.get(key)
+    if plan is None:
+        if len(_plans) > 1024:
+            _plans.clear()
+        plan = _plans[key] = runtime.ext().TokGemmPlan(mode, epi, w, x, out, gu, granule, BAND_ROWS)
+    n = scratch.ctas if scratch is not None else _ctas()
+    counter_ptr, target = gate or (0, None)
+    if scratch is None:
+        plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows)
+    else:
+        scratch.parity ^= 1
+        plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, scratch.counters, scratch.parity)
+
+
 def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, swiglu: bool = False,
                      gate_up_out: Optional[torch.Tensor] = None, timeout_s: float = 5.0, gate=None, a_scales: Optional[torch.Tensor] = None,
-                     group_rows: Optional[torch.Tensor] = None, gate_tile_rows: int = 0, ctas: Optional[int] = None) -> torch.Tensor:
+                     group_rows: Optional[torch.Tensor] = None, gate_tile_rows: int = 0, ctas: Optional[int] = None,
+                     live_rows: Optional[torch.Tensor] = None, granule: int = 32, scratch: Optional[TokScratch] = None) -> torch.Tensor:
     """out[rows of g] = a[rows of g] @ w[g].T  (a [R, K], w [G, N, K], out [R, N]).
 
     With ``swiglu`` the N columns of every 256-wide tile are [128 gate | 128 up] of the same 128
@@ -105,10 +136,17 @@ def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, 
     the CTA-pair kernel then converts them to bf16 tiles in shared memory on the way to the tensor
     core (no dequantised copy of ``a`` exists in global memory). ``group_rows`` (int32[G], real rows
     per group) makes that path treat the rows between a group's real and padded end as zeros.
+
+    ``live_rows`` (int32[G], real rows per group; CTA-pair kernels, bf16 ``a``): only these rows, up to a multiple of
+    ``granule`` (32 or 64), are computed and written. ``scratch``: see ``TokScratch``.
     """
     G, N, K = w.shape
     assert a.shape[1] == K and K % _BK == 0 and N % _BN == 0 and a.shape[0] % _BM == 0
     assert out.shape[0] == a.shape[0] and out.shape[1] == (N // 2 if swiglu else N)
+    if USE_PAIR and a.dtype == torch.bfloat16:
+        assert a_scales is None
+        _tok_run(FORWARD, SWIGLU if swiglu else STORE, w, a, out, gate_up_out, group_off, live_rows, granule, timeout_s, ctas, gate, gate_tile_rows, scratch)
+        return out
     C = runtime.ext()
     map_b = _tmap(w.view(G * N, K), 128 if USE_PAIR else _BN)
     if a.dtype == torch.uint8:
@@ -124,33 +162,36 @@ def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, 
 
 
 def grouped_gemm_dgrad(dy: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, timeout_s: float = 5.0, gate=None,
-                       swiglu_bwd_of: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       swiglu_bwd_of: Optional[torch.Tensor] = None, live_rows: Optional[torch.Tensor] = None, granule: int = 64,
+                       scratch: Optional[TokScratch] = None) -> torch.Tensor:
     """out[rows of g] = dy[rows of g] @ w[g]  (dy [R, N], w [G, N, K], out [R, K]).
 
     With ``swiglu_bwd_of`` (the saved gate|up tiles [R, 2K]) the product is taken as d(act) and the
     epilogue writes d(gate|up) [R, 2K] into ``out`` instead (CTA-pair kernel only): the SwiGLU
-    backward costs no extra pass over memory.
+    backward costs no extra pass over memory. ``live_rows``, ``granule``, ``scratch``: as in ``grouped_gemm_fwd``.
     """
     G, N, K = w.shape
     assert dy.shape[1] == N and N % _BK == 0 and K % _BN == 0 and dy.shape[0] % _BM == 0
-    C = runtime.ext()
     if swiglu_bwd_of is not None:
         assert USE_PAIR and out.shape[1] == 2 * K and swiglu_bwd_of.shape == out.shape
-        C.grouped_gemm(DGRAD, SWIGLU_BWD, _tmap(dy, _BM), _tmap(w.view(G * N, K), _BK), group_off, K // _BN, 0, N, N, 0, out, swiglu_bwd_of,
-                       _st().ptr(), int(timeout_s * 1e9), _ctas(), *(gate or (0, None)), USE_PAIR, BAND_ROWS, *_out_maps(out, swiglu_bwd_of), DIRECT_EPILOGUE)
+    if USE_PAIR:
+        _tok_run(DGRAD, SWIGLU_BWD if swiglu_bwd_of is not None else STORE, w, dy, out, swiglu_bwd_of, group_off, live_rows, granule, timeout_s, None, gate, 0, scratch)
         return out
+    C = runtime.ext()
     C.grouped_gemm(DGRAD, STORE, _tmap(dy, _BM), _tmap(w.view(G * N, K), _BK), group_off, K // _BN, 0, N, N, 0, out, None, _st().ptr(),
                    int(timeout_s * 1e9), _ctas(), *(gate or (0, None)), USE_PAIR, BAND_ROWS, *_out_maps(out, None), DIRECT_EPILOGUE)
     return out
 
 
-def grouped_gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, timeout_s: float = 5.0) -> torch.Tensor:
+def grouped_gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, timeout_s: float = 5.0,
+                       live_rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[g] = dy[rows of g].T @ x[rows of g]  (dy [R, N], x [R, K], out [G, N, K]). Rows between a
-    group's real end and its padded end must be zero in at least one operand and finite in both."""
+    group's real end and its padded end must be zero in at least one operand and finite in both; with ``live_rows``
+    (int32[G], real rows per group) that holds for the rows up to the next multiple of 64, the others are not read."""
     G, N, K = out.shape
     bm = 256 if USE_PAIR else _BM
     assert dy.shape[1] == N and x.shape[1] == K and N % bm == 0 and K % _BN == 0
     C = runtime.ext()
     C.grouped_gemm(WGRAD, STORE, _tmap(dy, _BK), _tmap(x, _BK), group_off, K // _BN, N // bm, 0, 0, N, out.view(G * N, K), None, _st().ptr(),
-                   int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *_out_maps(out.view(G * N, K), None), DIRECT_EPILOGUE)
+                   int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *_out_maps(out.view(G * N, K), None), DIRECT_EPILOGUE, None, live_rows)
     return out

@@ -143,6 +143,11 @@ class ExpertParallel:
         if graph_mode:
             self._static_route = (torch.empty(max_tokens, top_k, **i32), torch.empty(max_tokens, top_k, dtype=torch.float32, device=dev),
                                   torch.empty(max_tokens, top_k, **i32))
+        # CTA-pair GEMMs take only the real rows of an expert, up to a multiple of 64 where a weight gradient will reduce over
+        # them (those rows are zeroed in its inputs), of 32 elsewhere (what lies in the rows past the real ones is never used).
+        self.granule = 64 if training else 32
+        self.pad_align = 64 if gemm.USE_PAIR else 0
+        self.scratch = gemm.TokScratch(dev) if gemm.USE_PAIR else None
         self.status = comm.status
         self.timeout_ns = comm.timeout_ns
         torch.cuda.synchronize(dev)
@@ -169,6 +174,13 @@ class ExpertParallel:
 
     def _arrive_ptr(self, ch: int) -> int:
         return self.arrive.data_ptr() + ch * self.arrive.shape[1] * 8
+
+    def _needs_zero_pads(self) -> bool:
+        """Whether rows past an expert's real ones are computed with: by the one-CTA GEMM always, else by weight gradients only."""
+        return self.training or not gemm.USE_PAIR
+
+    def _live(self, rs: RouteState) -> dict:
+        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch) if self.scratch is not None else {}
 
     def traffic_matrix(self) -> torch.Tensor:
         """Token traffic matrix [src, dst] of the last routed step (device tensor)."""
@@ -226,8 +238,8 @@ class ExpertParallel:
     def dispatch(self, x: torch.Tensor, rs: RouteState) -> None:
         C = self._C
         send_list = xq = xs = None
-        if not self.fp8:
-            C.zero_pad_rows(self.x_recv, rs.group_off, rs.group_rows)  # on the main stream: ordered before any consumer
+        if not self.fp8 and self._needs_zero_pads():
+            C.zero_pad_rows(self.x_recv, rs.group_off, rs.group_rows, self.pad_align)  # on the main stream: ordered before any consumer
         if self.overlap:
             # The sending order and (fp8) the quantised rows are made on the main stream, with the whole GPU, before the
             # gated GEMM is queued behind them. Only the sends themselves go to the side stream: ordered after routing,
@@ -284,12 +296,13 @@ class ExpertParallel:
             if self.fp8:
                 C.wait_counters(self._arrive_ptr(0), self.tile_target[0] if self.tile_rows else self.arrive_target[0], self.status, self.timeout_ns)
                 C.dequant_fp8(self.xq_recv, self.xs_recv, self.x_recv, rs.group_off.data_ptr() + 4 * self.El)
-                C.zero_pad_rows(self.x_recv, rs.group_off, rs.group_rows)
+                if self._needs_zero_pads():
+                    C.zero_pad_rows(self.x_recv, rs.group_off, rs.group_rows, self.pad_align)
                 gate = None
             # A gated GEMM leaves SMs to the dispatch it waits for; an ungated one (every row is in) takes them all.
             gemm.grouped_gemm_fwd(self.x_recv, w13, rs.group_off, self.act, swiglu=True, gate_up_out=self.gu if self.training else None, gate=gate,
-                                  gate_tile_rows=gate_tile, ctas=self.gemm1_ctas if gate is not None else None)
-        gemm.grouped_gemm_fwd(self.act, w2, rs.group_off, self.y)
+                                  gate_tile_rows=gate_tile, ctas=self.gemm1_ctas if gate is not None else None, **self._live(rs))
+        gemm.grouped_gemm_fwd(self.act, w2, rs.group_off, self.y, **self._live(rs))
         self._join_dispatch()
         C.peer_signal(self.comm.heap, self._flag_off(1), rs.epoch, self.epoch_dev.data_ptr() if self.graph_mode else 0)
 
@@ -340,22 +353,23 @@ class ExpertParallel:
         C.combine_pull(self.comm.heap, self.E, rs.topk_idx, rs.dest_row, None, self._off(self.y), self._flag_off(1), rs.epoch, None, grad_out, grad_w,
                        self.H, self.status, self.timeout_ns, self.comm_ctas, 0)
         # Transposed combine: push w * grad_out to the expert rows (channel 1).
-        C.zero_pad_rows(self.dy_recv, rs.group_off, rs.group_rows)
+        C.zero_pad_rows(self.dy_recv, rs.group_off, rs.group_rows, self.pad_align)
         C.dispatch_push(self.comm.heap, grad_out, rs.topk_idx, weights, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, False, False,
                         self._off(self.dy_recv), 0, self.arrive._symm_off + self.El * 8, self._flag_off(2), rs.epoch, self.status, self.timeout_ns,
                         self.comm_ctas, None)
         gate = (self._arrive_ptr(1), self.arrive_target[1])
         if gemm.USE_PAIR:  # d(act) never leaves the tensor memory: the dgrad epilogue applies the SwiGLU backward
-            gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dgu, gate=gate, swiglu_bwd_of=self.gu)
+            gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dgu, gate=gate, swiglu_bwd_of=self.gu, **self._live(rs))
         else:
-            gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dact, gate=gate)
-        gemm.grouped_gemm_wgrad(self.dy_recv, self.act, rs.group_off, dw2)
+            gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dact, gate=gate, **self._live(rs))
+        live = rs.group_rows if self.scratch is not None else None
+        gemm.grouped_gemm_wgrad(self.dy_recv, self.act, rs.group_off, dw2, live_rows=live)
         if after_dw2 is not None:
             after_dw2()
         if not gemm.USE_PAIR:
             C.swiglu_bwd(self.gu, self.dact, self.dgu, rs.group_off.data_ptr() + 4 * self.El)
-        gemm.grouped_gemm_dgrad(self.dgu, w13, rs.group_off, self.dx_recv)
-        gemm.grouped_gemm_wgrad(self.dgu, self.x_recv, rs.group_off, dw13)
+        gemm.grouped_gemm_dgrad(self.dgu, w13, rs.group_off, self.dx_recv, **self._live(rs))
+        gemm.grouped_gemm_wgrad(self.dgu, self.x_recv, rs.group_off, dw13, live_rows=live)
         C.peer_signal(self.comm.heap, self._flag_off(3), rs.epoch, 0)
         grad_x = torch.empty(T, self.H, dtype=torch.bfloat16, device=dev)
         # Transposed dispatch: every token pulls and sums the gradients of its k rows.

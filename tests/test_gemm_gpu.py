@@ -139,6 +139,79 @@ def test_dgrad_with_fused_swiglu_backward(kernel_variant):
         _close(got[:, :, 1].reshape(e - s, I), ut.grad)
 
 
+@pytest.mark.parametrize("counts,N,K,granule,keep_counters", [
+    ([1], 256, 64, 32, False),                                       # one tile of the narrowest width, one block
+    ([1, 0, 2], 1024, 14336, 32, True),                              # few tiles: the reduction is cut as a stream, several parts per tile
+    ([31, 32, 33, 255, 256, 257, 513], 512, 1024, 32, True),         # widths around the 32-row steps and the 256-token tile
+    ([63, 64, 65, 1000, 2100], 768, 2048, 64, True),                 # several token tiles per group: cut in equal parts
+    ([(7 * i) % 70 for i in range(300)], 256, 256, 64, False),       # more groups than prefix entries
+])
+def test_live_rows_and_cut_reductions(counts, N, K, granule, keep_counters, kernel_variant):
+    """Forward (plain, SwiGLU with and without the kept tiles) and dgrad (plain, SwiGLU backward) on the real rows only: those
+    match fp32, the rows past their granule stay untouched. Twice with kept counters: they are clean for the next launch."""
+    if kernel_variant != "cta_pair":
+        pytest.skip("live rows belong to the CTA-pair kernels")
+    from fast_b200.ops import gemm
+
+    G = len(counts)
+    counts_t, off, R, a, w = _setup(G, N, K, counts, seed=21)
+    g = torch.Generator(device="cuda").manual_seed(23)
+    live, scratch = counts_t.to(torch.int32), gemm.TokScratch(a.device) if keep_counters else None
+    kw = dict(live_rows=live, granule=granule, scratch=scratch)
+    new = lambda cols: torch.full((R, cols), 7.0, device="cuda", dtype=torch.bfloat16)
+    dy = torch.randn(R, N, generator=g, device="cuda").to(torch.bfloat16)
+    gu = torch.randn(R, 2 * K, generator=g, device="cuda").to(torch.bfloat16)
+    for _ in range(2 if keep_counters else 1):
+        out, act, act2, kept, dx, dgu = new(N), new(N // 2), new(N // 2), new(N), new(K), new(2 * K)
+        gemm.grouped_gemm_fwd(a, w, off, out, **kw)
+        gemm.grouped_gemm_fwd(a, w, off, act, swiglu=True, gate_up_out=kept, **kw)
+        gemm.grouped_gemm_fwd(a, w, off, act2, swiglu=True, **kw)
+        if K % 256 == 0:
+            gemm.grouped_gemm_dgrad(dy, w, off, dx, **kw)
+            gemm.grouped_gemm_dgrad(dy, w, off, dgu, swiglu_bwd_of=gu, **kw)
+    gemm.check()
+    o = off.tolist()
+    for i in range(G):
+        s, e, n = o[i], o[i + 1], counts[i]
+        if n == 0:
+            continue
+        end = s + (n + granule - 1) // granule * granule
+        full = a[s:s + n].float() @ w[i].float().T
+        t = full.view(n, N // 256, 2, 128)
+        _close(out[s:s + n], full)
+        _close(kept[s:s + n], full)
+        _close(act[s:s + n], (torch.nn.functional.silu(t[:, :, 0]) * t[:, :, 1]).reshape(n, N // 2))
+        assert torch.equal(act[s:s + n], act2[s:s + n])
+        assert all(bool((x[end:e] == 7).all()) for x in (out, act, act2, kept, dx, dgu))
+        if K % 256 == 0:
+            dact = dy[s:s + n].float() @ w[i].float()
+            _close(dx[s:s + n], dact)
+            q = gu[s:s + n].float().view(n, K // 128, 2, 128)
+            gt, ut = q[:, :, 0].reshape(n, K).requires_grad_(), q[:, :, 1].reshape(n, K).requires_grad_()
+            (torch.nn.functional.silu(gt) * ut).backward(dact.to(torch.bfloat16).float())
+            got = dgu[s:s + n].float().view(n, K // 128, 2, 128)
+            _close(got[:, :, 0].reshape(n, K), gt.grad)
+            _close(got[:, :, 1].reshape(n, K), ut.grad)
+
+
+def test_wgrad_stops_at_the_live_rows(kernel_variant):
+    """Rows past the next multiple of 64 are not read: what lies there (here NaN) does not reach the gradient."""
+    from fast_b200.ops import gemm
+
+    counts, N, K = [1, 64, 65, 0, 300], 256, 256
+    counts_t, off, R, x, _ = _setup(5, 256, K, counts, seed=25)
+    dy = torch.randn(R, N, generator=torch.Generator(device="cuda").manual_seed(27), device="cuda").to(torch.bfloat16)
+    for i, n in enumerate(counts):
+        s = int(off[i])
+        x[s + (n + 63) // 64 * 64:int(off[i + 1])] = float("nan")
+    out = torch.full((5, N, K), float("nan"), device="cuda", dtype=torch.bfloat16)
+    gemm.grouped_gemm_wgrad(dy, x, off, out, live_rows=counts_t.to(torch.int32))
+    gemm.check()
+    for i, n in enumerate(counts):
+        s = int(off[i])
+        _close(out[i], dy[s:s + n].float().T @ x[s:s + n].float())
+
+
 def test_custom_operators_run_the_same_kernels():
     """torch.ops.fast_b200.* (schemas, mutation annotations) give the same bits as the direct calls."""
     from fast_b200.ops import gemm, registry  # noqa: F401
