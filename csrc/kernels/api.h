@@ -141,9 +141,12 @@ struct TokGemmArgs {
   int m_tiles;               // 256-feature tiles of the output's columns (SwiGLU forward: of gate|up)
   int red_blocks;            // 64-wide blocks of the reduction
   int w_rows_per_group;      // rows of a group's slice in w's matrix (forward: features, dgrad: reduction)
+  int tile_n;                // most tokens of a tile: 64, 128 or 256
+  int stages;                // set by the launcher
   int band_tiles;            // token tiles of a raster band
   int granule;               // tile widths are multiples of this (32 or 64); rows up to a multiple of it are written
   int keep_gate_up;
+  int early;                 // 1: weights, group_off and group_rows were written by no kernel later than the last but one of the stream
   float* partials;           // tok_partial_floats(ctas)
   unsigned int* counters;    // num_counters >= tok_counters(ctas), zero before the launch and after it
   unsigned int* counters_next;   // num_counters; cleared by the launch
@@ -168,7 +171,6 @@ struct SplitsArgs {
   int rank, world, num_experts, num_blocks, num_channels;
   int row_align;               // group row ranges are padded to this many rows (128 or 256)
   int cap_rows;                // rows of the receive buffers; a step that needs more is refused on every rank
-  int counts_in_smem;          // set by the launcher: the [world][E] count matrix fits in shared memory
   long long counts_heap_off;   // int [world][E] on every rank
   long long flags_heap_off;    // u64 [world] on every rank: epoch of the last counts row received from each rank
   unsigned long long epoch;
@@ -193,6 +195,22 @@ struct SplitsArgs {
   unsigned long long timeout_ns;
 };
 cudaError_t launch_splits_scan(const SplitsArgs& a, cudaStream_t stream);
+// launch_route_topk with the split scan in its last block (sp.block_cnt is written, then scanned). ticket: one zeroed word that
+// the launches of one stream share; it is zero again after each.
+cudaError_t launch_route_splits(const float* logits, const float* bias, int T, int K, int* topk_idx, float* topk_w, int* slot_in_block, const SplitsArgs& sp,
+                                unsigned int* ticket, cudaStream_t stream);
+// The same from the activations, for T <= kRouteTokensPerBlock: logits = bf16(x . gate^T).
+struct GateRouteArgs {
+  const __nv_bfloat16* x;       // [T, H]
+  const __nv_bfloat16* gate;    // [E, H]
+  const float* bias;            // [E] or null: added for the expert choice only
+  int T, H, K;
+  int* topk_idx;                // [T, K] out
+  float* topk_w;                // [T, K] out
+  int* slot_in_block;
+  int* block_cnt;               // [E], the same as SplitsArgs::block_cnt
+};
+cudaError_t launch_gate_route(const GateRouteArgs& g, const SplitsArgs& sp, unsigned int* ticket, cudaStream_t stream);
 // list[send_pos[e] + rank of (t, j) among my entries for e] = t*K + j  (see SplitsArgs::send_pos).
 // Entries whose expert id is outside [0, E) are skipped and reported in `status` (kSiteExpertId).
 cudaError_t launch_build_send_list(const int* topk_idx, const int* slot_in_block, const int* block_base, const int* send_pos, int T, int K, int E,
@@ -218,7 +236,8 @@ struct NormGateArgs {
   int* slot_in_block;           // as launch_route_topk
   int* block_cnt;
 };
-cudaError_t launch_norm_gate_route(const NormGateArgs& a, cudaStream_t stream);
+// With sp, the last block goes on with the split scan (sp->block_cnt = a.block_cnt).
+cudaError_t launch_norm_gate_route(const NormGateArgs& a, const SplitsArgs* sp, unsigned int* ticket, cudaStream_t stream);
 struct NormGateBwdArgs {
   const __nv_bfloat16* h;       // [T, H] input of the forward pass
   const __nv_bfloat16* norm_w;  // [H]
@@ -251,6 +270,9 @@ struct DispatchArgs {
   int fp8;                     // 1: send e4m3 bytes + one fp32 scale per 128 elements
   const unsigned char* xq;     // fp8 only, optional: rows already quantised by launch_quantise_rows ([T, H] e4m3); x is then not read
   const float* xq_scales;      // their scales [T, H/128]
+  __nv_bfloat16* local_rows;   // fp8, unsorted, a world of one rank, optional: the rows are stored here as the bf16 values a receiver would make of
+                               // them, instead of as e4m3 in the receive buffer
+  int warps_per_row;           // set by the launcher
   long long recv_heap_off;     // destination rows: bf16 [cap, H] (or u8 [cap, H] when fp8)
   long long scale_heap_off;    // fp8 only: float [cap, H/128]
   long long arrive_heap_off;   // u64 arrival counters of this channel: [E/world] per expert, or [num_tiles] per tile
@@ -274,6 +296,8 @@ struct CombineArgs {
   long long src_heap_off;      // bf16 [cap, H] on every rank
   long long ready_flags_heap_off;  // u64 [world] in my slab: peer d's rows are final once flags[d] >= ready_epoch
   unsigned long long ready_epoch;
+  int signal;                  // 1: first write ready_epoch into slot `rank` of every rank's flags (my own rows are final)
+  int segments;                // set by the launcher: warps that share a token's row
   const unsigned long long* epoch_dev;  // when non-null, *epoch_dev replaces ready_epoch (see SplitsArgs)
   __nv_bfloat16* out;          // [T, H] sum_j w * row_j (null in dot mode)
   const __nv_bfloat16* dot_with;  // dot mode: [T, H]
@@ -283,9 +307,6 @@ struct CombineArgs {
 };
 cudaError_t launch_combine_pull(const CombineArgs& a, int ctas, cudaStream_t stream);
 
-// Writes `epoch` (release, system scope) into slot `rank` of the flag array of every rank.
-cudaError_t launch_peer_signal(void* const* peer_table, int rank, int world, long long flags_heap_off, unsigned long long epoch,
-                               const unsigned long long* epoch_dev, cudaStream_t stream);
 // Bounded wait until counter[i] >= target[i] for all i < n (one thread each).
 cudaError_t launch_wait_counters(const unsigned long long* counter, const unsigned long long* target, int n, DeviceStatus* status,
                                  unsigned long long timeout_ns, cudaStream_t stream);

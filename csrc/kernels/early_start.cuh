@@ -1,0 +1,39 @@
+// Programmatic dependent launch: a kernel of the forward chain may be set up (blocks placed, barriers and tensor memory made)
+// while the kernel before it in the stream still runs. Rules that keep it safe:
+//   * grid_dependency_wait() comes before the first access to anything an earlier kernel reads or writes. The one exception, where its
+//     caller vouches for it (TokGemmArgs::early), is the expert GEMM's weights and group table: at least one kernel lies
+//     between their writers and the GEMM, and that kernel gives leave after its own wait or not at all.
+//   * launch_dependents() comes after the wait, so leave is given only by kernels whose own predecessors are complete.
+// A kernel that gives no leave lets its successor start when it ends, as always.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace fastb {
+
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+inline cudaLaunchAttribute early_start_attribute() {
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+
+// kern<<<grid, block, smem, stream>>>(args...), allowed to start early. The kernel calls grid_dependency_wait().
+template <class... P, class... A>
+cudaError_t launch_early(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1] = {early_start_attribute()};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+}  // namespace fastb

@@ -27,6 +27,7 @@
 //
 // Barriers as in grouped_gemm_pair.cu. Every wait is bounded. No load is multicast.
 #include "gemm_epilogue_tma.cuh"
+#include "early_start.cuh"
 #include "token_walker.h"
 
 namespace fastb {
@@ -37,26 +38,33 @@ using namespace ptx;
 using namespace gemm;
 
 constexpr int kPairM = 256, kHalfM = 128;
-constexpr int kStages = 6;
+constexpr int kMaxStages = 10;
 constexpr int kAccStages = 2;
 constexpr int kTmemCols = 512;
 constexpr int kABytes = kHalfM * BK * 2;          // 16 KiB
-constexpr int kBBytes = kTokTileN / 2 * BK * 2;   // 16 KiB: half of the widest tile's tokens
-constexpr int kStageBytes = kABytes + kBBytes;
+__host__ __device__ constexpr int stage_bytes(int tile_n) { return kABytes + tile_n / 2 * BK * 2; }   // B: half of the widest tile's tokens
 constexpr int kThreads = 192;
 constexpr int kStepTokens = 32;                   // tokens per epilogue step = rows of a TMA store
 constexpr int kBox = kStepTokens * 128;           // 4 KiB: 32 tokens x 64 features
 constexpr int kPrefix = 256;                      // entries of the tile-count prefix (several groups each when there are more)
 
 struct __align__(8) TokCtl {
-  uint64_t full[kStages], empty[kStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load[2];
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load[2];
   uint32_t tmem_base;
   int abort_flag, last_arrived, widest, share_weights;
   int base[kPrefix + 1];                          // tiles of the groups before entry i
 };
 __host__ __device__ constexpr int epi_boxes(GemmEpilogue e) { return e == GemmEpilogue::kStore ? 2 : e == GemmEpilogue::kSwiGLU ? 3 : 4; }
-__host__ __device__ constexpr int smem_bytes(GemmEpilogue e) { return kStages * kStageBytes + 2 * epi_boxes(e) * kBox + 1024 + static_cast<int>(sizeof(TokCtl)); }
-static_assert(smem_bytes(GemmEpilogue::kSwiGLUBwd) <= 227 * 1024, "dynamic shared memory of one CTA on sm_100a");
+constexpr int kSmemLimit = 227 * 1024;
+constexpr int other_bytes(GemmEpilogue e) { return 2 * epi_boxes(e) * kBox + 1024 + static_cast<int>(sizeof(TokCtl)); }
+// Operand stages that fit. Tiles of up to 256 tokens: 6 of 32 KiB. Where few tokens meet the weights, the loop is bound by
+// HBM and wants weight bytes in flight: tiles of up to 64 tokens leave room for 10 stages of 20 KiB.
+constexpr int stages_for(GemmEpilogue e, int tile_n) {
+  const int n = (kSmemLimit - other_bytes(e)) / stage_bytes(tile_n);
+  return n < kMaxStages ? n : kMaxStages;
+}
+constexpr int smem_bytes(GemmEpilogue e, int tile_n) { return stages_for(e, tile_n) * stage_bytes(tile_n) + other_bytes(e); }
+static_assert(stages_for(GemmEpilogue::kSwiGLUBwd, kTokTileN) == 6 && stages_for(GemmEpilogue::kSwiGLU, 64) == 10, "stages at both ends of the range");
 static_assert(kAccStages * kTokTileN <= kTmemCols, "two accumulators of 256 columns");
 static_assert(kTokPartialFloats == kHalfM * kTokTileN, "a partial is one CTA's accumulator");
 
@@ -78,9 +86,9 @@ struct TokTiles {
       g = entry * per_entry; g_base = base[entry];
     }
     int rows = rows_of(g);
-    while (tile >= g_base + tok_tiles(rows) * p.m_tiles) { g_base += tok_tiles(rows) * p.m_tiles; rows = rows_of(++g); }
-    const TokPlace at = tok_place(tile - g_base, p.m_tiles, tok_tiles(rows), p.band_tiles);
-    const int per = tok_tile_size(rows), t0 = at.t * per;
+    while (tile >= g_base + tok_tiles(rows, p.tile_n) * p.m_tiles) { g_base += tok_tiles(rows, p.tile_n) * p.m_tiles; rows = rows_of(++g); }
+    const TokPlace at = tok_place(tile - g_base, p.m_tiles, tok_tiles(rows, p.tile_n), p.band_tiles);
+    const int per = tok_tile_size(rows, p.tile_n), t0 = at.t * per;
     return Tile{g, at.m, p.group_off[g] + t0, min(per, rows - t0)};
   }
 };
@@ -127,14 +135,16 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   constexpr int kRing = epi_boxes(EPI) * kBox;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* ring = tiles + kStages * kStageBytes;
+  const int stages = p.stages, stage_size = stage_bytes(p.tile_n);
+  uint8_t* ring = tiles + stages * stage_size;
   TokCtl* ctl = reinterpret_cast<TokCtl*>(ring + 2 * kRing);
+  if (!p.early) grid_dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = static_cast<int>(cluster_cta_rank());  // 0 = leader
   const bool leader = cta == 0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
+    for (int s = 0; s < stages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
     for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * 4); mbar_init(&ctl->epi_load[a], 1); }
     ctl->abort_flag = 0;
     mbar_fence_init();
@@ -155,9 +165,9 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       int mine = 0;
       for (int q = (e0 + lane) * per_entry; q < min((e0 + lane + 1) * per_entry, p.num_groups); ++q) {
         const int rows = tok_rows(p, q);
-        mine += tok_tiles(rows) * p.m_tiles;
-        widest = max(widest, tok_tile_size(rows));
-        most = max(most, tok_tiles(rows));
+        mine += tok_tiles(rows, p.tile_n) * p.m_tiles;
+        widest = max(widest, tok_tile_size(rows, p.tile_n));
+        most = max(most, tok_tiles(rows, p.tile_n));
       }
       int incl = mine;
 #pragma unroll
@@ -181,10 +191,6 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   TokSegments segs(split, pair);
   TokTiles walk{p, ctl->base, per_entry};
   TokSegment sg;
-  // The other arrival counters are cleared for the next launch; this launch's are back at zero once all parts have arrived.
-  if (blockIdx.x == 0)
-    for (int i = threadIdx.x; i < p.num_counters; i += blockDim.x) p.counters_next[i] = 0u;
-
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs, each for its own halves) ----------------
     if (elect_one()) {
@@ -192,8 +198,30 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       uint32_t ph = 0;
       bool ok = true;
       int gated = -1;
+      // The first stages' weights do not depend on the kernel before this one: with p.early they are on their way before it has ended.
+      bool first = true;
       while (ok && segs.next(sg)) {
         const TokTiles::Tile tc = walk.locate(sg.tile);
+        const int half = tc.n >> 1, x_row = tc.row0 + cta * half;
+        const int n32 = half == 128 ? 0 : half >> 5, n16 = half == 128 ? 0 : (half >> 4) & 1;
+        const uint32_t bytes = 2u * (kABytes + static_cast<uint32_t>(half) * 128u);
+        auto load_w = [&](int kb, int st) {
+          uint8_t* sa = tiles + st * stage_size;
+          const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[st]), 0);
+          if (leader) mbar_arrive_expect_tx(&ctl->full[st], bytes);
+          if (A_MN) {
+#pragma unroll
+            for (int j = 0; j < kHalfM / 64; ++j)
+              tma_load_2d_pair(sa + j * (BK * 128), &map_w, tc.m * kPairM + cta * kHalfM + j * 64, tc.g * p.w_rows_per_group + kb * BK, full_leader);
+          } else if (EPI == GemmEpilogue::kSwiGLU) {
+            tma_load_5d_pair(sa, &map_w, kb * BK, 0, 0, cta * 4, tc.g * p.m_tiles + tc.m, full_leader);
+          } else {
+            tma_load_2d_pair(sa, &map_w, kb * BK, tc.g * p.w_rows_per_group + tc.m * kPairM + cta * kHalfM, full_leader);
+          }
+        };
+        const int early = first ? min(sg.kb1, sg.kb0 + stages) : sg.kb0;   // blocks whose weights are requested now
+        for (int kb = sg.kb0; kb < early; ++kb) load_w(kb, kb - sg.kb0);
+        if (first) { grid_dependency_wait(); first = false; }
         if (p.gate_counter != nullptr) {
           // Arrival gate: per group, or (gate_tile_rows > 0) per tile of that many rows of the grouped matrix that this one touches.
           const int lo = p.gate_tile_rows > 0 ? tc.row0 / p.gate_tile_rows : tc.g, hi = p.gate_tile_rows > 0 ? (tc.row0 + tc.n - 1) / p.gate_tile_rows : tc.g;
@@ -206,28 +234,17 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
           }
           if (!ok) break;
         }
-        const int half = tc.n >> 1, x_row = tc.row0 + cta * half;
-        const int n32 = half == 128 ? 0 : half >> 5, n16 = half == 128 ? 0 : (half >> 4) & 1;
-        const uint32_t bytes = 2u * (kABytes + static_cast<uint32_t>(half) * 128u);
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          if (!(ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1, abort_flag, p.status, 100 + s, p.timeout_ns))) break;
-          uint8_t* sa = tiles + s * kStageBytes;
-          uint8_t* sb = sa + kABytes;
-          const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
-          if (leader) mbar_arrive_expect_tx(&ctl->full[s], bytes);
-          if (A_MN) {
-#pragma unroll
-            for (int j = 0; j < kHalfM / 64; ++j)
-              tma_load_2d_pair(sa + j * (BK * 128), &map_w, tc.m * kPairM + cta * kHalfM + j * 64, tc.g * p.w_rows_per_group + kb * BK, full_leader);
-          } else if (EPI == GemmEpilogue::kSwiGLU) {
-            tma_load_5d_pair(sa, &map_w, kb * BK, 0, 0, cta * 4, tc.g * p.m_tiles + tc.m, full_leader);
-          } else {
-            tma_load_2d_pair(sa, &map_w, kb * BK, tc.g * p.w_rows_per_group + tc.m * kPairM + cta * kHalfM, full_leader);
+          if (kb >= early) {
+            if (!(ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1, abort_flag, p.status, 100 + s, p.timeout_ns))) break;
+            load_w(kb, s);
           }
+          uint8_t* sb = tiles + s * stage_size + kABytes;
+          const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
           if (half == 128) tma_load_2d_pair(sb, &map_x128, kb * BK, x_row, full_leader);
           for (int j = 0; j < n32; ++j) tma_load_2d_pair(sb + j * 4096, &map_x32, kb * BK, x_row + 32 * j, full_leader);
           if (n16) tma_load_2d_pair(sb + n32 * 4096, &map_x16, kb * BK, x_row + 32 * n32, full_leader);
-          if (++s == kStages) { s = 0; ph ^= 1; }
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -249,7 +266,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
           if (!(ok = mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.status, 300 + s, p.timeout_ns))) break;
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(tiles + s * kStageBytes), sb = sa + kABytes;
+          const uint32_t sa = smem_u32(tiles + s * stage_size), sb = sa + kABytes;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t da = A_MN ? make_smem_desc(sa + k * 2048, BK * 128, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
@@ -257,7 +274,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
             mma_bf16_ss_pair(d_tmem, da, db, idesc, (kb != sg.kb0 || k != 0) ? 1u : 0u);
           }
           mma_commit_pair(&ctl->empty[s], 0x3);
-          if (++s == kStages) { s = 0; ph ^= 1; }
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
         if (ok) mma_commit_pair(&ctl->acc_full[a], 0x3);
       }
@@ -267,6 +284,11 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     const int quarter = warp & 3;
     const int et = threadIdx.x - 64;              // 0..127 among the epilogue threads
     const bool issuer = threadIdx.x == 64;
+    grid_dependency_wait();   // what is written below may still be read by earlier kernels
+    launch_dependents();
+    // The other arrival counters are cleared for the next launch; this launch's are back at zero once all parts have arrived.
+    if (blockIdx.x == 0)
+      for (int i = et; i < p.num_counters; i += 128) p.counters_next[i] = 0u;
     uint32_t acc_it = 0, ring_n = 0, load_ph = 0u;   // load_ph: one parity bit per half of the ring
     bool ok = true;
     while (ok && segs.next(sg)) {
@@ -313,7 +335,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         release_acc();
         __threadfence();
         epi_bar();
-        if (issuer) ctl->last_arrived = atomicInc(p.counters + (sg.tile - split.whole_tiles) * 2 + cta, static_cast<unsigned>(sg.parts - 1)) == static_cast<unsigned>(sg.parts - 1);
+        if (issuer) ctl->last_arrived = atomicInc(p.counters + sg.tile * 2 + cta, static_cast<unsigned>(sg.parts - 1)) == static_cast<unsigned>(sg.parts - 1);
         epi_bar();
         if (!ctl->last_arrived) continue;
         __threadfence();
@@ -455,20 +477,23 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
 }
 
 template <GemmMode MODE, GemmEpilogue EPI>
-cudaError_t launch(const TokGemmMaps& m, const TokGemmArgs& args, int ctas, cudaStream_t stream) {
+cudaError_t launch(const TokGemmMaps& m, TokGemmArgs args, int ctas, cudaStream_t stream) {
   auto kern = grouped_gemm_tokens_kernel<MODE, EPI>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(EPI));
+  args.stages = stages_for(EPI, args.tile_n);
+  const int smem = smem_bytes(EPI, args.tile_n);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas & ~1);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem_bytes(EPI);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1] = early_start_attribute();
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   e = cudaLaunchKernelEx(&cfg, kern, *m.w, *m.x128, *m.x32, *m.x16, *m.c, m.c2 ? *m.c2 : *m.c, args);
   if (e == cudaSuccess) note_launch();
   return e;
@@ -478,6 +503,7 @@ cudaError_t launch(const TokGemmMaps& m, const TokGemmArgs& args, int ctas, cuda
 
 cudaError_t launch_grouped_gemm_tokens(GemmMode mode, GemmEpilogue epi, const TokGemmMaps& maps, const TokGemmArgs& args, int ctas, cudaStream_t stream) {
   if (ctas < 2 || args.num_groups < 1 || args.m_tiles < 1 || args.red_blocks < 1 || args.band_tiles < 1) return cudaErrorInvalidValue;
+  if (args.tile_n != 64 && args.tile_n != 128 && args.tile_n != 256) return cudaErrorInvalidValue;
   if ((args.granule != 32 && args.granule != 64) || args.partials == nullptr || args.counters == nullptr || args.counters_next == nullptr) return cudaErrorInvalidValue;
   if (args.num_counters < tok_counters(ctas)) return cudaErrorInvalidValue;
   if (mode == GemmMode::kForward && epi == GemmEpilogue::kStore) return launch<GemmMode::kForward, GemmEpilogue::kStore>(maps, args, ctas, stream);

@@ -9,9 +9,13 @@
 // In FAST's terms these are the all-to-all of the forward pass and its transpose
 // (amd/flash.cpp:400-408 `backward` flag) with the permute / reduce fused in; the reference moves
 // opaque bytes with ncclSend/ncclRecv groups or NVSHMEM puts and leaves the packing to the caller.
+#include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "api.h"
+#include "early_start.cuh"
 
 namespace fastb {
 
@@ -60,6 +64,27 @@ __device__ __forceinline__ uint4 quantise16(const uint4 (&raw)[2], float& sc) {
   return q;
 }
 
+// 8 bf16 elements of a lane (16 consecutive lanes = 128 elements share a scale) -> what a receiver makes of their e4m3 values:
+// quantised as in quantise16, multiplied back in fp32 as dequant_fp8_kernel does, rounded to bf16.
+__device__ __forceinline__ uint4 through_e4m3(const uint4& raw) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  __nv_bfloat162 m2 = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+  float amax = fmaxf(__low2float(m2), __high2float(m2));
+#pragma unroll
+  for (int o = 8; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float sc = __uint_as_float((__float_as_uint(fmaxf(amax, 1e-12f) * (1.0f / 448.0f)) + 0xFFFFu) & 0xFFFF0000u), inv = 1.0f / sc;
+  float f[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = __bfloat1622float2(h[i]);
+    const __half2_raw r = __nv_cvt_fp8x2_to_halfraw2(__nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3), __NV_E4M3);
+    const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&r));
+    f[2 * i] = d.x * sc;
+    f[2 * i + 1] = d.y * sc;
+  }
+  return pack8(f);
+}
+
 // One warp per row: x [T, H] bf16 -> q [T, H] e4m3 bytes + scales [T, H / 128], in this GPU's own memory.
 // The sorted dispatch sends every (token, slot) entry from a warp of its own; with the rows quantised
 // here first, a token's K entries copy bytes instead of each repeating the reduction and the conversions.
@@ -99,18 +124,22 @@ __global__ void __launch_bounds__(kCommThreads) quantise_rows_kernel(const __nv_
 // FP8: rows leave as e4m3 + scales; SORTED: one warp per (token, slot) entry of send_list (one destination per warp, so the
 // per-slot arrays shrink to one element); SCALED: bf16 rows are multiplied by row_scale on the way. The variants exist for
 // their register counts: the copy loops are bound by the stores a SM keeps in flight, i.e. by resident warps.
-template <bool FP8, bool SORTED, bool SCALED>
+// ROUNDED (one rank alone): nothing crosses a wire, so the rows go straight to the GEMM's bf16 operand, as the values that a
+// receiver would make of their e4m3 form. Sent as e4m3 and converted afterwards, 32768 rows of 7168 took 85 + 145 us.
+template <bool FP8, bool SORTED, bool SCALED, bool ROUNDED = false>
 __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_kernel(const DispatchArgs a) {
   extern __shared__ int s_cnt[];  // rows this CTA sent: [E] per expert, or [world][num_tiles] per destination tile
   __shared__ int s_ok;
   __shared__ __align__(16) float s_scales[(kCommThreads / 32) * kMaxScaleGroups];  // fp8 mode: the 1x128 scales of the row each warp is sending
+  grid_dependency_wait();
+  launch_dependents();
   const int E = a.num_experts, El = E / a.world;
   const int n_cnt = a.tile_rows > 0 ? a.world * a.num_tiles : E;
   for (int e = threadIdx.x; e < n_cnt; e += blockDim.x) s_cnt[e] = 0;
   if (threadIdx.x == 0) s_ok = 1;
   if (*reinterpret_cast<volatile unsigned long long*>(&a.status->abort) != 0ull) return;  // an earlier kernel of this rank refused the step
   __syncthreads();
-  if (a.entry_epoch != 0) {
+  if (a.entry_epoch != 0 && a.world > 1) {
     // Entry handshake: publish that my receive buffers may be written, then wait for the peers.
     unsigned long long* my_flags = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[a.rank]) + a.entry_flags_heap_off);
     if (blockIdx.x == 0 && threadIdx.x < a.world) {
@@ -121,10 +150,14 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
     __syncthreads();
     if (!s_ok) return;
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  // a.warps_per_row warps of a CTA share a row (1, or all of them when there are fewer rows than CTAs: a few rows of 4096 took one
+  // warp each through 16 dependent rounds). Warp `part` of them takes the rounds [part, part + 1) / warps_per_row.
+  const int lane = threadIdx.x & 31, wpr = SORTED ? 1 : a.warps_per_row, wpb = (blockDim.x >> 5) / wpr;
+  const int warp = (threadIdx.x >> 5) / wpr, part = (threadIdx.x >> 5) % wpr;
+  const bool first = lane == 0 && part == 0;
   constexpr int tpb = kRouteTokensPerBlock;
   const int chunks = a.H / 8;  // 16-byte chunks per row
-  // Unsorted mode: one warp per token, the row is read once and stored to its K destinations.
+  // Unsorted mode: one warp (or warps_per_row) per token, the row is read once and stored to its K destinations.
   // Sorted mode (send_list != null): one warp per (token, slot) entry, entries ordered by
   // (local expert index, destination rank counted from the sender upwards), so that every rank's expert 0 fills first, then
   // expert 1, ... and the gated GEMM of the receivers can start while later experts still arrive.
@@ -169,20 +202,21 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
           const long long tj = static_cast<long long>(t) * a.K + jbeg + j;
           const int e = a.topk_idx[tj];
           if (e < 0 || e >= E) {  // not an expert: nothing is indexed with it; the step is flagged and the entry skipped
-            if (lane == 0) report_failure(a.status, kStatusBadArg, kSiteExpertId, static_cast<unsigned long long>(tj), static_cast<unsigned long long>(static_cast<unsigned int>(e)), static_cast<unsigned long long>(E));
+            if (first) report_failure(a.status, kStatusBadArg, kSiteExpertId, static_cast<unsigned long long>(tj), static_cast<unsigned long long>(static_cast<unsigned int>(e)), static_cast<unsigned long long>(E));
             continue;
           }
           int row;
           if (a.compute_rows) {
             row = a.send_base[e] + a.block_base[static_cast<long long>(t / tpb) * E + e] + a.slot_in_block[tj];
-            if (lane == 0) a.dest_row[tj] = row;
+            if (first) a.dest_row[tj] = row;
           } else {
             row = a.dest_row[tj];
           }
           row_of[j] = row;
-          out_row[j] = static_cast<unsigned char*>(a.peer_table[e / El]) + a.recv_heap_off + static_cast<long long>(row) * a.H * (FP8 ? 1 : 2);
+          if (ROUNDED) out_row[j] = reinterpret_cast<unsigned char*>(a.local_rows + static_cast<long long>(row) * a.H);
+          else out_row[j] = static_cast<unsigned char*>(a.peer_table[e / El]) + a.recv_heap_off + static_cast<long long>(row) * a.H * (FP8 ? 1 : 2);
           if (SCALED) scale[j] = a.row_scale[tj];
-          if (lane == 0) atomicAdd(&s_cnt[a.tile_rows > 0 ? (e / El) * a.num_tiles + min(row / a.tile_rows, a.num_tiles - 1) : e], 1);
+          if (first) atomicAdd(&s_cnt[a.tile_rows > 0 ? (e / El) * a.num_tiles + min(row / a.tile_rows, a.num_tiles - 1) : e], 1);
         }
       }
       const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<long long>(t) * a.H);
@@ -190,15 +224,17 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
         // Four 16-byte chunks per lane in flight before the first store: the loop is bound by the
         // latency of the local loads otherwise.
         constexpr int U = 4;
-        for (int c0 = lane; c0 < chunks; c0 += 32 * U) {
+        const int rounds = chunks / 32, c_end = rounds * (part + 1) / wpr * 32;   // H is a multiple of 256
+        for (int c0 = rounds * part / wpr * 32 + lane; c0 < c_end; c0 += 32 * U) {
           uint4 v[U];
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            if (c0 + 32 * u < chunks) v[u] = __ldg(src + c0 + 32 * u);
+            if (c0 + 32 * u < c_end) v[u] = __ldg(src + c0 + 32 * u);
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const int c = c0 + 32 * u;
-            if (c >= chunks) break;
+            if (c >= c_end) break;
+            if (ROUNDED) v[u] = through_e4m3(v[u]);   // every lane of the warp is here: rounds are whole
             float f[8];
             if (SCALED) unpack8(v[u], f);
 #pragma unroll
@@ -251,19 +287,20 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
           // (8, 16 or 24 per SM), nor requesting the next pass before reducing this one, nor packed arithmetic
           // moves this path off about 600 GB/s to one peer; a plain copy of already quantised rows reaches 624.
           constexpr int U = 2;
-          for (int c0 = 0; c0 < chunks16; c0 += 32 * U) {
+          const int rounds = (chunks16 + 31) / 32, c_end = min(chunks16, rounds * (part + 1) / wpr * 32);
+          for (int c0 = rounds * part / wpr * 32; c0 < c_end; c0 += 32 * U) {
             uint4 raw[U][2];
             bool active[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
               const int c = c0 + 32 * u + lane;
-              active[u] = c < chunks16;
+              active[u] = c < c_end;
               raw[u][0] = active[u] ? __ldg(src + 2 * c) : make_uint4(0, 0, 0, 0);
               raw[u][1] = active[u] ? __ldg(src + 2 * c + 1) : make_uint4(0, 0, 0, 0);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-              if (c0 + 32 * u >= chunks16) break;  // warp-uniform: the second block of the last pass may not exist
+              if (c0 + 32 * u >= c_end) break;  // warp-uniform: the second block of the last pass may not exist
               const int c = c0 + 32 * u + lane;
               float sc;
               const uint4 q = quantise16(raw[u], sc);
@@ -276,12 +313,12 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
             }
           }
         }
-        __syncwarp();
+        if (wpr > 1) __syncthreads(); else __syncwarp();   // the row's scales are complete (all warps of the CTA are in this round)
         // sgroups is a multiple of 2 (H % 256 == 0): pairs of scales always; quads when the row's scale block is 16-byte aligned.
         const bool quad = (sgroups & 3) == 0;
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-          if (j >= nj || out_row[j] == nullptr) continue;
+          if (part != 0 || j >= nj || out_row[j] == nullptr) continue;
           // the receiver's slab base is the row pointer minus the row's offset in the receive buffer
           float* srow = reinterpret_cast<float*>(out_row[j] - a.recv_heap_off - static_cast<long long>(row_of[j]) * a.H + a.scale_heap_off) + static_cast<long long>(row_of[j]) * sgroups;
           if (quad) {
@@ -290,7 +327,7 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
             for (int g = lane * 2; g < sgroups; g += 64) *reinterpret_cast<float2*>(srow + g) = *reinterpret_cast<const float2*>(my_scales + g);
           }
         }
-        __syncwarp();  // the next row reuses my_scales
+        if (wpr > 1) __syncthreads(); else __syncwarp();  // the next row reuses my_scales
       }
     }  // wi < n_work
     if (SORTED && (++round % kPublishRounds) == 0 && base + round_stride < n_work) publish_counts();
@@ -300,20 +337,31 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
 
 __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const CombineArgs a) {
   __shared__ int s_ok;
+  grid_dependency_wait();
+  launch_dependents();
   const int El = a.num_experts / a.world;
   if (threadIdx.x == 0) s_ok = 1;
   if (*reinterpret_cast<volatile unsigned long long*>(&a.status->abort) != 0ull) return;
   __syncthreads();
   const unsigned long long ready_epoch = a.epoch_dev ? *a.epoch_dev : a.ready_epoch;
-  if (ready_epoch != 0) {
+  if (ready_epoch != 0 && a.world > 1) {   // alone, the rows were written by earlier kernels of this stream
+    if (a.signal && blockIdx.x == 0 && threadIdx.x < a.world) {
+      // My rows are final (this kernel follows their producer): say so to every rank. Block 0 is always resident, so no rank's
+      // wait below can keep this from happening.
+      __threadfence_system();
+      st_release_sys(reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[threadIdx.x]) + a.ready_flags_heap_off) + a.rank, ready_epoch);
+    }
     const unsigned long long* flags = reinterpret_cast<const unsigned long long*>(static_cast<unsigned char*>(a.peer_table[a.rank]) + a.ready_flags_heap_off);
     if (threadIdx.x < a.world && !wait_ge_bounded(flags + threadIdx.x, ready_epoch, a.status, kSiteCombineReady, threadIdx.x, a.timeout_ns)) s_ok = 0;
     __syncthreads();
     if (!s_ok) return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  const int chunks = a.H / 8;
-  for (int t = blockIdx.x * wpb + warp; t < a.T; t += gridDim.x * wpb) {
+  const int chunks = a.H / 8, rounds = chunks / 32, segs = a.segments;
+  // A warp takes one of `segs` column ranges of a token's row (1 in dot mode, whose sums span the row).
+  for (long long u = blockIdx.x * wpb + warp; u < static_cast<long long>(a.T) * segs; u += gridDim.x * wpb) {
+    const int t = static_cast<int>(u / segs), seg = static_cast<int>(u % segs);
+    const int c_end = rounds * (seg + 1) / segs * 32;
     const uint4* rows[kMaxK];
     float w[kMaxK];
 #pragma unroll
@@ -334,17 +382,17 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
     if (a.dot_out == nullptr) {
       uint4* out = reinterpret_cast<uint4*>(a.out + static_cast<long long>(t) * a.H);
       constexpr int U = 2;  // two chunks x K rows of peer loads in flight per lane
-      for (int c0 = lane; c0 < chunks; c0 += 32 * U) {
+      for (int c0 = rounds * seg / segs * 32 + lane; c0 < c_end; c0 += 32 * U) {
         uint4 v[U][kMaxK];
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
           for (int j = 0; j < kMaxK; ++j)
-            if (j < a.K && c0 + 32 * u < chunks) v[u][j] = rows[j] ? __ldcg(rows[j] + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
+            if (j < a.K && c0 + 32 * u < c_end) v[u][j] = rows[j] ? __ldcg(rows[j] + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int c = c0 + 32 * u;
-          if (c >= chunks) break;
+          if (c >= c_end) break;
           float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
           for (int j = 0; j < kMaxK; ++j) {
@@ -386,16 +434,6 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
   }
 }
 
-__global__ void peer_signal_kernel(void* const* peer_table, int rank, int world, long long flags_heap_off, unsigned long long epoch,
-                                   const unsigned long long* epoch_dev) {
-  if (epoch_dev) epoch = *epoch_dev;
-  if (threadIdx.x < world) {
-    __threadfence_system();
-    unsigned long long* dst = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(peer_table[threadIdx.x]) + flags_heap_off);
-    st_release_sys(dst + rank, epoch);
-  }
-}
-
 __global__ void wait_counters_kernel(const unsigned long long* counter, const unsigned long long* target, int n, DeviceStatus* st,
                                      unsigned long long timeout_ns) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -410,6 +448,12 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
   if ((a.xq != nullptr) != (a.xq_scales != nullptr) || (a.xq != nullptr && !a.fp8)) return cudaErrorInvalidValue;
   if (a.T == 0) return cudaSuccess;
   if (a.tile_rows < 0 || (a.tile_rows > 0 && a.num_tiles < 1)) return cudaErrorInvalidValue;
+  if (a.local_rows != nullptr && (!a.fp8 || a.send_list != nullptr || a.row_scale != nullptr || a.world != 1)) return cudaErrorInvalidValue;
+  DispatchArgs b = a;
+  b.warps_per_row = a.send_list == nullptr && a.T <= ctas ? kCommThreads / 32 : 1;
+  // No more CTAs than there is work for (entries of the sorted list, rows per CTA otherwise).
+  const long long work = a.send_list != nullptr ? static_cast<long long>(a.T) * a.K : static_cast<long long>(a.T) * b.warps_per_row;
+  ctas = static_cast<int>(std::min<long long>(ctas, (work + kCommThreads / 32 - 1) / (kCommThreads / 32)));
   const size_t smem = sizeof(int) * (a.tile_rows > 0 ? static_cast<size_t>(a.world) * a.num_tiles : static_cast<size_t>(a.num_experts));
   if (smem > 200 * 1024) return cudaErrorInvalidValue;  // per-CTA histogram of destination tiles must fit in shared memory
   auto go = [&](auto kern) {
@@ -417,11 +461,12 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
       if (e != cudaSuccess) return e;
     }
-    kern<<<ctas, kCommThreads, smem, stream>>>(a);
-    note_launch();
-    return cudaGetLastError();
+    cudaError_t e = launch_early(kern, dim3(ctas), kCommThreads, smem, stream, b);
+    if (e == cudaSuccess) note_launch();
+    return e;
   };
   const bool sorted = a.send_list != nullptr, scaled = a.row_scale != nullptr;
+  if (a.local_rows != nullptr) return go(dispatch_push_kernel<false, false, false, true>);
   if (a.fp8) return sorted ? go(dispatch_push_kernel<true, true, false>) : go(dispatch_push_kernel<true, false, false>);
   if (sorted) return scaled ? go(dispatch_push_kernel<false, true, true>) : go(dispatch_push_kernel<false, true, false>);
   return scaled ? go(dispatch_push_kernel<false, false, true>) : go(dispatch_push_kernel<false, false, false>);
@@ -438,16 +483,12 @@ cudaError_t launch_quantise_rows(const __nv_bfloat16* x, int T, int H, unsigned 
 cudaError_t launch_combine_pull(const CombineArgs& a, int ctas, cudaStream_t stream) {
   if (a.K < 1 || a.K > kMaxK || a.H % 256 || a.world < 1 || a.num_experts % a.world || ctas < 1) return cudaErrorInvalidValue;
   if (a.T == 0) return cudaSuccess;
-  combine_pull_kernel<<<ctas, kCommThreads, 0, stream>>>(a);
-  note_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_peer_signal(void* const* peer_table, int rank, int world, long long flags_heap_off, unsigned long long epoch,
-                               const unsigned long long* epoch_dev, cudaStream_t stream) {
-  peer_signal_kernel<<<1, 64, 0, stream>>>(peer_table, rank, world, flags_heap_off, epoch, epoch_dev);
-  note_launch();
-  return cudaGetLastError();
+  CombineArgs b = a;
+  // Few tokens: as many warps per row as fill the grid, down to one round of loads per warp.
+  b.segments = a.dot_out != nullptr ? 1 : static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / a.T, 1, a.H / 256));
+  cudaError_t e = launch_early(combine_pull_kernel, dim3(ctas), kCommThreads, 0, stream, b);
+  if (e == cudaSuccess) note_launch();
+  return e;
 }
 
 cudaError_t launch_wait_counters(const unsigned long long* counter, const unsigned long long* target, int n, DeviceStatus* status,

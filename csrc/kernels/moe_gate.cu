@@ -10,7 +10,10 @@
 // GEMM, top-k, gather, softmax and their backward kernels with the activations re-read each time.
 // Limits: num_experts <= 32 (one logit per lane), hidden % 256 == 0, and the gate matrix (forward)
 // or the gate matrix plus the fp32 gradient accumulators (backward) must fit in shared memory.
+#include <algorithm>
+
 #include "route_rank.cuh"
+#include "route_splits.cuh"
 
 namespace fastb {
 
@@ -43,7 +46,7 @@ __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(_
 // Dynamic shared memory: gate [E][H] bf16, norm weight [H] bf16, then int s_eid[kTokensPerBlock * K].
 // A warp takes two tokens per pass: every gate chunk is read and unpacked once for both rows.
 template <int EMAX>
-__global__ void __launch_bounds__(kGateThreads) norm_gate_route_kernel(const NormGateArgs a) {
+__global__ void __launch_bounds__(kGateThreads) norm_gate_route_kernel(const NormGateArgs a, const SplitsArgs sp, unsigned int* ticket) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int E = a.num_experts, H = a.H, K = a.K;
   uint4* s_gate = reinterpret_cast<uint4*>(smem);                            // [E][H / 8]
@@ -133,6 +136,7 @@ __global__ void __launch_bounds__(kGateThreads) norm_gate_route_kernel(const Nor
   __syncthreads();
   route::block_stable_ranks(s_eid, reinterpret_cast<unsigned short*>(s_eid + kTokensPerBlock * K), E, K, a.slot_in_block + static_cast<long long>(t0) * K,
                             a.block_cnt + static_cast<long long>(blockIdx.x) * E);
+  if (ticket != nullptr && route::last_block(ticket)) route::splits_block(sp, reinterpret_cast<int*>(smem));
 }
 
 // Dynamic shared memory: gate [E][H] bf16, norm weight [H] bf16, then fp32 accumulators d_gate [E][H], d_nw [H].
@@ -273,16 +277,17 @@ size_t norm_gate_smem_bytes(int E, int H, int K, bool backward) {
   return backward ? base + (static_cast<size_t>(E) + 1) * H * 4 : base + route::rank_smem_bytes(E, K);
 }
 
-cudaError_t launch_norm_gate_route(const NormGateArgs& a, cudaStream_t stream) {
+cudaError_t launch_norm_gate_route(const NormGateArgs& a, const SplitsArgs* sp, unsigned int* ticket, cudaStream_t stream) {
   if (a.num_experts < 1 || a.num_experts > 32 || a.K < 1 || a.K > a.num_experts || a.K > 32 || a.H % 256) return cudaErrorInvalidValue;
-  const size_t smem = norm_gate_smem_bytes(a.num_experts, a.H, a.K, false);
+  if ((sp != nullptr) != (ticket != nullptr) || (sp != nullptr && (sp->num_experts != a.num_experts || sp->block_cnt != a.block_cnt))) return cudaErrorInvalidValue;
+  const size_t smem = std::max(norm_gate_smem_bytes(a.num_experts, a.H, a.K, false), sp ? route::splits_smem_bytes(sp->world, a.num_experts) : size_t{0});
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   const int blocks = (a.T + kTokensPerBlock - 1) / kTokensPerBlock;
   if (blocks == 0) return cudaSuccess;
   auto go = [&](auto kern) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    kern<<<blocks, kGateThreads, smem, stream>>>(a);
+    kern<<<blocks, kGateThreads, smem, stream>>>(a, sp ? *sp : SplitsArgs{}, ticket);
     note_launch();
     return cudaGetLastError();
   };

@@ -6,7 +6,11 @@
 //                  group offsets for the grouped GEMM and cumulative arrival targets.
 // The reference has no router; its counterpart of the count exchange is the host-side workload
 // broadcast (nvidia/alltoall_nvshmem.cpp:452-472), which this replaces with ~1 KB of NVLink stores.
+#include <algorithm>
+
+#include "early_start.cuh"
 #include "route_rank.cuh"
+#include "route_splits.cuh"
 
 namespace fastb {
 
@@ -17,11 +21,15 @@ constexpr int kRouteThreads = 1024;
 
 // One warp per token at a time. E <= 256 (8 values per lane). 32 warps: a block owns 128 tokens whatever T is, so at small T
 // the warps of one block are all the parallelism there is.
-template <int MAX_PER_LANE>
+// SPLITS: the last block goes on with the split scan.
+template <int MAX_PER_LANE, bool SPLITS>
 __global__ void __launch_bounds__(kRouteThreads) route_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E,
                                                                    int K, int* __restrict__ topk_idx, float* __restrict__ topk_w,
-                                                                   int* __restrict__ slot_in_block, int* __restrict__ block_cnt) {
-  extern __shared__ int s_eid[];  // [kTokensPerBlock * K], then the counts of block_stable_ranks
+                                                                   int* __restrict__ slot_in_block, int* __restrict__ block_cnt, const SplitsArgs sp,
+                                                                   unsigned int* ticket) {
+  extern __shared__ int s_eid[];  // [kTokensPerBlock * K], then the counts of block_stable_ranks; later the split scan's tables
+  grid_dependency_wait();
+  launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kRouteThreads / 32;
   const int t0 = blockIdx.x * kTokensPerBlock;
   const int nt = min(kTokensPerBlock, T - t0);
@@ -57,128 +65,92 @@ __global__ void __launch_bounds__(kRouteThreads) route_topk_kernel(const float* 
   __syncthreads();
   route::block_stable_ranks(s_eid, reinterpret_cast<unsigned short*>(s_eid + kTokensPerBlock * K), E, K, slot_in_block + static_cast<long long>(t0) * K,
                             block_cnt + static_cast<long long>(blockIdx.x) * E);
+  if (SPLITS && route::last_block(ticket)) route::splits_block(sp, s_eid);
 }
 
-// Single CTA. Thread e owns expert e (E <= 1024).
 __global__ void __launch_bounds__(1024) splits_scan_kernel(const SplitsArgs a) {
-  extern __shared__ int s_tot[];  // [E] padded totals per expert, then [world] scratch
-  const int e = threadIdx.x;
-  const int E = a.num_experts, W = a.world, El = E / W;
-  unsigned char* my_slab = static_cast<unsigned char*>(a.peer_table[a.rank]);
-  int* my_counts = reinterpret_cast<int*>(my_slab + a.counts_heap_off);                       // [W][E]
-  unsigned long long* my_flags = reinterpret_cast<unsigned long long*>(my_slab + a.flags_heap_off);  // [W]
-  __shared__ unsigned long long s_epoch;
-  if (e == 0) s_epoch = a.epoch_dev ? (*a.epoch_dev = *a.epoch_dev + 1ull) : a.epoch;
-  __syncthreads();
-  const unsigned long long epoch = s_epoch;
-  int mine = 0;
-  if (e < E) {
-    // Eight independent loads in flight per round (the running sum is the only serial part).
-    for (int b0 = 0; b0 < a.num_blocks; b0 += 8) {
-      int c[8];
+  extern __shared__ int s_splits[];
+  route::splits_block(a, s_splits);
+}
+
+// Router logits of a few tokens with the whole routing behind them, in one launch: a block per token computes its logits (fp32
+// sums of bf16 products, rounded to bf16 as a bf16 GEMM returns them) and chooses its experts; the last block then ranks
+// all entries and does the split scan. Up to kRouteTokensPerBlock tokens. A library GEMM, a conversion, route_topk and
+// splits_scan took 20 us for one token, 35 us for 64; this is bound by each block's read of the gate from L2.
+constexpr int kGateSmallThreads = 1024;
+__global__ void __launch_bounds__(kGateSmallThreads) gate_route_kernel(const GateRouteArgs g, const SplitsArgs sp, unsigned int* ticket) {
+  extern __shared__ int s_mem[];   // first the logits of the token, later the entries' expert ids, their counts and the split scan's tables
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kGateSmallThreads / 32;
+  grid_dependency_wait();
+  launch_dependents();
+  const int E = sp.num_experts, K = g.K, chunks = g.H / 8, t = blockIdx.x;
+  float* s_part = reinterpret_cast<float*>(s_mem);              // [parts][E]
+  const int parts = max(1, kWarps / E);                         // warps that share an expert's row
+  const uint4* x = reinterpret_cast<const uint4*>(g.x + static_cast<long long>(t) * g.H);
+  for (int u = warp; u < E * parts; u += kWarps) {
+    const int e = u % E, part = u / E;
+    const uint4* w = reinterpret_cast<const uint4*>(g.gate + static_cast<long long>(e) * g.H);
+    const int c1 = chunks * (part + 1) / parts;
+    float acc = 0.0f;
+    constexpr int U = 4;   // chunks of both rows in flight: one at a time, 28 rounds of 7168 elements took 16 us
+    for (int c0 = chunks * part / parts + lane; c0 < c1; c0 += 32 * U) {
+      uint4 a[U], b[U];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) c[u] = b0 + u < a.num_blocks ? __ldg(a.block_cnt + static_cast<long long>(b0 + u) * E + e) : 0;
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (b0 + u < a.num_blocks) { a.block_base[static_cast<long long>(b0 + u) * E + e] = mine; mine += c[u]; }
-    }
-    // All-gather by stores: my row of the count matrix goes to every rank (myself included).
-    for (int r = 0; r < W; ++r) {
-      int* dst = reinterpret_cast<int*>(static_cast<unsigned char*>(a.peer_table[r]) + a.counts_heap_off);
-      dst[a.rank * E + e] = mine;
-    }
-  }
-  __threadfence_system();
-  __syncthreads();
-  if (e < W) {
-    unsigned long long* dst = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[e]) + a.flags_heap_off);
-    st_release_sys(dst + a.rank, epoch);
-  }
-  __shared__ int s_ok;
-  if (e == 0) s_ok = 1;
-  __syncthreads();
-  if (e < W) {
-    if (!wait_ge_bounded(my_flags + e, epoch, a.status, kSiteCountsArrive, e, a.timeout_ns)) s_ok = 0;
-  }
-  __syncthreads();
-  if (!s_ok) return;
-  // The count matrix is read once (coalesced, W independent loads per thread) and kept in shared
-  // memory when it fits; every later loop reads the copy.
-  int* s_cnt = s_tot + E;  // [W][E] when a.counts_in_smem
-  int tot = 0, before_me = 0;
-  if (e < E) {
-    for (int s = 0; s < W; ++s) {
-      const int c = *reinterpret_cast<volatile int*>(my_counts + s * E + e);
-      if (a.counts_in_smem) s_cnt[s * E + e] = c;
-      tot += c;
-      if (s < a.rank) before_me += c;
-    }
-    s_tot[e] = (tot + a.row_align - 1) / a.row_align * a.row_align;
-  }
-  auto count_at = [&](int s, int q) { return a.counts_in_smem ? s_cnt[s * E + q] : *reinterpret_cast<volatile int*>(my_counts + s * E + q); };
-  __shared__ int s_over;
-  if (e == 0) s_over = 0;
-  __syncthreads();
-  // Every rank sees the same count matrix, so every rank reaches the same verdict: if any rank's
-  // padded rows exceed the receive capacity, the step is refused everywhere (no rows are sent, the
-  // GEMMs get empty groups) and the status block says how many rows were needed.
-  if (e < W) {
-    int need = 0;
-    for (int q = 0; q < El; ++q) need += s_tot[e * El + q];
-    if (need > a.cap_rows) { atomicMax(&s_over, need); }
-  }
-  __syncthreads();
-  if (s_over) {
-    if (e == 0) report_failure(a.status, kStatusBadArg, kSiteCapacity, a.rank, static_cast<unsigned long long>(s_over), static_cast<unsigned long long>(a.cap_rows));
-    if (e < E) { a.send_base[e] = 0; a.send_cnt[e] = 0; }
-    if (e <= El) a.group_off[e] = 0;
-    if (e < El) a.group_rows[e] = 0;
-    return;
-  }
-  if (e < E) {
-    // Row where my first token for expert e lands on its owner: padded sizes of the owner's
-    // earlier experts plus the rows of lower-ranked sources for e.
-    const int d = e / El, le = e % El;
-    int base = 0;
-    for (int q = 0; q < le; ++q) base += s_tot[d * El + q];
-    a.send_base[e] = base + before_me;
-    a.send_cnt[e] = mine;
-    if (a.send_pos) {
-      // Entries are sent expert-slot by expert-slot: all ranks' local expert 0, then 1, ... Within a
-      // slot every sender starts with itself and walks the ranks upwards, so that at any moment the
-      // senders aim at different receivers.
-      int pos = 0;
-      for (int q = 0; q < E; ++q) {
-        const int key_q = (q % El) * W + (q / El - a.rank + W) % W, key_e = le * W + (d - a.rank + W) % W;
-        if (key_q < key_e) pos += count_at(a.rank, q);
+      for (int k = 0; k < U; ++k) {
+        const bool in = c0 + 32 * k < c1;
+        b[k] = in ? __ldg(w + c0 + 32 * k) : make_uint4(0, 0, 0, 0);
+        a[k] = in ? __ldg(x + c0 + 32 * k) : make_uint4(0, 0, 0, 0);
       }
-      a.send_pos[e] = pos;
-    }
-    if (d == a.rank) {
-      a.group_off[le] = base;
-      a.group_rows[le] = tot;
-      if (le == El - 1) a.group_off[El] = base + s_tot[e];
-      // Monotone arrival targets, one per channel (forward dispatch, backward dispatch).
-      for (int ch = 0; ch < a.num_channels; ++ch) a.arrive_target[ch * El + le] += static_cast<unsigned long long>(tot);
-      if (a.tile_target != nullptr) {
-        // The same per tile of the receive buffer: this expert's rows fill its tiles from `base` on.
-        for (int r0 = 0; r0 < tot; r0 += a.tile_rows) {
-          const int t = (base + r0) / a.tile_rows;
-          if (t >= a.num_tiles) break;
-          const unsigned long long rows = static_cast<unsigned long long>(min(a.tile_rows, tot - r0));
-          for (int ch = 0; ch < a.num_channels; ++ch) a.tile_target[static_cast<long long>(ch) * a.num_tiles + t] += rows;
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&a[k]);
+        const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&b[k]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 f = __bfloat1622float2(p[i]), h = __bfloat1622float2(q[i]);
+          acc = fmaf(f.x, h.x, acc);
+          acc = fmaf(f.y, h.y, acc);
         }
       }
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) s_part[part * E + e] = acc;
   }
-  // Token traffic matrix of this step, [src][dst], for the scheduler / observability.
-  if (a.traffic_matrix)
-    for (int i = threadIdx.x; i < W * W; i += blockDim.x) {
-      const int s = i / W, d = i % W;
-      int sent = 0;
-      for (int q = 0; q < El; ++q) sent += count_at(s, d * El + q);
-      a.traffic_matrix[i] = sent;
+  __syncthreads();
+  if (warp == 0) {
+    constexpr int kPerLane = 8;   // E <= 256
+    float sel[kPerLane], raw[kPerLane];
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+      const int e = lane + 32 * i;
+      float r = -INFINITY, s = -INFINITY;
+      if (e < E) {
+        r = 0.0f;
+        for (int j = 0; j < parts; ++j) r += s_part[j * E + e];
+        r = __bfloat162float(__float2bfloat16_rn(r));
+        if (r != r) r = -INFINITY;
+        s = r + (g.bias ? g.bias[e] : 0.0f);
+        if (s != s) s = -INFINITY;
+      }
+      raw[i] = r;
+      sel[i] = s;
     }
+    int my_e;
+    float my_w;
+    route::warp_topk<kPerLane>(sel, raw, E, K, my_e, my_w);
+    if (lane < K) {
+      g.topk_idx[static_cast<long long>(t) * K + lane] = my_e;
+      g.topk_w[static_cast<long long>(t) * K + lane] = my_w;
+    }
+  }
+  if (!route::last_block(ticket)) return;
+  for (int i = threadIdx.x; i < kTokensPerBlock * K; i += blockDim.x) s_mem[i] = i < static_cast<int>(gridDim.x) * K ? __ldcg(g.topk_idx + i) : -1;
+  __syncthreads();
+  route::block_stable_ranks(s_mem, reinterpret_cast<unsigned short*>(s_mem + kTokensPerBlock * K), E, K, g.slot_in_block, g.block_cnt);
+  __syncthreads();
+  route::splits_block(sp, s_mem);
 }
 
 __global__ void build_send_list_kernel(const int* __restrict__ topk_idx, const int* __restrict__ slot_in_block, const int* __restrict__ block_base,
@@ -208,35 +180,66 @@ __global__ void zero_pad_rows_kernel(unsigned char* buf, long long row_bytes, co
 
 }  // namespace
 
-cudaError_t launch_route_topk(const float* logits, const float* bias, int T, int E, int K, int* topk_idx, float* topk_w, int* slot_in_block,
-                              int* block_cnt, cudaStream_t stream) {
+namespace {
+
+bool splits_args_ok(const SplitsArgs& a) {
+  if (a.tile_target != nullptr && (a.tile_rows < 1 || a.row_align % a.tile_rows || a.num_tiles < 1)) return false;
+  return (a.row_align == 128 || a.row_align == 256) && a.num_experts >= 1 && a.num_experts <= 1024 && a.world >= 1 && a.world <= a.num_experts && a.num_experts % a.world == 0;
+}
+
+template <bool SPLITS>
+cudaError_t route_topk_any(const float* logits, const float* bias, int T, int E, int K, int* topk_idx, float* topk_w, int* slot_in_block, int* block_cnt,
+                           const SplitsArgs& sp, unsigned int* ticket, cudaStream_t stream) {
   if (E < 1 || E > 256 || K < 1 || K > 32 || K > E) return cudaErrorInvalidValue;
   const int blocks = (T + kTokensPerBlock - 1) / kTokensPerBlock;
   if (blocks == 0) return cudaSuccess;
-  const size_t smem = route::rank_smem_bytes(E, K);
+  const size_t smem = std::max(route::rank_smem_bytes(E, K), SPLITS ? route::splits_smem_bytes(sp.world, E) : size_t{0});
   auto go = [&](auto kern) {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
       if (e != cudaSuccess) return e;
     }
-    kern<<<blocks, kRouteThreads, smem, stream>>>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt);
-    note_launch();
-    return cudaGetLastError();
+    cudaError_t e = launch_early(kern, dim3(blocks), kRouteThreads, smem, stream, logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt, sp, ticket);
+    if (e == cudaSuccess) note_launch();
+    return e;
   };
-  if (E <= 32) return go(route_topk_kernel<1>);
-  if (E <= 64) return go(route_topk_kernel<2>);
-  if (E <= 128) return go(route_topk_kernel<4>);
-  return go(route_topk_kernel<8>);
+  if (E <= 32) return go(route_topk_kernel<1, SPLITS>);
+  if (E <= 64) return go(route_topk_kernel<2, SPLITS>);
+  if (E <= 128) return go(route_topk_kernel<4, SPLITS>);
+  return go(route_topk_kernel<8, SPLITS>);
+}
+
+}  // namespace
+
+cudaError_t launch_route_topk(const float* logits, const float* bias, int T, int E, int K, int* topk_idx, float* topk_w, int* slot_in_block,
+                              int* block_cnt, cudaStream_t stream) {
+  return route_topk_any<false>(logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt, SplitsArgs{}, nullptr, stream);
+}
+
+cudaError_t launch_route_splits(const float* logits, const float* bias, int T, int K, int* topk_idx, float* topk_w, int* slot_in_block, const SplitsArgs& sp,
+                                unsigned int* ticket, cudaStream_t stream) {
+  if (T < 1 || ticket == nullptr || !splits_args_ok(sp) || sp.num_blocks != (T + kTokensPerBlock - 1) / kTokensPerBlock) return cudaErrorInvalidValue;
+  return route_topk_any<true>(logits, bias, T, sp.num_experts, K, topk_idx, topk_w, slot_in_block, const_cast<int*>(sp.block_cnt), sp, ticket, stream);
+}
+
+cudaError_t launch_gate_route(const GateRouteArgs& g, const SplitsArgs& sp, unsigned int* ticket, cudaStream_t stream) {
+  const int E = sp.num_experts;
+  if (g.T < 1 || g.T > kTokensPerBlock || E > 256 || g.K < 1 || g.K > 32 || g.K > E || g.H % 8 || ticket == nullptr || !splits_args_ok(sp) || sp.num_blocks != 1) return cudaErrorInvalidValue;
+  const size_t smem = std::max({route::rank_smem_bytes(E, g.K), route::splits_smem_bytes(sp.world, E), sizeof(float) * std::max(E, kGateSmallThreads / 32)});
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(gate_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
+  cudaError_t e = launch_early(gate_route_kernel, dim3(g.T), kGateSmallThreads, smem, stream, g, sp, ticket);
+  if (e == cudaSuccess) note_launch();
+  return e;
 }
 
 cudaError_t launch_splits_scan(const SplitsArgs& a, cudaStream_t stream) {
-  if (a.tile_target != nullptr && (a.tile_rows < 1 || a.row_align % a.tile_rows || a.num_tiles < 1)) return cudaErrorInvalidValue;
-  if ((a.row_align != 128 && a.row_align != 256) || a.num_experts < 1 || a.num_experts > 1024 || a.world < 1 || a.world > a.num_experts || a.num_experts % a.world) return cudaErrorInvalidValue;
-  int threads = (std::max(a.num_experts, a.world) + 31) / 32 * 32;
-  SplitsArgs b = a;
-  b.counts_in_smem = static_cast<long long>(a.world) * a.num_experts <= 8192 ? 1 : 0;  // 32 KiB of the 48 KiB default
-  const size_t smem = sizeof(int) * (a.num_experts + a.world + (b.counts_in_smem ? a.world * a.num_experts : 0));
-  splits_scan_kernel<<<1, threads, smem, stream>>>(b);
+  if (!splits_args_ok(a)) return cudaErrorInvalidValue;
+  // a thread per expert at least; more warps take experts and routing blocks in parallel
+  const int threads = std::max(256, (std::max(a.num_experts, a.world) + 31) / 32 * 32);
+  splits_scan_kernel<<<1, threads, route::splits_smem_bytes(a.world, a.num_experts), stream>>>(a);
   note_launch();
   return cudaGetLastError();
 }

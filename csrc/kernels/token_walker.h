@@ -19,9 +19,9 @@ FASTB_HD constexpr int div_up(int a, int b) { return (a + b - 1) / b; }
 // Token tiles of a group whose tokens are taken up to `rows` (real rows rounded up to the granule, a multiple of 32): as few
 // as hold them, all but the last of one width, in multiples of 32. 640 tokens are 3 tiles of 224, 224 and 192 instead of
 // 256, 256 and 128: tiles that run side by side then advance at one pace and keep sharing operand panels.
-FASTB_HD inline int tok_tiles(int rows) { return div_up(rows, kTokTileN); }
-FASTB_HD inline int tok_tile_size(int rows) {
-  const int t = tok_tiles(rows);
+FASTB_HD inline int tok_tiles(int rows, int tile_n) { return div_up(rows, tile_n); }
+FASTB_HD inline int tok_tile_size(int rows, int tile_n) {
+  const int t = tok_tiles(rows, tile_n);
   return t > 0 ? ceil_to(div_up(rows, t), 32) : 0;
 }
 
@@ -38,8 +38,8 @@ FASTB_HD inline int tok_tile_size(int rows) {
 // tokens of the tile, i.e. its fp32 sums written and read once at an SM's share of L2.
 struct TokSplit {
   int pairs, kb_tile;
-  int whole_tiles;     // tiles done whole, tile i by pair i % pairs
-  int cut_tiles;       // tiles from whole_tiles on, done in parts
+  int whole_tiles;     // tiles done whole: the i-th of them, tile cut_tiles + i, by pair i % pairs
+  int cut_tiles;       // the first tiles, done in parts, before the whole ones: their exchange then hides behind the others
   int shares;          // stream: pairs that take a share; parts: parts per tile
   bool stream;
   FASTB_HD static TokSplit make(int tiles, int kb_tile, int pairs, int widest_n, bool share_weights) {
@@ -80,15 +80,15 @@ struct TokSegments {
     else if (pair < s.shares) { u = s.share_begin(pair); u_end = s.share_begin(pair + 1); }
   }
   FASTB_HD bool next(TokSegment& g) {
-    if (next_whole < s.whole_tiles) {
-      g = TokSegment{next_whole, 0, s.kb_tile, 1, 0, pair, 1};
+    if (u >= u_end) {
+      if (next_whole >= s.whole_tiles) return false;
+      g = TokSegment{s.cut_tiles + next_whole, 0, s.kb_tile, 1, 0, pair, 1};
       next_whole += s.pairs;
       return true;
     }
-    if (u >= u_end) return false;
     if (!s.stream) {
       const int t = pair % s.cut_tiles, j = pair / s.cut_tiles;
-      g = TokSegment{s.whole_tiles + t, static_cast<int>(static_cast<long long>(s.kb_tile) * j / s.shares), static_cast<int>(static_cast<long long>(s.kb_tile) * (j + 1) / s.shares),
+      g = TokSegment{t, static_cast<int>(static_cast<long long>(s.kb_tile) * j / s.shares), static_cast<int>(static_cast<long long>(s.kb_tile) * (j + 1) / s.shares),
                      s.shares, j, t, s.cut_tiles};
       u = u_end;
       return true;
@@ -96,7 +96,7 @@ struct TokSegments {
     const int t = u / s.kb_tile, kb0 = u - t * s.kb_tile;
     const int left = s.kb_tile - kb0, kb1 = kb0 + (u_end - u < left ? u_end - u : left);
     const int lo = s.share_of(t * s.kb_tile), hi = s.share_of((t + 1) * s.kb_tile - 1);
-    g = TokSegment{s.whole_tiles + t, kb0, kb1, hi - lo + 1, pair - lo, lo, 1};
+    g = TokSegment{t, kb0, kb1, hi - lo + 1, pair - lo, lo, 1};
     u += kb1 - kb0;
     return true;
   }

@@ -127,9 +127,11 @@ struct TokGemmPlan {
 
   // counters: int32 [2, >= tok_counters(ctas)], kept by the caller, parity alternating from launch to launch; none = cleared for this launch.
   void run(torch::Tensor group_off, c10::optional<torch::Tensor> group_rows, int64_t status_ptr, uint64_t timeout_ns, int ctas, int64_t gate_counter_ptr,
-           c10::optional<torch::Tensor> gate_target, int gate_tile_rows, c10::optional<torch::Tensor> counters, int parity) const {
+           c10::optional<torch::Tensor> gate_target, int gate_tile_rows, c10::optional<torch::Tensor> counters, int parity, int tile_n, bool early) const {
     TORCH_CHECK(group_off.is_cuda() && group_off.dtype() == torch::kInt32 && group_off.is_contiguous() && group_off.numel() == groups + 1, "group_off: cuda int32[G+1]");
     TokGemmArgs g = a;
+    g.tile_n = tile_n;
+    g.early = early ? 1 : 0;
     g.group_off = group_off.data_ptr<int>();
     if (group_rows.has_value()) {
       want(*group_rows, torch::kInt32, "group_rows");
@@ -221,36 +223,91 @@ void route_topk(torch::Tensor logits, c10::optional<torch::Tensor> bias, int K, 
                              slot_in_block.data_ptr<int>(), block_cnt.data_ptr<int>(), stream_now()), "route_topk");
 }
 
-void splits_scan(const HeapPy& heap, int64_t counts_off, int64_t flags_off, uint64_t epoch, torch::Tensor block_cnt, torch::Tensor block_base,
-                 torch::Tensor send_base, torch::Tensor send_cnt, torch::Tensor group_off, torch::Tensor group_rows, torch::Tensor arrive_target,
-                 c10::optional<torch::Tensor> traffic, int num_channels, int row_align, int cap_rows, const StatusPy& st, uint64_t timeout_ns,
-                 c10::optional<torch::Tensor> send_pos, int64_t epoch_dev_ptr, c10::optional<torch::Tensor> tile_target, int tile_rows) {
+// The split scan of one engine: everything that stays the same from step to step (and the tensors it points into).
+struct SplitsPlan {
   SplitsArgs a{};
-  if (tile_target.has_value()) {
-    want(*tile_target, torch::kInt64, "tile_target");
-    TORCH_CHECK(tile_target->dim() == 2 && tile_target->size(0) == num_channels && tile_rows > 0, "tile_target: int64 [channels, tiles]");
-    a.tile_target = reinterpret_cast<unsigned long long*>(tile_target->data_ptr());
-    a.tile_rows = tile_rows;
-    a.num_tiles = static_cast<int>(tile_target->size(1));
+  unsigned int* ticket = nullptr;
+  std::vector<torch::Tensor> keep;
+  int max_blocks = 0;
+
+  SplitsPlan(const HeapPy& heap, int64_t counts_off, int64_t flags_off, torch::Tensor block_cnt, torch::Tensor block_base, torch::Tensor send_base, torch::Tensor send_cnt,
+             torch::Tensor group_off, torch::Tensor group_rows, torch::Tensor arrive_target, c10::optional<torch::Tensor> traffic, int num_channels, int row_align, int cap_rows,
+             const StatusPy& st, uint64_t timeout_ns, c10::optional<torch::Tensor> send_pos, int64_t epoch_dev_ptr, c10::optional<torch::Tensor> tile_target, int tile_rows,
+             torch::Tensor ticket_word) {
+    if (tile_target.has_value()) {
+      want(*tile_target, torch::kInt64, "tile_target");
+      TORCH_CHECK(tile_target->dim() == 2 && tile_target->size(0) == num_channels && tile_rows > 0, "tile_target: int64 [channels, tiles]");
+      a.tile_target = reinterpret_cast<unsigned long long*>(tile_target->data_ptr());
+      a.tile_rows = tile_rows;
+      a.num_tiles = static_cast<int>(tile_target->size(1));
+      keep.push_back(*tile_target);
+    }
+    a.row_align = row_align;
+    a.cap_rows = cap_rows;
+    a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
+    a.num_experts = static_cast<int>(send_base.numel()); a.num_channels = num_channels;
+    max_blocks = static_cast<int>(block_cnt.numel() / a.num_experts);
+    a.counts_heap_off = counts_off; a.flags_heap_off = flags_off;
+    want(block_cnt, torch::kInt32, "block_cnt"); want(block_base, torch::kInt32, "block_base"); want(send_base, torch::kInt32, "send_base");
+    want(send_cnt, torch::kInt32, "send_cnt"); want(group_off, torch::kInt32, "group_off"); want(group_rows, torch::kInt32, "group_rows");
+    want(arrive_target, torch::kInt64, "arrive_target"); want(ticket_word, torch::kInt32, "ticket");
+    const int El = a.num_experts / a.world;
+    TORCH_CHECK(group_off.numel() == El + 1 && group_rows.numel() == El && arrive_target.numel() == static_cast<int64_t>(num_channels) * El && block_base.numel() >= block_cnt.numel(),
+                "split scan: shapes");
+    a.block_cnt = block_cnt.data_ptr<int>(); a.block_base = block_base.data_ptr<int>(); a.send_base = send_base.data_ptr<int>();
+    a.send_cnt = send_cnt.data_ptr<int>(); a.group_off = group_off.data_ptr<int>(); a.group_rows = group_rows.data_ptr<int>();
+    a.arrive_target = reinterpret_cast<unsigned long long*>(arrive_target.data_ptr());
+    a.traffic_matrix = ptr_or_null<int>(traffic);
+    a.send_pos = ptr_or_null<int>(send_pos);
+    a.epoch_dev = reinterpret_cast<unsigned long long*>(epoch_dev_ptr);
+    a.status = st.d; a.timeout_ns = timeout_ns;
+    ticket = reinterpret_cast<unsigned int*>(ticket_word.data_ptr<int>());
+    for (const auto& t : {block_cnt, block_base, send_base, send_cnt, group_off, group_rows, arrive_target, ticket_word}) keep.push_back(t);
+    if (traffic.has_value()) keep.push_back(*traffic);
+    if (send_pos.has_value()) keep.push_back(*send_pos);
   }
-  a.row_align = row_align;
-  a.cap_rows = cap_rows;
-  a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
-  a.num_experts = static_cast<int>(send_base.numel()); a.num_blocks = static_cast<int>(block_cnt.numel() / a.num_experts); a.num_channels = num_channels;
-  a.counts_heap_off = counts_off; a.flags_heap_off = flags_off; a.epoch = epoch;
-  want(block_cnt, torch::kInt32, "block_cnt"); want(block_base, torch::kInt32, "block_base"); want(send_base, torch::kInt32, "send_base");
-  want(send_cnt, torch::kInt32, "send_cnt"); want(group_off, torch::kInt32, "group_off"); want(group_rows, torch::kInt32, "group_rows");
-  want(arrive_target, torch::kInt64, "arrive_target");
-  const int El = a.num_experts / a.world;
-  TORCH_CHECK(group_off.numel() == El + 1 && group_rows.numel() == El && arrive_target.numel() == static_cast<int64_t>(num_channels) * El, "splits_scan: shapes");
-  a.block_cnt = block_cnt.data_ptr<int>(); a.block_base = block_base.data_ptr<int>(); a.send_base = send_base.data_ptr<int>();
-  a.send_cnt = send_cnt.data_ptr<int>(); a.group_off = group_off.data_ptr<int>(); a.group_rows = group_rows.data_ptr<int>();
-  a.arrive_target = reinterpret_cast<unsigned long long*>(arrive_target.data_ptr());
-  a.traffic_matrix = ptr_or_null<int>(traffic);
-  a.send_pos = ptr_or_null<int>(send_pos);
-  a.epoch_dev = reinterpret_cast<unsigned long long*>(epoch_dev_ptr);
-  a.status = st.d; a.timeout_ns = timeout_ns;
-  cu_check(launch_splits_scan(a, stream_now()), "splits_scan");
+  SplitsArgs for_tokens(int64_t T, uint64_t epoch) const {
+    SplitsArgs b = a;
+    b.num_blocks = static_cast<int>((T + kRouteTokensPerBlock - 1) / kRouteTokensPerBlock);
+    TORCH_CHECK(b.num_blocks <= max_blocks, "more tokens than the engine was made for");
+    b.epoch = epoch;
+    return b;
+  }
+};
+
+void check_route_outputs(const SplitsPlan& p, int64_t T, int K, const torch::Tensor& topk_idx, const torch::Tensor& topk_w, const torch::Tensor& slot_in_block) {
+  want(topk_idx, torch::kInt32, "topk_idx"); want(topk_w, torch::kFloat32, "topk_w"); want(slot_in_block, torch::kInt32, "slot_in_block");
+  const int64_t blocks = (T + kRouteTokensPerBlock - 1) / kRouteTokensPerBlock;
+  TORCH_CHECK(topk_idx.numel() == T * K && topk_w.numel() == T * K && slot_in_block.numel() >= blocks * kRouteTokensPerBlock * K, "route: output shapes");
+}
+
+// Top-k of ready-made logits and the split scan, one launch.
+void route_splits(const SplitsPlan& p, torch::Tensor logits, c10::optional<torch::Tensor> bias, int K, torch::Tensor topk_idx, torch::Tensor topk_w,
+                  torch::Tensor slot_in_block, uint64_t epoch) {
+  want(logits, torch::kFloat32, "logits");
+  const int64_t T = logits.size(0);
+  TORCH_CHECK(logits.dim() == 2 && logits.size(1) == p.a.num_experts, "logits: float [T, experts]");
+  check_route_outputs(p, T, K, topk_idx, topk_w, slot_in_block);
+  const SplitsArgs a = p.for_tokens(T, epoch);
+  if (T == 0) cu_check(launch_splits_scan(a, stream_now()), "splits_scan");   // no tokens of my own: the peers still want my counts
+  else
+    cu_check(launch_route_splits(logits.data_ptr<float>(), ptr_or_null<const float>(bias), static_cast<int>(T), K, topk_idx.data_ptr<int>(), topk_w.data_ptr<float>(),
+                                 slot_in_block.data_ptr<int>(), a, p.ticket, stream_now()), "route_splits");
+}
+
+// The same from the activations of at most ROUTE_TOKENS_PER_BLOCK tokens: logits = bf16(x . gate^T).
+void gate_route(const SplitsPlan& p, torch::Tensor x, torch::Tensor gate, c10::optional<torch::Tensor> bias, int K, torch::Tensor topk_idx, torch::Tensor topk_w,
+                torch::Tensor slot_in_block, uint64_t epoch) {
+  want(x, torch::kBFloat16, "x"); want(gate, torch::kBFloat16, "gate");
+  const int64_t T = x.size(0);
+  TORCH_CHECK(x.dim() == 2 && gate.dim() == 2 && gate.size(0) == p.a.num_experts && gate.size(1) == x.size(1) && T >= 1 && T <= kRouteTokensPerBlock, "gate_route: shapes");
+  check_route_outputs(p, T, K, topk_idx, topk_w, slot_in_block);
+  const SplitsArgs a = p.for_tokens(T, epoch);
+  GateRouteArgs g{};
+  g.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()); g.gate = reinterpret_cast<const __nv_bfloat16*>(gate.data_ptr()); g.bias = ptr_or_null<const float>(bias);
+  g.T = static_cast<int>(T); g.H = static_cast<int>(x.size(1)); g.K = K;
+  g.topk_idx = topk_idx.data_ptr<int>(); g.topk_w = topk_w.data_ptr<float>(); g.slot_in_block = slot_in_block.data_ptr<int>(); g.block_cnt = const_cast<int*>(a.block_cnt);
+  cu_check(launch_gate_route(g, a, p.ticket, stream_now()), "gate_route");
 }
 
 void zero_pad_rows(torch::Tensor buf, torch::Tensor group_off, torch::Tensor group_rows, int align) {
@@ -263,7 +320,7 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
                    torch::Tensor block_base, torch::Tensor send_base, torch::Tensor dest_row, bool compute_rows, bool fp8, int64_t recv_off,
                    int64_t scale_off, int64_t arrive_off, int64_t entry_flags_off, uint64_t entry_epoch, const StatusPy& st, uint64_t timeout_ns, int ctas,
                    c10::optional<torch::Tensor> send_list, int tile_rows, int num_tiles, c10::optional<torch::Tensor> xq,
-                   c10::optional<torch::Tensor> xq_scales) {
+                   c10::optional<torch::Tensor> xq_scales, c10::optional<torch::Tensor> local_rows) {
   want(x, torch::kBFloat16, "x"); want(topk_idx, torch::kInt32, "topk_idx"); want(dest_row, torch::kInt32, "dest_row");
   DispatchArgs a{};
   a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
@@ -280,6 +337,11 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
     TORCH_CHECK(xq->numel() >= x.numel() && xq_scales->numel() >= x.numel() / 128, "dispatch_push: xq / xq_scales too small");
     a.xq = xq->data_ptr<uint8_t>(); a.xq_scales = xq_scales->data_ptr<float>();
   }
+  if (local_rows.has_value()) {
+    want(*local_rows, torch::kBFloat16, "local_rows");
+    TORCH_CHECK(fp8 && local_rows->dim() == 2 && local_rows->size(1) == a.H, "dispatch_push: local_rows belongs to the fp8 rows");
+    a.local_rows = reinterpret_cast<__nv_bfloat16*>(local_rows->data_ptr());
+  }
   a.recv_heap_off = recv_off; a.scale_heap_off = scale_off; a.arrive_heap_off = arrive_off;
   a.entry_flags_heap_off = entry_flags_off; a.entry_epoch = entry_epoch; a.status = st.d; a.timeout_ns = timeout_ns;
   cu_check(launch_dispatch_push(a, ctas, stream_now()), "dispatch_push");
@@ -287,8 +349,9 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
 
 void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, torch::Tensor dest_row, c10::optional<torch::Tensor> weights, int64_t src_off,
                   int64_t ready_off, uint64_t ready_epoch, c10::optional<torch::Tensor> out, c10::optional<torch::Tensor> dot_with,
-                  c10::optional<torch::Tensor> dot_out, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr) {
+                  c10::optional<torch::Tensor> dot_out, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr, bool signal) {
   CombineArgs a{};
+  a.signal = signal ? 1 : 0;
   a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world(); a.num_experts = num_experts;
   a.T = static_cast<int>(topk_idx.size(0)); a.K = static_cast<int>(topk_idx.size(1)); a.H = H;
   a.topk_idx = topk_idx.data_ptr<int>(); a.dest_row = dest_row.data_ptr<int>(); a.weights = ptr_or_null<const float>(weights);
@@ -307,7 +370,7 @@ void bind_moe(py::module_& m) {
   py::class_<TokGemmPlan>(m, "TokGemmPlan")
       .def(py::init<int, int, torch::Tensor, torch::Tensor, torch::Tensor, c10::optional<torch::Tensor>, int, int>())
       .def("run", &TokGemmPlan::run, py::arg("group_off"), py::arg("group_rows"), py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"),
-           py::arg("gate_counter_ptr") = 0, py::arg("gate_target") = py::none(), py::arg("gate_tile_rows") = 0, py::arg("counters") = py::none(), py::arg("parity") = 0);
+           py::arg("gate_counter_ptr") = 0, py::arg("gate_target") = py::none(), py::arg("gate_tile_rows") = 0, py::arg("counters") = py::none(), py::arg("parity") = 0, py::arg("tile_n") = 256, py::arg("early") = false);
   m.attr("TOK_COUNTERS_PER_CTA") = tok_counters(1);
   m.def("grouped_gemm", &grouped_gemm, py::arg("mode"), py::arg("epilogue"), py::arg("a"), py::arg("b"), py::arg("group_off"), py::arg("tiles_n"),
         py::arg("fixed_m_tiles"), py::arg("red_len"), py::arg("b_rows_per_group"), py::arg("c_rows_per_group"), py::arg("c"), py::arg("c2"),
@@ -317,10 +380,14 @@ void bind_moe(py::module_& m) {
   m.def("grouped_gemm_smem_bytes", &grouped_gemm_smem_bytes);
   m.attr("ROUTE_TOKENS_PER_BLOCK") = kRouteTokensPerBlock;
   m.def("route_topk", &route_topk);
-  m.def("splits_scan", &splits_scan, py::arg("heap"), py::arg("counts_off"), py::arg("flags_off"), py::arg("epoch"), py::arg("block_cnt"), py::arg("block_base"),
-        py::arg("send_base"), py::arg("send_cnt"), py::arg("group_off"), py::arg("group_rows"), py::arg("arrive_target"), py::arg("traffic"),
-        py::arg("num_channels"), py::arg("row_align"), py::arg("cap_rows"), py::arg("status"), py::arg("timeout_ns"), py::arg("send_pos"),
-        py::arg("epoch_dev_ptr"), py::arg("tile_target") = py::none(), py::arg("tile_rows") = 0);
+  py::class_<SplitsPlan>(m, "SplitsPlan")
+      .def(py::init<const HeapPy&, int64_t, int64_t, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor,
+                    c10::optional<torch::Tensor>, int, int, int, const StatusPy&, uint64_t, c10::optional<torch::Tensor>, int64_t, c10::optional<torch::Tensor>, int, torch::Tensor>(),
+           py::arg("heap"), py::arg("counts_off"), py::arg("flags_off"), py::arg("block_cnt"), py::arg("block_base"), py::arg("send_base"), py::arg("send_cnt"),
+           py::arg("group_off"), py::arg("group_rows"), py::arg("arrive_target"), py::arg("traffic"), py::arg("num_channels"), py::arg("row_align"), py::arg("cap_rows"),
+           py::arg("status"), py::arg("timeout_ns"), py::arg("send_pos"), py::arg("epoch_dev_ptr"), py::arg("tile_target"), py::arg("tile_rows"), py::arg("ticket"));
+  m.def("route_splits", &route_splits);
+  m.def("gate_route", &gate_route);
   m.def("zero_pad_rows", &zero_pad_rows, py::arg("buf"), py::arg("group_off"), py::arg("group_rows"), py::arg("align") = 0);
   m.def("build_send_list", [](torch::Tensor topk_idx, torch::Tensor slot_in_block, torch::Tensor block_base, torch::Tensor send_pos, torch::Tensor list, const StatusPy& st) {
     want(topk_idx, torch::kInt32, "topk_idx"); want(send_pos, torch::kInt32, "send_pos"); want(list, torch::kInt32, "list");
@@ -332,7 +399,7 @@ void bind_moe(py::module_& m) {
   m.def("norm_gate_smem_bytes", [](int E, int H, int K, bool backward) { return static_cast<int64_t>(norm_gate_smem_bytes(E, H, K, backward)); });
   m.def("norm_gate_route", [](torch::Tensor h, torch::Tensor norm_w, torch::Tensor gate, c10::optional<torch::Tensor> bias, int K, double eps, torch::Tensor hn,
                               torch::Tensor rstd, torch::Tensor logits, torch::Tensor topk_idx, torch::Tensor topk_w, torch::Tensor slot_in_block,
-                              torch::Tensor block_cnt) {
+                              torch::Tensor block_cnt, const SplitsPlan* splits, uint64_t epoch) {
     want(h, torch::kBFloat16, "h"); want(norm_w, torch::kBFloat16, "norm_w"); want(gate, torch::kBFloat16, "gate"); want(hn, torch::kBFloat16, "hn");
     want(rstd, torch::kFloat32, "rstd"); want(logits, torch::kFloat32, "logits"); want(topk_idx, torch::kInt32, "topk_idx"); want(topk_w, torch::kFloat32, "topk_w");
     want(slot_in_block, torch::kInt32, "slot_in_block"); want(block_cnt, torch::kInt32, "block_cnt");
@@ -347,8 +414,12 @@ void bind_moe(py::module_& m) {
     a.gate = reinterpret_cast<const __nv_bfloat16*>(gate.data_ptr()); a.bias = ptr_or_null<const float>(bias);
     a.hn = reinterpret_cast<__nv_bfloat16*>(hn.data_ptr()); a.rstd = rstd.data_ptr<float>(); a.logits = logits.data_ptr<float>();
     a.topk_idx = topk_idx.data_ptr<int>(); a.topk_w = topk_w.data_ptr<float>(); a.slot_in_block = slot_in_block.data_ptr<int>(); a.block_cnt = block_cnt.data_ptr<int>();
-    cu_check(launch_norm_gate_route(a, stream_now()), "norm_gate_route");
-  });
+    if (splits == nullptr) { cu_check(launch_norm_gate_route(a, nullptr, nullptr, stream_now()), "norm_gate_route"); return; }
+    const SplitsArgs sp = splits->for_tokens(a.T, epoch);
+    if (a.T == 0) cu_check(launch_splits_scan(sp, stream_now()), "splits_scan");
+    else cu_check(launch_norm_gate_route(a, &sp, splits->ticket, stream_now()), "norm_gate_route");
+  }, py::arg("h"), py::arg("norm_w"), py::arg("gate"), py::arg("bias"), py::arg("k"), py::arg("eps"), py::arg("hn"), py::arg("rstd"), py::arg("logits"), py::arg("topk_idx"),
+     py::arg("topk_w"), py::arg("slot_in_block"), py::arg("block_cnt"), py::arg("splits") = nullptr, py::arg("epoch") = 0);
   m.def("norm_gate_bwd", [](torch::Tensor h, torch::Tensor norm_w, torch::Tensor gate, torch::Tensor rstd, torch::Tensor topk_idx, torch::Tensor topk_w,
                             torch::Tensor grad_w, torch::Tensor grad_hn, torch::Tensor grad_h, torch::Tensor d_gate, torch::Tensor d_norm_w) {
     want(h, torch::kBFloat16, "h"); want(norm_w, torch::kBFloat16, "norm_w"); want(gate, torch::kBFloat16, "gate"); want(rstd, torch::kFloat32, "rstd");
@@ -367,18 +438,16 @@ void bind_moe(py::module_& m) {
   m.def("dispatch_push", &dispatch_push, py::arg("heap"), py::arg("x"), py::arg("topk_idx"), py::arg("row_scale"), py::arg("slot_in_block"), py::arg("block_base"),
         py::arg("send_base"), py::arg("dest_row"), py::arg("compute_rows"), py::arg("fp8"), py::arg("recv_off"), py::arg("scale_off"), py::arg("arrive_off"),
         py::arg("entry_flags_off"), py::arg("entry_epoch"), py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"), py::arg("send_list"),
-        py::arg("tile_rows") = 0, py::arg("num_tiles") = 0, py::arg("xq") = py::none(), py::arg("xq_scales") = py::none());
+        py::arg("tile_rows") = 0, py::arg("num_tiles") = 0, py::arg("xq") = py::none(), py::arg("xq_scales") = py::none(), py::arg("local_rows") = py::none());
   m.def("quantise_rows", [](torch::Tensor x, torch::Tensor q, torch::Tensor scales, int ctas) {
     want(x, torch::kBFloat16, "x"); want(q, torch::kUInt8, "q"); want(scales, torch::kFloat32, "scales");
     TORCH_CHECK(x.dim() == 2 && q.numel() >= x.numel() && scales.numel() >= x.numel() / 128, "quantise_rows: q / scales too small");
     cu_check(launch_quantise_rows(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), static_cast<int>(x.size(0)), static_cast<int>(x.size(1)),
                                   q.data_ptr<uint8_t>(), scales.data_ptr<float>(), ctas, stream_now()), "quantise_rows");
   });
-  m.def("combine_pull", &combine_pull);
-  m.def("peer_signal", [](const HeapPy& heap, int64_t flags_off, uint64_t epoch, int64_t epoch_dev_ptr) {
-    cu_check(launch_peer_signal(heap.h->device_peer_table(), heap.h->rank(), heap.h->world(), flags_off, epoch,
-                                reinterpret_cast<const unsigned long long*>(epoch_dev_ptr), stream_now()), "peer_signal");
-  });
+  m.def("combine_pull", &combine_pull, py::arg("heap"), py::arg("num_experts"), py::arg("topk_idx"), py::arg("dest_row"), py::arg("weights"), py::arg("src_off"), py::arg("ready_off"),
+        py::arg("ready_epoch"), py::arg("out"), py::arg("dot_with"), py::arg("dot_out"), py::arg("hidden"), py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"),
+        py::arg("epoch_dev_ptr"), py::arg("signal") = false);
   m.def("wait_counters", [](int64_t counter_ptr, torch::Tensor target, const StatusPy& st, uint64_t timeout_ns) {
     cu_check(launch_wait_counters(reinterpret_cast<const unsigned long long*>(counter_ptr), reinterpret_cast<const unsigned long long*>(target.data_ptr()),
                                   static_cast<int>(target.numel()), st.d, timeout_ns, stream_now()), "wait_counters");

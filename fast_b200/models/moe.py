@@ -148,8 +148,7 @@ class MoELayer(nn.Module):
         return self._gout
 
     def _infer(self, x: torch.Tensor) -> torch.Tensor:
-        logits = (x @ self.gate.t()).float()
-        rs = self.engine.route(logits, self.router_bias)
+        rs = self.engine.route_gate(x, self.gate, self.router_bias)
         self.last_route = rs
         self.engine.dispatch(x, rs)
         self.engine.experts_forward(self.w13, self.w2, rs)
@@ -172,15 +171,14 @@ class MoELayer(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """x: [tokens, hidden] bf16 -> [tokens, hidden] bf16."""
+        if not (torch.is_grad_enabled() and self.training):
+            with torch.no_grad():
+                return self._infer(x)
         logits = (x @ self.gate.t()).float()
         rs = self.engine.route(logits.detach(), self.router_bias)
         self.last_route = rs
-        if torch.is_grad_enabled() and self.training:
-            w = torch.softmax(logits.gather(1, rs.topk_idx.long()), dim=-1)
-            return _MoEFunction.apply(x, w, self.w13, self.w2, self.engine, rs)
-        self.engine.dispatch(x, rs)
-        self.engine.experts_forward(self.w13, self.w2, rs)
-        return self.engine.combine(rs, rs.topk_w)
+        w = torch.softmax(logits.gather(1, rs.topk_idx.long()), dim=-1)
+        return _MoEFunction.apply(x, w, self.w13, self.w2, self.engine, rs)
 
 
 class MixtralBlockModel(nn.Module):

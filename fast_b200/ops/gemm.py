@@ -97,13 +97,16 @@ class TokScratch:
         self.ctas = torch.cuda.get_device_properties(device).multi_processor_count
         self.counters = torch.zeros(2, self.ctas * runtime.ext().TOK_COUNTERS_PER_CTA, dtype=torch.int32, device=device)
         self.parity = 0
+        # True while weights and group tables are older than the kernel that a launch follows in the stream (an engine whose routing
+        # lies behind its dispatch): the launch may then start on them before that kernel has ended.
+        self.early = False
 
 
 _plans: dict = {}
 
 
 def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
-             granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch]) -> None:
+             granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch], most_rows: int = 0) -> None:
     key = (mode, epi, granule, BAND_ROWS, w.data_ptr(), w.shape, x.data_ptr(), x.shape, x.stride(0), out.data_ptr(), out.stride(0), gu.data_ptr() if gu is not None else 0)
     plan = _plans.get(key)
     if plan is None:
@@ -112,17 +115,19 @@ def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.T
         plan = _plans[key] = runtime.ext().TokGemmPlan(mode, epi, w, x, out, gu, granule, BAND_ROWS)
     n = scratch.ctas if scratch is not None else _ctas()
     counter_ptr, target = gate or (0, None)
-    if scratch is None:
-        plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows)
-    else:
+    counters, parity, early = None, 0, False
+    if scratch is not None:
         scratch.parity ^= 1
-        plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, scratch.counters, scratch.parity)
+        counters, parity, early = scratch.counters, scratch.parity, scratch.early
+    # Where no group can have more tokens than a narrow tile holds, narrow tiles leave shared memory to the weights in flight.
+    tile_n = 64 if 0 < most_rows <= 64 else 128 if 0 < most_rows <= 128 else 256
+    plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, counters, parity, tile_n, early)
 
 
 def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, swiglu: bool = False,
                      gate_up_out: Optional[torch.Tensor] = None, timeout_s: float = 5.0, gate=None, a_scales: Optional[torch.Tensor] = None,
                      group_rows: Optional[torch.Tensor] = None, gate_tile_rows: int = 0, ctas: Optional[int] = None,
-                     live_rows: Optional[torch.Tensor] = None, granule: int = 32, scratch: Optional[TokScratch] = None) -> torch.Tensor:
+                     live_rows: Optional[torch.Tensor] = None, granule: int = 32, scratch: Optional[TokScratch] = None, most_rows: int = 0) -> torch.Tensor:
     """out[rows of g] = a[rows of g] @ w[g].T  (a [R, K], w [G, N, K], out [R, N]).
 
     With ``swiglu`` the N columns of every 256-wide tile are [128 gate | 128 up] of the same 128
@@ -138,14 +143,15 @@ def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, 
     per group) makes that path treat the rows between a group's real and padded end as zeros.
 
     ``live_rows`` (int32[G], real rows per group; CTA-pair kernels, bf16 ``a``): only these rows, up to a multiple of
-    ``granule`` (32 or 64), are computed and written. ``scratch``: see ``TokScratch``.
+    ``granule`` (32 or 64), are computed and written. ``scratch``: see ``TokScratch``. ``most_rows`` > 0: no group has more real
+    rows than this (a hint that sizes the tiles; the result does not depend on it).
     """
     G, N, K = w.shape
     assert a.shape[1] == K and K % _BK == 0 and N % _BN == 0 and a.shape[0] % _BM == 0
     assert out.shape[0] == a.shape[0] and out.shape[1] == (N // 2 if swiglu else N)
     if USE_PAIR and a.dtype == torch.bfloat16:
         assert a_scales is None
-        _tok_run(FORWARD, SWIGLU if swiglu else STORE, w, a, out, gate_up_out, group_off, live_rows, granule, timeout_s, ctas, gate, gate_tile_rows, scratch)
+        _tok_run(FORWARD, SWIGLU if swiglu else STORE, w, a, out, gate_up_out, group_off, live_rows, granule, timeout_s, ctas, gate, gate_tile_rows, scratch, most_rows)
         return out
     C = runtime.ext()
     map_b = _tmap(w.view(G * N, K), 128 if USE_PAIR else _BN)
@@ -163,19 +169,19 @@ def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, 
 
 def grouped_gemm_dgrad(dy: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, timeout_s: float = 5.0, gate=None,
                        swiglu_bwd_of: Optional[torch.Tensor] = None, live_rows: Optional[torch.Tensor] = None, granule: int = 64,
-                       scratch: Optional[TokScratch] = None) -> torch.Tensor:
+                       scratch: Optional[TokScratch] = None, most_rows: int = 0) -> torch.Tensor:
     """out[rows of g] = dy[rows of g] @ w[g]  (dy [R, N], w [G, N, K], out [R, K]).
 
     With ``swiglu_bwd_of`` (the saved gate|up tiles [R, 2K]) the product is taken as d(act) and the
     epilogue writes d(gate|up) [R, 2K] into ``out`` instead (CTA-pair kernel only): the SwiGLU
-    backward costs no extra pass over memory. ``live_rows``, ``granule``, ``scratch``: as in ``grouped_gemm_fwd``.
+    backward costs no extra pass over memory. ``live_rows``, ``granule``, ``scratch``, ``most_rows``: as in ``grouped_gemm_fwd``.
     """
     G, N, K = w.shape
     assert dy.shape[1] == N and N % _BK == 0 and K % _BN == 0 and dy.shape[0] % _BM == 0
     if swiglu_bwd_of is not None:
         assert USE_PAIR and out.shape[1] == 2 * K and swiglu_bwd_of.shape == out.shape
     if USE_PAIR:
-        _tok_run(DGRAD, SWIGLU_BWD if swiglu_bwd_of is not None else STORE, w, dy, out, swiglu_bwd_of, group_off, live_rows, granule, timeout_s, None, gate, 0, scratch)
+        _tok_run(DGRAD, SWIGLU_BWD if swiglu_bwd_of is not None else STORE, w, dy, out, swiglu_bwd_of, group_off, live_rows, granule, timeout_s, None, gate, 0, scratch, most_rows)
         return out
     C = runtime.ext()
     C.grouped_gemm(DGRAD, STORE, _tmap(dy, _BM), _tmap(w.view(G * N, K), _BK), group_off, K // _BN, 0, N, N, 0, out, None, _st().ptr(),

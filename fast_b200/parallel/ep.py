@@ -140,6 +140,13 @@ class ExpertParallel:
         self.traffic = torch.zeros(W, W, **i32)
         self.epoch = 0
         self.epoch_dev = torch.zeros(1, dtype=torch.int64, device=dev)
+        channels = 2 if training else 1
+        self.splits = C.SplitsPlan(comm.heap, self._off(self.counts), self._flag_off(0), self.block_cnt, self.block_base, self.send_base, self.send_cnt, self.group_off,
+                                   self.group_rows, self.arrive_target[:channels], self.traffic, channels, gemm.row_align(), self.cap, comm.status, comm.timeout_ns,
+                                   self.send_pos if overlap_dispatch else None, self.epoch_dev.data_ptr() if graph_mode else 0, self.tile_target, self.tile_rows,
+                                   torch.zeros(1, **i32))
+        # One rank alone: nothing crosses a wire, so the fp8 dispatch stores the bf16 values that a receiver would make of its rows.
+        self.local_bf16 = fp8_dispatch and W == 1 and not self.fp8_direct and not overlap_dispatch
         if graph_mode:
             self._static_route = (torch.empty(max_tokens, top_k, **i32), torch.empty(max_tokens, top_k, dtype=torch.float32, device=dev),
                                   torch.empty(max_tokens, top_k, **i32))
@@ -180,33 +187,48 @@ class ExpertParallel:
         return self.training or not gemm.USE_PAIR
 
     def _live(self, rs: RouteState) -> dict:
-        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch) if self.scratch is not None else {}
+        if self.scratch is None:
+            return {}
+        self.scratch.early = rs.topk_idx.shape[0] > 0   # without tokens there is no dispatch kernel between routing and GEMM
+        # a token picks an expert at most once; other ranks may have up to max_tokens of them
+        most = rs.topk_idx.shape[0] if self.comm.world == 1 else self.T * self.comm.world
+        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch, most_rows=most)
 
     def traffic_matrix(self) -> torch.Tensor:
         """Token traffic matrix [src, dst] of the last routed step (device tensor)."""
         return self.traffic
 
     # ---- forward ---------------------------------------------------------------------------------
-    def route(self, logits: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
-        C = self._C
-        T = logits.shape[0]
-        assert T <= self.T and logits.shape[1] == self.E and logits.dtype == torch.float32
+    def _route_outputs(self, T: int, device):
         if self.graph_mode:
-            topk_idx, topk_w, dest_row = (t[:T] for t in self._static_route)
-        else:
-            topk_idx = torch.empty(T, self.K, dtype=torch.int32, device=logits.device)
-            topk_w = torch.empty(T, self.K, dtype=torch.float32, device=logits.device)
-            dest_row = torch.empty(T, self.K, dtype=torch.int32, device=logits.device)
-        nb = (T + C.ROUTE_TOKENS_PER_BLOCK - 1) // C.ROUTE_TOKENS_PER_BLOCK
-        C.route_topk(logits.contiguous(), bias, self.K, topk_idx, topk_w, self.slot_in_block, self.block_cnt[:nb])
-        self.epoch += 1
-        ed = self.epoch_dev.data_ptr() if self.graph_mode else 0
-        C.splits_scan(self.comm.heap, self._off(self.counts), self._flag_off(0), self.epoch, self.block_cnt[:nb], self.block_base[:nb], self.send_base,
-                      self.send_cnt, self.group_off, self.group_rows, self.arrive_target[: 2 if self.training else 1], self.traffic, 2 if self.training else 1,
-                      gemm.row_align(), self.cap, self.status,
-                      self.timeout_ns, self.send_pos if self.overlap else None, ed, self.tile_target, self.tile_rows)
+            return tuple(t[:T] for t in self._static_route)
+        return (torch.empty(T, self.K, dtype=torch.int32, device=device), torch.empty(T, self.K, dtype=torch.float32, device=device),
+                torch.empty(T, self.K, dtype=torch.int32, device=device))
+
+    def _route_state(self, topk_idx, topk_w, dest_row) -> RouteState:
         return RouteState(topk_idx, topk_w, dest_row, self.slot_in_block, self.block_base, self.send_base, self.group_off, self.group_rows,
                           0 if self.graph_mode else self.epoch)
+
+    def route(self, logits: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
+        T = logits.shape[0]
+        assert T <= self.T and logits.shape[1] == self.E and logits.dtype == torch.float32
+        topk_idx, topk_w, dest_row = self._route_outputs(T, logits.device)
+        self.epoch += 1
+        self._C.route_splits(self.splits, logits.contiguous(), bias, self.K, topk_idx, topk_w, self.slot_in_block, self.epoch)
+        return self._route_state(topk_idx, topk_w, dest_row)
+
+    def route_gate(self, x: torch.Tensor, gate: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
+        """Route on the router logits ``x @ gate.T`` (bf16, as a GEMM returns them). For a few tokens the logits are made in the
+        routing kernel itself: one block per token, each reading the whole gate, so up to a block's worth of tokens and
+        64 MiB of such reads; beyond that a GEMM reads the gate less often than it costs a launch."""
+        T = x.shape[0]
+        if (1 <= T <= self._C.ROUTE_TOKENS_PER_BLOCK and 2 * T * self.E * self.H <= 64 << 20 and self.E <= 256 and x.dtype == gate.dtype == torch.bfloat16
+                and x.is_contiguous() and gate.is_contiguous() and T <= self.T):
+            topk_idx, topk_w, dest_row = self._route_outputs(T, x.device)
+            self.epoch += 1
+            self._C.gate_route(self.splits, x, gate, bias, self.K, topk_idx, topk_w, self.slot_in_block, self.epoch)
+            return self._route_state(topk_idx, topk_w, dest_row)
+        return self.route((x @ gate.t()).float(), bias)
 
     def can_fuse_gate(self) -> bool:
         """Whether ``route_fused`` (RMSNorm + router logits + top-k in one kernel) covers this layer."""
@@ -226,13 +248,9 @@ class ExpertParallel:
         hn = torch.empty_like(h)
         rstd = torch.empty(T, dtype=torch.float32, device=dev)
         logits = torch.empty(T, self.E, dtype=torch.float32, device=dev)
-        nb = (T + C.ROUTE_TOKENS_PER_BLOCK - 1) // C.ROUTE_TOKENS_PER_BLOCK
-        C.norm_gate_route(h, norm_w, gate, bias, self.K, eps, hn, rstd, logits, topk_idx, topk_w, self.slot_in_block, self.block_cnt[:nb])
         self.epoch += 1
-        C.splits_scan(self.comm.heap, self._off(self.counts), self._flag_off(0), self.epoch, self.block_cnt[:nb], self.block_base[:nb], self.send_base,
-                      self.send_cnt, self.group_off, self.group_rows, self.arrive_target[: 2 if self.training else 1], self.traffic, 2 if self.training else 1,
-                      gemm.row_align(), self.cap, self.status, self.timeout_ns, self.send_pos if self.overlap else None, 0, self.tile_target, self.tile_rows)
-        rs = RouteState(topk_idx, topk_w, dest_row, self.slot_in_block, self.block_base, self.send_base, self.group_off, self.group_rows, self.epoch)
+        C.norm_gate_route(h, norm_w, gate, bias, self.K, eps, hn, rstd, logits, topk_idx, topk_w, self.slot_in_block, self.block_cnt, self.splits, self.epoch)
+        rs = self._route_state(topk_idx, topk_w, dest_row)
         return rs, hn, rstd, logits
 
     def dispatch(self, x: torch.Tensor, rs: RouteState) -> None:
@@ -264,7 +282,8 @@ class ExpertParallel:
             if self.fp8:
                 C.dispatch_push(self.comm.heap, x, rs.topk_idx, None, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, True, True,
                                 self._off(self.xq_recv), self._off(self.xs_recv), self.arrive._symm_off, 0, 0, self.status, self.timeout_ns,
-                                4 * self.overlap_reserve_sms if self.overlap else self.comm_ctas, send_list, self.tile_rows, self.ntiles, xq, xs)
+                                4 * self.overlap_reserve_sms if self.overlap else self.comm_ctas, send_list, self.tile_rows, self.ntiles, xq, xs,
+                                self.x_recv if self.local_bf16 else None)
             else:
                 C.dispatch_push(self.comm.heap, x, rs.topk_idx, None, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, True, False,
                                 self._off(self.x_recv), 0, self.arrive._symm_off, 0, 0, self.status, self.timeout_ns,
@@ -283,7 +302,9 @@ class ExpertParallel:
 
     def experts_forward(self, w13: torch.Tensor, w2: torch.Tensor, rs: RouteState) -> None:
         C = self._C
-        if self.tile_rows:   # forward-only layer: the producer of the first GEMM waits tile by tile
+        if self.comm.world == 1 and not self.overlap:   # alone, every row is in once the dispatch kernel is over
+            gate, gate_tile = None, 0
+        elif self.tile_rows:   # forward-only layer: the producer of the first GEMM waits tile by tile
             gate, gate_tile = (self._arrive_ptr(0), self.tile_target[0]), self.tile_rows
         else:
             gate, gate_tile = (self._arrive_ptr(0), self.arrive_target[0]), 0
@@ -294,8 +315,9 @@ class ExpertParallel:
                                   gate_tile_rows=gate_tile, ctas=self.gemm1_ctas)
         else:
             if self.fp8:
-                C.wait_counters(self._arrive_ptr(0), self.tile_target[0] if self.tile_rows else self.arrive_target[0], self.status, self.timeout_ns)
-                C.dequant_fp8(self.xq_recv, self.xs_recv, self.x_recv, rs.group_off.data_ptr() + 4 * self.El)
+                if not self.local_bf16:
+                    C.wait_counters(self._arrive_ptr(0), self.tile_target[0] if self.tile_rows else self.arrive_target[0], self.status, self.timeout_ns)
+                    C.dequant_fp8(self.xq_recv, self.xs_recv, self.x_recv, rs.group_off.data_ptr() + 4 * self.El)
                 if self._needs_zero_pads():
                     C.zero_pad_rows(self.x_recv, rs.group_off, rs.group_rows, self.pad_align)
                 gate = None
@@ -304,14 +326,13 @@ class ExpertParallel:
                                   gate_tile_rows=gate_tile, ctas=self.gemm1_ctas if gate is not None else None, **self._live(rs))
         gemm.grouped_gemm_fwd(self.act, w2, rs.group_off, self.y, **self._live(rs))
         self._join_dispatch()
-        C.peer_signal(self.comm.heap, self._flag_off(1), rs.epoch, self.epoch_dev.data_ptr() if self.graph_mode else 0)
 
     def combine(self, rs: RouteState, weights: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         T = rs.topk_idx.shape[0]
         if out is None:
             out = torch.empty(T, self.H, dtype=torch.bfloat16, device=rs.topk_idx.device)
         self._C.combine_pull(self.comm.heap, self.E, rs.topk_idx, rs.dest_row, weights, self._off(self.y), self._flag_off(1), rs.epoch, out, None, None,
-                             self.H, self.status, self.timeout_ns, self.comm_ctas, self.epoch_dev.data_ptr() if self.graph_mode else 0)
+                             self.H, self.status, self.timeout_ns, self.comm_ctas, self.epoch_dev.data_ptr() if self.graph_mode else 0, True)
         return out
 
     def forward(self, x: torch.Tensor, logits: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -357,7 +378,7 @@ class ExpertParallel:
         C.dispatch_push(self.comm.heap, grad_out, rs.topk_idx, weights, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, False, False,
                         self._off(self.dy_recv), 0, self.arrive._symm_off + self.El * 8, self._flag_off(2), rs.epoch, self.status, self.timeout_ns,
                         self.comm_ctas, None)
-        gate = (self._arrive_ptr(1), self.arrive_target[1])
+        gate = (self._arrive_ptr(1), self.arrive_target[1]) if self.comm.world > 1 else None
         if gemm.USE_PAIR:  # d(act) never leaves the tensor memory: the dgrad epilogue applies the SwiGLU backward
             gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dgu, gate=gate, swiglu_bwd_of=self.gu, **self._live(rs))
         else:
@@ -370,9 +391,8 @@ class ExpertParallel:
             C.swiglu_bwd(self.gu, self.dact, self.dgu, rs.group_off.data_ptr() + 4 * self.El)
         gemm.grouped_gemm_dgrad(self.dgu, w13, rs.group_off, self.dx_recv, **self._live(rs))
         gemm.grouped_gemm_wgrad(self.dgu, self.x_recv, rs.group_off, dw13, live_rows=live)
-        C.peer_signal(self.comm.heap, self._flag_off(3), rs.epoch, 0)
         grad_x = torch.empty(T, self.H, dtype=torch.bfloat16, device=dev)
         # Transposed dispatch: every token pulls and sums the gradients of its k rows.
         C.combine_pull(self.comm.heap, self.E, rs.topk_idx, rs.dest_row, None, self._off(self.dx_recv), self._flag_off(3), rs.epoch, grad_x, None, None,
-                       self.H, self.status, self.timeout_ns, self.comm_ctas, 0)
+                       self.H, self.status, self.timeout_ns, self.comm_ctas, 0, True)
         return grad_x, grad_w

@@ -297,6 +297,40 @@ def test_moe_forward_single_rank(E, K, H, I, T, fp8, overlap):
     assert int(tm.sum().item()) == T * K
 
 
+@pytest.mark.parametrize("E,K,H,I,T,fp8", [(8, 2, 512, 384, 1, False), (5, 3, 768, 256, 7, False), (32, 8, 256, 128, 128, False), (256, 8, 256, 128, 33, False),
+                                            (8, 2, 512, 384, 64, True), (8, 2, 512, 384, 129, False), (40, 4, 7168, 256, 2, True)])
+def test_forward_layer_of_few_tokens(E, K, H, I, T, fp8):
+    """The routes a decode step takes: logits, choice, ranks and split scan in one kernel (up to 128 tokens), rows shared by
+    the warps of a block, narrow GEMM tiles with cut reductions. Three steps in a row on other tokens; the routing tables
+    agree with each other and the output with fp32."""
+    from fast_b200.models import MoELayer
+    from fast_b200.parallel import Communicator
+
+    comm = Communicator(heap_bytes=256 << 20, device=0)
+    layer = MoELayer(comm, H, I, E, K, max_tokens=max(T, 200), fp8_dispatch=fp8, router_bias=True, training=False).eval()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    layer.router_bias.data.copy_(torch.randn(E, generator=g, device="cuda") * 0.5)
+    for n in (T, max(1, T - 1), T):
+        x = torch.randn(n, H, generator=g, device="cuda").to(torch.bfloat16)
+        with torch.no_grad():
+            y = layer(x)
+        comm.check()
+        rs, eng = layer.last_route, layer.engine
+        idx = rs.topk_idx.long()
+        want, _, w = _ref_forward(x, layer.gate, layer.w13, layer.w2, K, idx=idx)
+        assert _rel(y, want) < (8e-2 if fp8 else 2e-2)
+        sel = (x @ layer.gate.t()).float() + layer.router_bias
+        top = sel.topk(K, dim=-1)
+        assert bool((sel.gather(1, idx) >= top.values[:, -1:] - 2e-2).all()) and all(len(set(r)) == K for r in idx.tolist())
+        assert torch.allclose(rs.topk_w, w, atol=2e-2)
+        counts = torch.bincount(idx.reshape(-1), minlength=E)
+        assert torch.equal(rs.group_rows.long(), counts) and int(eng.traffic_matrix()[0, 0]) == n * K
+        off = torch.cat([torch.zeros(1, dtype=torch.long, device="cuda"), torch.cumsum((counts + 255) // 256 * 256, 0)])
+        assert torch.equal(rs.group_off.long(), off)
+        rows = rs.dest_row.long()
+        assert bool(((rows >= off[idx]) & (rows < off[idx] + counts[idx])).all()) and rows.unique().numel() == n * K
+
+
 def test_forward_layer_in_cuda_graph():
     """The forward-only layer captured in a CUDA graph replays correctly on new inputs (the step's
     epoch lives in device memory, so a replay is a new step)."""
