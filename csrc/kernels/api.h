@@ -337,8 +337,21 @@ cudaError_t launch_embedding_bwd(const long long* sorted_ids, const long long* p
 cudaError_t launch_embedding_index(const long long* ids, long long T, int V, int* hist, int* rank_in_block, int* total, int* start, long long* sorted_ids,
                                    long long* perm, cudaStream_t stream);
 int embedding_index_block();
-// AdamW on bf16 parameters with fp32 master weights and moments.
-cudaError_t launch_adamw(__nv_bfloat16* param, float* master, float* m, float* v, const __nv_bfloat16* grad, long long n, float lr, float beta1,
-                         float beta2, float eps, float weight_decay, float bias_c1, float bias_c2, float grad_scale, cudaStream_t stream);
+// AdamW on bf16 parameters with fp32 master weights and moments, several tensors per launch.
+struct AdamWTensor {
+  __nv_bfloat16* param;
+  float *master, *m, *v;
+  const __nv_bfloat16* grad;
+  long long n;               // multiple of 8
+  float c1, c2;              // bias corrections 1 / (1 - beta^step)
+  unsigned int blocks;       // set by the launcher
+};
+constexpr int kAdamWTensors = 16;
+struct AdamWArgs {
+  AdamWTensor t[kAdamWTensors];
+  int count;
+  float lr, b1, b2, eps, wd, gscale;
+};
+cudaError_t launch_adamw(AdamWArgs args, cudaStream_t stream);
 
 }  // namespace fastb

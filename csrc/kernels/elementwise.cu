@@ -84,47 +84,53 @@ __global__ void dequant_fp8_kernel(const uint2* __restrict__ q, const float* __r
   }
 }
 
-// One thread owns groups of 4 consecutive parameters: its fp32 accesses are 16 bytes, contiguous across the warp
-// (512 bytes per instruction), its bf16 accesses 8 bytes. Two groups are in flight per iteration. Nothing is read
-// twice, so every access is marked streaming (evict first).
-__global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ master, float4* __restrict__ m, float4* __restrict__ v,
-                             const uint2* __restrict__ grad, long long n4, float lr, float b1, float b2, float eps, float wd, float c1, float c2,
-                             float gscale) {
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  constexpr int U = 2;
-  for (long long i0 = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i0 < n4; i0 += U * stride) {
-    float4 w[U], mm[U], vv[U];
-    uint2 g[U];
+// A block takes kAdamChunk consecutive parameters of one tensor, four of them a thread at a time: fp32 accesses are 16 bytes,
+// contiguous across the warp, bf16 accesses 8 bytes. Nothing is read twice, so every access is marked streaming. Bound by
+// HBM (28 bytes a parameter): one short block per chunk, as many as there are, keeps the seven streams of all resident
+// blocks within a narrow moving window: 6.9 TB/s over 0.94 G parameters. A grid of resident blocks that strides through
+// the same arrays reaches 6.1, bulk copies through shared memory 6.4. All tensors of an optimizer step are one launch.
+constexpr int kAdamThreads = 256, kAdamPerThread = 2, kAdamChunk = 4 * kAdamThreads * kAdamPerThread;
+__global__ void __launch_bounds__(kAdamThreads) adamw_kernel(const __grid_constant__ AdamWArgs a) {
+  int k = 0;
+  unsigned int block = blockIdx.x;
+  while (block >= a.t[k].blocks) block -= a.t[k++].blocks;
+  const AdamWTensor& t = a.t[k];
+  const long long n4 = t.n / 4, base = static_cast<long long>(block) * (kAdamChunk / 4) + threadIdx.x;
+  uint2* param = reinterpret_cast<uint2*>(t.param);
+  float4 *master = reinterpret_cast<float4*>(t.master), *m = reinterpret_cast<float4*>(t.m), *v = reinterpret_cast<float4*>(t.v);
+  const uint2* grad = reinterpret_cast<const uint2*>(t.grad);
+  constexpr int U = kAdamPerThread;
+  float4 w[U], mm[U], vv[U];
+  uint2 g[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long i = i0 + u * stride;
-      if (i < n4) { g[u] = __ldcs(grad + i); w[u] = __ldcs(master + i); mm[u] = __ldcs(m + i); vv[u] = __ldcs(v + i); }
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + u * kAdamThreads;
+    if (i < n4) { g[u] = __ldcs(grad + i); w[u] = __ldcs(master + i); mm[u] = __ldcs(m + i); vv[u] = __ldcs(v + i); }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + u * kAdamThreads;
+    if (i >= n4) break;
+    const float2 g01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g[u].x));
+    const float2 g23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g[u].y));
+    const float gk[4] = {g01.x * a.gscale, g01.y * a.gscale, g23.x * a.gscale, g23.y * a.gscale};
+    float* wp = reinterpret_cast<float*>(&w[u]);
+    float* mp = reinterpret_cast<float*>(&mm[u]);
+    float* vp = reinterpret_cast<float*>(&vv[u]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      mp[q] = a.b1 * mp[q] + (1.0f - a.b1) * gk[q];
+      vp[q] = a.b2 * vp[q] + (1.0f - a.b2) * gk[q] * gk[q];
+      const float upd = (mp[q] * t.c1) / (sqrtf(vp[q] * t.c2) + a.eps);
+      wp[q] = wp[q] - a.lr * (upd + a.wd * wp[q]);
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long i = i0 + u * stride;
-      if (i >= n4) break;
-      const float2 g01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g[u].x));
-      const float2 g23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g[u].y));
-      const float gk[4] = {g01.x * gscale, g01.y * gscale, g23.x * gscale, g23.y * gscale};
-      float* wp = reinterpret_cast<float*>(&w[u]);
-      float* mp = reinterpret_cast<float*>(&mm[u]);
-      float* vp = reinterpret_cast<float*>(&vv[u]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        mp[k] = b1 * mp[k] + (1.0f - b1) * gk[k];
-        vp[k] = b2 * vp[k] + (1.0f - b2) * gk[k] * gk[k];
-        const float upd = (mp[k] * c1) / (sqrtf(vp[k] * c2) + eps);
-        wp[k] = wp[k] - lr * (upd + wd * wp[k]);
-      }
-      __stcs(master + i, w[u]);
-      __stcs(m + i, mm[u]);
-      __stcs(v + i, vv[u]);
-      uint2 pb;
-      *reinterpret_cast<__nv_bfloat162*>(&pb.x) = __floats2bfloat162_rn(wp[0], wp[1]);
-      *reinterpret_cast<__nv_bfloat162*>(&pb.y) = __floats2bfloat162_rn(wp[2], wp[3]);
-      __stcs(param + i, pb);
-    }
+    __stcs(master + i, w[u]);
+    __stcs(m + i, mm[u]);
+    __stcs(v + i, vv[u]);
+    uint2 pb;
+    *reinterpret_cast<__nv_bfloat162*>(&pb.x) = __floats2bfloat162_rn(wp[0], wp[1]);
+    *reinterpret_cast<__nv_bfloat162*>(&pb.y) = __floats2bfloat162_rn(wp[2], wp[3]);
+    __stcs(param + i, pb);
   }
 }
 
@@ -365,13 +371,18 @@ cudaError_t launch_dequant_fp8(const unsigned char* q, const float* scales, __nv
   note_launch();
   return cudaGetLastError();
 }
-cudaError_t launch_adamw(__nv_bfloat16* param, float* master, float* m, float* v, const __nv_bfloat16* grad, long long n, float lr, float beta1,
-                         float beta2, float eps, float weight_decay, float bias_c1, float bias_c2, float grad_scale, cudaStream_t stream) {
-  if (n % 8) return cudaErrorInvalidValue;
-  if (n == 0) return cudaSuccess;
-  adamw_kernel<<<grid_for(n / 8), 256, 0, stream>>>(reinterpret_cast<uint2*>(param), reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m),
-                                                    reinterpret_cast<float4*>(v), reinterpret_cast<const uint2*>(grad), n / 4, lr, beta1, beta2, eps,
-                                                    weight_decay, bias_c1, bias_c2, grad_scale);
+cudaError_t launch_adamw(AdamWArgs args, cudaStream_t stream) {
+  if (args.count < 0 || args.count > kAdamWTensors) return cudaErrorInvalidValue;
+  long long blocks = 0;
+  for (int k = 0; k < args.count; ++k) {
+    AdamWTensor& t = args.t[k];
+    if (t.n < 0 || t.n % 8) return cudaErrorInvalidValue;
+    t.blocks = static_cast<unsigned int>((t.n + kAdamChunk - 1) / kAdamChunk);
+    blocks += t.blocks;
+  }
+  if (blocks == 0) return cudaSuccess;
+  if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
+  adamw_kernel<<<static_cast<unsigned>(blocks), kAdamThreads, 0, stream>>>(args);
   note_launch();
   return cudaGetLastError();
 }

@@ -498,14 +498,31 @@ void bind_moe(py::module_& m) {
              "embedding_index");
     return std::make_tuple(sorted_ids, perm);
   });
-  m.def("adamw", [](torch::Tensor param, torch::Tensor master, torch::Tensor m1, torch::Tensor v, torch::Tensor grad, double lr, double b1, double b2,
-                    double eps, double wd, int64_t step, double grad_scale) {
-    want(param, torch::kBFloat16, "param"); want(master, torch::kFloat32, "master"); want(m1, torch::kFloat32, "m"); want(v, torch::kFloat32, "v");
-    want(grad, torch::kBFloat16, "grad");
-    const double c1 = 1.0 / (1.0 - std::pow(b1, static_cast<double>(step))), c2 = 1.0 / (1.0 - std::pow(b2, static_cast<double>(step)));
-    cu_check(launch_adamw(reinterpret_cast<__nv_bfloat16*>(param.data_ptr()), master.data_ptr<float>(), m1.data_ptr<float>(), v.data_ptr<float>(),
-                          reinterpret_cast<const __nv_bfloat16*>(grad.data_ptr()), param.numel(), static_cast<float>(lr), static_cast<float>(b1),
-                          static_cast<float>(b2), static_cast<float>(eps), static_cast<float>(wd), static_cast<float>(c1), static_cast<float>(c2),
-                          static_cast<float>(grad_scale), stream_now()), "adamw");
-  });
+  // One step of several tensors: lists of equal length, steps[k] = the step number that tensor k takes now.
+  const auto adamw_step = [](const std::vector<torch::Tensor>& params, const std::vector<torch::Tensor>& masters, const std::vector<torch::Tensor>& ms, const std::vector<torch::Tensor>& vs,
+                    const std::vector<torch::Tensor>& grads, const std::vector<int64_t>& steps, double lr, double b1, double b2, double eps, double wd, double grad_scale) {
+    const size_t n = params.size();
+    TORCH_CHECK(masters.size() == n && ms.size() == n && vs.size() == n && grads.size() == n && steps.size() == n, "adamw: lists of equal length");
+    for (size_t k0 = 0; k0 < n; k0 += kAdamWTensors) {
+      AdamWArgs a{};
+      a.lr = static_cast<float>(lr); a.b1 = static_cast<float>(b1); a.b2 = static_cast<float>(b2); a.eps = static_cast<float>(eps); a.wd = static_cast<float>(wd);
+      a.gscale = static_cast<float>(grad_scale);
+      for (size_t k = k0; k < std::min(n, k0 + kAdamWTensors); ++k) {
+        want(params[k], torch::kBFloat16, "param"); want(masters[k], torch::kFloat32, "master"); want(ms[k], torch::kFloat32, "m"); want(vs[k], torch::kFloat32, "v");
+        want(grads[k], torch::kBFloat16, "grad");
+        const int64_t len = params[k].numel();
+        TORCH_CHECK(masters[k].numel() == len && ms[k].numel() == len && vs[k].numel() == len && grads[k].numel() == len, "adamw: sizes");
+        AdamWTensor& t = a.t[a.count++];
+        t.param = reinterpret_cast<__nv_bfloat16*>(params[k].data_ptr());
+        t.master = masters[k].data_ptr<float>(); t.m = ms[k].data_ptr<float>(); t.v = vs[k].data_ptr<float>();
+        t.grad = reinterpret_cast<const __nv_bfloat16*>(grads[k].data_ptr());
+        t.n = len;
+        t.c1 = static_cast<float>(1.0 / (1.0 - std::pow(b1, static_cast<double>(steps[k])))); t.c2 = static_cast<float>(1.0 / (1.0 - std::pow(b2, static_cast<double>(steps[k]))));
+      }
+      cu_check(launch_adamw(a, stream_now()), "adamw");
+    }
+  };
+  m.def("adamw_step", adamw_step);
+  m.def("adamw", [adamw_step](torch::Tensor param, torch::Tensor master, torch::Tensor m1, torch::Tensor v, torch::Tensor grad, double lr, double b1, double b2, double eps, double wd,
+                              int64_t step, double grad_scale) { adamw_step({param}, {master}, {m1}, {v}, {grad}, {step}, lr, b1, b2, eps, wd, grad_scale); });
 }

@@ -1,4 +1,4 @@
-"""AdamW for bf16 parameters with fp32 master weights and moments, one fused kernel per tensor."""
+"""AdamW for bf16 parameters with fp32 master weights and moments, one fused kernel per step."""
 from __future__ import annotations
 
 from typing import Optional
@@ -35,23 +35,27 @@ class FusedAdamW:
             elif p.grad is not None:
                 p.grad.zero_()
 
+    def _update(self, params, grads, grad_scale: float) -> None:
+        state = [self.state[p] for p in params]
+        for p in params:
+            self.steps[p] += 1
+        runtime.ext().adamw_step([p.data for p in params], [s[0] for s in state], [s[1] for s in state], [s[2] for s in state],
+                            [g.to(torch.bfloat16).contiguous() for g in grads], [self.steps[p] for p in params], self.lr, self.betas[0], self.betas[1], self.eps, self.wd,
+                            grad_scale)
+
     @torch.no_grad()
     def step_param(self, p, grad: torch.Tensor, grad_scale: float = 1.0, stream: Optional[torch.cuda.Stream] = None, early: bool = False):
-        master, m, v = self.state[p]
-        self.steps[p] += 1
-        g = grad if grad.dtype == torch.bfloat16 else grad.to(torch.bfloat16)
         if stream is None:
-            runtime.ext().adamw(p.data, master, m, v, g.contiguous(), self.lr, self.betas[0], self.betas[1], self.eps, self.wd, self.steps[p], grad_scale)
+            self._update([p], [grad], grad_scale)
         else:
             with torch.cuda.stream(stream):
-                runtime.ext().adamw(p.data, master, m, v, g.contiguous(), self.lr, self.betas[0], self.betas[1], self.eps, self.wd, self.steps[p], grad_scale)
+                self._update([p], [grad], grad_scale)
         if early:
             self._stepped_early.add(p)
 
     @torch.no_grad()
     def step(self, grad_scale: float = 1.0):
-        for p in self.params:
-            if p in self._stepped_early or p.grad is None:
-                continue
-            self.step_param(p, p.grad, grad_scale)
+        due = [p for p in self.params if p not in self._stepped_early and p.grad is not None]
+        if due:
+            self._update(due, [p.grad for p in due], grad_scale)
         self._stepped_early.clear()

@@ -212,6 +212,27 @@ def test_elementwise_kernels():
     assert torch.equal(pb, master.to(torch.bfloat16))
 
 
+def test_adamw_of_several_tensors_is_the_single_update():
+    """One launch over tensors of all kinds of lengths (less than a block's chunk, its multiples, one past; more tensors than one
+    launch takes; different step numbers) gives the bits of one call per tensor."""
+    from fast_b200 import runtime
+
+    C = runtime.ext()
+    g = torch.Generator(device="cuda").manual_seed(4)
+    sizes = [8, 2040, 2048, 2056, 4096, 10000] * 3
+    make = lambda: [torch.randn(n, generator=g, device="cuda") for n in sizes]
+    grads = [x.to(torch.bfloat16) for x in make()]
+    masters, ms, vs = make(), make(), [x.abs() for x in make()]
+    steps = [1 + i % 5 for i in range(len(sizes))]
+    clone = lambda ts: [t.clone() for t in ts]
+    got = [[torch.empty_like(x) for x in grads], clone(masters), clone(ms), clone(vs)]
+    want = [[torch.empty_like(x) for x in grads], clone(masters), clone(ms), clone(vs)]
+    C.adamw_step(*got, grads, steps, 1e-2, 0.9, 0.95, 1e-8, 0.1, 0.5)
+    for i in range(len(sizes)):
+        C.adamw(want[0][i], want[1][i], want[2][i], want[3][i], grads[i], 1e-2, 0.9, 0.95, 1e-8, 0.1, steps[i], 0.5)
+    assert all(torch.equal(a, b) for x, y in zip(got, want) for a, b in zip(x, y))
+
+
 def test_quantise_rows_matches_a_torch_restatement():
     """Rows to e4m3 in 1 x 128 blocks: the scale is amax / 448 rounded up to a bf16 value, the bytes are
     round-to-nearest e4m3 of value / scale; value x scale comes back within e4m3's half-ulp."""
