@@ -131,13 +131,35 @@ RankProgram lower_for_rank(const Plan& p, int rank, const LowerOptions& lo) {
     c = (c + 15) / 16 * 16;
     return c;
   };
+  struct Slice { double key; size_t pc; int64_t begin, bytes; };
+  std::vector<Slice> slices;
+  auto emit = [&](const Piece& pc, int64_t begin, int64_t bytes) {
+    const Op& o = *pc.op;
+    WorkItem w{};
+    w.src_off = o.src_off * ub + pc.begin + begin;
+    w.dst_off = o.dst_off * ub + pc.begin + begin;
+    w.bytes = bytes;
+    w.dst_rank = o.dst_rank;
+    w.src_buf = static_cast<uint8_t>(o.src_buf);
+    w.dst_buf = static_cast<uint8_t>(o.dst_buf);
+    w.wait_kind = o.src_buf == Buf::kBalance ? 1 : o.src_buf == Buf::kRail ? 2 : 0;
+    w.signal_kind = o.dst_buf == Buf::kBalance ? 1 : o.dst_buf == Buf::kRail ? 2 : 3;
+    w.stage = pc.signal_slot;
+    w.wait_stage = pc.wait_slot;
+    prog.items.push_back(w);
+  };
   auto emit_interleaved = [&](const std::vector<Piece>& pcs) {
+    if (pcs.empty()) return;
+    if (pcs.size() == 1) {  // a stage of a flat plan: one transfer, its chunks in order
+      const int64_t total = pcs[0].bytes, c = chunk_of(total);
+      for (int64_t at = 0; at < total; at += c) emit(pcs[0], at, std::min(c, total - at));
+      return;
+    }
     // Proportional interleave: chunk j of a piece with c chunks gets key (j + 1/2) / c and chunks are
     // issued in key order, so every transfer of the slot advances at a rate proportional to its size
     // and all of them finish together (equal ones degenerate to plain round-robin). A heavy pair
     // is then in flight from the first chunk on instead of trailing alone at the end.
-    struct Slice { double key; size_t pc; int64_t begin, bytes; };
-    std::vector<Slice> slices;
+    slices.clear();
     for (size_t k = 0; k < pcs.size(); ++k) {
       const int64_t total = pcs[k].bytes;
       const int64_t c = chunk_of(total);
@@ -146,23 +168,15 @@ RankProgram lower_for_rank(const Plan& p, int rank, const LowerOptions& lo) {
         slices.push_back(Slice{(static_cast<double>(j) + 0.5) / static_cast<double>(pieces), k, j * c, std::min(c, total - j * c)});
     }
     std::stable_sort(slices.begin(), slices.end(), [](const Slice& x, const Slice& y) { return x.key < y.key; });
-    for (const Slice& sl : slices) {
-      const Piece& pc = pcs[sl.pc];
-      const Op& o = *pc.op;
-      WorkItem w{};
-      w.src_off = o.src_off * ub + pc.begin + sl.begin;
-      w.dst_off = o.dst_off * ub + pc.begin + sl.begin;
-      w.bytes = sl.bytes;
-      w.dst_rank = o.dst_rank;
-      w.src_buf = static_cast<uint8_t>(o.src_buf);
-      w.dst_buf = static_cast<uint8_t>(o.dst_buf);
-      w.wait_kind = o.src_buf == Buf::kBalance ? 1 : o.src_buf == Buf::kRail ? 2 : 0;
-      w.signal_kind = o.dst_buf == Buf::kBalance ? 1 : o.dst_buf == Buf::kRail ? 2 : 3;
-      w.stage = pc.signal_slot;
-      w.wait_stage = pc.wait_slot;
-      prog.items.push_back(w);
-    }
+    for (const Slice& sl : slices) emit(pcs[sl.pc], sl.begin, sl.bytes);
   };
+  {  // one allocation for the whole list
+    size_t items = 0;
+    for (const auto* slots_of : {&push_slot, &fwd_slot})
+      for (const auto& pcs : *slots_of)
+        for (const Piece& pc : pcs) { const int64_t c = chunk_of(pc.bytes); items += static_cast<size_t>((pc.bytes + c - 1) / c); }
+    prog.items.reserve(items);
+  }
   for (int s = 0; s < K + 3; ++s) {
     emit_interleaved(push_slot[s]);
     emit_interleaved(fwd_slot[s]);

@@ -1,7 +1,6 @@
 #include "plan.h"
 
 #include <algorithm>
-#include <deque>
 #include <stdexcept>
 
 namespace fastb {
@@ -13,6 +12,16 @@ struct Piece {
   int64_t pair_off, len;
   Buf buf;
   int64_t off;  // units, inside `buf` of the GPU currently holding the piece
+};
+
+// Pieces waiting at one (source server, destination server, GPU): appended at the back, taken at the front. A vector and a
+// cursor: a std::deque allocates half a kilobyte for each of the S * S * G queues, most of which hold one piece.
+struct PieceQueue {
+  std::vector<Piece> v;
+  size_t head = 0;
+  bool empty() const { return head == v.size(); }
+  Piece& front() { return v[head]; }
+  void pop_front() { ++head; }
 };
 
 // Largest cut <= want that keeps the remainder of `p` aligned inside its segment, or the whole
@@ -84,19 +93,20 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
 
   // ---- balance: equalise the per-GPU load of every (src server, dst server) tile -------------
   // hold[(s*S+t)*G+i] = pieces GPU i of server s will put on its rail toward server t.
-  std::vector<std::deque<Piece>> hold(static_cast<size_t>(S) * S * G);
-  auto hold_at = [&](int s, int t, int i) -> std::deque<Piece>& { return hold[(static_cast<size_t>(s) * S + t) * G + i]; };
+  std::vector<PieceQueue> hold(static_cast<size_t>(S) * S * G);
+  auto hold_at = [&](int s, int t, int i) -> PieceQueue& { return hold[(static_cast<size_t>(s) * S + t) * G + i]; };
 
+  std::vector<int64_t> load(G, 0);
   for (int s = 0; s < S; ++s) {
     for (int t = 0; t < S; ++t) {
       if (s == t) continue;
-      std::vector<int64_t> load(G, 0);
+      std::fill(load.begin(), load.end(), 0);
       int64_t sum = 0;
       for (int i = 0; i < G; ++i) {
         for (int j = 0; j < G; ++j) {
           const int64_t x = M.at(s * G + i, t * G + j);
           if (x == 0) continue;
-          hold_at(s, t, i).push_back(Piece{i, j, 0, x, Buf::kInput, in_at(s * G + i, t * G + j)});
+          hold_at(s, t, i).v.push_back(Piece{i, j, 0, x, Buf::kInput, in_at(s * G + i, t * G + j)});
           load[i] += x;
         }
         sum += load[i];
@@ -116,7 +126,7 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
       for (int big = 0; big < G && balance; ++big) {
         for (int small = 0; small < G && load[big] > target; ++small) {
           if (small == big || load[small] >= target) continue;
-          auto& src = hold_at(s, t, big);
+          std::vector<Piece>& src = hold_at(s, t, big).v;   // nothing is taken from the front yet
           // Walk the heavy GPU's own pieces (only data still in its input buffer can be relayed).
           for (size_t k = 0; k < src.size() && load[big] > target && load[small] < target;) {
             Piece& pc = src[k];
@@ -129,7 +139,7 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
             if (keep(src_rank, dst_rank))
               p.ops.push_back(Op{Phase::kBalance, Buf::kInput, Buf::kBalance, -1, src_rank, dst_rank,
                                  src_rank, t * G + pc.final_local, pc.off, cursor, mv, pc.pair_off});
-            hold_at(s, t, small).push_back(Piece{pc.origin_local, pc.final_local, pc.pair_off, mv, Buf::kBalance, cursor});
+            hold_at(s, t, small).v.push_back(Piece{pc.origin_local, pc.final_local, pc.pair_off, mv, Buf::kBalance, cursor});
             cursor += mv;
             load[big] -= mv;
             load[small] += mv;
@@ -152,32 +162,30 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
       for (int i = 0; i < G; ++i) direct(s * G + i, s * G + (i + step) % G, -1);
 
   // ---- inter-server stages ----------------------------------------------------------------------
-  std::vector<Stage> stages;
+  Stage all;                // kSingleBurst: every server pair at once, unlimited budget
+  all.weight = -1;
+  const Stage* stages = &all;
+  int K = 1;
   if (opt.kind == PlanKind::kStaged) {
     int64_t scale = opt.scale > 0 ? opt.scale
                                   : choose_scale(p.server_matrix, G, opt.scale_policy, opt.inter, opt.intra, opt.mb_per_unit);
     if (scale < 1) scale = 1;
     p.decomp = decompose(p.server_matrix, opt.match, scale);
-    stages = p.decomp.stages;
-  } else {  // kSingleBurst: every server pair at once, unlimited budget
-    Stage all;
-    all.weight = -1;
-    stages.push_back(all);
+    stages = p.decomp.stages.data();
+    K = static_cast<int>(p.decomp.stages.size());
   }
 
   std::vector<int> last_stage_of_pair(static_cast<size_t>(S) * S, -1);
-  
-  const int K = static_cast<int>(stages.size());
-  // Rail and redistribution ops are collected per stage and concatenated at the end, so that the
+
+  // Rail and redistribution ops are collected as they come and filed by stage at the end, so that the
   // final list is [balance][intrinsic][rail 0][redis 0][rail 1][redis 1]...
-  std::vector<std::vector<Op>> rail_of_stage(K), redis_of_stage(K);
+  std::vector<Op> later;
+  later.reserve(std::min<size_t>(static_cast<size_t>(K) * S * G, 4096));
 
   auto emit_rail = [&](int k, int s, int t, int i, int64_t budget) {
     auto& q = hold_at(s, t, i);
     if (q.empty()) return;
     const int src_rank = s * G + i, dst_rank = t * G + i;
-    std::vector<Op>& rail = rail_of_stage[k];
-    std::vector<Op>& redis = redis_of_stage[k];
     while (!q.empty() && budget != 0) {
       Piece& pc = q.front();
       const int64_t take = budget < 0 ? pc.len : aligned_cut(pc, budget, opt.split_align);
@@ -185,15 +193,15 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
       const int origin = s * G + pc.origin_local, fin = t * G + pc.final_local;
       if (pc.final_local == i) {
         if (keep(src_rank, dst_rank))
-          rail.push_back(Op{Phase::kRail, pc.buf, Buf::kOutput, k, src_rank, dst_rank, origin, fin, pc.off,
+          later.push_back(Op{Phase::kRail, pc.buf, Buf::kOutput, k, src_rank, dst_rank, origin, fin, pc.off,
                             out_at(fin, origin) + pc.pair_off, take, pc.pair_off});
       } else {
         int64_t& cursor = p.buffers[dst_rank].rail_units;
         if (keep(src_rank, dst_rank))
-          rail.push_back(Op{Phase::kRail, pc.buf, Buf::kRail, k, src_rank, dst_rank, origin, fin, pc.off, cursor,
+          later.push_back(Op{Phase::kRail, pc.buf, Buf::kRail, k, src_rank, dst_rank, origin, fin, pc.off, cursor,
                             take, pc.pair_off});
         if (keep(dst_rank, fin))
-          redis.push_back(Op{Phase::kRedistribute, Buf::kRail, Buf::kOutput, k, dst_rank, fin, origin, fin, cursor,
+          later.push_back(Op{Phase::kRedistribute, Buf::kRail, Buf::kOutput, k, dst_rank, fin, origin, fin, cursor,
                              out_at(fin, origin) + pc.pair_off, take, pc.pair_off});
         cursor += take;
       }
@@ -233,15 +241,14 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
         }
       }
   }
-  size_t total = p.ops.size();
-  for (int k = 0; k < K; ++k) total += rail_of_stage[k].size() + redis_of_stage[k].size();
-  p.ops.reserve(total);
-  for (int k = 0; k < K; ++k) {
-    p.ops.insert(p.ops.end(), rail_of_stage[k].begin(), rail_of_stage[k].end());
-    p.ops.insert(p.ops.end(), redis_of_stage[k].begin(), redis_of_stage[k].end());
-    std::vector<Op>().swap(rail_of_stage[k]);
-    std::vector<Op>().swap(redis_of_stage[k]);
-  }
+  // Stable counting sort by (stage, rail before redistribution).
+  auto slot_of = [](const Op& o) { return static_cast<size_t>(o.stage) * 2 + (o.phase == Phase::kRedistribute ? 1 : 0); };
+  std::vector<size_t> at(static_cast<size_t>(K) * 2 + 1, 0);
+  for (const Op& o : later) ++at[slot_of(o) + 1];
+  for (size_t q = 1; q < at.size(); ++q) at[q] += at[q - 1];
+  const size_t first = p.ops.size();
+  p.ops.resize(first + later.size());
+  for (const Op& o : later) p.ops[first + at[slot_of(o)]++] = o;
   p.num_stages = K;
   return p;
 }

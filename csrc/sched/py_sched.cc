@@ -97,6 +97,7 @@ PYBIND11_MODULE(_sched, m) {
     return choose_scale(to_matrix(a), gpus, sp, inter, intra, mbpu);
   });
   m.def("matrix_hash", [](const I64Array& a) { return to_matrix(a).hash(); });
+  m.def("max_line_sum", [](const I64Array& a) { return to_matrix(a).max_line_sum(); });
 
   py::class_<Plan>(m, "Plan")
       .def_property_readonly("servers", [](const Plan& p) { return p.topo.servers; })

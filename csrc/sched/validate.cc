@@ -1,7 +1,7 @@
 // Plan validation and host replay (the CPU oracle for every executor).
 #include <algorithm>
 #include <cstring>
-#include <sstream>
+#include <string>
 
 #include "plan.h"
 
@@ -16,23 +16,37 @@ int64_t buf_units(const RankBuffers& b, Buf k) {
     default: return b.rail_units;
   }
 }
-using Interval = std::pair<int64_t, int64_t>;  // [begin, end)
+struct Interval { int64_t begin, end; };
 
-// Empty string if `iv` tiles [0, total) exactly once.
-std::string tiles_exactly(std::vector<Interval>& iv, int64_t total) {
-  std::sort(iv.begin(), iv.end());
-  int64_t pos = 0;
-  for (const Interval& x : iv) {
-    if (x.first != pos) return x.first < pos ? "overlap" : "gap";
-    pos = x.second;
+// Intervals filed by cell: count them, fix the cells' places, file them. Two passes over the ops and two allocations,
+// where a vector per cell allocated (and grew) n * n times.
+struct Filed {
+  std::vector<size_t> start;      // [cells + 1] once filed
+  std::vector<Interval> iv;
+  explicit Filed(size_t cells) : start(cells + 2, 0) {}
+  void count(size_t cell) { ++start[cell + 2]; }
+  void places() {
+    for (size_t c = 2; c < start.size(); ++c) start[c] += start[c - 1];
+    iv.resize(start.back());
   }
-  return pos == total ? "" : "short";
-}
+  void file(size_t cell, int64_t begin, int64_t end) { iv[start[cell + 1]++] = Interval{begin, end}; }
+  // Empty string if the intervals of `cell` tile [0, total) exactly once.
+  const char* tiles_exactly(size_t cell, int64_t total) {
+    Interval *b = iv.data() + start[cell], *e = iv.data() + start[cell + 1];
+    auto before = [](const Interval& x, const Interval& y) { return x.begin != y.begin ? x.begin < y.begin : x.end < y.end; };
+    if (!std::is_sorted(b, e, before)) std::sort(b, e, before);
+    int64_t pos = 0;
+    for (const Interval* x = b; x != e; ++x) {
+      if (x->begin != pos) return x->begin < pos ? "overlap" : "gap";
+      pos = x->end;
+    }
+    return pos == total ? "" : "short";
+  }
+};
 }  // namespace
 
 std::string validate_plan(const Plan& p) {
   const int n = p.matrix.n, G = p.topo.gpus, S = p.topo.servers;
-  std::ostringstream err;
   // Structure first (a plan may come from a file): everything below indexes by these sizes.
   if (n < 0 || G < 1 || S < 1 || static_cast<int64_t>(S) * G != n) return "topology does not match the matrix";
   if (static_cast<int>(p.buffers.size()) != n) return "buffers: wrong rank count";
@@ -59,15 +73,16 @@ std::string validate_plan(const Plan& p) {
   const int only = p.opt.only_rank;  // >= 0: a one-rank view, only that rank's deliveries and staging can be complete
   if (only >= n) return "only_rank out of range";
   // Flat tables instead of maps: validation runs on every new plan, and a 512-rank plan has millions of ops.
-  std::vector<std::vector<Interval>> delivered(static_cast<size_t>(n) * n);  // origin * n + final -> segment intervals
-  std::vector<std::vector<Interval>> staged_w(static_cast<size_t>(n) * 2), staged_r(static_cast<size_t>(n) * 2);  // rank * 2 + (rail ? 1 : 0)
+  Filed delivered(static_cast<size_t>(n) * n);                                   // origin * n + final -> segment intervals
+  Filed staged_w(static_cast<size_t>(n) * 2), staged_r(static_cast<size_t>(n) * 2);  // rank * 2 + (rail ? 1 : 0)
   const size_t stage_cells = p.opt.kind == PlanKind::kStaged ? static_cast<size_t>(std::max(p.num_stages, 0)) * S : 0;
   std::vector<int> stage_to(stage_cells, -1), stage_from(stage_cells, -1);   // stage * S + server -> peer server
   auto staging_slot = [](int rank, Buf b) { return static_cast<size_t>(rank) * 2 + (b == Buf::kRail ? 1 : 0); };
 
+  bool any_rail = false;
   for (size_t k = 0; k < p.ops.size(); ++k) {
     const Op& o = p.ops[k];
-    auto bad = [&](const char* what) { err << "op " << k << ": " << what; return err.str(); };
+    auto bad = [&](const char* what) { return "op " + std::to_string(k) + ": " + what; };
     if (o.len <= 0) return bad("non-positive length");
     if (only >= 0 && o.src_rank != only && o.dst_rank != only) return bad("op of another rank in a one-rank view");
     if (static_cast<unsigned>(o.phase) > 3u || static_cast<unsigned>(o.src_buf) > 3u || static_cast<unsigned>(o.dst_buf) > 3u) return bad("unknown phase or buffer");
@@ -100,41 +115,47 @@ std::string validate_plan(const Plan& p) {
       if (o.src_rank != o.origin) return bad("input read on a rank that is not the origin");
       if (o.src_off != p.in_disp[static_cast<size_t>(o.origin) * n + o.final_dst] + o.pair_off) return bad("input offset does not match the pair segment");
     } else {
-      staged_r[staging_slot(o.src_rank, o.src_buf)].push_back({o.src_off, o.src_off + o.len});
+      staged_r.count(staging_slot(o.src_rank, o.src_buf));
     }
     if (o.dst_buf == Buf::kOutput) {
       if (o.dst_rank != o.final_dst) return bad("output written on a rank that is not the final destination");
       if (o.dst_off != p.out_disp[static_cast<size_t>(o.final_dst) * n + o.origin] + o.pair_off) return bad("output offset does not match the pair segment");
-      delivered[static_cast<size_t>(o.origin) * n + o.final_dst].push_back({o.pair_off, o.pair_off + o.len});
+      delivered.count(static_cast<size_t>(o.origin) * n + o.final_dst);
     } else {
-      staged_w[staging_slot(o.dst_rank, o.dst_buf)].push_back({o.dst_off, o.dst_off + o.len});
+      staged_w.count(staging_slot(o.dst_rank, o.dst_buf));
+      any_rail |= o.dst_buf == Buf::kRail;
     }
   }
-  {  // up to rail_tail_start the regions of a rank's rail staging follow the stage order
+  delivered.places(); staged_w.places(); staged_r.places();
+  for (const Op& o : p.ops) {
+    if (o.src_buf != Buf::kInput) staged_r.file(staging_slot(o.src_rank, o.src_buf), o.src_off, o.src_off + o.len);
+    if (o.dst_buf == Buf::kOutput) delivered.file(static_cast<size_t>(o.origin) * n + o.final_dst, o.pair_off, o.pair_off + o.len);
+    else staged_w.file(staging_slot(o.dst_rank, o.dst_buf), o.dst_off, o.dst_off + o.len);
+  }
+  if (any_rail) {  // up to rail_tail_start the regions of a rank's rail staging follow the stage order
     std::vector<std::vector<std::pair<int64_t, int>>> by_off(n);
     for (const Op& o : p.ops)
       if (o.dst_buf == Buf::kRail && o.dst_off < p.rail_tail_start[o.dst_rank]) by_off[o.dst_rank].push_back({o.dst_off, o.stage});
     for (int r = 0; r < n; ++r) {
       std::sort(by_off[r].begin(), by_off[r].end());
       for (size_t k = 1; k < by_off[r].size(); ++k)
-        if (by_off[r][k].second < by_off[r][k - 1].second) { err << "rank " << r << ": rail staging is not in stage order before its tail"; return err.str(); }
+        if (by_off[r][k].second < by_off[r][k - 1].second) return "rank " + std::to_string(r) + ": rail staging is not in stage order before its tail";
     }
   }
   for (int i = 0; i < n; ++i)
     for (int j = 0; j < n; ++j) {
       if (only >= 0 && j != only) continue;
-      std::string r = tiles_exactly(delivered[static_cast<size_t>(i) * n + j], p.matrix.at(i, j));
-      if (!r.empty()) { err << "pair " << i << "->" << j << ": delivery has a " << r; return err.str(); }
+      const char* r = delivered.tiles_exactly(static_cast<size_t>(i) * n + j, p.matrix.at(i, j));
+      if (*r) return "pair " + std::to_string(i) + "->" + std::to_string(j) + ": delivery has a " + r;
     }
   for (int r = 0; r < n; ++r)
     for (Buf b : {Buf::kBalance, Buf::kRail}) {
       if (only >= 0 && r != only) continue;
-      std::vector<Interval>&w = staged_w[staging_slot(r, b)], &rd = staged_r[staging_slot(r, b)];
-      std::string a = tiles_exactly(w, buf_units(p.buffers[r], b));
-      if (!a.empty()) { err << "rank " << r << " staging " << static_cast<int>(b) << ": writes have a " << a; return err.str(); }
+      const char* a = staged_w.tiles_exactly(staging_slot(r, b), buf_units(p.buffers[r], b));
+      if (*a) return "rank " + std::to_string(r) + " staging " + std::to_string(static_cast<int>(b)) + ": writes have a " + a;
       // Reads may split a written piece, but together they must cover the same bytes once.
-      a = tiles_exactly(rd, buf_units(p.buffers[r], b));
-      if (!a.empty()) { err << "rank " << r << " staging " << static_cast<int>(b) << ": forwards have a " << a; return err.str(); }
+      a = staged_r.tiles_exactly(staging_slot(r, b), buf_units(p.buffers[r], b));
+      if (*a) return "rank " + std::to_string(r) + " staging " + std::to_string(static_cast<int>(b)) + ": forwards have a " + a;
     }
   return "";
 }

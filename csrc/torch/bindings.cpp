@@ -20,7 +20,8 @@ namespace {
 
 // ---- a2a program ----------------------------------------------------------------------------------
 struct A2AProgramPy {
-  torch::Tensor items_dev, expect_rail_dev;
+  torch::Tensor program_dev;     // the work list, then the expected rail bytes from rail_off on
+  int64_t rail_off = 0;
   int n_items = 0, num_stages = 0;
   bool has_waits = false;  // some item waits for bytes another item of a peer's (or this) launch forwards
   unsigned long long expect_output = 0, expect_balance = 0;
@@ -28,37 +29,44 @@ struct A2AProgramPy {
   int64_t input_bytes = 0, output_bytes = 0;  // what the rank's input and output hold (set by the owner, checked by the group launch)
 
   // items: int64[k, 10] as produced by Plan.lower(); expect_rail: list of bytes per stage.
-  A2AProgramPy(torch::Tensor items, std::vector<int64_t> expect_rail, int64_t exp_out, int64_t exp_bal, int device) {
+  A2AProgramPy(torch::Tensor items, const std::vector<int64_t>& expect_rail, int64_t exp_out, int64_t exp_bal, int device) {
     TORCH_CHECK(items.dim() == 2 && items.size(1) == 10 && items.dtype() == torch::kInt64 && items.is_cpu(), "items must be CPU int64[k, 10]");
     TORCH_CHECK(static_cast<int>(expect_rail.size()) <= kSigMaxStages, "too many stages for the signal block");
     n_items = static_cast<int>(items.size(0));
     num_stages = static_cast<int>(expect_rail.size());
     expect_output = static_cast<unsigned long long>(exp_out);
     expect_balance = static_cast<unsigned long long>(exp_bal);
-    auto host = torch::empty({std::max(n_items, 1), static_cast<int64_t>(sizeof(A2AWork))}, torch::kUInt8);
+    // Work list and expected rail bytes go up in one copy from pinned memory, in stream order: nothing here waits for the GPU.
+    const int64_t list_bytes = std::max<int64_t>(n_items, 1) * static_cast<int64_t>(sizeof(A2AWork)), all_bytes = list_bytes + std::max(num_stages, 1) * 8;
+    const auto u8 = torch::TensorOptions().dtype(torch::kUInt8);
+    auto host = torch::empty({all_bytes}, u8.pinned_memory(true));
     A2AWork* w = reinterpret_cast<A2AWork*>(host.data_ptr());
     auto it = items.contiguous();
     const int64_t* q = it.data_ptr<int64_t>();
-    for (int i = 0; i < n_items; ++i, q += 10) {
-      w[i].src_off = q[0]; w[i].dst_off = q[1]; w[i].bytes = q[2]; w[i].dst_rank = static_cast<int>(q[3]);
-      w[i].src_buf = static_cast<unsigned char>(q[4]); w[i].dst_buf = static_cast<unsigned char>(q[5]);
-      w[i].wait_kind = static_cast<unsigned char>(q[6]); w[i].signal_kind = static_cast<unsigned char>(q[7]);
-      w[i].stage = static_cast<int>(q[8]); w[i].wait_stage = static_cast<int>(q[9]); w[i].pad_ = 0;
-      total_bytes += q[2];
-      largest_item = std::max(largest_item, q[2]);
-      if (q[6] != 0) has_waits = true;
+    int64_t total = 0, largest = 0, waits = 0;   // locals: stores through w could alias the members
+    for (int i = 0, n = n_items; i < n; ++i, q += 10) {
+      A2AWork x;
+      x.src_off = q[0]; x.dst_off = q[1]; x.bytes = q[2]; x.dst_rank = static_cast<int>(q[3]);
+      x.src_buf = static_cast<unsigned char>(q[4]); x.dst_buf = static_cast<unsigned char>(q[5]);
+      x.wait_kind = static_cast<unsigned char>(q[6]); x.signal_kind = static_cast<unsigned char>(q[7]);
+      x.stage = static_cast<int>(q[8]); x.wait_stage = static_cast<int>(q[9]); x.pad_ = 0;
+      total += q[2];
+      largest = std::max(largest, q[2]);
+      waits |= q[6];
+      w[i] = x;
     }
-    auto dev = torch::Device(torch::kCUDA, device);
-    items_dev = host.to(dev);
-    auto er = torch::empty({std::max(num_stages, 1)}, torch::kInt64);
-    for (int k = 0; k < num_stages; ++k) er[k] = expect_rail[k];
-    expect_rail_dev = er.to(dev);
+    total_bytes = total; largest_item = largest; has_waits = waits != 0;
+    std::copy(expect_rail.begin(), expect_rail.end(), reinterpret_cast<int64_t*>(host.data_ptr<uint8_t>() + list_bytes));
+    c10::cuda::CUDAGuard g(device);
+    program_dev = torch::empty({all_bytes}, u8.device(torch::kCUDA, device));
+    program_dev.copy_(host, /*non_blocking=*/true);
+    rail_off = list_bytes;
   }
 
   A2ARankArgs args(const HeapPy& heap, std::array<int64_t, 4> src_ptrs, std::array<int64_t, 4> dst_offs, int64_t sig_off,
                    uint64_t epoch, const StatusPy& st, uint64_t timeout_ns, int64_t stamps_ptr = 0) const {
     A2ARankArgs a{};
-    a.items = reinterpret_cast<const A2AWork*>(items_dev.data_ptr());
+    a.items = reinterpret_cast<const A2AWork*>(program_dev.data_ptr());
     a.n_items = n_items; a.rank = heap.h->rank(); a.world = heap.h->world(); a.num_stages = num_stages;
     // Slices of 128 KiB (two passes of the copy loop: 512 threads x 8 x 16 bytes each), at most 16 per item.
     a.slice_bytes = std::max<int64_t>(128 << 10, (largest_item / 16 + 0xFFFF) & ~int64_t{0xFFFF});
@@ -66,7 +74,7 @@ struct A2AProgramPy {
     a.peer_table = heap.h->device_peer_table();
     for (int i = 0; i < 4; ++i) { a.src_base[i] = reinterpret_cast<const unsigned char*>(src_ptrs[i]); a.dst_heap_off[i] = dst_offs[i]; }
     a.sig_heap_off = sig_off; a.epoch = epoch; a.expect_output = expect_output; a.expect_balance = expect_balance;
-    a.expect_rail = reinterpret_cast<const unsigned long long*>(expect_rail_dev.data_ptr());
+    a.expect_rail = reinterpret_cast<const unsigned long long*>(program_dev.data_ptr<uint8_t>() + rail_off);
     a.status = st.d; a.timeout_ns = timeout_ns;
     a.phase_stamps = reinterpret_cast<unsigned long long*>(stamps_ptr);
     return a;

@@ -8,6 +8,7 @@ exposes self-tests (nvidia/alltoall_nvshmem.cpp:508-601); this one is a general 
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -197,12 +198,12 @@ class Communicator:
         if chunk_bytes is None:
             # Work items: about 8 per CTA for the busiest rank (an uneven last round of 1 MiB items costs
             # up to half the bandwidth at 148 CTAs), between 64 KiB and 1 MiB, a power of two.
-            busiest = int(max(m.sum(1).max(), m.sum(0).max())) * unit_bytes
+            busiest = sched.max_line_sum(m) * unit_bytes
             chunk_bytes = 1 << 16
             while chunk_bytes < (1 << 20) and chunk_bytes * 2 * self.ctas * 8 <= busiest:
                 chunk_bytes *= 2
         if "split_align" not in plan_opts:
-            plan_opts["split_align"] = max(1, 16 // np.gcd(16, unit_bytes))
+            plan_opts["split_align"] = 16 // math.gcd(16, unit_bytes)
         key = (sched.matrix_hash(m), unit_bytes, transpose, str(kind), chunk_bytes, rail_segment_bytes, tuple(sorted((k, str(v)) for k, v in plan_opts.items())))
         s = self._sched_cache.get(key)
         if s is None:
@@ -217,7 +218,7 @@ class Communicator:
             if err:
                 raise RuntimeError(f"scheduler produced an invalid plan: {err}")
             low = plan.lower(self.rank, unit_bytes, chunk_bytes, rail_segment_bytes, MAX_RAIL_COUNTERS)
-            prog = self._C.A2AProgram(torch.from_numpy(low["items"]), [int(x) for x in low["expect_rail_bytes"]],
+            prog = self._C.A2AProgram(torch.from_numpy(low["items"]), low["expect_rail_bytes"],
                                       int(low["expect_output_bytes"]), int(low["expect_balance_bytes"]), self.device.index)
             prog.input_bytes, prog.output_bytes = int(low["input_bytes"]), int(low["output_bytes"])
             s = Schedule(plan, unit_bytes, prog, low, self.rank)

@@ -64,6 +64,11 @@ def inter_link(name: str) -> "LinkModel":
     return LinkModel(a, b)
 
 
+def max_line_sum(matrix) -> int:
+    """Largest row or column sum: the units through the busiest port."""
+    return _S.max_line_sum(matrix)
+
+
 BUF_INPUT, BUF_OUTPUT, BUF_BALANCE, BUF_RAIL = 0, 1, 2, 3
 PHASE_BALANCE, PHASE_INTRINSIC, PHASE_RAIL, PHASE_REDISTRIBUTE = 0, 1, 2, 3
 
