@@ -252,39 +252,48 @@ __global__ void emb_scan_blocks_kernel(int* __restrict__ hist, int blocks, int V
   total[v] = run;
 }
 
-// Single block: start[v] = sum of total[< v]; start[V] = number of tokens that took part. Four ids per thread and pass.
+// Single block: start[v] = sum of total[< v]; start[V] = number of tokens that took part. Tiles of 4096 ids, each
+// warp 128 of them with coalesced 16-byte accesses; all tiles of a batch are requested before the first is summed (eight
+// dependent passes over 32000 ids took 25 us).
 __global__ void __launch_bounds__(1024) emb_scan_ids_kernel(const int* __restrict__ total, int V, int* __restrict__ start) {
-  __shared__ int s_warp[32];
-  __shared__ int s_carry;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
+  constexpr int N = 8;                       // tiles of a batch
+  __shared__ int s_warp[N][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int v0 = 0; v0 < V; v0 += 4096) {
-    const int v = v0 + 4 * threadIdx.x;
-    int x[4];
+  int carry = 0;
+  for (int v0 = 0; v0 < V; v0 += 4096 * N) {
+    int x[N][4], incl[N];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) x[u] = v + u < V ? total[v + u] : 0;
-    const int mine = x[0] + x[1] + x[2] + x[3];
-    int incl = mine;
+    for (int n = 0; n < N; ++n) {
+      const int v = v0 + 4096 * n + 4 * static_cast<int>(threadIdx.x);
+      if (v + 3 < V) {
+        const int4 q = __ldg(reinterpret_cast<const int4*>(total + v));   // v is a multiple of 4
+        x[n][0] = q.x; x[n][1] = q.y; x[n][2] = q.z; x[n][3] = q.w;
+      } else {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      int w = s_warp[lane];
+        for (int u = 0; u < 4; ++u) x[n][u] = v + u < V ? __ldg(total + v + u) : 0;
+      }
+    }
+    __syncthreads();   // the previous batch has read s_warp
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += y; }
-      s_warp[lane] = w;  // inclusive over warps
+    for (int n = 0; n < N; ++n) {
+      incl[n] = x[n][0] + x[n][1] + x[n][2] + x[n][3];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl[n], o); if (lane >= o) incl[n] += y; }
+      if (lane == 31) s_warp[n][warp] = incl[n];
     }
     __syncthreads();
-    int before = s_carry + (warp ? s_warp[warp - 1] : 0) + incl - mine;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) { if (v + u < V) start[v + u] = before; before += x[u]; }
-    __syncthreads();
-    if (threadIdx.x == 1023) s_carry = before;
-    __syncthreads();
+    for (int n = 0; n < N; ++n) {
+      const int w = s_warp[n][lane];
+      const int before = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(lane < warp ? w : 0))), all = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(w)));
+      int at = carry + before + incl[n] - (x[n][0] + x[n][1] + x[n][2] + x[n][3]);
+      const int v = v0 + 4096 * n + 4 * static_cast<int>(threadIdx.x);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { if (v + u < V) start[v + u] = at; at += x[n][u]; }
+      carry += all;
+    }
   }
-  if (threadIdx.x == 0) start[V] = s_carry;
+  if (threadIdx.x == 0) start[V] = carry;
 }
 
 __global__ void emb_scatter_kernel(const long long* __restrict__ ids, const int* __restrict__ rank_in_block, const int* __restrict__ hist,
@@ -297,6 +306,109 @@ __global__ void emb_scatter_kernel(const long long* __restrict__ ids, const int*
   const long long slot = start[id] + hist[(p / kIdxBlock) * V + id] + r;
   sorted_ids[slot] = id;
   perm[slot] = p;
+}
+
+// ---- the whole gradient of an embedding table ------------------------------------------------------------------
+// A warp per table row, after the counting sort: every row is written once, its sum or zeros (cleared beforehand by a kernel of
+// its own, the table cost one more pass of writes: 91 us for 32000 x 4096).
+__global__ void embedding_rows_kernel(const int* __restrict__ start, const long long* __restrict__ perm, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int V, int H) {
+  const long long v = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, chunks = H / 8;
+  if (v >= V) return;
+  const int begin = __ldg(start + v), end = __ldg(start + v + 1);
+  uint4* out = grad_table + v * chunks;
+  constexpr int U = 4;   // chunks in flight per row
+  for (int c0 = lane; c0 < chunks; c0 += 32 * U) {
+    float acc[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[u][k] = 0.0f;
+    for (int j = begin; j < end; ++j) {
+      const uint4* row = grad_out + __ldg(perm + j) * chunks;
+      uint4 x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = c0 + 32 * u < chunks ? __ldg(row + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float f[8];
+        unpack8(x[u], f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + 32 * u < chunks) __stcs(out + c0 + 32 * u, pack8(acc[u]));
+  }
+}
+
+// Few tokens, on a table that is zero already: a warp per position looks for its id among the earlier ones; the first of an id sums
+// all of its rows, in position order. T * T / 32 comparisons a warp's width replace the sort's six launches. The ids are
+// compared in shared memory (read from global memory every 32 of them were a trip to L2: 69 us at 4096 tokens).
+constexpr int kLeaderTokens = 4096;
+__global__ void __launch_bounds__(256) embedding_leaders_kernel(const long long* __restrict__ ids, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int T, int V, int H) {
+  __shared__ int s_id[kLeaderTokens];   // ids outside [0, V) take no part: each gets a value of its own
+  for (int i = threadIdx.x; i < T; i += blockDim.x) {
+    const long long x = __ldg(ids + i);
+    s_id[i] = x >= 0 && x < V ? static_cast<int>(x) : -1 - i;
+  }
+  __syncthreads();
+  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, chunks = H / 8;
+  if (p >= T) return;
+  const int id = s_id[p];
+  if (id < 0) return;
+  bool earlier = false;
+#pragma unroll 4
+  for (int q = lane; q < p; q += 32) earlier |= s_id[q] == id;
+  if (__any_sync(0xffffffffu, earlier)) return;
+  // My id's later positions: kept one per lane where there are at most 32 of them, else looked up again for every chunk.
+  int mine = -1, found = 0;
+  for (int q0 = p / 32 * 32; q0 < T; q0 += 32) {
+    unsigned m = __ballot_sync(0xffffffffu, q0 + lane > p && q0 + lane < T && s_id[min(q0 + lane, T - 1)] == id);
+    while (m) {
+      const int q = q0 + __ffs(m) - 1;
+      m &= m - 1;
+      if (found == lane) mine = q;
+      ++found;
+    }
+  }
+  uint4* out = grad_table + static_cast<long long>(id) * chunks;
+  constexpr int U = 4;
+  for (int c0 = 0; c0 < chunks; c0 += 32 * U) {
+    float acc[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[u][k] = 0.0f;
+    auto add = [&](int q) {
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c = c0 + 32 * u + lane;
+        v[u] = c < chunks ? __ldg(grad_out + static_cast<long long>(q) * chunks + c) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float f[8];
+        unpack8(v[u], f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+      }
+    };
+    add(p);
+    if (found <= 32) {
+      for (int j = 0; j < found; ++j) add(__shfl_sync(0xffffffffu, mine, j));
+    } else {
+      for (int q0 = p / 32 * 32; q0 < T; q0 += 32) {
+        unsigned m = __ballot_sync(0xffffffffu, q0 + lane > p && q0 + lane < T && s_id[min(q0 + lane, T - 1)] == id);
+        while (m) { add(q0 + __ffs(m) - 1); m &= m - 1; }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + 32 * u + lane < chunks) out[c0 + 32 * u + lane] = pack8(acc[u]);
+  }
 }
 
 int grid_for(long long items) { return static_cast<int>(std::min<long long>((items + 255) / 256, 148 * 8)); }
@@ -363,6 +475,20 @@ cudaError_t launch_embedding_index(const long long* ids, long long T, int V, int
   return cudaGetLastError();
 }
 int embedding_index_block() { return kIdxBlock; }
+cudaError_t launch_embedding_rows(const int* start, const long long* perm, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int V, int H, cudaStream_t stream) {
+  if (H % 8) return cudaErrorInvalidValue;
+  embedding_rows_kernel<<<static_cast<unsigned>((V * 32ll + 255) / 256), 256, 0, stream>>>(start, perm, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), V, H);
+  note_launch();
+  return cudaGetLastError();
+}
+cudaError_t launch_embedding_leaders(const long long* ids, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int T, int V, int H, cudaStream_t stream) {
+  if (H % 8 || T > kLeaderTokens) return cudaErrorInvalidValue;
+  cudaError_t e = cudaMemsetAsync(grad_table, 0, static_cast<size_t>(V) * H * 2, stream);
+  if (e != cudaSuccess || T == 0) return e;
+  embedding_leaders_kernel<<<static_cast<unsigned>((T * 32ll + 255) / 256), 256, 0, stream>>>(ids, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), T, V, H);
+  note_launch();
+  return cudaGetLastError();
+}
 cudaError_t launch_dequant_fp8(const unsigned char* q, const float* scales, __nv_bfloat16* out, long long rows, int H, const int* rows_dev,
                                cudaStream_t stream) {
   if (H % 128) return cudaErrorInvalidValue;

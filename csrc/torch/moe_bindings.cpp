@@ -486,6 +486,29 @@ void bind_moe(py::module_& m) {
                                   reinterpret_cast<const __nv_bfloat16*>(grad_out.data_ptr()), reinterpret_cast<__nv_bfloat16*>(grad_table.data_ptr()),
                                   sorted_ids.numel(), static_cast<int>(grad_out.size(1)), stream_now()), "embedding_bwd");
   });
+  // grad_out [T, H] summed by id in position order -> a new table gradient [V, H] (rows that no id names are zero).
+  m.def("embedding_grad", [](torch::Tensor ids, int V, torch::Tensor grad_out) {
+    want(ids, torch::kInt64, "ids"); want(grad_out, torch::kBFloat16, "grad_out");
+    const int64_t T = ids.numel(), H = grad_out.size(1);
+    TORCH_CHECK(grad_out.dim() == 2 && grad_out.size(0) == T, "embedding_grad: one gradient row per id");
+    auto table = torch::empty({V, H}, grad_out.options());
+    const long long* idp = reinterpret_cast<const long long*>(ids.data_ptr());
+    const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(grad_out.data_ptr());
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(table.data_ptr());
+    // Up to here comparing all pairs of positions (5 us at 4096) is cheaper than the sort's six launches.
+    if (T <= 4096) {
+      cu_check(launch_embedding_leaders(idp, g, out, static_cast<int>(T), V, static_cast<int>(H), stream_now()), "embedding_grad");
+      return table;
+    }
+    const int64_t blocks = (T + embedding_index_block() - 1) / embedding_index_block();
+    auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(ids.device());
+    auto hist = torch::empty({blocks, V}, i32), rank = torch::empty({T}, i32), total = torch::empty({V}, i32), start = torch::empty({V + 1}, i32);
+    auto sorted_ids = torch::empty({T}, ids.options()), perm = torch::empty({T}, ids.options());
+    cu_check(launch_embedding_index(idp, T, V, hist.data_ptr<int>(), rank.data_ptr<int>(), total.data_ptr<int>(), start.data_ptr<int>(),
+                                    reinterpret_cast<long long*>(sorted_ids.data_ptr()), reinterpret_cast<long long*>(perm.data_ptr()), stream_now()), "embedding_grad");
+    cu_check(launch_embedding_rows(start.data_ptr<int>(), reinterpret_cast<const long long*>(perm.data_ptr()), g, out, V, static_cast<int>(H), stream_now()), "embedding_grad");
+    return table;
+  });
   m.def("embedding_index", [](torch::Tensor ids, int V) {
     want(ids, torch::kInt64, "ids");
     const int64_t T = ids.numel();

@@ -17,10 +17,8 @@ class _Embedding(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         (ids,) = ctx.saved_tensors
-        grad_table = torch.zeros(ctx.shape, dtype=grad_out.dtype, device=grad_out.device)
         # positions grouped by id by this library's counting sort (stable, cost independent of duplicates)
-        sorted_ids, perm = runtime.ext().embedding_index(ids.reshape(-1).contiguous(), ctx.shape[0])
-        runtime.ext().embedding_bwd(sorted_ids, perm, grad_out.reshape(-1, ctx.shape[1]).contiguous(), grad_table)
+        grad_table = runtime.ext().embedding_grad(ids.reshape(-1).contiguous(), ctx.shape[0], grad_out.reshape(-1, ctx.shape[1]).contiguous())
         return None, grad_table
 
 

@@ -274,6 +274,22 @@ def test_embedding_index_is_a_stable_sort_by_id():
         assert torch.equal(sid, rs) and torch.equal(perm, rp)
 
 
+@pytest.mark.parametrize("T,V,H,spread", [(1, 7, 256, 7), (33, 50, 264, 50), (300, 40, 256, 3), (4096, 1000, 256, 1000), (4097, 40000, 256, 40000), (5000, 33, 512, 2)])
+def test_embedding_gradient_of_any_length(T, V, H, spread):
+    """Pairwise search (up to 4096 tokens) and counting sort, rare and heavy duplicates: position-order fp32 sums, zeros elsewhere."""
+    from fast_b200.ops import fused
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.randint(0, spread, (T,), generator=g, device="cuda") * (V // spread)
+    table = torch.randn(V, H, generator=g, device="cuda").to(torch.bfloat16).requires_grad_()
+    go = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    table.grad = None
+    fused.embedding(ids, table).backward(go)
+    want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids, go.double())
+    assert _rel(table.grad, want.float()) < 1e-2
+    assert bool((table.grad[torch.bincount(ids, minlength=V) == 0] == 0).all())
+
+
 def test_fused_embedding_and_loss_match_torch():
     from fast_b200.ops import fused
 
