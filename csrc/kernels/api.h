@@ -236,8 +236,10 @@ struct NormGateArgs {
   int* slot_in_block;           // as launch_route_topk
   int* block_cnt;
 };
-// With sp, the last block goes on with the split scan (sp->block_cnt = a.block_cnt).
-cudaError_t launch_norm_gate_route(const NormGateArgs& a, const SplitsArgs* sp, unsigned int* ticket, cudaStream_t stream);
+// With sp, the last block goes on with the split scan (sp->block_cnt = a.block_cnt). tickets: norm_gate_tickets(T) zeroed words that the
+// launches of one stream share; they are zero again after each.
+int norm_gate_tickets(int T);
+cudaError_t launch_norm_gate_route(const NormGateArgs& a, const SplitsArgs* sp, unsigned int* tickets, cudaStream_t stream);
 struct NormGateBwdArgs {
   const __nv_bfloat16* h;       // [T, H] input of the forward pass
   const __nv_bfloat16* norm_w;  // [H]
@@ -249,10 +251,16 @@ struct NormGateBwdArgs {
   const __nv_bfloat16* grad_hn; // [T, H] gradient of hn from its other consumer (the MoE input)
   int T, H, num_experts, K;
   __nv_bfloat16* grad_h;        // [T, H] out
-  float* d_gate;                // [E, H] fp32, accumulated into (zero it first)
-  float* d_norm_w;              // [H] fp32, accumulated into
+  const __nv_bfloat16* residual;  // [T, H] or null: gradient that reaches h past the norm, added to grad_h
+  float* partials;              // [blocks][(E + 1) * H] scratch
+  // Either fp32, accumulated into, or bf16, written:
+  float* d_gate;                // [E, H]
+  float* d_norm_w;              // [H]
+  __nv_bfloat16* d_gate_bf16;
+  __nv_bfloat16* d_norm_w_bf16;
 };
-cudaError_t launch_norm_gate_bwd(const NormGateBwdArgs& a, cudaStream_t stream);
+int norm_gate_bwd_blocks(int T, int H, int E, int sms);
+cudaError_t launch_norm_gate_bwd(const NormGateBwdArgs& a, int blocks, cudaStream_t stream);
 size_t norm_gate_smem_bytes(int E, int H, int K, bool backward);
 
 struct DispatchArgs {
@@ -273,6 +281,14 @@ struct DispatchArgs {
   __nv_bfloat16* local_rows;   // fp8, unsorted, a world of one rank, optional: the rows are stored here as the bf16 values a receiver would make of
                                // them, instead of as e4m3 in the receive buffer
   int warps_per_row;           // set by the launcher
+  // Backward, bf16 rows with row_scale: dot_out [T, K] = <x row, row of the forward output at y_heap_off that lies where the row is sent>.
+  float* dot_out;
+  long long y_heap_off;
+  // With it, optional: x row := bf16(x + sum_with) * *grad_loss * grad_factor, also stored to grad_out (gradient of mean((x + sum_with)^2)).
+  const __nv_bfloat16* sum_with;
+  __nv_bfloat16* grad_out;     // [T, H]
+  const float* grad_loss;
+  float grad_factor;
   long long recv_heap_off;     // destination rows: bf16 [cap, H] (or u8 [cap, H] when fp8)
   long long scale_heap_off;    // fp8 only: float [cap, H/128]
   long long arrive_heap_off;   // u64 arrival counters of this channel: [E/world] per expert, or [num_tiles] per tile
@@ -287,6 +303,7 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
 // quantisation the fp8 dispatch otherwise does per entry, done once per row.
 cudaError_t launch_quantise_rows(const __nv_bfloat16* x, int T, int H, unsigned char* q, float* scales, int ctas, cudaStream_t stream);
 
+constexpr int kMaxLossPartials = 2048;   // blocks of a combine launch that also makes the loss
 struct CombineArgs {
   void* const* peer_table;
   int rank, world, num_experts, T, K, H;
@@ -302,6 +319,12 @@ struct CombineArgs {
   __nv_bfloat16* out;          // [T, H] sum_j w * row_j (null in dot mode)
   const __nv_bfloat16* dot_with;  // dot mode: [T, H]
   float* dot_out;              // dot mode: [T, K] = <dot_with[t], row_j>
+  // Optional, with out: *loss = loss_scale * sum((residual + out)^2), the sum rounded to bf16 first.
+  const __nv_bfloat16* residual;   // [T, H]
+  float* loss_partials;        // [kMaxLossPartials] scratch
+  unsigned int* ticket;        // one zeroed word; zero again afterwards
+  float* loss;
+  float loss_scale;
   DeviceStatus* status;
   unsigned long long timeout_ns;
 };

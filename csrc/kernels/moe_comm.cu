@@ -16,6 +16,7 @@
 
 #include "api.h"
 #include "early_start.cuh"
+#include "route_splits.cuh"
 
 namespace fastb {
 
@@ -33,6 +34,12 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
 #pragma unroll
   for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  return v;
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -126,13 +133,18 @@ __global__ void __launch_bounds__(kCommThreads) quantise_rows_kernel(const __nv_
 // their register counts: the copy loops are bound by the stores a SM keeps in flight, i.e. by resident warps.
 // ROUNDED (one rank alone): nothing crosses a wire, so the rows go straight to the GEMM's bf16 operand, as the values that a
 // receiver would make of their e4m3 form. Sent as e4m3 and converted afterwards, 32768 rows of 7168 took 85 + 145 us.
-template <bool FP8, bool SORTED, bool SCALED, bool ROUNDED = false>
-__global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_kernel(const DispatchArgs a) {
+// DOT (backward): the row on its way out (w * grad) meets the expert's output row that lies at the same place of the owner's
+// forward buffer, and their product is the gradient of w: one reading of the gradient rows serves both. With a.sum_with
+// the gradient itself is made here, from the two terms whose mean square is the loss.
+template <bool FP8, bool SORTED, bool SCALED, bool ROUNDED = false, bool DOT = false>
+__global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispatch_push_kernel(const DispatchArgs a) {
   extern __shared__ int s_cnt[];  // rows this CTA sent: [E] per expert, or [world][num_tiles] per destination tile
   __shared__ int s_ok;
   __shared__ __align__(16) float s_scales[(kCommThreads / 32) * kMaxScaleGroups];  // fp8 mode: the 1x128 scales of the row each warp is sending
   grid_dependency_wait();
   launch_dependents();
+  __shared__ float s_dot[DOT ? kCommThreads / 32 : 1][kMaxK];
+  const float gscale = DOT && a.sum_with != nullptr ? *a.grad_loss * a.grad_factor : 0.0f;
   const int E = a.num_experts, El = E / a.world;
   const int n_cnt = a.tile_rows > 0 ? a.world * a.num_tiles : E;
   for (int e = threadIdx.x; e < n_cnt; e += blockDim.x) s_cnt[e] = 0;
@@ -220,7 +232,75 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
         }
       }
       const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<long long>(t) * a.H);
-      if constexpr (!FP8) {
+      if constexpr (DOT) {
+        const uint4* sum_with = a.sum_with ? reinterpret_cast<const uint4*>(a.sum_with + static_cast<long long>(t) * a.H) : nullptr;
+        uint4* grad_out = a.sum_with ? reinterpret_cast<uint4*>(a.grad_out + static_cast<long long>(t) * a.H) : nullptr;
+        const long long to_y = a.y_heap_off - a.recv_heap_off;
+        float dots[NJ];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) dots[j] = 0.0f;
+        constexpr int U = 4;
+        const int rounds = chunks / 32, c_end = rounds * (part + 1) / wpr * 32;
+        for (int c0 = rounds * part / wpr * 32 + lane; c0 < c_end; c0 += 32 * U) {
+          uint4 v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (c0 + 32 * u < c_end) v[u] = __ldg(src + c0 + 32 * u);
+          if (sum_with != nullptr) {
+            uint4 w[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (c0 + 32 * u < c_end) w[u] = __ldg(sum_with + c0 + 32 * u);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              if (c0 + 32 * u >= c_end) break;
+              float f[8], h[8];
+              unpack8(v[u], f);
+              unpack8(w[u], h);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(__float2bfloat16_rn(f[i] + h[i])) * gscale;
+              v[u] = pack8(f);
+              grad_out[c0 + 32 * u] = v[u];
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) {
+            if (j >= nj || out_row[j] == nullptr) continue;
+            uint4 y[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (c0 + 32 * u < c_end) y[u] = __ldcg(reinterpret_cast<const uint4*>(out_row[j] + to_y) + c0 + 32 * u);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              if (c0 + 32 * u >= c_end) break;
+              float f[8], h[8];
+              unpack8(v[u], f);
+              unpack8(y[u], h);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) { dots[j] = fmaf(f[i], h[i], dots[j]); f[i] *= scale[j]; }
+              reinterpret_cast<uint4*>(out_row[j])[c0 + 32 * u] = pack8(f);
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          if (j >= nj) break;
+          float d = dots[j];
+#pragma unroll
+          for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+          if (wpr == 1) { if (lane == 0) a.dot_out[static_cast<long long>(t) * a.K + j] = d; }
+          else if (lane == 0) s_dot[part][j] = d;
+        }
+        if (wpr > 1) {   // the CTA's warps share this row
+          __syncthreads();
+          if (part == 0 && lane < nj) {
+            float d = 0.0f;
+            for (int q = 0; q < wpr; ++q) d += s_dot[q][lane];
+            a.dot_out[static_cast<long long>(t) * a.K + lane] = d;
+          }
+          __syncthreads();
+        }
+      } else if constexpr (!FP8) {
         // Four 16-byte chunks per lane in flight before the first store: the loop is bound by the
         // latency of the local loads otherwise.
         constexpr int U = 4;
@@ -335,16 +415,17 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : 3) dispatch_push_ke
   publish_counts();
 }
 
+// LOSS: the rows are also added to a.residual and squared on their way out.
+template <bool LOSS>
 __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const CombineArgs a) {
   __shared__ int s_ok;
   grid_dependency_wait();
   launch_dependents();
   const int El = a.num_experts / a.world;
-  if (threadIdx.x == 0) s_ok = 1;
-  if (*reinterpret_cast<volatile unsigned long long*>(&a.status->abort) != 0ull) return;
+  if (threadIdx.x == 0) s_ok = *reinterpret_cast<volatile unsigned long long*>(&a.status->abort) == 0ull;
   __syncthreads();
   const unsigned long long ready_epoch = a.epoch_dev ? *a.epoch_dev : a.ready_epoch;
-  if (ready_epoch != 0 && a.world > 1) {   // alone, the rows were written by earlier kernels of this stream
+  if (s_ok && ready_epoch != 0 && a.world > 1) {   // alone, the rows were written by earlier kernels of this stream
     if (a.signal && blockIdx.x == 0 && threadIdx.x < a.world) {
       // My rows are final (this kernel follows their producer): say so to every rank. Block 0 is always resident, so no rank's
       // wait below can keep this from happening.
@@ -354,10 +435,14 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
     const unsigned long long* flags = reinterpret_cast<const unsigned long long*>(static_cast<unsigned char*>(a.peer_table[a.rank]) + a.ready_flags_heap_off);
     if (threadIdx.x < a.world && !wait_ge_bounded(flags + threadIdx.x, ready_epoch, a.status, kSiteCombineReady, threadIdx.x, a.timeout_ns)) s_ok = 0;
     __syncthreads();
-    if (!s_ok) return;
+  }
+  if (!s_ok) {
+    if (LOSS) route::last_block(a.ticket);   // the count of blocks stays whole
+    return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int chunks = a.H / 8, rounds = chunks / 32, segs = a.segments;
+  float square = 0.0f;   // my share of sum((residual + out)^2)
   // A warp takes one of `segs` column ranges of a token's row (1 in dot mode, whose sums span the row).
   for (long long u = blockIdx.x * wpb + warp; u < static_cast<long long>(a.T) * segs; u += gridDim.x * wpb) {
     const int t = static_cast<int>(u / segs), seg = static_cast<int>(u % segs);
@@ -383,7 +468,13 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
       uint4* out = reinterpret_cast<uint4*>(a.out + static_cast<long long>(t) * a.H);
       constexpr int U = 2;  // two chunks x K rows of peer loads in flight per lane
       for (int c0 = rounds * seg / segs * 32 + lane; c0 < c_end; c0 += 32 * U) {
-        uint4 v[U][kMaxK];
+        uint4 v[U][kMaxK], res[U];
+        if (LOSS) {
+          const uint4* h = reinterpret_cast<const uint4*>(a.residual + static_cast<long long>(t) * a.H);
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (c0 + 32 * u < c_end) res[u] = __ldg(h + c0 + 32 * u);
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -402,7 +493,15 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[i] = fmaf(w[j], f[i], acc[i]);
           }
-          out[c] = pack8(acc);
+          const uint4 o = pack8(acc);
+          out[c] = o;
+          if (LOSS) {
+            float f[8], h[8];
+            unpack8(o, f);
+            unpack8(res[u], h);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { const float q = __bfloat162float(__float2bfloat16_rn(h[i] + f[i])); square = fmaf(q, q, square); }
+          }
         }
       }
     } else {
@@ -432,6 +531,29 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
       }
     }
   }
+  if constexpr (LOSS) {
+    // Block sums, then the last block adds them up in a fixed order.
+    __shared__ float s_sum[kCommThreads / 32];
+    square = warp_sum(square);
+    if (lane == 0) s_sum[warp] = square;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float v = 0.0f;
+      for (int i = 0; i < wpb; ++i) v += s_sum[i];
+      a.loss_partials[blockIdx.x] = v;
+    }
+    if (!route::last_block(a.ticket)) return;
+    float v = 0.0f;
+    for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) v += __ldcg(a.loss_partials + i);
+    v = warp_sum(v);
+    if (lane == 0) s_sum[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      v = 0.0f;
+      for (int i = 0; i < wpb; ++i) v += s_sum[i];
+      *a.loss = v * a.loss_scale;
+    }
+  }
 }
 
 __global__ void wait_counters_kernel(const unsigned long long* counter, const unsigned long long* target, int n, DeviceStatus* st,
@@ -449,6 +571,8 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
   if (a.T == 0) return cudaSuccess;
   if (a.tile_rows < 0 || (a.tile_rows > 0 && a.num_tiles < 1)) return cudaErrorInvalidValue;
   if (a.local_rows != nullptr && (!a.fp8 || a.send_list != nullptr || a.row_scale != nullptr || a.world != 1)) return cudaErrorInvalidValue;
+  if (a.dot_out != nullptr && (a.fp8 || a.send_list != nullptr || a.row_scale == nullptr)) return cudaErrorInvalidValue;
+  if (a.sum_with != nullptr && (a.dot_out == nullptr || a.grad_out == nullptr || a.grad_loss == nullptr)) return cudaErrorInvalidValue;
   DispatchArgs b = a;
   b.warps_per_row = a.send_list == nullptr && a.T <= ctas ? kCommThreads / 32 : 1;
   // No more CTAs than there is work for (entries of the sorted list, rows per CTA otherwise).
@@ -466,6 +590,7 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
     return e;
   };
   const bool sorted = a.send_list != nullptr, scaled = a.row_scale != nullptr;
+  if (a.dot_out != nullptr) return go(dispatch_push_kernel<false, false, true, false, true>);
   if (a.local_rows != nullptr) return go(dispatch_push_kernel<false, false, false, true>);
   if (a.fp8) return sorted ? go(dispatch_push_kernel<true, true, false>) : go(dispatch_push_kernel<true, false, false>);
   if (sorted) return scaled ? go(dispatch_push_kernel<false, true, true>) : go(dispatch_push_kernel<false, true, false>);
@@ -482,11 +607,12 @@ cudaError_t launch_quantise_rows(const __nv_bfloat16* x, int T, int H, unsigned 
 
 cudaError_t launch_combine_pull(const CombineArgs& a, int ctas, cudaStream_t stream) {
   if (a.K < 1 || a.K > kMaxK || a.H % 256 || a.world < 1 || a.num_experts % a.world || ctas < 1) return cudaErrorInvalidValue;
+  if (a.residual != nullptr && (a.out == nullptr || a.loss_partials == nullptr || a.ticket == nullptr || a.loss == nullptr || ctas > kMaxLossPartials)) return cudaErrorInvalidValue;
   if (a.T == 0) return cudaSuccess;
   CombineArgs b = a;
   // Few tokens: as many warps per row as fill the grid, down to one round of loads per warp.
   b.segments = a.dot_out != nullptr ? 1 : static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / a.T, 1, a.H / 256));
-  cudaError_t e = launch_early(combine_pull_kernel, dim3(ctas), kCommThreads, 0, stream, b);
+  cudaError_t e = launch_early(a.residual != nullptr ? combine_pull_kernel<true> : combine_pull_kernel<false>, dim3(ctas), kCommThreads, 0, stream, b);
   if (e == cudaSuccess) note_launch();
   return e;
 }

@@ -320,7 +320,8 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
                    torch::Tensor block_base, torch::Tensor send_base, torch::Tensor dest_row, bool compute_rows, bool fp8, int64_t recv_off,
                    int64_t scale_off, int64_t arrive_off, int64_t entry_flags_off, uint64_t entry_epoch, const StatusPy& st, uint64_t timeout_ns, int ctas,
                    c10::optional<torch::Tensor> send_list, int tile_rows, int num_tiles, c10::optional<torch::Tensor> xq,
-                   c10::optional<torch::Tensor> xq_scales, c10::optional<torch::Tensor> local_rows) {
+                   c10::optional<torch::Tensor> xq_scales, c10::optional<torch::Tensor> local_rows, c10::optional<torch::Tensor> dot_out, int64_t y_off,
+                   c10::optional<torch::Tensor> sum_with, c10::optional<torch::Tensor> grad_out, c10::optional<torch::Tensor> grad_loss, double grad_factor) {
   want(x, torch::kBFloat16, "x"); want(topk_idx, torch::kInt32, "topk_idx"); want(dest_row, torch::kInt32, "dest_row");
   DispatchArgs a{};
   a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
@@ -337,6 +338,19 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
     TORCH_CHECK(xq->numel() >= x.numel() && xq_scales->numel() >= x.numel() / 128, "dispatch_push: xq / xq_scales too small");
     a.xq = xq->data_ptr<uint8_t>(); a.xq_scales = xq_scales->data_ptr<float>();
   }
+  if (dot_out.has_value()) {
+    want(*dot_out, torch::kFloat32, "dot_out");
+    TORCH_CHECK(dot_out->numel() == topk_idx.numel(), "dispatch_push: dot_out is [T, K]");
+    a.dot_out = dot_out->data_ptr<float>();
+    a.y_heap_off = y_off;
+    if (sum_with.has_value()) {
+      TORCH_CHECK(grad_out.has_value() && grad_loss.has_value(), "dispatch_push: sum_with needs grad_out and grad_loss");
+      want(*sum_with, torch::kBFloat16, "sum_with"); want(*grad_out, torch::kBFloat16, "grad_out"); want(*grad_loss, torch::kFloat32, "grad_loss");
+      TORCH_CHECK(sum_with->sizes() == x.sizes() && grad_out->sizes() == x.sizes(), "dispatch_push: sum_with / grad_out shapes");
+      a.sum_with = reinterpret_cast<const __nv_bfloat16*>(sum_with->data_ptr()); a.grad_out = reinterpret_cast<__nv_bfloat16*>(grad_out->data_ptr());
+      a.grad_loss = grad_loss->data_ptr<float>(); a.grad_factor = static_cast<float>(grad_factor);
+    }
+  }
   if (local_rows.has_value()) {
     want(*local_rows, torch::kBFloat16, "local_rows");
     TORCH_CHECK(fp8 && local_rows->dim() == 2 && local_rows->size(1) == a.H, "dispatch_push: local_rows belongs to the fp8 rows");
@@ -349,8 +363,18 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
 
 void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, torch::Tensor dest_row, c10::optional<torch::Tensor> weights, int64_t src_off,
                   int64_t ready_off, uint64_t ready_epoch, c10::optional<torch::Tensor> out, c10::optional<torch::Tensor> dot_with,
-                  c10::optional<torch::Tensor> dot_out, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr, bool signal) {
+                  c10::optional<torch::Tensor> dot_out, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr, bool signal,
+                  c10::optional<torch::Tensor> residual, c10::optional<torch::Tensor> loss, double loss_scale, c10::optional<torch::Tensor> ticket) {
   CombineArgs a{};
+  torch::Tensor partials;
+  if (residual.has_value()) {
+    TORCH_CHECK(loss.has_value() && ticket.has_value(), "combine_pull: residual needs loss and ticket");
+    want(*residual, torch::kBFloat16, "residual"); want(*loss, torch::kFloat32, "loss"); want(*ticket, torch::kInt32, "ticket");
+    TORCH_CHECK(residual->dim() == 2 && residual->size(0) == topk_idx.size(0) && residual->size(1) == H, "combine_pull: residual shape");
+    partials = torch::empty({kMaxLossPartials}, loss->options());
+    a.residual = reinterpret_cast<const __nv_bfloat16*>(residual->data_ptr()); a.loss = loss->data_ptr<float>(); a.loss_scale = static_cast<float>(loss_scale);
+    a.loss_partials = partials.data_ptr<float>(); a.ticket = reinterpret_cast<unsigned int*>(ticket->data_ptr<int>());
+  }
   a.signal = signal ? 1 : 0;
   a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world(); a.num_experts = num_experts;
   a.T = static_cast<int>(topk_idx.size(0)); a.K = static_cast<int>(topk_idx.size(1)); a.H = H;
@@ -414,17 +438,24 @@ void bind_moe(py::module_& m) {
     a.gate = reinterpret_cast<const __nv_bfloat16*>(gate.data_ptr()); a.bias = ptr_or_null<const float>(bias);
     a.hn = reinterpret_cast<__nv_bfloat16*>(hn.data_ptr()); a.rstd = rstd.data_ptr<float>(); a.logits = logits.data_ptr<float>();
     a.topk_idx = topk_idx.data_ptr<int>(); a.topk_w = topk_w.data_ptr<float>(); a.slot_in_block = slot_in_block.data_ptr<int>(); a.block_cnt = block_cnt.data_ptr<int>();
-    if (splits == nullptr) { cu_check(launch_norm_gate_route(a, nullptr, nullptr, stream_now()), "norm_gate_route"); return; }
+    if (splits == nullptr) {
+      auto tickets = torch::zeros({norm_gate_tickets(a.T)}, topk_idx.options());
+      cu_check(launch_norm_gate_route(a, nullptr, reinterpret_cast<unsigned int*>(tickets.data_ptr<int>()), stream_now()), "norm_gate_route");
+      return;
+    }
     const SplitsArgs sp = splits->for_tokens(a.T, epoch);
     if (a.T == 0) cu_check(launch_splits_scan(sp, stream_now()), "splits_scan");
     else cu_check(launch_norm_gate_route(a, &sp, splits->ticket, stream_now()), "norm_gate_route");
   }, py::arg("h"), py::arg("norm_w"), py::arg("gate"), py::arg("bias"), py::arg("k"), py::arg("eps"), py::arg("hn"), py::arg("rstd"), py::arg("logits"), py::arg("topk_idx"),
      py::arg("topk_w"), py::arg("slot_in_block"), py::arg("block_cnt"), py::arg("splits") = nullptr, py::arg("epoch") = 0);
   m.def("norm_gate_bwd", [](torch::Tensor h, torch::Tensor norm_w, torch::Tensor gate, torch::Tensor rstd, torch::Tensor topk_idx, torch::Tensor topk_w,
-                            torch::Tensor grad_w, torch::Tensor grad_hn, torch::Tensor grad_h, torch::Tensor d_gate, torch::Tensor d_norm_w) {
+                            torch::Tensor grad_w, torch::Tensor grad_hn, torch::Tensor grad_h, torch::Tensor d_gate, torch::Tensor d_norm_w,
+                            c10::optional<torch::Tensor> residual) {
     want(h, torch::kBFloat16, "h"); want(norm_w, torch::kBFloat16, "norm_w"); want(gate, torch::kBFloat16, "gate"); want(rstd, torch::kFloat32, "rstd");
     want(topk_idx, torch::kInt32, "topk_idx"); want(topk_w, torch::kFloat32, "topk_w"); want(grad_w, torch::kFloat32, "grad_w");
-    want(grad_hn, torch::kBFloat16, "grad_hn"); want(grad_h, torch::kBFloat16, "grad_h"); want(d_gate, torch::kFloat32, "d_gate"); want(d_norm_w, torch::kFloat32, "d_norm_w");
+    want(grad_hn, torch::kBFloat16, "grad_hn"); want(grad_h, torch::kBFloat16, "grad_h");
+    const bool as_bf16 = d_gate.scalar_type() == torch::kBFloat16;   // written as bf16, or accumulated into as fp32
+    want(d_gate, as_bf16 ? torch::kBFloat16 : torch::kFloat32, "d_gate"); want(d_norm_w, as_bf16 ? torch::kBFloat16 : torch::kFloat32, "d_norm_w");
     NormGateBwdArgs a{};
     a.T = static_cast<int>(h.size(0)); a.H = static_cast<int>(h.size(1)); a.num_experts = static_cast<int>(gate.size(0)); a.K = static_cast<int>(topk_idx.size(1));
     TORCH_CHECK(gate.size(1) == a.H && grad_hn.sizes() == h.sizes() && grad_h.sizes() == h.sizes() && d_gate.numel() == gate.numel() && d_norm_w.numel() == a.H &&
@@ -432,13 +463,26 @@ void bind_moe(py::module_& m) {
     a.h = reinterpret_cast<const __nv_bfloat16*>(h.data_ptr()); a.norm_w = reinterpret_cast<const __nv_bfloat16*>(norm_w.data_ptr());
     a.gate = reinterpret_cast<const __nv_bfloat16*>(gate.data_ptr()); a.rstd = rstd.data_ptr<float>(); a.topk_idx = topk_idx.data_ptr<int>();
     a.topk_w = topk_w.data_ptr<float>(); a.grad_w = grad_w.data_ptr<float>(); a.grad_hn = reinterpret_cast<const __nv_bfloat16*>(grad_hn.data_ptr());
-    a.grad_h = reinterpret_cast<__nv_bfloat16*>(grad_h.data_ptr()); a.d_gate = d_gate.data_ptr<float>(); a.d_norm_w = d_norm_w.data_ptr<float>();
-    cu_check(launch_norm_gate_bwd(a, stream_now()), "norm_gate_bwd");
-  });
+    a.grad_h = reinterpret_cast<__nv_bfloat16*>(grad_h.data_ptr());
+    if (as_bf16) { a.d_gate_bf16 = reinterpret_cast<__nv_bfloat16*>(d_gate.data_ptr()); a.d_norm_w_bf16 = reinterpret_cast<__nv_bfloat16*>(d_norm_w.data_ptr()); }
+    else { a.d_gate = d_gate.data_ptr<float>(); a.d_norm_w = d_norm_w.data_ptr<float>(); }
+    if (residual.has_value()) {
+      want(*residual, torch::kBFloat16, "residual");
+      TORCH_CHECK(residual->sizes() == h.sizes(), "norm_gate_bwd: residual shape");
+      a.residual = reinterpret_cast<const __nv_bfloat16*>(residual->data_ptr());
+    }
+    const int blocks = norm_gate_bwd_blocks(a.T, a.H, a.num_experts, at::cuda::getCurrentDeviceProperties()->multiProcessorCount);
+    auto partials = torch::empty({blocks, a.num_experts + 1, a.H}, h.options().dtype(torch::kFloat32));
+    a.partials = partials.data_ptr<float>();
+    if (a.T == 0 && as_bf16) { d_gate.zero_(); d_norm_w.zero_(); }
+    cu_check(launch_norm_gate_bwd(a, blocks, stream_now()), "norm_gate_bwd");
+  }, py::arg("h"), py::arg("norm_w"), py::arg("gate"), py::arg("rstd"), py::arg("topk_idx"), py::arg("topk_w"), py::arg("grad_w"), py::arg("grad_hn"), py::arg("grad_h"),
+     py::arg("d_gate"), py::arg("d_norm_w"), py::arg("residual") = py::none());
   m.def("dispatch_push", &dispatch_push, py::arg("heap"), py::arg("x"), py::arg("topk_idx"), py::arg("row_scale"), py::arg("slot_in_block"), py::arg("block_base"),
         py::arg("send_base"), py::arg("dest_row"), py::arg("compute_rows"), py::arg("fp8"), py::arg("recv_off"), py::arg("scale_off"), py::arg("arrive_off"),
         py::arg("entry_flags_off"), py::arg("entry_epoch"), py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"), py::arg("send_list"),
-        py::arg("tile_rows") = 0, py::arg("num_tiles") = 0, py::arg("xq") = py::none(), py::arg("xq_scales") = py::none(), py::arg("local_rows") = py::none());
+        py::arg("tile_rows") = 0, py::arg("num_tiles") = 0, py::arg("xq") = py::none(), py::arg("xq_scales") = py::none(), py::arg("local_rows") = py::none(), py::arg("dot_out") = py::none(),
+        py::arg("y_off") = 0, py::arg("sum_with") = py::none(), py::arg("grad_out") = py::none(), py::arg("grad_loss") = py::none(), py::arg("grad_factor") = 0.0);
   m.def("quantise_rows", [](torch::Tensor x, torch::Tensor q, torch::Tensor scales, int ctas) {
     want(x, torch::kBFloat16, "x"); want(q, torch::kUInt8, "q"); want(scales, torch::kFloat32, "scales");
     TORCH_CHECK(x.dim() == 2 && q.numel() >= x.numel() && scales.numel() >= x.numel() / 128, "quantise_rows: q / scales too small");
@@ -447,7 +491,7 @@ void bind_moe(py::module_& m) {
   });
   m.def("combine_pull", &combine_pull, py::arg("heap"), py::arg("num_experts"), py::arg("topk_idx"), py::arg("dest_row"), py::arg("weights"), py::arg("src_off"), py::arg("ready_off"),
         py::arg("ready_epoch"), py::arg("out"), py::arg("dot_with"), py::arg("dot_out"), py::arg("hidden"), py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"),
-        py::arg("epoch_dev_ptr"), py::arg("signal") = false);
+        py::arg("epoch_dev_ptr"), py::arg("signal") = false, py::arg("residual") = py::none(), py::arg("loss") = py::none(), py::arg("loss_scale") = 1.0, py::arg("ticket") = py::none());
   m.def("wait_counters", [](int64_t counter_ptr, torch::Tensor target, const StatusPy& st, uint64_t timeout_ns) {
     cu_check(launch_wait_counters(reinterpret_cast<const unsigned long long*>(counter_ptr), reinterpret_cast<const unsigned long long*>(target.data_ptr()),
                                   static_cast<int>(target.numel()), st.d, timeout_ns, stream_now()), "wait_counters");

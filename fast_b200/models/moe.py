@@ -45,9 +45,10 @@ class _MoEFunction(torch.autograd.Function):
         return gx, gw.to(weights.dtype), dw13, dw2, None, None
 
 
-def _experts_backward(eng, grad_out, rs, weights, w13, w2, w2_param):
+def _experts_backward(eng, grad_out, rs, weights, w13, w2, w2_param, mean_square=None):
     """Backward of dispatch -> experts -> combine through the engine. Returns (grad_x, grad_weights, dW13,
-    dW2 or None); dW2 is None when an attached optimizer applied W2's update inside the pass."""
+    dW2 or None); dW2 is None when an attached optimizer applied W2's update inside the pass.
+    ``mean_square``: see ``ExpertParallel.backward``."""
     # New tensors each time, held by nobody else when they are returned: autograd then keeps them as the parameters' .grad.
     # Buffers that the engine kept were cloned instead (a pass over all expert gradients: 0.9 ms for 8 x 4096 x 14336).
     dw13, dw2 = torch.empty_like(w13), torch.empty_like(w2)
@@ -59,7 +60,7 @@ def _experts_backward(eng, grad_out, rs, weights, w13, w2, w2_param):
         # W2 wgrad nothing in this pass reads W2 any more.
         main = torch.cuda.current_stream()
         if not hasattr(eng, "_opt_stream"):
-            eng._opt_stream = torch.cuda.Stream(device=grad_out.device)
+            eng._opt_stream = torch.cuda.Stream(device=w2.device)
 
         def after():
             ev = torch.cuda.Event()
@@ -67,7 +68,7 @@ def _experts_backward(eng, grad_out, rs, weights, w13, w2, w2_param):
             eng._opt_stream.wait_event(ev)
             opt.step_param(w2_param, dw2, stream=eng._opt_stream, early=True)
 
-    gx, gw = eng.backward(grad_out.contiguous(), rs, weights, w13, w2, dw13, dw2, after_dw2=after)
+    gx, gw = eng.backward(grad_out.contiguous() if grad_out is not None else None, rs, weights, w13, w2, dw13, dw2, after_dw2=after, mean_square=mean_square)
     if early:
         done = torch.cuda.Event()
         done.record(eng._opt_stream)
@@ -96,10 +97,37 @@ class _NormRouteMoEFunction(torch.autograd.Function):
         eng, rs = ctx.engine, ctx.rs
         gx, gw, dw13, dw2 = _experts_backward(eng, grad_out, rs, rs.topk_w, w13, w2, ctx.w2_param)
         grad_h = torch.empty_like(h)
-        d_gate = torch.zeros(gate.shape, dtype=torch.float32, device=h.device)
-        d_nw = torch.zeros(norm_w.shape, dtype=torch.float32, device=h.device)
+        d_gate, d_nw = torch.empty_like(gate), torch.empty_like(norm_w)
         eng._C.norm_gate_bwd(h, norm_w, gate, rstd, rs.topk_idx, rs.topk_w, gw, gx, grad_h, d_gate, d_nw)
-        return grad_h, d_nw.to(norm_w.dtype), d_gate.to(gate.dtype), dw13, dw2, None, None, None
+        return grad_h, d_nw, d_gate, dw13, dw2, None, None, None
+
+
+class _NormRouteMoELossFunction(torch.autograd.Function):
+    """mean((h + MoE(RMSNorm(h)))^2): the chain above with the residual sum, the loss and their gradients inside the
+    kernels that handle the rows anyway (combine; the backward dispatch; the norm's backward)."""
+
+    @staticmethod
+    def forward(ctx, h, norm_w, gate, w13, w2, engine, eps, layer):
+        rs, hn, rstd, _ = engine.route_fused(h, norm_w, gate, eps, layer.router_bias)
+        layer.last_route = rs
+        engine.dispatch(hn, rs)
+        engine.experts_forward(w13, w2, rs)
+        loss = torch.empty(1, dtype=torch.float32, device=h.device)
+        out = engine.combine(rs, rs.topk_w, residual=h, loss=loss)
+        ctx.engine, ctx.rs, ctx.w2_param = engine, rs, w2
+        ctx.save_for_backward(h, norm_w, gate, rstd, w13, w2, out)
+        return loss.reshape(())
+
+    @staticmethod
+    def backward(ctx, grad_loss):
+        h, norm_w, gate, rstd, w13, w2, out = ctx.saved_tensors
+        eng, rs = ctx.engine, ctx.rs
+        g = torch.empty_like(h)
+        gx, gw, dw13, dw2 = _experts_backward(eng, None, rs, rs.topk_w, w13, w2, ctx.w2_param, (h, out, grad_loss.reshape(1).float().contiguous(), g))
+        grad_h = torch.empty_like(h)
+        d_gate, d_nw = torch.empty_like(gate), torch.empty_like(norm_w)
+        eng._C.norm_gate_bwd(h, norm_w, gate, rstd, rs.topk_idx, rs.topk_w, gw, gx, grad_h, d_gate, d_nw, g)
+        return grad_h, d_nw, d_gate, dw13, dw2, None, None, None
 
 
 class MoELayer(nn.Module):
@@ -158,10 +186,18 @@ class MoELayer(nn.Module):
         """MoE(RMSNorm(h; norm_w)) for h [tokens, hidden] bf16. When the layer's shapes allow it the norm,
         the router logits, the top-k and their backward run as one fused kernel each way; otherwise this is
         ``self(rms_norm(h))`` with stock ops in front."""
-        fused = self.engine.can_fuse_gate() and torch.is_grad_enabled() and self.training and h.dtype == torch.bfloat16
-        if not fused:
+        if not self._fuses(h):
             return self(torch.nn.functional.rms_norm(h, (h.shape[-1],), norm_w, eps))
         return _NormRouteMoEFunction.apply(h.contiguous(), norm_w, self.gate, self.w13, self.w2, self.engine, eps, self)
+
+    def _fuses(self, h: torch.Tensor) -> bool:
+        return self.engine.can_fuse_gate() and torch.is_grad_enabled() and self.training and h.dtype == torch.bfloat16
+
+    def mean_square_from_residual(self, h: torch.Tensor, norm_w: torch.Tensor, eps: float) -> torch.Tensor:
+        """mean((h + MoE(RMSNorm(h; norm_w)))^2), the sum rounded to bf16, as a scalar fp32 tensor."""
+        if not (self._fuses(h) and h.shape[0] > 0):
+            return fused.residual_mean_square(h, self.forward_from_residual(h, norm_w, eps))
+        return _NormRouteMoELossFunction.apply(h.contiguous(), norm_w, self.gate, self.w13, self.w2, self.engine, eps, self)
 
     def attach_optimizer(self, opt) -> None:
         """Optimizer-in-backward: ``opt`` (a FusedAdamW owning ``w2``) applies W2's update as soon as
@@ -202,7 +238,7 @@ class MixtralBlockModel(nn.Module):
 
     def forward(self, token_ids: torch.Tensor) -> torch.Tensor:
         h = fused.embedding(token_ids.reshape(-1), self.embed)
-        return fused.residual_mean_square(h, self.moe.forward_from_residual(h, self.norm_w, self.eps))
+        return self.moe.mean_square_from_residual(h, self.norm_w, self.eps)
 
 
 @torch.no_grad()

@@ -144,7 +144,8 @@ class ExpertParallel:
         self.splits = C.SplitsPlan(comm.heap, self._off(self.counts), self._flag_off(0), self.block_cnt, self.block_base, self.send_base, self.send_cnt, self.group_off,
                                    self.group_rows, self.arrive_target[:channels], self.traffic, channels, gemm.row_align(), self.cap, comm.status, comm.timeout_ns,
                                    self.send_pos if overlap_dispatch else None, self.epoch_dev.data_ptr() if graph_mode else 0, self.tile_target, self.tile_rows,
-                                   torch.zeros(1, **i32))
+                                   torch.zeros(1 + blocks, **i32))
+        self.ticket = torch.zeros(1, **i32)
         # One rank alone: nothing crosses a wire, so the fp8 dispatch stores the bf16 values that a receiver would make of its rows.
         self.local_bf16 = fp8_dispatch and W == 1 and not self.fp8_direct and not overlap_dispatch
         if graph_mode:
@@ -327,12 +328,16 @@ class ExpertParallel:
         gemm.grouped_gemm_fwd(self.act, w2, rs.group_off, self.y, **self._live(rs))
         self._join_dispatch()
 
-    def combine(self, rs: RouteState, weights: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def combine(self, rs: RouteState, weights: torch.Tensor, out: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
+                loss: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``out[t] = sum_j weights[t, j] * y_row(t, j)``. With ``residual`` ([T, H] bf16), ``loss`` (float [1]) receives
+        mean((residual + out)^2), the sum rounded to bf16."""
         T = rs.topk_idx.shape[0]
         if out is None:
             out = torch.empty(T, self.H, dtype=torch.bfloat16, device=rs.topk_idx.device)
         self._C.combine_pull(self.comm.heap, self.E, rs.topk_idx, rs.dest_row, weights, self._off(self.y), self._flag_off(1), rs.epoch, out, None, None,
-                             self.H, self.status, self.timeout_ns, self.comm_ctas, self.epoch_dev.data_ptr() if self.graph_mode else 0, True)
+                             self.H, self.status, self.timeout_ns, self.comm_ctas, self.epoch_dev.data_ptr() if self.graph_mode else 0, True,
+                             residual, loss, 1.0 / max(T * self.H, 1), self.ticket if residual is not None else None)
         return out
 
     def forward(self, x: torch.Tensor, logits: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -362,22 +367,25 @@ class ExpertParallel:
         return plan, plan.cost(nv, nv, 1e-6)
 
     # ---- backward --------------------------------------------------------------------------------
-    def backward(self, grad_out: torch.Tensor, rs: RouteState, weights: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, dw13: torch.Tensor,
-                 dw2: torch.Tensor, after_dw2=None):
+    def backward(self, grad_out: Optional[torch.Tensor], rs: RouteState, weights: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, dw13: torch.Tensor,
+                 dw2: torch.Tensor, after_dw2=None, mean_square=None):
         """Returns (grad_x [T, H], grad_weights [T, K]); fills dw13 / dw2. ``after_dw2()`` is called
-        as soon as the W2 gradient kernel is queued (nothing later in the pass reads W2)."""
+        as soon as the W2 gradient kernel is queued (nothing later in the pass reads W2).
+        ``mean_square = (h, out, grad_loss, grad_out)``: the gradient to start from is that of mean((h + out)^2); it is made on
+        the way and left in ``grad_out``."""
         C = self._C
         T = rs.topk_idx.shape[0]
+        if mean_square is not None:
+            h, out, grad_loss, grad_out = mean_square
         dev = grad_out.device
         grad_w = torch.empty(T, self.K, dtype=torch.float32, device=dev)
-        # d(weights): <grad_out[t], y_row(t, j)> - the expert outputs are still in place on the peers.
-        C.combine_pull(self.comm.heap, self.E, rs.topk_idx, rs.dest_row, None, self._off(self.y), self._flag_off(1), rs.epoch, None, grad_out, grad_w,
-                       self.H, self.status, self.timeout_ns, self.comm_ctas, 0)
-        # Transposed combine: push w * grad_out to the expert rows (channel 1).
         C.zero_pad_rows(self.dy_recv, rs.group_off, rs.group_rows, self.pad_align)
-        C.dispatch_push(self.comm.heap, grad_out, rs.topk_idx, weights, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, False, False,
+        # Transposed combine: push w * grad_out to the expert rows (channel 1); on the way d(weights): <grad_out[t], y_row(t, j)> -
+        # the expert outputs are still in place on the peers.
+        src, extra = (grad_out, ()) if mean_square is None else (h, (out, grad_out, grad_loss, 2.0 / max(T * self.H, 1)))
+        C.dispatch_push(self.comm.heap, src, rs.topk_idx, weights, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, False, False,
                         self._off(self.dy_recv), 0, self.arrive._symm_off + self.El * 8, self._flag_off(2), rs.epoch, self.status, self.timeout_ns,
-                        self.comm_ctas, None)
+                        self.comm_ctas, None, 0, 0, None, None, None, grad_w, self._off(self.y), *extra)
         gate = (self._arrive_ptr(1), self.arrive_target[1]) if self.comm.world > 1 else None
         if gemm.USE_PAIR:  # d(act) never leaves the tensor memory: the dgrad epilogue applies the SwiGLU backward
             gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dgu, gate=gate, swiglu_bwd_of=self.gu, **self._live(rs))

@@ -290,6 +290,34 @@ def test_embedding_gradient_of_any_length(T, V, H, spread):
     assert bool((table.grad[torch.bincount(ids, minlength=V) == 0] == 0).all())
 
 
+@pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 256, 4, 2), (127, 512, 256, 8, 2), (130, 1024, 256, 12, 3), (700, 2048, 256, 8, 2)])
+def test_loss_inside_the_layer_matches_the_separate_ops(T, H, I, E, K):
+    """mean((h + MoE(RMSNorm(h)))^2) with loss and gradients made inside combine, the backward dispatch and the norm's backward,
+    against the same layer followed by the separate residual loss. Twice: tickets are clean for the next step."""
+    from fast_b200.models import MoELayer
+    from fast_b200.ops import fused
+    from fast_b200.parallel import Communicator
+
+    comm = Communicator(heap_bytes=256 << 20, device=0)
+    layer = MoELayer(comm, H, I, E, K, max_tokens=T)
+    assert layer.engine.can_fuse_gate()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    nw = (1.0 + 0.1 * torch.randn(H, generator=g, device="cuda")).to(torch.bfloat16).requires_grad_()
+    for _ in range(2):
+        h0 = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+        got = []
+        for inside in (True, False):
+            h = h0.clone().requires_grad_()
+            for p in (nw, layer.gate, layer.w13, layer.w2):
+                p.grad = None
+            loss = layer.mean_square_from_residual(h, nw, 1e-5) if inside else fused.residual_mean_square(h, layer.forward_from_residual(h, nw, 1e-5))
+            (loss * 3.0).backward()
+            comm.check()
+            got.append([loss.detach(), h.grad, nw.grad, layer.gate.grad, layer.w13.grad, layer.w2.grad])
+        for a, b in zip(*got):
+            assert _rel(a, b) < 2e-2
+
+
 def test_fused_embedding_and_loss_match_torch():
     from fast_b200.ops import fused
 
