@@ -291,7 +291,8 @@ struct DispatchArgs {
   float grad_factor;
   long long recv_heap_off;     // destination rows: bf16 [cap, H] (or u8 [cap, H] when fp8)
   long long scale_heap_off;    // fp8 only: float [cap, H/128]
-  long long arrive_heap_off;   // u64 arrival counters of this channel: [E/world] per expert, or [num_tiles] per tile
+  long long arrive_heap_off;   // u64 arrival counters of this channel: [E/world] per expert, or [num_tiles] per tile;
+                               // < 0: not counted, nobody waits for single rows
   int tile_rows, num_tiles;    // tile_rows > 0: arrivals are counted per tile of that many destination rows (num_tiles per rank)
   long long entry_flags_heap_off;  // u64 [world]; used when entry_epoch != 0
   unsigned long long entry_epoch;

@@ -37,6 +37,15 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return v;
 }
 
+__device__ __forceinline__ uint4 add8(const uint4& a, const uint4& b) {
+  uint4 v;
+  const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&a), *y = reinterpret_cast<const __nv_bfloat162*>(&b);
+  __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = __hadd2_rn(x[i], y[i]);
+  return v;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -136,8 +145,10 @@ __global__ void __launch_bounds__(kCommThreads) quantise_rows_kernel(const __nv_
 // DOT (backward): the row on its way out (w * grad) meets the expert's output row that lies at the same place of the owner's
 // forward buffer, and their product is the gradient of w: one reading of the gradient rows serves both. With a.sum_with
 // the gradient itself is made here, from the two terms whose mean square is the loss.
-template <bool FP8, bool SORTED, bool SCALED, bool ROUNDED = false, bool DOT = false>
-__global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispatch_push_kernel(const DispatchArgs a) {
+// KM: most destinations of a token, K <= KM (2 or 8): with 2 the rows of all of them are requested at once, and no empty slots
+// are walked.
+template <bool FP8, bool SORTED, bool SCALED, bool ROUNDED = false, bool DOT = false, int KM = kMaxK>
+__global__ void __launch_bounds__(kCommThreads, DOT ? (KM <= 2 ? 3 : 2) : SORTED || KM <= 2 ? 4 : 3) dispatch_push_kernel(const DispatchArgs a) {
   extern __shared__ int s_cnt[];  // rows this CTA sent: [E] per expert, or [world][num_tiles] per destination tile
   __shared__ int s_ok;
   __shared__ __align__(16) float s_scales[(kCommThreads / 32) * kMaxScaleGroups];  // fp8 mode: the 1x128 scales of the row each warp is sending
@@ -147,7 +158,9 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispat
   const float gscale = DOT && a.sum_with != nullptr ? *a.grad_loss * a.grad_factor : 0.0f;
   const int E = a.num_experts, El = E / a.world;
   const int n_cnt = a.tile_rows > 0 ? a.world * a.num_tiles : E;
-  for (int e = threadIdx.x; e < n_cnt; e += blockDim.x) s_cnt[e] = 0;
+  const bool counted = a.arrive_heap_off >= 0;   // somebody waits for the rows while this kernel runs
+  if (counted)
+    for (int e = threadIdx.x; e < n_cnt; e += blockDim.x) s_cnt[e] = 0;
   if (threadIdx.x == 0) s_ok = 1;
   if (*reinterpret_cast<volatile unsigned long long*>(&a.status->abort) != 0ull) return;  // an earlier kernel of this rank refused the step
   __syncthreads();
@@ -173,7 +186,7 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispat
   // Sorted mode (send_list != null): one warp per (token, slot) entry, entries ordered by
   // (local expert index, destination rank counted from the sender upwards), so that every rank's expert 0 fills first, then
   // expert 1, ... and the gated GEMM of the receivers can start while later experts still arrive.
-  constexpr int NJ = SORTED ? 1 : kMaxK;  // destinations one warp serves
+  constexpr int NJ = SORTED ? 1 : KM;  // destinations one warp serves
   const long long n_work = SORTED ? static_cast<long long>(a.T) * a.K : a.T;
   // Adds this CTA's row counts to the receivers' arrival counters (release: the rows are stored before the counters move)
   // and clears them. Called by every thread of the CTA.
@@ -228,7 +241,7 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispat
           if (ROUNDED) out_row[j] = reinterpret_cast<unsigned char*>(a.local_rows + static_cast<long long>(row) * a.H);
           else out_row[j] = static_cast<unsigned char*>(a.peer_table[e / El]) + a.recv_heap_off + static_cast<long long>(row) * a.H * (FP8 ? 1 : 2);
           if (SCALED) scale[j] = a.row_scale[tj];
-          if (first) atomicAdd(&s_cnt[a.tile_rows > 0 ? (e / El) * a.num_tiles + min(row / a.tile_rows, a.num_tiles - 1) : e], 1);
+          if (first && counted) atomicAdd(&s_cnt[a.tile_rows > 0 ? (e / El) * a.num_tiles + min(row / a.tile_rows, a.num_tiles - 1) : e], 1);
         }
       }
       const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<long long>(t) * a.H);
@@ -239,46 +252,43 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispat
         float dots[NJ];
 #pragma unroll
         for (int j = 0; j < NJ; ++j) dots[j] = 0.0f;
-        constexpr int U = 4;
+        constexpr int U = KM <= 2 ? 2 : 1;
         const int rounds = chunks / 32, c_end = rounds * (part + 1) / wpr * 32;
         for (int c0 = rounds * part / wpr * 32 + lane; c0 < c_end; c0 += 32 * U) {
-          uint4 v[U];
+          uint4 v[U], w[U], y[NJ][U];   // every load of the pass is in flight before the first value is used
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            if (c0 + 32 * u < c_end) v[u] = __ldg(src + c0 + 32 * u);
-          if (sum_with != nullptr) {
-            uint4 w[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (c0 + 32 * u < c_end) w[u] = __ldg(sum_with + c0 + 32 * u);
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              if (c0 + 32 * u >= c_end) break;
-              float f[8], h[8];
-              unpack8(v[u], f);
-              unpack8(w[u], h);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(__float2bfloat16_rn(f[i] + h[i])) * gscale;
-              v[u] = pack8(f);
-              grad_out[c0 + 32 * u] = v[u];
+            if (c0 + 32 * u < c_end) {
+              v[u] = __ldg(src + c0 + 32 * u);
+              if (sum_with != nullptr) w[u] = __ldg(sum_with + c0 + 32 * u);
             }
-          }
 #pragma unroll
           for (int j = 0; j < NJ; ++j) {
             if (j >= nj || out_row[j] == nullptr) continue;
-            uint4 y[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-              if (c0 + 32 * u < c_end) y[u] = __ldcg(reinterpret_cast<const uint4*>(out_row[j] + to_y) + c0 + 32 * u);
+              if (c0 + 32 * u < c_end) y[j][u] = __ldcg(reinterpret_cast<const uint4*>(out_row[j] + to_y) + c0 + 32 * u);
+          }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              if (c0 + 32 * u >= c_end) break;
-              float f[8], h[8];
-              unpack8(v[u], f);
-              unpack8(y[u], h);
+          for (int u = 0; u < U; ++u) {
+            if (c0 + 32 * u >= c_end) break;
+            float f[8];
+            if (sum_with != nullptr) {
+              unpack8(add8(v[u], w[u]), f);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) { dots[j] = fmaf(f[i], h[i], dots[j]); f[i] *= scale[j]; }
-              reinterpret_cast<uint4*>(out_row[j])[c0 + 32 * u] = pack8(f);
+              for (int i = 0; i < 8; ++i) f[i] *= gscale;
+              v[u] = pack8(f);
+              grad_out[c0 + 32 * u] = v[u];
+            }
+            unpack8(v[u], f);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+              if (j >= nj || out_row[j] == nullptr) continue;
+              float h[8];
+              unpack8(y[j][u], h);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) { dots[j] = fmaf(f[i], h[i], dots[j]); h[i] = f[i] * scale[j]; }
+              reinterpret_cast<uint4*>(out_row[j])[c0 + 32 * u] = pack8(h);
             }
           }
         }
@@ -410,14 +420,16 @@ __global__ void __launch_bounds__(kCommThreads, SORTED ? 4 : DOT ? 2 : 3) dispat
         if (wpr > 1) __syncthreads(); else __syncwarp();  // the next row reuses my_scales
       }
     }  // wi < n_work
-    if (SORTED && (++round % kPublishRounds) == 0 && base + round_stride < n_work) publish_counts();
+    if (SORTED && counted && (++round % kPublishRounds) == 0 && base + round_stride < n_work) publish_counts();
   }
-  publish_counts();
+  if (counted) publish_counts();
 }
 
-// LOSS: the rows are also added to a.residual and squared on their way out.
-template <bool LOSS>
-__global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const CombineArgs a) {
+// LOSS: the rows are also added to a.residual and squared on their way out. KM: most rows a token has, K <= KM. With 2 the kernel
+// keeps 3 or 4 blocks on an SM, with 8 two, and walks no slots that are not there: under the GEMMs'
+// power cap the issue slots of an SM are as short as its bandwidth.
+template <bool LOSS, int KM>
+__global__ void __launch_bounds__(kCommThreads, KM > 2 ? 2 : LOSS ? 3 : 4) combine_pull_kernel(const CombineArgs a) {
   __shared__ int s_ok;
   grid_dependency_wait();
   launch_dependents();
@@ -447,10 +459,10 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
   for (long long u = blockIdx.x * wpb + warp; u < static_cast<long long>(a.T) * segs; u += gridDim.x * wpb) {
     const int t = static_cast<int>(u / segs), seg = static_cast<int>(u % segs);
     const int c_end = rounds * (seg + 1) / segs * 32;
-    const uint4* rows[kMaxK];
-    float w[kMaxK];
+    const uint4* rows[KM];
+    float w[KM];
 #pragma unroll
-    for (int j = 0; j < kMaxK; ++j) {
+    for (int j = 0; j < KM; ++j) {
       rows[j] = nullptr; w[j] = 0.0f;
       if (j < a.K) {
         const long long tj = static_cast<long long>(t) * a.K + j;
@@ -468,7 +480,7 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
       uint4* out = reinterpret_cast<uint4*>(a.out + static_cast<long long>(t) * a.H);
       constexpr int U = 2;  // two chunks x K rows of peer loads in flight per lane
       for (int c0 = rounds * seg / segs * 32 + lane; c0 < c_end; c0 += 32 * U) {
-        uint4 v[U][kMaxK], res[U];
+        uint4 v[U][KM], res[U];
         if (LOSS) {
           const uint4* h = reinterpret_cast<const uint4*>(a.residual + static_cast<long long>(t) * a.H);
 #pragma unroll
@@ -478,7 +490,7 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
-          for (int j = 0; j < kMaxK; ++j)
+          for (int j = 0; j < KM; ++j)
             if (j < a.K && c0 + 32 * u < c_end) v[u][j] = rows[j] ? __ldcg(rows[j] + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -486,7 +498,7 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
           if (c >= c_end) break;
           float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-          for (int j = 0; j < kMaxK; ++j) {
+          for (int j = 0; j < KM; ++j) {
             if (j >= a.K) break;
             float f[8];
             unpack8(v[u][j], f);
@@ -496,24 +508,23 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
           const uint4 o = pack8(acc);
           out[c] = o;
           if (LOSS) {
-            float f[8], h[8];
-            unpack8(o, f);
-            unpack8(res[u], h);
+            float q[8];
+            unpack8(add8(o, res[u]), q);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { const float q = __bfloat162float(__float2bfloat16_rn(h[i] + f[i])); square = fmaf(q, q, square); }
+            for (int i = 0; i < 8; ++i) square = fmaf(q[i], q[i], square);
           }
         }
       }
     } else {
       const uint4* g = reinterpret_cast<const uint4*>(a.dot_with + static_cast<long long>(t) * a.H);
-      float dots[kMaxK];
+      float dots[KM];
 #pragma unroll
-      for (int j = 0; j < kMaxK; ++j) dots[j] = 0.0f;
+      for (int j = 0; j < KM; ++j) dots[j] = 0.0f;
       for (int c = lane; c < chunks; c += 32) {
         float gf[8];
         unpack8(__ldg(g + c), gf);
 #pragma unroll
-        for (int j = 0; j < kMaxK; ++j) {
+        for (int j = 0; j < KM; ++j) {
           if (j >= a.K) break;
           float f[8];
           unpack8(rows[j] ? __ldcg(rows[j] + c) : make_uint4(0, 0, 0, 0), f);
@@ -522,7 +533,7 @@ __global__ void __launch_bounds__(kCommThreads) combine_pull_kernel(const Combin
         }
       }
 #pragma unroll
-      for (int j = 0; j < kMaxK; ++j) {
+      for (int j = 0; j < KM; ++j) {
         if (j >= a.K) break;
         float d = dots[j];
 #pragma unroll
@@ -590,10 +601,12 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
     return e;
   };
   const bool sorted = a.send_list != nullptr, scaled = a.row_scale != nullptr;
-  if (a.dot_out != nullptr) return go(dispatch_push_kernel<false, false, true, false, true>);
+  const bool few = a.K <= 2 && !sorted && !a.fp8;
+  if (a.dot_out != nullptr) return few ? go(dispatch_push_kernel<false, false, true, false, true, 2>) : go(dispatch_push_kernel<false, false, true, false, true>);
   if (a.local_rows != nullptr) return go(dispatch_push_kernel<false, false, false, true>);
   if (a.fp8) return sorted ? go(dispatch_push_kernel<true, true, false>) : go(dispatch_push_kernel<true, false, false>);
   if (sorted) return scaled ? go(dispatch_push_kernel<false, true, true>) : go(dispatch_push_kernel<false, true, false>);
+  if (few) return scaled ? go(dispatch_push_kernel<false, false, true, false, false, 2>) : go(dispatch_push_kernel<false, false, false, false, false, 2>);
   return scaled ? go(dispatch_push_kernel<false, false, true>) : go(dispatch_push_kernel<false, false, false>);
 }
 
@@ -609,10 +622,13 @@ cudaError_t launch_combine_pull(const CombineArgs& a, int ctas, cudaStream_t str
   if (a.K < 1 || a.K > kMaxK || a.H % 256 || a.world < 1 || a.num_experts % a.world || ctas < 1) return cudaErrorInvalidValue;
   if (a.residual != nullptr && (a.out == nullptr || a.loss_partials == nullptr || a.ticket == nullptr || a.loss == nullptr || ctas > kMaxLossPartials)) return cudaErrorInvalidValue;
   if (a.T == 0) return cudaSuccess;
+  if (a.residual != nullptr) ctas = std::max(1, ctas * 3 / 4);   // a grid of four blocks per SM; three of this variant fit
   CombineArgs b = a;
   // Few tokens: as many warps per row as fill the grid, down to one round of loads per warp.
   b.segments = a.dot_out != nullptr ? 1 : static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / a.T, 1, a.H / 256));
-  cudaError_t e = launch_early(a.residual != nullptr ? combine_pull_kernel<true> : combine_pull_kernel<false>, dim3(ctas), kCommThreads, 0, stream, b);
+  cudaError_t e = launch_early(a.K <= 2 ? (a.residual != nullptr ? combine_pull_kernel<true, 2> : combine_pull_kernel<false, 2>)
+                                      : (a.residual != nullptr ? combine_pull_kernel<true, kMaxK> : combine_pull_kernel<false, kMaxK>),
+                               dim3(ctas), kCommThreads, 0, stream, b);
   if (e == cudaSuccess) note_launch();
   return e;
 }

@@ -183,6 +183,11 @@ class ExpertParallel:
     def _arrive_ptr(self, ch: int) -> int:
         return self.arrive.data_ptr() + ch * self.arrive.shape[1] * 8
 
+    def _arrive_off(self, ch: int) -> int:
+        """Where a dispatch counts its rows in; nowhere when the rows are complete with the kernel anyway (one rank, one stream):
+        a system-wide fence and an atomic per block and expert cost more than the few rows of a block."""
+        return -1 if self.comm.world == 1 and not self.overlap else self.arrive._symm_off + ch * self.El * 8
+
     def _needs_zero_pads(self) -> bool:
         """Whether rows past an expert's real ones are computed with: by the one-CTA GEMM always, else by weight gradients only."""
         return self.training or not gemm.USE_PAIR
@@ -282,12 +287,12 @@ class ExpertParallel:
         try:
             if self.fp8:
                 C.dispatch_push(self.comm.heap, x, rs.topk_idx, None, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, True, True,
-                                self._off(self.xq_recv), self._off(self.xs_recv), self.arrive._symm_off, 0, 0, self.status, self.timeout_ns,
+                                self._off(self.xq_recv), self._off(self.xs_recv), self._arrive_off(0), 0, 0, self.status, self.timeout_ns,
                                 4 * self.overlap_reserve_sms if self.overlap else self.comm_ctas, send_list, self.tile_rows, self.ntiles, xq, xs,
                                 self.x_recv if self.local_bf16 else None)
             else:
                 C.dispatch_push(self.comm.heap, x, rs.topk_idx, None, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, True, False,
-                                self._off(self.x_recv), 0, self.arrive._symm_off, 0, 0, self.status, self.timeout_ns,
+                                self._off(self.x_recv), 0, self._arrive_off(0), 0, 0, self.status, self.timeout_ns,
                                 4 * self.overlap_reserve_sms if self.overlap else self.comm_ctas, send_list, self.tile_rows, self.ntiles)
         finally:
             if self.overlap:
@@ -384,7 +389,7 @@ class ExpertParallel:
         # the expert outputs are still in place on the peers.
         src, extra = (grad_out, ()) if mean_square is None else (h, (out, grad_out, grad_loss, 2.0 / max(T * self.H, 1)))
         C.dispatch_push(self.comm.heap, src, rs.topk_idx, weights, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, False, False,
-                        self._off(self.dy_recv), 0, self.arrive._symm_off + self.El * 8, self._flag_off(2), rs.epoch, self.status, self.timeout_ns,
+                        self._off(self.dy_recv), 0, self._arrive_off(1), self._flag_off(2), rs.epoch, self.status, self.timeout_ns,
                         self.comm_ctas, None, 0, 0, None, None, None, grad_w, self._off(self.y), *extra)
         gate = (self._arrive_ptr(1), self.arrive_target[1]) if self.comm.world > 1 else None
         if gemm.USE_PAIR:  # d(act) never leaves the tensor memory: the dgrad epilogue applies the SwiGLU backward
