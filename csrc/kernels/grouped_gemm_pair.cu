@@ -136,7 +136,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             gated = slot;
           }
         }
-        for (int kb = 0; kb < tc.red_blocks; ++kb, ++it) {
+        // Weight gradients: every other wave walks the reduction backwards, from the panel ends that the wave before left in L2.
+        const bool back = MODE == GemmMode::kWgrad && ((tile / pairs) & 1);
+        for (int kbi = 0; kbi < tc.red_blocks; ++kbi, ++it) {
+          const int kb = back ? tc.red_blocks - 1 - kbi : kbi;
           const int s = it % NS;
           const uint32_t ph = (it / NS) & 1;
           if (!(ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1, abort_flag, p.status, 100 + s, p.timeout_ns))) break;

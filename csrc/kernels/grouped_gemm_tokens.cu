@@ -205,6 +205,9 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         const int half = tc.n >> 1, x_row = tc.row0 + cta * half;
         const int n32 = half == 128 ? 0 : half >> 5, n16 = half == 128 ? 0 : (half >> 4) & 1;
         const uint32_t bytes = 2u * (kABytes + static_cast<uint32_t>(half) * 128u);
+        // Every other wave walks the reduction backwards: it starts on the ends of the panels that the wave before left in L2.
+        const bool back = sg.parts == 1 && (((sg.tile - split.cut_tiles) / pairs) & 1);
+        auto k_of = [&](int kb) { return (back ? p.red_blocks - 1 - kb : kb) * BK; };
         auto load_w = [&](int kb, int st) {
           uint8_t* sa = tiles + st * stage_size;
           const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[st]), 0);
@@ -212,11 +215,11 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
           if (A_MN) {
 #pragma unroll
             for (int j = 0; j < kHalfM / 64; ++j)
-              tma_load_2d_pair(sa + j * (BK * 128), &map_w, tc.m * kPairM + cta * kHalfM + j * 64, tc.g * p.w_rows_per_group + kb * BK, full_leader);
+              tma_load_2d_pair(sa + j * (BK * 128), &map_w, tc.m * kPairM + cta * kHalfM + j * 64, tc.g * p.w_rows_per_group + k_of(kb), full_leader);
           } else if (EPI == GemmEpilogue::kSwiGLU) {
-            tma_load_5d_pair(sa, &map_w, kb * BK, 0, 0, cta * 4, tc.g * p.m_tiles + tc.m, full_leader);
+            tma_load_5d_pair(sa, &map_w, k_of(kb), 0, 0, cta * 4, tc.g * p.m_tiles + tc.m, full_leader);
           } else {
-            tma_load_2d_pair(sa, &map_w, kb * BK, tc.g * p.w_rows_per_group + tc.m * kPairM + cta * kHalfM, full_leader);
+            tma_load_2d_pair(sa, &map_w, k_of(kb), tc.g * p.w_rows_per_group + tc.m * kPairM + cta * kHalfM, full_leader);
           }
         };
         const int early = first ? min(sg.kb1, sg.kb0 + stages) : sg.kb0;   // blocks whose weights are requested now
@@ -241,9 +244,9 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
           }
           uint8_t* sb = tiles + s * stage_size + kABytes;
           const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
-          if (half == 128) tma_load_2d_pair(sb, &map_x128, kb * BK, x_row, full_leader);
-          for (int j = 0; j < n32; ++j) tma_load_2d_pair(sb + j * 4096, &map_x32, kb * BK, x_row + 32 * j, full_leader);
-          if (n16) tma_load_2d_pair(sb + n32 * 4096, &map_x16, kb * BK, x_row + 32 * n32, full_leader);
+          if (half == 128) tma_load_2d_pair(sb, &map_x128, k_of(kb), x_row, full_leader);
+          for (int j = 0; j < n32; ++j) tma_load_2d_pair(sb + j * 4096, &map_x32, k_of(kb), x_row + 32 * j, full_leader);
+          if (n16) tma_load_2d_pair(sb + n32 * 4096, &map_x16, k_of(kb), x_row + 32 * n32, full_leader);
           if (++s == stages) { s = 0; ph ^= 1; }
         }
       }

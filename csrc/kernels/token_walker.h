@@ -104,6 +104,15 @@ struct TokSegments {
 
 // Place of tile `local` inside its group: bands of `band` token tiles, token tiles fastest inside a band, so that the
 // tiles that run together cover a squarish patch and share their operand panels in L2.
+// How many: as the reduction grows, fewer, so that the token panels of a band take at most half of the L2 while the weights
+// stream past them; at most 8, where a wave of 74 tiles is square. What this saves is the power that moving operands costs,
+// and with it clock: 8 experts of 8192 tokens, seconds at the power cap, TFLOP/s at
+// bands of 16, 8, 4 tiles: reduction of 4096 1312, 1396, 1340; of 14336 1115, 1353, 1356; of 28672 1050, 1267, 1315.
+constexpr int kTokBandBytes = 60 << 20, kTokBandTiles = 8;
+FASTB_HD inline int tok_band_tiles(int red_len) {
+  const long long fit = kTokBandBytes / (2ll * red_len * kTokTileN);
+  return fit < 1 ? 1 : fit > kTokBandTiles ? kTokBandTiles : static_cast<int>(fit);
+}
 struct TokPlace { int m, t; };
 FASTB_HD inline TokPlace tok_place(int local, int m_tiles, int t_tiles, int band_tiles) {
   const int per_band = band_tiles * m_tiles, band = local / per_band, rem = local - band * per_band;

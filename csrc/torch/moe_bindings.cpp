@@ -2,6 +2,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "../kernels/token_walker.h"
 #include "py_types.h"
 
 namespace py = pybind11;
@@ -121,7 +122,7 @@ struct TokGemmPlan {
     if (has_c2) c2 = bf16_map_2d(*gate_up, 32);
     a.num_groups = static_cast<int>(G);
     a.m_tiles = static_cast<int>(feats / 256); a.red_blocks = static_cast<int>(red / 64); a.w_rows_per_group = static_cast<int>(N);
-    a.band_tiles = std::max(1, (band_rows > 0 ? band_rows : 4096) / 256);
+    a.band_tiles = band_rows > 0 ? std::max(1, band_rows / 256) : gemm::tok_band_tiles(static_cast<int>(red));
     a.granule = granule; a.keep_gate_up = fwd && has_c2 ? 1 : 0;
   }
 
