@@ -1,5 +1,5 @@
 // Threaded host twin of the expert-parallel MoE step: the synchronisation structure of
-// splits_scan / dispatch_push / gated grouped GEMMs / peer_signal / combine_pull and of the backward
+// splits_scan / dispatch_push / gated grouped GEMMs / combine_pull with its ready flags and of the backward
 // pass (fast_b200/parallel/ep.py, csrc/kernels/moe_route.cu, moe_comm.cu), with std::atomic for
 // every flag and counter and plain memory for every payload buffer that peers read or write.
 // One thread per rank plays the stream (kernels in order, each kernel = a few worker threads that
@@ -207,7 +207,7 @@ void run_rank(World& w, int me) {
     parallel(kWorkers, gemms);
     if (side.joinable()) side.join();  // the main stream re-joins the side stream before it signals
     if (w.abort.load()) return;
-    for (int p = 0; p < W; ++p) w.r[p]->flags[1 * W + me].store(epoch, std::memory_order_release);  // peer_signal: my y is complete
+    for (int p = 0; p < W; ++p) w.r[p]->flags[1 * W + me].store(epoch, std::memory_order_release);  // combine's block 0: my y is complete
     // ---- combine_pull: every token pulls its K rows from the owners and sums them ------------------
     auto pull = [&](int flag_row, bool from_dx, const std::function<uint32_t(int, int, int)>& expect) {
 #ifndef FASTB_MOE_TWIN_NO_READY_WAIT  // defining it drops the wait for the owners' ready flags: the race detector must object
