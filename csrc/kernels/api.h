@@ -128,9 +128,12 @@ cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUte
 constexpr int kTokPartialFloats = 128 * 256;   // fp32 sums of one CTA's part of a tile
 constexpr int tok_counters(int ctas) { return 2 * ctas; }                                  // arrival counters a launch needs
 constexpr long long tok_partial_floats(int ctas) { return 2ll * ctas * kTokPartialFloats; }  // two partial tiles per CTA
+// Maps of the tokens: entry j loads boxes of {64, 16 << j}. Half a tile's tokens (a multiple of 16 up to 128) are at most three.
+constexpr int kTokBoxes = 4;
+struct TokMapsX { CUtensorMap box[kTokBoxes]; };
 struct TokGemmMaps {   // bf16, 128-byte swizzle; boxes {inner, outer}
   const CUtensorMap* w;      // forward store {64,128}; forward SwiGLU 5-D {64,16,2,4,1} over [tile][16-row group][gate|up][16][K]; dgrad {64,64}
-  const CUtensorMap *x128, *x32, *x16;   // tokens: {64,128}, {64,32}, {64,16}
+  const TokMapsX* x;
   const CUtensorMap* c;      // output {64,32}
   const CUtensorMap* c2;     // gate|up: written by the SwiGLU forward (keep_gate_up), read by the SwiGLU backward {64,32}; else null
 };
@@ -144,6 +147,7 @@ struct TokGemmArgs {
   int tile_n;                // most tokens of a tile: 64, 128 or 256
   int stages;                // set by the launcher
   int band_tiles;            // token tiles of a raster band
+  int back_tiles;            // groups of more token tiles than this alternate the direction of the reduction from wave to wave
   int granule;               // tile widths are multiples of this (32 or 64); rows up to a multiple of it are written
   int keep_gate_up;
   int early;                 // 1: weights, group_off and group_rows were written by no kernel later than the last but one of the stream

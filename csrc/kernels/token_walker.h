@@ -17,12 +17,17 @@ FASTB_HD constexpr int ceil_to(int x, int q) { return (x + q - 1) / q * q; }
 FASTB_HD constexpr int div_up(int a, int b) { return (a + b - 1) / b; }
 
 // Token tiles of a group whose tokens are taken up to `rows` (real rows rounded up to the granule, a multiple of 32): as few
-// as hold them, all but the last of one width, in multiples of 32. 640 tokens are 3 tiles of 224, 224 and 192 instead of
-// 256, 256 and 128: tiles that run side by side then advance at one pace and keep sharing operand panels.
+// as hold them, their widths as even as multiples of 32 allow. 1056 tokens are 3 tiles of 224 and 2 of 192, not 4 of 224 and one
+// of 160: tiles that run side by side then advance at about one pace and keep sharing operand panels.
 FASTB_HD inline int tok_tiles(int rows, int tile_n) { return div_up(rows, tile_n); }
-FASTB_HD inline int tok_tile_size(int rows, int tile_n) {
+FASTB_HD inline int tok_tile_size(int rows, int tile_n) {   // the widest
   const int t = tok_tiles(rows, tile_n);
   return t > 0 ? ceil_to(div_up(rows, t), 32) : 0;
+}
+struct TokSpan { int begin, n; };
+FASTB_HD inline TokSpan tok_span(int rows, int tile_n, int i) {
+  const int t = tok_tiles(rows, tile_n), units = rows / 32, base = units / t, extra = units - base * t;
+  return TokSpan{32 * (i * base + (i < extra ? i : extra)), 32 * (base + (i < extra ? 1 : 0))};
 }
 
 // How `tiles` tiles of kb_tile reduction blocks are spread over `pairs` CTA pairs. Whole tiles go round robin; where the last
@@ -112,6 +117,10 @@ constexpr int kTokBandBytes = 60 << 20, kTokBandTiles = 8;
 FASTB_HD inline int tok_band_tiles(int red_len) {
   const long long fit = kTokBandBytes / (2ll * red_len * kTokTileN);
   return fit < 1 ? 1 : fit > kTokBandTiles ? kTokBandTiles : static_cast<int>(fit);
+}
+// From how many token tiles of a group on alternating the direction of the reduction pays (grouped_gemm_tokens.cu).
+FASTB_HD inline int tok_back_tiles(int red_len, int band_tiles) {
+  return 2ll * red_len * kTokTileN * band_tiles > kTokBandBytes / 2 ? band_tiles : 1 << 30;
 }
 struct TokPlace { int m, t; };
 FASTB_HD inline TokPlace tok_place(int local, int m_tiles, int t_tiles, int band_tiles) {

@@ -88,7 +88,8 @@ CUtensorMap bf16_map_2d(const torch::Tensor& t, int box_rows) {
 // One contraction on fixed buffers (weights, tokens, outputs): everything about the launch of grouped_gemm_tokens that does not
 // change from call to call, the tensor maps above all.
 struct TokGemmPlan {
-  alignas(64) CUtensorMap w, x128, x32, x16, c, c2;
+  alignas(64) CUtensorMap w, c, c2;
+  TokMapsX x;
   GemmMode mode;
   GemmEpilogue epi;
   bool has_c2;
@@ -117,12 +118,13 @@ struct TokGemmPlan {
     } else {
       w = bf16_map_2d(weights.view({G * N, K}), fwd ? 128 : 64);
     }
-    x128 = bf16_map_2d(tokens, 128); x32 = bf16_map_2d(tokens, 32); x16 = bf16_map_2d(tokens, 16);
+    for (int j = 0; j < kTokBoxes; ++j) x.box[j] = bf16_map_2d(tokens, 16 << j);
     c = bf16_map_2d(out, 32);
     if (has_c2) c2 = bf16_map_2d(*gate_up, 32);
     a.num_groups = static_cast<int>(G);
     a.m_tiles = static_cast<int>(feats / 256); a.red_blocks = static_cast<int>(red / 64); a.w_rows_per_group = static_cast<int>(N);
     a.band_tiles = band_rows > 0 ? std::max(1, band_rows / 256) : gemm::tok_band_tiles(static_cast<int>(red));
+    a.back_tiles = gemm::tok_back_tiles(static_cast<int>(red), a.band_tiles);
     a.granule = granule; a.keep_gate_up = fwd && has_c2 ? 1 : 0;
   }
 
@@ -159,7 +161,7 @@ struct TokGemmPlan {
     g.num_counters = static_cast<int>(cnt.size(1));
     g.counters = base + (parity & 1) * g.num_counters;
     g.counters_next = base + (~parity & 1) * g.num_counters;
-    const TokGemmMaps maps{&w, &x128, &x32, &x16, &c, has_c2 ? &c2 : nullptr};
+    const TokGemmMaps maps{&w, &x, &c, has_c2 ? &c2 : nullptr};
     cu_check(launch_grouped_gemm_tokens(mode, epi, maps, g, ctas, stream_now()), "grouped_gemm_tokens launch");
   }
 };

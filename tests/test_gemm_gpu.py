@@ -212,6 +212,31 @@ def test_wgrad_stops_at_the_live_rows(kernel_variant):
         _close(out[i], dy[s:s + n].float().T @ x[s:s + n].float())
 
 
+@pytest.mark.parametrize("counts,N,K", [
+    ([2049, 33], 4608, 8192),   # forward: 9 token tiles in bands of at most 8, more than two waves, 2049 tokens in tiles of unequal width
+    ([4097, 4096, 65], 2560, 2048),   # weight gradient: 65, 64 and 2 reduction blocks, 80 tiles each
+])
+def test_reductions_walked_backwards(counts, N, K, kernel_variant):
+    """Sizes at which every other wave walks the reduction from its end: forward and weight gradient equal the fp32 product."""
+    if kernel_variant != "cta_pair":
+        pytest.skip("belongs to the CTA-pair kernels")
+    from fast_b200.ops import gemm
+
+    G = len(counts)
+    counts_t, off, R, a, w = _setup(G, N, K, counts, seed=29)
+    live = counts_t.to(torch.int32)
+    dy = torch.randn(R, N, generator=torch.Generator(device="cuda").manual_seed(31), device="cuda").to(torch.bfloat16)
+    o = off.tolist()
+    out, dw = torch.zeros(R, N, device="cuda", dtype=torch.bfloat16), torch.zeros_like(w)
+    gemm.grouped_gemm_fwd(a, w, off, out, live_rows=live, granule=32)
+    gemm.grouped_gemm_wgrad(dy, a, off, dw, live_rows=live)
+    gemm.check()
+    for i, n in enumerate(counts):
+        s = o[i]
+        _close(out[s:s + n], a[s:s + n].float() @ w[i].float().T)
+        _close(dw[i], dy[s:s + n].float().T @ a[s:s + n].float())
+
+
 def test_custom_operators_run_the_same_kernels():
     """torch.ops.fast_b200.* (schemas, mutation annotations) give the same bits as the direct calls."""
     from fast_b200.ops import gemm, registry  # noqa: F401
