@@ -14,14 +14,11 @@ struct Piece {
   int64_t off;  // units, inside `buf` of the GPU currently holding the piece
 };
 
-// Pieces waiting at one (source server, destination server, GPU): appended at the back, taken at the front. A vector and a
-// cursor: a std::deque allocates half a kilobyte for each of the S * S * G queues, most of which hold one piece.
+// Pieces waiting at one (source server, destination server, GPU): a range of one list, taken from the front. A container per
+// queue allocates S * S * G times, mostly for a single piece.
 struct PieceQueue {
-  std::vector<Piece> v;
-  size_t head = 0;
-  bool empty() const { return head == v.size(); }
-  Piece& front() { return v[head]; }
-  void pop_front() { ++head; }
+  size_t head = 0, end = 0;
+  bool empty() const { return head == end; }
 };
 
 // Largest cut <= want that keeps the remainder of `p` aligned inside its segment, or the whole
@@ -29,7 +26,8 @@ struct PieceQueue {
 int64_t aligned_cut(const Piece& p, int64_t want, int64_t align) {
   if (want >= p.len) return p.len;
   if (align <= 1) return want;
-  const int64_t end = (p.pair_off + want) / align * align;  // absolute cut position in the segment
+  const int64_t at = p.pair_off + want;
+  const int64_t end = (align & (align - 1)) == 0 ? at & -align : at / align * align;  // absolute cut position in the segment; no division per cut
   return end > p.pair_off ? end - p.pair_off : 0;
 }
 
@@ -94,6 +92,9 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
   // ---- balance: equalise the per-GPU load of every (src server, dst server) tile -------------
   // hold[(s*S+t)*G+i] = pieces GPU i of server s will put on its rail toward server t.
   std::vector<PieceQueue> hold(static_cast<size_t>(S) * S * G);
+  std::vector<Piece> pieces;
+  pieces.reserve(static_cast<size_t>(n) * n);   // about one piece per rank pair; balancing adds a few
+  std::vector<std::vector<Piece>> tile(G);      // the queues of the server pair at hand
   auto hold_at = [&](int s, int t, int i) -> PieceQueue& { return hold[(static_cast<size_t>(s) * S + t) * G + i]; };
 
   std::vector<int64_t> load(G, 0);
@@ -101,12 +102,13 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
     for (int t = 0; t < S; ++t) {
       if (s == t) continue;
       std::fill(load.begin(), load.end(), 0);
+      for (auto& q : tile) q.clear();
       int64_t sum = 0;
       for (int i = 0; i < G; ++i) {
         for (int j = 0; j < G; ++j) {
           const int64_t x = M.at(s * G + i, t * G + j);
           if (x == 0) continue;
-          hold_at(s, t, i).v.push_back(Piece{i, j, 0, x, Buf::kInput, in_at(s * G + i, t * G + j)});
+          tile[i].push_back(Piece{i, j, 0, x, Buf::kInput, in_at(s * G + i, t * G + j)});
           load[i] += x;
         }
         sum += load[i];
@@ -126,7 +128,7 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
       for (int big = 0; big < G && balance; ++big) {
         for (int small = 0; small < G && load[big] > target; ++small) {
           if (small == big || load[small] >= target) continue;
-          std::vector<Piece>& src = hold_at(s, t, big).v;   // nothing is taken from the front yet
+          std::vector<Piece>& src = tile[big];
           // Walk the heavy GPU's own pieces (only data still in its input buffer can be relayed).
           for (size_t k = 0; k < src.size() && load[big] > target && load[small] < target;) {
             Piece& pc = src[k];
@@ -139,7 +141,7 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
             if (keep(src_rank, dst_rank))
               p.ops.push_back(Op{Phase::kBalance, Buf::kInput, Buf::kBalance, -1, src_rank, dst_rank,
                                  src_rank, t * G + pc.final_local, pc.off, cursor, mv, pc.pair_off});
-            hold_at(s, t, small).v.push_back(Piece{pc.origin_local, pc.final_local, pc.pair_off, mv, Buf::kBalance, cursor});
+            tile[small].push_back(Piece{pc.origin_local, pc.final_local, pc.pair_off, mv, Buf::kBalance, cursor});
             cursor += mv;
             load[big] -= mv;
             load[small] += mv;
@@ -151,6 +153,11 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
             }
           }
         }
+      }
+      for (int i = 0; i < G; ++i) {
+        const size_t head = pieces.size();
+        pieces.insert(pieces.end(), tile[i].begin(), tile[i].end());
+        hold_at(s, t, i) = PieceQueue{head, pieces.size()};
       }
       p.server_matrix.at(s, t) = *std::max_element(load.begin(), load.end());
     }
@@ -187,7 +194,7 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
     if (q.empty()) return;
     const int src_rank = s * G + i, dst_rank = t * G + i;
     while (!q.empty() && budget != 0) {
-      Piece& pc = q.front();
+      Piece& pc = pieces[q.head];
       const int64_t take = budget < 0 ? pc.len : aligned_cut(pc, budget, opt.split_align);
       if (take == 0) break;
       const int origin = s * G + pc.origin_local, fin = t * G + pc.final_local;
@@ -206,7 +213,7 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
         cursor += take;
       }
       if (budget > 0) budget -= take;
-      if (take == pc.len) q.pop_front();
+      if (take == pc.len) ++q.head;
       else { pc.pair_off += take; pc.off += take; pc.len -= take; }
     }
   };

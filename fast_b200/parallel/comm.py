@@ -204,7 +204,7 @@ class Communicator:
                 chunk_bytes *= 2
         if "split_align" not in plan_opts:
             plan_opts["split_align"] = 16 // math.gcd(16, unit_bytes)
-        key = (sched.matrix_hash(m), unit_bytes, transpose, str(kind), chunk_bytes, rail_segment_bytes, tuple(sorted((k, str(v)) for k, v in plan_opts.items())))
+        key = (sched.matrix_hash(m), unit_bytes, transpose, sched.option_text(kind), chunk_bytes, rail_segment_bytes, tuple(sorted((k, sched.option_text(v)) for k, v in plan_opts.items())))
         s = self._sched_cache.get(key)
         if s is None:
             if kind == "auto":

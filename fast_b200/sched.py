@@ -43,6 +43,14 @@ workload_balanced = _S.workload_balanced
 workload_zipf_rows = _S.workload_zipf_rows
 workload_zipf_entries = _S.workload_zipf_entries
 
+_KIND_TEXT = {k.value: str(k) for k in (PlanKind.STAGED, PlanKind.FANOUT, PlanKind.SPREAD_OUT, PlanKind.SINGLE_BURST)}
+
+
+def option_text(v) -> str:
+    """``str(v)``; a plan kind's text is kept, because composing it takes 2.5 us and it is part of every plan's key, twice."""
+    return _KIND_TEXT[v.value] if type(v) is PlanKind else str(v)
+
+
 # Link presets: (alpha in us, beta in us per MB). The intra-server and inter-server classes and their
 # figures are those of the reference simulator's tables (simulation/scheduler/config.cpp:8-59), plus
 # the measured NVLink-5 port of a B200 (770 GB/s peer copy, ~2 us per hop).
@@ -52,6 +60,9 @@ INTRA_LINKS = {"DGX2": (0.1, 8.0), "FAST": (0.1, 1.0), "B100": (0.1, 1.2), "H100
                # measured 8-GPU skewed all-to-all(v) completion times (64 MiB - 1 GiB rows, Zipf 0 - 1.5)
                "B200_MEASURED": (44.0, 1e3 / 644.0)}
 INTER_LINKS = {"INFB": (1.7, 106.0), "ETHER100": (0.7, 84.0), "ETHER400": (0.7, 22.0)}
+
+
+_DEFAULT_INTER, _DEFAULT_INTRA = gbps_model(400.0, 0.7), nvlink_model(900.0, 0.1)
 
 
 def intra_link(name: str) -> "LinkModel":
@@ -104,7 +115,7 @@ def build_plan(matrix, topo: Topology, kind=PlanKind.STAGED, match=MatchPolicy.F
     """
     m = np.ascontiguousarray(matrix, dtype=np.int64)
     return _S.build_plan(m, topo.servers, topo.gpus, kind, match, scale_policy, scale, split_align, transpose,
-                         inter or gbps_model(400.0, 0.7), intra or nvlink_model(900.0, 0.1), mb_per_unit, balance_alpha_beta, only_rank)
+                         inter or _DEFAULT_INTER, intra or _DEFAULT_INTRA, mb_per_unit, balance_alpha_beta, only_rank)
 
 
 def select_plan(matrix, topo: Topology, inter: LinkModel, intra: LinkModel, mb_per_unit: float = 1.0, kinds=None,
@@ -140,7 +151,7 @@ class PlanCache:
 
     def get(self, matrix, topo: Topology, **opts) -> Plan:
         m = np.ascontiguousarray(matrix, dtype=np.int64)
-        key = (matrix_hash(m), topo.servers, topo.gpus, tuple(sorted((k, str(v)) for k, v in opts.items())))
+        key = (matrix_hash(m), topo.servers, topo.gpus, tuple(sorted((k, option_text(v)) for k, v in opts.items())))
         p = self._d.get(key)
         if p is None:
             self.misses += 1
