@@ -14,6 +14,7 @@
 
 #include <algorithm>
 
+#include "announce_blocks.h"
 #include "api.h"
 #include "early_start.cuh"
 #include "route_splits.cuh"
@@ -579,7 +580,8 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
   if (a.K < 1 || a.K > kMaxK || a.H % 256 || a.world < 1 || a.num_experts % a.world || ctas < 1) return cudaErrorInvalidValue;
   if (a.fp8 && a.H / 128 > kMaxScaleGroups) return cudaErrorInvalidValue;
   if ((a.xq != nullptr) != (a.xq_scales != nullptr) || (a.xq != nullptr && !a.fp8)) return cudaErrorInvalidValue;
-  if (a.T == 0) return cudaSuccess;
+  const bool announces = a.entry_epoch != 0 && a.world > 1;   // the peers wait for my entry flag, rows or none
+  if (a.T == 0 && !announces) return cudaSuccess;
   if (a.tile_rows < 0 || (a.tile_rows > 0 && a.num_tiles < 1)) return cudaErrorInvalidValue;
   if (a.local_rows != nullptr && (!a.fp8 || a.send_list != nullptr || a.row_scale != nullptr || a.world != 1)) return cudaErrorInvalidValue;
   if (a.dot_out != nullptr && (a.fp8 || a.send_list != nullptr || a.row_scale == nullptr)) return cudaErrorInvalidValue;
@@ -588,7 +590,7 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
   b.warps_per_row = a.send_list == nullptr && a.T <= ctas ? kCommThreads / 32 : 1;
   // No more CTAs than there is work for (entries of the sorted list, rows per CTA otherwise).
   const long long work = a.send_list != nullptr ? static_cast<long long>(a.T) * a.K : static_cast<long long>(a.T) * b.warps_per_row;
-  ctas = static_cast<int>(std::min<long long>(ctas, (work + kCommThreads / 32 - 1) / (kCommThreads / 32)));
+  ctas = announce_blocks(static_cast<int>(std::min<long long>(ctas, (work + kCommThreads / 32 - 1) / (kCommThreads / 32))), announces);
   const size_t smem = sizeof(int) * (a.tile_rows > 0 ? static_cast<size_t>(a.world) * a.num_tiles : static_cast<size_t>(a.num_experts));
   if (smem > 200 * 1024) return cudaErrorInvalidValue;  // per-CTA histogram of destination tiles must fit in shared memory
   auto go = [&](auto kern) {
@@ -621,11 +623,13 @@ cudaError_t launch_quantise_rows(const __nv_bfloat16* x, int T, int H, unsigned 
 cudaError_t launch_combine_pull(const CombineArgs& a, int ctas, cudaStream_t stream) {
   if (a.K < 1 || a.K > kMaxK || a.H % 256 || a.world < 1 || a.num_experts % a.world || ctas < 1) return cudaErrorInvalidValue;
   if (a.residual != nullptr && (a.out == nullptr || a.loss_partials == nullptr || a.ticket == nullptr || a.loss == nullptr || ctas > kMaxLossPartials)) return cudaErrorInvalidValue;
-  if (a.T == 0) return cudaSuccess;
   if (a.residual != nullptr) ctas = std::max(1, ctas * 3 / 4);   // a grid of four blocks per SM; three of this variant fit
+  // Without tokens of my own: the peers still wait for my ready flag.
+  ctas = announce_blocks(a.T > 0 ? ctas : 0, a.signal && a.world > 1 && (a.ready_epoch != 0 || a.epoch_dev != nullptr));
+  if (ctas == 0) return cudaSuccess;
   CombineArgs b = a;
   // Few tokens: as many warps per row as fill the grid, down to one round of loads per warp.
-  b.segments = a.dot_out != nullptr ? 1 : static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / a.T, 1, a.H / 256));
+  b.segments = a.dot_out != nullptr ? 1 : static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / std::max(a.T, 1), 1, a.H / 256));
   cudaError_t e = launch_early(a.K <= 2 ? (a.residual != nullptr ? combine_pull_kernel<true, 2> : combine_pull_kernel<false, 2>)
                                       : (a.residual != nullptr ? combine_pull_kernel<true, kMaxK> : combine_pull_kernel<false, kMaxK>),
                                dim3(ctas), kCommThreads, 0, stream, b);

@@ -21,13 +21,17 @@
 #include <thread>
 #include <vector>
 
+#include "../kernels/announce_blocks.h"
+
 namespace {
 
 constexpr int H = 4;        // words per row
 constexpr int RA = 4;       // group rows are padded to a multiple of this
 constexpr int kWorkers = 3;
 
-struct Cfg { int W, El, K, T, steps; bool training; bool bwd_entry_handshake; bool fp8 = false; bool overlap = false; bool tiles = false; };
+struct Cfg { int W, El, K, T, steps; bool training; bool bwd_entry_handshake; bool fp8 = false; bool overlap = false; bool tiles = false;
+             int empty_rank = -1;   // this rank has no tokens (its experts still get the others')
+};
 
 uint64_t mix(uint64_t x) { x += 0x9e3779b97f4a7c15ull; x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull; x = (x ^ (x >> 27)) * 0x94d049bb133111ebull; return x ^ (x >> 31); }
 
@@ -76,7 +80,7 @@ uint32_t g_word(int rank, int step, int t, int i) { return static_cast<uint32_t>
 
 void run_rank(World& w, int me) {
   const Cfg& c = w.c;
-  const int W = c.W, El = c.El, E = w.E, K = c.K, T = c.T;
+  const int W = c.W, El = c.El, E = w.E, K = c.K, T = me == c.empty_rank ? 0 : c.T;
   Rank& my = *w.r[me];
   std::vector<int> topk(static_cast<size_t>(T) * K), dest_row(static_cast<size_t>(T) * K);
   for (int step = 1; step <= c.steps && !w.abort.load(); ++step) {
@@ -191,9 +195,11 @@ void run_rank(World& w, int me) {
           }
       }
     };
+    // The blocks of a transport kernel, as its launcher counts them; `announces`: it also sets flags that the peers wait for.
+    auto blocks = [&](bool announces) { return fastb::announce_blocks(T > 0 ? kWorkers : 0, announces && W > 1); };
     std::thread side;
-    if (c.overlap) side = std::thread([&] { parallel(kWorkers, dispatch); });
-    else parallel(kWorkers, dispatch);
+    if (c.overlap) side = std::thread([&] { parallel(blocks(false), dispatch); });
+    else parallel(blocks(false), dispatch);
     if (c.fp8 && !c.tiles) {
       // wait_counters + dequant: all local experts complete, then quantised rows -> x_recv (real rows only), pad rows zeroed
       bool ok = true;
@@ -207,13 +213,16 @@ void run_rank(World& w, int me) {
     parallel(kWorkers, gemms);
     if (side.joinable()) side.join();  // the main stream re-joins the side stream before it signals
     if (w.abort.load()) return;
-    for (int p = 0; p < W; ++p) w.r[p]->flags[1 * W + me].store(epoch, std::memory_order_release);  // combine's block 0: my y is complete
-    // ---- combine_pull: every token pulls its K rows from the owners and sums them ------------------
-    auto pull = [&](int flag_row, bool from_dx, const std::function<uint32_t(int, int, int)>& expect) {
+    // ---- combine_pull: block 0 says that my rows are final; every token pulls its K rows from the owners and sums them ----
+    auto pull = [&](int flag_row, bool from_dx, bool signal, const std::function<uint32_t(int, int, int)>& expect) {
+      parallel(blocks(signal), [&](int k, int n) {
+        if (W > 1) {
+          if (signal && k == 0)
+            for (int p = 0; p < W; ++p) w.r[p]->flags[flag_row * W + me].store(epoch, std::memory_order_release);
 #ifndef FASTB_MOE_TWIN_NO_READY_WAIT  // defining it drops the wait for the owners' ready flags: the race detector must object
-      for (int p = 0; p < W; ++p) if (!wait_ge(w, my.flags[flag_row * W + p], epoch)) return;
+          for (int p = 0; p < W; ++p) if (!wait_ge(w, my.flags[flag_row * W + p], epoch)) return;
 #endif
-      parallel(kWorkers, [&](int k, int n) {
+        }
         for (int t = k; t < T; t += n)
           for (int i = 0; i < H; ++i) {
             uint32_t acc = 0, want = 0;
@@ -229,17 +238,18 @@ void run_rank(World& w, int me) {
       });
     };
     auto y_expect = [&](int t, int j, int i) { return x_word(me, step, t, i) * 3 + static_cast<uint32_t>(topk[t * K + j] + 1); };
-    pull(1, false, y_expect);
+    pull(1, false, true, y_expect);
     if (!c.training || w.abort.load()) continue;
     // ---- backward: router-weight gradients read y again (still in place on the owners) --------------
-    pull(1, false, y_expect);
+    pull(1, false, false, y_expect);
     // ---- transposed combine: push grad rows to the owners (second arrival channel) ------------------
     zero_pad(my.dy_recv);
-    if (c.bwd_entry_handshake) {
-      for (int p = 0; p < W; ++p) w.r[p]->flags[2 * W + me].store(epoch, std::memory_order_release);
-      for (int p = 0; p < W; ++p) if (!wait_ge(w, my.flags[2 * W + p], epoch)) return;
-    }
-    parallel(kWorkers, [&](int k, int n) {
+    parallel(blocks(c.bwd_entry_handshake), [&](int k, int n) {
+      if (c.bwd_entry_handshake && W > 1) {
+        if (k == 0)
+          for (int p = 0; p < W; ++p) w.r[p]->flags[2 * W + me].store(epoch, std::memory_order_release);
+        for (int p = 0; p < W; ++p) if (!wait_ge(w, my.flags[2 * W + p], epoch)) return;
+      }
       std::vector<int> sent(E, 0);
       for (int t = k; t < T; t += n)
         for (int j = 0; j < K; ++j) {
@@ -263,9 +273,8 @@ void run_rank(World& w, int me) {
       }
     });
     if (w.abort.load()) return;
-    for (int p = 0; p < W; ++p) w.r[p]->flags[3 * W + me].store(epoch, std::memory_order_release);  // my dx is complete
     // ---- transposed dispatch: every token pulls and sums the gradients of its K rows -----------------
-    pull(3, true, [&](int t, int j, int i) { const uint32_t x = x_word(me, step, t, i); return (g_word(me, step, t, i) + static_cast<uint32_t>(j)) * 2 + (x + 7) + x; });
+    pull(3, true, true, [&](int t, int j, int i) { const uint32_t x = x_word(me, step, t, i); return (g_word(me, step, t, i) + static_cast<uint32_t>(j)) * 2 + (x + 7) + x; });
   }
 }
 
@@ -308,6 +317,11 @@ int main(int argc, char** argv) {
           Cfg c{W, El, K, 10 + 3 * W, steps, training, !no_handshake};
           failures += run(c);
           ++runs;
+          for (int empty : {0, W - 1}) {   // the first or the last rank has no tokens
+            Cfg e = c; e.empty_rank = empty;
+            failures += run(e);
+            ++runs;
+          }
           if (!training) {  // the forward-only variants: fp8 receive path, dispatch overlapped with the gated GEMMs
             Cfg f = c; f.fp8 = true;
             failures += run(f);

@@ -385,7 +385,7 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
   a.src_heap_off = src_off; a.ready_flags_heap_off = ready_off; a.ready_epoch = ready_epoch;
   a.epoch_dev = reinterpret_cast<const unsigned long long*>(epoch_dev_ptr);
   a.out = ptr_or_null<__nv_bfloat16>(out); a.dot_with = ptr_or_null<const __nv_bfloat16>(dot_with); a.dot_out = ptr_or_null<float>(dot_out);
-  TORCH_CHECK((a.out != nullptr) != (a.dot_out != nullptr), "combine_pull: give either out or dot_out");
+  TORCH_CHECK(out.has_value() != dot_out.has_value(), "combine_pull: give either out or dot_out");   // no pointers: without tokens both are null
   a.status = st.d; a.timeout_ns = timeout_ns;
   cu_check(launch_combine_pull(a, ctas, stream_now()), "combine_pull");
 }

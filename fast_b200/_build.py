@@ -83,7 +83,7 @@ def build_moe_twin(force=False, tsan=True, broken=False):
     out = ROOT / "build" / (("fastb-moe-twin-tsan" if tsan else "fastb-moe-twin") + ("-broken" if broken else ""))
     out.parent.mkdir(exist_ok=True)
     srcs = [CSRC / "sched" / "moe_twin.cc"]
-    if force or _stale(out, srcs):
+    if force or _stale(out, srcs + [CSRC / "kernels" / "announce_blocks.h"]):
         flags = ["-O1", "-g", "-fsanitize=thread"] if tsan else ["-O2"]
         if broken:
             flags.append("-DFASTB_MOE_TWIN_NO_READY_WAIT")

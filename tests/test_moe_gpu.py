@@ -396,6 +396,85 @@ def test_forward_layer_of_few_tokens(E, K, H, I, T, fp8):
         assert bool(((rows >= off[idx]) & (rows < off[idx] + counts[idx])).all()) and rows.unique().numel() == n * K
 
 
+@pytest.mark.parametrize("fp8,overlap", [(False, False), (True, False), (False, True), (True, True)])
+def test_forward_layer_without_tokens(fp8, overlap):
+    """A step of no tokens returns no rows, and the step after it is as if it had not been."""
+    from fast_b200.models import MoELayer
+    from fast_b200.parallel import Communicator
+
+    comm = Communicator(heap_bytes=128 << 20, device=0)
+    layer = MoELayer(comm, 256, 256, 8, 2, max_tokens=512, fp8_dispatch=fp8, training=False, overlap_dispatch=overlap).eval()
+    x = torch.randn(300, 256, device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        want = layer(x)
+        assert layer(x[:0]).shape == (0, 256) and int(layer.engine.traffic_matrix().sum()) == 0
+        got = layer(x)
+    comm.check()
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_training_layer_without_tokens(fused):
+    """Forward and backward of no tokens: every parameter's gradient is zero, the input's has no rows."""
+    from fast_b200.models import MoELayer
+    from fast_b200.parallel import Communicator
+
+    comm = Communicator(heap_bytes=128 << 20, device=0)
+    layer = MoELayer(comm, 256, 256, 8, 2, max_tokens=512)
+    norm = torch.ones(256, dtype=torch.bfloat16, device="cuda", requires_grad=True)
+    x = torch.empty(0, 256, dtype=torch.bfloat16, device="cuda", requires_grad=True)
+    out = layer.forward_from_residual(x, norm, 1e-5) if fused else layer(x)
+    assert out.shape == x.shape
+    out.sum().backward()
+    comm.check()
+    assert x.grad.shape == x.shape
+    for p in (layer.gate, layer.w13, layer.w2) + ((norm,) if fused else ()):
+        assert int(p.grad.count_nonzero()) == 0
+
+
+def _two_ranks_words(C, flags=4):
+    """Heaps of two ranks in this process, and where `flags` words per rank lie in both."""
+    heaps = C.SymmHeap.create_local_group(2, 1 << 20, 0)
+    off = [h.alloc(64 * 8) for h in heaps][0]
+    return heaps, off, [h.tensor(off, [flags], torch.int64) for h in heaps]
+
+
+@pytest.mark.parametrize("epoch_on_device", [False, True])
+def test_rank_without_tokens_says_that_its_rows_are_final(epoch_on_device):
+    """Combine of a rank without tokens writes its ready flag on every rank (their tokens may have gone to its experts). The
+    peer's flag is there before the launch, so nothing waits."""
+    from fast_b200 import runtime
+
+    C = runtime.ext()
+    heaps, off, flags = _two_ranks_words(C)
+    st = C.StatusBlock()
+    flags[0][1] = 7
+    none = torch.empty(0, 2, dtype=torch.int32, device="cuda")
+    epoch = torch.full((1,), 7, dtype=torch.int64, device="cuda")
+    out = torch.empty(0, 256, dtype=torch.bfloat16, device="cuda")
+    C.combine_pull(heaps[0], 2, none, none, none.float(), 0, off, 0 if epoch_on_device else 7, out, None, None, 256, st, int(1e9), 8,
+                   epoch.data_ptr() if epoch_on_device else 0, True)
+    assert st.read()[0] == 0
+    assert flags[1].tolist() == [7, 0, 0, 0] and flags[0].tolist() == [7, 7, 0, 0]
+
+
+def test_rank_without_tokens_joins_the_entry_handshake():
+    """The backward dispatch of a rank without tokens publishes that its receive buffers may be written."""
+    from fast_b200 import runtime
+
+    C = runtime.ext()
+    heaps, off, flags = _two_ranks_words(C)
+    st = C.StatusBlock()
+    flags[0][1] = 7
+    none = torch.empty(0, 2, dtype=torch.int32, device="cuda")
+    x = torch.empty(0, 256, dtype=torch.bfloat16, device="cuda")
+    send_base = torch.zeros(2, dtype=torch.int32, device="cuda")
+    C.dispatch_push(heaps[0], x, none, none.float(), none, none, send_base, none, False, False, 0, 0, -1, off, 7, st, int(1e9), 8, None, 0, 0,
+                    None, None, None, none.float(), 0)
+    assert st.read()[0] == 0
+    assert flags[1].tolist() == [7, 0, 0, 0] and flags[0].tolist() == [7, 7, 0, 0]
+
+
 def test_forward_layer_in_cuda_graph():
     """The forward-only layer captured in a CUDA graph replays correctly on new inputs (the step's
     epoch lives in device memory, so a replay is a new step)."""
