@@ -3,6 +3,9 @@
 // flash_comm_t (nvidia/alltoall_nvshmem.cpp:390-662) and pybind module flash_t
 // (amd/flash.cpp:650-666); the user-facing API built on top lives in fast_b200/parallel.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -27,11 +30,19 @@ struct A2AProgramPy {
   unsigned long long expect_output = 0, expect_balance = 0;
   int64_t total_bytes = 0, largest_item = 0;
   int64_t input_bytes = 0, output_bytes = 0;  // what the rank's input and output hold (set by the owner, checked by the group launch)
+  // The list goes up in order on the stream that is current when the schedule is made, `home`; launches may be on any stream.
+  c10::cuda::CUDAStream home;
+  mutable at::cuda::CUDAEvent upload;
+  mutable bool uploaded = false;   // the upload was seen complete: launches have nothing to wait for any more
 
   // items: int64[k, 10] as produced by Plan.lower(); expect_rail: list of bytes per stage.
-  A2AProgramPy(torch::Tensor items, const std::vector<int64_t>& expect_rail, int64_t exp_out, int64_t exp_bal, int device) {
+  A2AProgramPy(torch::Tensor items, const std::vector<int64_t>& expect_rail, int64_t exp_out, int64_t exp_bal, int device)
+      : home(c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device))) {
     TORCH_CHECK(items.dim() == 2 && items.size(1) == 10 && items.dtype() == torch::kInt64 && items.is_cpu(), "items must be CPU int64[k, 10]");
     TORCH_CHECK(static_cast<int>(expect_rail.size()) <= kSigMaxStages, "too many stages for the signal block");
+    c10::cuda::CUDAGuard g(static_cast<c10::DeviceIndex>(device));
+    // Captured, the upload would be read again at every replay from host memory that is somebody else's by then.
+    TORCH_CHECK(!capturing(), "a schedule cannot be made while its stream is being captured: make it before the capture");
     n_items = static_cast<int>(items.size(0));
     num_stages = static_cast<int>(expect_rail.size());
     expect_output = static_cast<unsigned long long>(exp_out);
@@ -57,10 +68,24 @@ struct A2AProgramPy {
     }
     total_bytes = total; largest_item = largest; has_waits = waits != 0;
     std::copy(expect_rail.begin(), expect_rail.end(), reinterpret_cast<int64_t*>(host.data_ptr<uint8_t>() + list_bytes));
-    c10::cuda::CUDAGuard g(device);
     program_dev = torch::empty({all_bytes}, u8.device(torch::kCUDA, device));
     program_dev.copy_(host, /*non_blocking=*/true);
+    upload.record(home);
     rail_off = list_bytes;
+  }
+
+  static bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
+  // Called before a launch on `stream` (the current one): the launch comes after the upload, and the list's memory is not given
+  // to anybody else before the launch has ended, also when the schedule is dropped earlier.
+  void ready_on(c10::cuda::CUDAStream stream) const {
+    if (!uploaded) {
+      c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);   // a capture elsewhere does not mind the query
+      if (upload.query()) uploaded = true;
+      else if (capturing()) { upload.synchronize(); uploaded = true; }   // a captured launch cannot wait for an event from outside of its graph
+      else upload.block(stream);
+    }
+    if (stream != home) c10::cuda::CUDACachingAllocator::recordStream(program_dev.storage().data_ptr(), stream);
   }
 
   A2ARankArgs args(const HeapPy& heap, std::array<int64_t, 4> src_ptrs, std::array<int64_t, 4> dst_offs, int64_t sig_off,
@@ -86,6 +111,7 @@ void a2a_launch(const A2AProgramPy& p, const HeapPy& heap, std::array<int64_t, 4
   TORCH_CHECK(heap.h->world() <= kSigMaxWorld, "world larger than the signal block supports");
   A2ARankArgs a = p.args(heap, src_ptrs, dst_offs, sig_off, epoch, st, timeout_ns, stamps_ptr);
   a.bulk = bulk ? 1 : 0;
+  p.ready_on(c10::cuda::getCurrentCUDAStream());
   cuda_check(launch_a2a_push(a, ctas, threads, cur_stream(), p.has_waits), "a2a_push launch");
 }
 
@@ -115,6 +141,8 @@ bool a2a_launch_group(const std::vector<const A2AProgramPy*>& progs, const std::
     const int64_t base = reinterpret_cast<int64_t>(heaps[r]->h->local_base());
     host[r] = progs[r]->args(*heaps[r], {reinterpret_cast<int64_t>(ins[r].data_ptr()), 0, base + dst[2], base + dst[3]}, dst, sig_off, epoch, *sts[r], timeout_ns);
   }
+  const auto stream = c10::cuda::getCurrentCUDAStream();
+  for (const A2AProgramPy* p : progs) p->ready_on(stream);
   // A rank with a handful of work items needs a handful of CTAs (every launched CTA takes a turn at the exit counter).
   cuda_check(launch_a2a_push_group(host.data(), static_cast<int>(n), std::min(ctas, most), threads, cur_stream()), "a2a_push group launch");
   return true;

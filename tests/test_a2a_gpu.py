@@ -65,6 +65,69 @@ def test_local_group_bit_exact(servers, gpus, kind):
             c.free(o)
 
 
+@pytest.mark.parametrize("how", ["eager", "dropped", "captured"])
+def test_new_schedule_runs_on_another_stream(how):
+    """A schedule's work list goes up on the stream on which it was made. A collective on another stream comes after that upload
+    ("eager": the first stream is still busy), keeps the list's memory when the schedule is dropped at once ("dropped"), and can be
+    captured in a graph before the upload was seen complete ("captured")."""
+    from fast_b200.parallel import LocalGroup
+
+    n = 4
+    grp = LocalGroup(n, heap_bytes=64 << 20, topo=Topology.flat(n), ctas=4, threads=256)
+    m = sched.workload_uniform(n, 3000, 11, zero_diag=False)
+    ins = _pattern_inputs(m, 4)
+    want = _expected_outputs(m, ins, 4)
+    d_in = [torch.from_numpy(x).cuda() for x in ins]
+    d_out = [c.alloc(max(int(m[:, r].sum()) for r in range(n)) * 4, torch.int32) for c in grp.comms]
+    warm = grp.schedule(np.ones((n, n), np.int64), unit_bytes=16)   # kernels loaded, staging made
+    grp.all_to_all_v(d_out, d_in, warm)
+    for o in d_out:
+        o.fill_(-1)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(100_000_000)   # about 50 ms before the upload's turn
+        ss = grp.schedule(m, unit_bytes=16, chunk_bytes=8192)
+    outs = [o[: s.output_bytes // 4] for o, s in zip(d_out, ss)]
+    if how == "captured":
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=second, capture_error_mode="thread_local"):
+            grp.all_to_all_v(outs, d_in, ss)
+        graph.replay()
+    else:
+        with torch.cuda.stream(second):
+            if how == "dropped":
+                torch.cuda._sleep(200_000_000)
+            grp.all_to_all_v(outs, d_in, ss)
+        if how == "dropped":
+            size = [s.program.n_items * 48 for s in ss]
+            del ss
+            for c in grp.comms:
+                c._sched_cache.clear()
+            with torch.cuda.stream(first):   # whoever gets the lists' memory next writes over it
+                junk = [torch.full((b + d,), 255, dtype=torch.uint8, device="cuda") for b in size for d in (0, 8, 16, 512)]
+    torch.cuda.synchronize()
+    grp.check()
+    for r in range(n):
+        assert np.array_equal(d_out[r][: want[r].size].cpu().numpy(), want[r]), f"rank {r} differs"
+
+
+def test_schedule_is_not_made_under_capture():
+    """A captured upload would read, at every replay, host memory that was given back: refused, and the capture goes on."""
+    from fast_b200.parallel import LocalGroup
+
+    grp = LocalGroup(2, heap_bytes=1 << 20, topo=Topology.flat(2), ctas=2, threads=64)
+    x = torch.zeros(8, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(RuntimeError, match="captured"):
+            grp.schedule(np.full((2, 2), 5, np.int64), unit_bytes=16)
+        x += 1
+    graph.replay()
+    assert float(x.sum()) == 8.0
+    assert grp.schedule(np.full((2, 2), 5, np.int64), unit_bytes=16)[0].output_bytes == 160
+
+
 def test_unaligned_byte_units():
     from fast_b200.parallel import LocalGroup
 
