@@ -105,9 +105,17 @@ class TokScratch:
 _plans: dict = {}
 
 
+def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor]) -> tuple:
+    """Everything that a ``TokGemmPlan`` is made from or refuses by: another view, shape, type or device at the same address is
+    another plan (or none)."""
+    return (mode, epi, granule, BAND_ROWS, w.data_ptr(), w.dtype, w.shape, w.stride(), w.get_device(), x.data_ptr(), x.dtype, x.shape, x.stride(), x.get_device(),
+            out.data_ptr(), out.dtype, out.shape, out.stride(), out.get_device(),
+            None if gu is None else (gu.data_ptr(), gu.dtype, gu.shape, gu.stride(), gu.get_device()))
+
+
 def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
              granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch], most_rows: int = 0) -> None:
-    key = (mode, epi, granule, BAND_ROWS, w.data_ptr(), w.shape, x.data_ptr(), x.shape, x.stride(0), out.data_ptr(), out.stride(0), gu.data_ptr() if gu is not None else 0)
+    key = _plan_key(mode, epi, granule, w, x, out, gu)
     plan = _plans.get(key)
     if plan is None:
         if len(_plans) > 1024:

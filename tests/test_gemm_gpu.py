@@ -52,6 +52,28 @@ def test_forward(G, N, K, counts):
         _close(out[s:e], a[s:e].float() @ w[i].float().T)
 
 
+def test_other_views_at_the_same_address():
+    """Calls on memory that an earlier call used in another way: refused views stay refused, other pitches are followed."""
+    from fast_b200.ops import gemm
+
+    G, N, K = 1, 256, 256
+    counts, off, R, a, w = _setup(G, N, K, [200], seed=8)
+    want = a.float() @ w[0].float().T
+    out = torch.empty(R, N, device="cuda", dtype=torch.bfloat16)
+    for _ in range(2):
+        gemm.grouped_gemm_fwd(a, w, off, out)
+        _close(out[:200], want[:200])
+        for bad in (w.transpose(1, 2), w.view(torch.float16)):
+            with pytest.raises((RuntimeError, AssertionError)):
+                gemm.grouped_gemm_fwd(a, bad, off, out)
+    act, buf = torch.empty(R, N // 2, device="cuda", dtype=torch.bfloat16), torch.empty(R, 2 * N, device="cuda", dtype=torch.bfloat16)
+    for gate_up in (buf[:, :N], buf.view(-1)[: R * N].view(R, N), buf[:, :N]):
+        gate_up.fill_(float("nan"))
+        gemm.grouped_gemm_fwd(a, w, off, act, swiglu=True, gate_up_out=gate_up)
+        _close(gate_up[:200], want[:200])
+    gemm.check()
+
+
 def test_forward_swiglu():
     from fast_b200.ops import gemm
 
