@@ -18,6 +18,12 @@ template <class T> T* ptr_or_null(const c10::optional<torch::Tensor>& t) { retur
 void want(const torch::Tensor& t, c10::ScalarType dt, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == dt, name, ": expected a contiguous CUDA tensor of the right dtype");
 }
+// ... that a kernel reads or writes in words of `word` bytes: a view may start at any element, and a misaligned access costs the context.
+void want_aligned(const torch::Tensor& t, c10::ScalarType dt, const char* name, int word) {
+  want(t, dt, name);
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % word == 0, name, ": must start at a multiple of ", word, " bytes (clone a view that does not)");
+}
+void want16(const torch::Tensor& t, c10::ScalarType dt, const char* name) { want_aligned(t, dt, name, 16); }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -301,7 +307,7 @@ void route_splits(const SplitsPlan& p, torch::Tensor logits, c10::optional<torch
 // The same from the activations of at most ROUTE_TOKENS_PER_BLOCK tokens: logits = bf16(x . gate^T).
 void gate_route(const SplitsPlan& p, torch::Tensor x, torch::Tensor gate, c10::optional<torch::Tensor> bias, int K, torch::Tensor topk_idx, torch::Tensor topk_w,
                 torch::Tensor slot_in_block, uint64_t epoch) {
-  want(x, torch::kBFloat16, "x"); want(gate, torch::kBFloat16, "gate");
+  want16(x, torch::kBFloat16, "x"); want16(gate, torch::kBFloat16, "gate");
   const int64_t T = x.size(0);
   TORCH_CHECK(x.dim() == 2 && gate.dim() == 2 && gate.size(0) == p.a.num_experts && gate.size(1) == x.size(1) && T >= 1 && T <= kRouteTokensPerBlock, "gate_route: shapes");
   check_route_outputs(p, T, K, topk_idx, topk_w, slot_in_block);
@@ -325,7 +331,7 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
                    c10::optional<torch::Tensor> send_list, int tile_rows, int num_tiles, c10::optional<torch::Tensor> xq,
                    c10::optional<torch::Tensor> xq_scales, c10::optional<torch::Tensor> local_rows, c10::optional<torch::Tensor> dot_out, int64_t y_off,
                    c10::optional<torch::Tensor> sum_with, c10::optional<torch::Tensor> grad_out, c10::optional<torch::Tensor> grad_loss, double grad_factor) {
-  want(x, torch::kBFloat16, "x"); want(topk_idx, torch::kInt32, "topk_idx"); want(dest_row, torch::kInt32, "dest_row");
+  want16(x, torch::kBFloat16, "x"); want(topk_idx, torch::kInt32, "topk_idx"); want(dest_row, torch::kInt32, "dest_row");
   DispatchArgs a{};
   a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
   a.num_experts = static_cast<int>(send_base.numel()); a.T = static_cast<int>(x.size(0)); a.H = static_cast<int>(x.size(1));
@@ -337,7 +343,7 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
   a.tile_rows = tile_rows; a.num_tiles = num_tiles;
   if (xq.has_value()) {
     TORCH_CHECK(fp8 && xq_scales.has_value(), "dispatch_push: xq needs fp8 and xq_scales");
-    want(*xq, torch::kUInt8, "xq"); want(*xq_scales, torch::kFloat32, "xq_scales");
+    want16(*xq, torch::kUInt8, "xq"); want(*xq_scales, torch::kFloat32, "xq_scales");
     TORCH_CHECK(xq->numel() >= x.numel() && xq_scales->numel() >= x.numel() / 128, "dispatch_push: xq / xq_scales too small");
     a.xq = xq->data_ptr<uint8_t>(); a.xq_scales = xq_scales->data_ptr<float>();
   }
@@ -348,14 +354,14 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
     a.y_heap_off = y_off;
     if (sum_with.has_value()) {
       TORCH_CHECK(grad_out.has_value() && grad_loss.has_value(), "dispatch_push: sum_with needs grad_out and grad_loss");
-      want(*sum_with, torch::kBFloat16, "sum_with"); want(*grad_out, torch::kBFloat16, "grad_out"); want(*grad_loss, torch::kFloat32, "grad_loss");
+      want16(*sum_with, torch::kBFloat16, "sum_with"); want16(*grad_out, torch::kBFloat16, "grad_out"); want(*grad_loss, torch::kFloat32, "grad_loss");
       TORCH_CHECK(sum_with->sizes() == x.sizes() && grad_out->sizes() == x.sizes(), "dispatch_push: sum_with / grad_out shapes");
       a.sum_with = reinterpret_cast<const __nv_bfloat16*>(sum_with->data_ptr()); a.grad_out = reinterpret_cast<__nv_bfloat16*>(grad_out->data_ptr());
       a.grad_loss = grad_loss->data_ptr<float>(); a.grad_factor = static_cast<float>(grad_factor);
     }
   }
   if (local_rows.has_value()) {
-    want(*local_rows, torch::kBFloat16, "local_rows");
+    want16(*local_rows, torch::kBFloat16, "local_rows");
     TORCH_CHECK(fp8 && local_rows->dim() == 2 && local_rows->size(1) == a.H, "dispatch_push: local_rows belongs to the fp8 rows");
     a.local_rows = reinterpret_cast<__nv_bfloat16*>(local_rows->data_ptr());
   }
@@ -372,7 +378,7 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
   torch::Tensor partials;
   if (residual.has_value()) {
     TORCH_CHECK(loss.has_value() && ticket.has_value(), "combine_pull: residual needs loss and ticket");
-    want(*residual, torch::kBFloat16, "residual"); want(*loss, torch::kFloat32, "loss"); want(*ticket, torch::kInt32, "ticket");
+    want16(*residual, torch::kBFloat16, "residual"); want(*loss, torch::kFloat32, "loss"); want(*ticket, torch::kInt32, "ticket");
     TORCH_CHECK(residual->dim() == 2 && residual->size(0) == topk_idx.size(0) && residual->size(1) == H, "combine_pull: residual shape");
     partials = torch::empty({kMaxLossPartials}, loss->options());
     a.residual = reinterpret_cast<const __nv_bfloat16*>(residual->data_ptr()); a.loss = loss->data_ptr<float>(); a.loss_scale = static_cast<float>(loss_scale);
@@ -385,6 +391,7 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
   a.src_heap_off = src_off; a.ready_flags_heap_off = ready_off; a.ready_epoch = ready_epoch;
   a.epoch_dev = reinterpret_cast<const unsigned long long*>(epoch_dev_ptr);
   a.out = ptr_or_null<__nv_bfloat16>(out); a.dot_with = ptr_or_null<const __nv_bfloat16>(dot_with); a.dot_out = ptr_or_null<float>(dot_out);
+  if (out.has_value()) want16(*out, torch::kBFloat16, "out");
   TORCH_CHECK(out.has_value() != dot_out.has_value(), "combine_pull: give either out or dot_out");   // no pointers: without tokens both are null
   a.status = st.d; a.timeout_ns = timeout_ns;
   cu_check(launch_combine_pull(a, ctas, stream_now()), "combine_pull");
@@ -427,7 +434,7 @@ void bind_moe(py::module_& m) {
   m.def("norm_gate_route", [](torch::Tensor h, torch::Tensor norm_w, torch::Tensor gate, c10::optional<torch::Tensor> bias, int K, double eps, torch::Tensor hn,
                               torch::Tensor rstd, torch::Tensor logits, torch::Tensor topk_idx, torch::Tensor topk_w, torch::Tensor slot_in_block,
                               torch::Tensor block_cnt, const SplitsPlan* splits, uint64_t epoch) {
-    want(h, torch::kBFloat16, "h"); want(norm_w, torch::kBFloat16, "norm_w"); want(gate, torch::kBFloat16, "gate"); want(hn, torch::kBFloat16, "hn");
+    want16(h, torch::kBFloat16, "h"); want16(norm_w, torch::kBFloat16, "norm_w"); want16(gate, torch::kBFloat16, "gate"); want16(hn, torch::kBFloat16, "hn");
     want(rstd, torch::kFloat32, "rstd"); want(logits, torch::kFloat32, "logits"); want(topk_idx, torch::kInt32, "topk_idx"); want(topk_w, torch::kFloat32, "topk_w");
     want(slot_in_block, torch::kInt32, "slot_in_block"); want(block_cnt, torch::kInt32, "block_cnt");
     NormGateArgs a{};
@@ -454,9 +461,9 @@ void bind_moe(py::module_& m) {
   m.def("norm_gate_bwd", [](torch::Tensor h, torch::Tensor norm_w, torch::Tensor gate, torch::Tensor rstd, torch::Tensor topk_idx, torch::Tensor topk_w,
                             torch::Tensor grad_w, torch::Tensor grad_hn, torch::Tensor grad_h, torch::Tensor d_gate, torch::Tensor d_norm_w,
                             c10::optional<torch::Tensor> residual) {
-    want(h, torch::kBFloat16, "h"); want(norm_w, torch::kBFloat16, "norm_w"); want(gate, torch::kBFloat16, "gate"); want(rstd, torch::kFloat32, "rstd");
+    want16(h, torch::kBFloat16, "h"); want16(norm_w, torch::kBFloat16, "norm_w"); want16(gate, torch::kBFloat16, "gate"); want(rstd, torch::kFloat32, "rstd");
     want(topk_idx, torch::kInt32, "topk_idx"); want(topk_w, torch::kFloat32, "topk_w"); want(grad_w, torch::kFloat32, "grad_w");
-    want(grad_hn, torch::kBFloat16, "grad_hn"); want(grad_h, torch::kBFloat16, "grad_h");
+    want16(grad_hn, torch::kBFloat16, "grad_hn"); want16(grad_h, torch::kBFloat16, "grad_h");
     const bool as_bf16 = d_gate.scalar_type() == torch::kBFloat16;   // written as bf16, or accumulated into as fp32
     want(d_gate, as_bf16 ? torch::kBFloat16 : torch::kFloat32, "d_gate"); want(d_norm_w, as_bf16 ? torch::kBFloat16 : torch::kFloat32, "d_norm_w");
     NormGateBwdArgs a{};
@@ -470,7 +477,7 @@ void bind_moe(py::module_& m) {
     if (as_bf16) { a.d_gate_bf16 = reinterpret_cast<__nv_bfloat16*>(d_gate.data_ptr()); a.d_norm_w_bf16 = reinterpret_cast<__nv_bfloat16*>(d_norm_w.data_ptr()); }
     else { a.d_gate = d_gate.data_ptr<float>(); a.d_norm_w = d_norm_w.data_ptr<float>(); }
     if (residual.has_value()) {
-      want(*residual, torch::kBFloat16, "residual");
+      want16(*residual, torch::kBFloat16, "residual");
       TORCH_CHECK(residual->sizes() == h.sizes(), "norm_gate_bwd: residual shape");
       a.residual = reinterpret_cast<const __nv_bfloat16*>(residual->data_ptr());
     }
@@ -487,7 +494,7 @@ void bind_moe(py::module_& m) {
         py::arg("tile_rows") = 0, py::arg("num_tiles") = 0, py::arg("xq") = py::none(), py::arg("xq_scales") = py::none(), py::arg("local_rows") = py::none(), py::arg("dot_out") = py::none(),
         py::arg("y_off") = 0, py::arg("sum_with") = py::none(), py::arg("grad_out") = py::none(), py::arg("grad_loss") = py::none(), py::arg("grad_factor") = 0.0);
   m.def("quantise_rows", [](torch::Tensor x, torch::Tensor q, torch::Tensor scales, int ctas) {
-    want(x, torch::kBFloat16, "x"); want(q, torch::kUInt8, "q"); want(scales, torch::kFloat32, "scales");
+    want16(x, torch::kBFloat16, "x"); want16(q, torch::kUInt8, "q"); want(scales, torch::kFloat32, "scales");
     TORCH_CHECK(x.dim() == 2 && q.numel() >= x.numel() && scales.numel() >= x.numel() / 128, "quantise_rows: q / scales too small");
     cu_check(launch_quantise_rows(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), static_cast<int>(x.size(0)), static_cast<int>(x.size(1)),
                                   q.data_ptr<uint8_t>(), scales.data_ptr<float>(), ctas, stream_now()), "quantise_rows");
@@ -500,34 +507,34 @@ void bind_moe(py::module_& m) {
                                   static_cast<int>(target.numel()), st.d, timeout_ns, stream_now()), "wait_counters");
   });
   m.def("swiglu_fwd", [](torch::Tensor gu, torch::Tensor act) {
-    want(gu, torch::kBFloat16, "gate_up"); want(act, torch::kBFloat16, "act");
+    want16(gu, torch::kBFloat16, "gate_up"); want16(act, torch::kBFloat16, "act");
     cu_check(launch_swiglu_fwd(reinterpret_cast<const __nv_bfloat16*>(gu.data_ptr()), reinterpret_cast<__nv_bfloat16*>(act.data_ptr()), gu.size(0),
                                static_cast<int>(act.size(1)), stream_now()), "swiglu_fwd");
   });
   m.def("swiglu_bwd", [](torch::Tensor gu, torch::Tensor dact, torch::Tensor dgu, int64_t rows_dev_ptr) {
-    want(gu, torch::kBFloat16, "gate_up"); want(dact, torch::kBFloat16, "d_act"); want(dgu, torch::kBFloat16, "d_gate_up");
+    want16(gu, torch::kBFloat16, "gate_up"); want16(dact, torch::kBFloat16, "d_act"); want16(dgu, torch::kBFloat16, "d_gate_up");
     cu_check(launch_swiglu_bwd(reinterpret_cast<const __nv_bfloat16*>(gu.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(dact.data_ptr()),
                                reinterpret_cast<__nv_bfloat16*>(dgu.data_ptr()), gu.size(0), static_cast<int>(dact.size(1)), reinterpret_cast<const int*>(rows_dev_ptr),
                                stream_now()), "swiglu_bwd");
   });
   m.def("dequant_fp8", [](torch::Tensor q, torch::Tensor scales, torch::Tensor out, int64_t rows_dev_ptr) {
-    want(q, torch::kUInt8, "q"); want(scales, torch::kFloat32, "scales"); want(out, torch::kBFloat16, "out");
+    want_aligned(q, torch::kUInt8, "q", 8); want(scales, torch::kFloat32, "scales"); want16(out, torch::kBFloat16, "out");
     cu_check(launch_dequant_fp8(q.data_ptr<uint8_t>(), scales.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(out.data_ptr()), q.size(0),
                                 static_cast<int>(q.size(1)), reinterpret_cast<const int*>(rows_dev_ptr), stream_now()), "dequant_fp8");
   });
   m.def("sumsq_add", [](torch::Tensor a, torch::Tensor b, double scale, torch::Tensor partial, torch::Tensor out) {
-    want(a, torch::kBFloat16, "a"); want(b, torch::kBFloat16, "b"); want(partial, torch::kFloat32, "partial"); want(out, torch::kFloat32, "out");
+    want16(a, torch::kBFloat16, "a"); want16(b, torch::kBFloat16, "b"); want(partial, torch::kFloat32, "partial"); want(out, torch::kFloat32, "out");
     TORCH_CHECK(a.numel() == b.numel(), "sumsq_add: shapes");
     cu_check(launch_sumsq_add(reinterpret_cast<const __nv_bfloat16*>(a.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(b.data_ptr()), a.numel(),
                               static_cast<float>(scale), partial.data_ptr<float>(), static_cast<int>(partial.numel()), out.data_ptr<float>(), stream_now()), "sumsq_add");
   });
   m.def("scaled_sum", [](torch::Tensor a, torch::Tensor b, torch::Tensor gscale, double factor, torch::Tensor out) {
-    want(a, torch::kBFloat16, "a"); want(b, torch::kBFloat16, "b"); want(gscale, torch::kFloat32, "gscale"); want(out, torch::kBFloat16, "out");
+    want16(a, torch::kBFloat16, "a"); want16(b, torch::kBFloat16, "b"); want(gscale, torch::kFloat32, "gscale"); want16(out, torch::kBFloat16, "out");
     cu_check(launch_scaled_sum(reinterpret_cast<const __nv_bfloat16*>(a.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(b.data_ptr()), a.numel(),
                                gscale.data_ptr<float>(), static_cast<float>(factor), reinterpret_cast<__nv_bfloat16*>(out.data_ptr()), stream_now()), "scaled_sum");
   });
   m.def("embedding_bwd", [](torch::Tensor sorted_ids, torch::Tensor perm, torch::Tensor grad_out, torch::Tensor grad_table) {
-    want(sorted_ids, torch::kInt64, "sorted_ids"); want(perm, torch::kInt64, "perm"); want(grad_out, torch::kBFloat16, "grad_out");
+    want(sorted_ids, torch::kInt64, "sorted_ids"); want(perm, torch::kInt64, "perm"); want16(grad_out, torch::kBFloat16, "grad_out");
     want(grad_table, torch::kBFloat16, "grad_table");
     cu_check(launch_embedding_bwd(reinterpret_cast<const long long*>(sorted_ids.data_ptr()), reinterpret_cast<const long long*>(perm.data_ptr()),
                                   reinterpret_cast<const __nv_bfloat16*>(grad_out.data_ptr()), reinterpret_cast<__nv_bfloat16*>(grad_table.data_ptr()),
@@ -535,7 +542,7 @@ void bind_moe(py::module_& m) {
   });
   // grad_out [T, H] summed by id in position order -> a new table gradient [V, H] (rows that no id names are zero).
   m.def("embedding_grad", [](torch::Tensor ids, int V, torch::Tensor grad_out) {
-    want(ids, torch::kInt64, "ids"); want(grad_out, torch::kBFloat16, "grad_out");
+    want(ids, torch::kInt64, "ids"); want16(grad_out, torch::kBFloat16, "grad_out");
     const int64_t T = ids.numel(), H = grad_out.size(1);
     TORCH_CHECK(grad_out.dim() == 2 && grad_out.size(0) == T, "embedding_grad: one gradient row per id");
     auto table = torch::empty({V, H}, grad_out.options());
@@ -578,8 +585,8 @@ void bind_moe(py::module_& m) {
       a.lr = static_cast<float>(lr); a.b1 = static_cast<float>(b1); a.b2 = static_cast<float>(b2); a.eps = static_cast<float>(eps); a.wd = static_cast<float>(wd);
       a.gscale = static_cast<float>(grad_scale);
       for (size_t k = k0; k < std::min(n, k0 + kAdamWTensors); ++k) {
-        want(params[k], torch::kBFloat16, "param"); want(masters[k], torch::kFloat32, "master"); want(ms[k], torch::kFloat32, "m"); want(vs[k], torch::kFloat32, "v");
-        want(grads[k], torch::kBFloat16, "grad");
+        want_aligned(params[k], torch::kBFloat16, "param", 8); want16(masters[k], torch::kFloat32, "master"); want16(ms[k], torch::kFloat32, "m"); want16(vs[k], torch::kFloat32, "v");
+        want_aligned(grads[k], torch::kBFloat16, "grad", 8);
         const int64_t len = params[k].numel();
         TORCH_CHECK(masters[k].numel() == len && ms[k].numel() == len && vs[k].numel() == len && grads[k].numel() == len, "adamw: sizes");
         AdamWTensor& t = a.t[a.count++];

@@ -226,10 +226,11 @@ class ExpertParallel:
     def route_gate(self, x: torch.Tensor, gate: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
         """Route on the router logits ``x @ gate.T`` (bf16, as a GEMM returns them). For a few tokens the logits are made in the
         routing kernel itself: one block per token, each reading the whole gate, so up to a block's worth of tokens and
-        64 MiB of such reads; beyond that a GEMM reads the gate less often than it costs a launch."""
+        64 MiB of such reads; beyond that a GEMM reads the gate less often than it costs a launch. The kernel reads 16-byte words;
+        a gate that is a view at another address goes through the GEMM too."""
         T = x.shape[0]
         if (1 <= T <= self._C.ROUTE_TOKENS_PER_BLOCK and 2 * T * self.E * self.H <= 64 << 20 and self.E <= 256 and x.dtype == gate.dtype == torch.bfloat16
-                and x.is_contiguous() and gate.is_contiguous() and T <= self.T):
+                and x.is_contiguous() and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and T <= self.T):
             topk_idx, topk_w, dest_row = self._route_outputs(T, x.device)
             self.epoch += 1
             self._C.gate_route(self.splits, x, gate, bias, self.K, topk_idx, topk_w, self.slot_in_block, self.epoch)

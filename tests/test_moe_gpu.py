@@ -475,6 +475,35 @@ def test_rank_without_tokens_joins_the_entry_handshake():
     assert flags[1].tolist() == [7, 0, 0, 0] and flags[0].tolist() == [7, 7, 0, 0]
 
 
+def test_views_that_start_between_16_byte_words():
+    """A router gate may be a view at any element (few tokens: the routing kernel's 16-byte reads give way to the GEMM); rows, which
+    every kernel of the chain reads in 16-byte words, are refused on the host."""
+    from fast_b200.models import MoELayer
+    from fast_b200.ops import fused
+    from fast_b200.parallel import Communicator
+
+    comm = Communicator(heap_bytes=128 << 20, device=0)
+    layer = MoELayer(comm, 256, 256, 8, 2, max_tokens=512, training=False).eval()
+    x = torch.randn(5, 256, device="cuda").to(torch.bfloat16)
+
+    def moved(t):
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view_as(t).copy_(t.detach())
+
+    with torch.no_grad():
+        layer(x)
+        want = layer.last_route.topk_idx.clone()
+        layer.gate.data = moved(layer.gate)
+        y = layer(x)
+        assert bool((layer.last_route.topk_idx == want).float().mean() > 0.9)   # the two sums round some logits differently
+        ref, _, _ = _ref_forward(x, layer.gate, layer.w13, layer.w2, 2, idx=layer.last_route.topk_idx.long())
+        assert _rel(y, ref) < 2e-2
+        with pytest.raises(RuntimeError, match="16 bytes"):
+            layer(moved(x))
+    with pytest.raises(RuntimeError, match="16 bytes"):
+        fused.residual_mean_square(x, moved(x))
+    comm.check()
+
+
 def test_forward_layer_in_cuda_graph():
     """The forward-only layer captured in a CUDA graph replays correctly on new inputs (the step's
     epoch lives in device memory, so a replay is a new step)."""
