@@ -321,10 +321,8 @@ struct CombineArgs {
   int signal;                  // 1: first write ready_epoch into slot `rank` of every rank's flags (my own rows are final)
   int segments;                // set by the launcher: warps that share a token's row
   const unsigned long long* epoch_dev;  // when non-null, *epoch_dev replaces ready_epoch (see SplitsArgs)
-  __nv_bfloat16* out;          // [T, H] sum_j w * row_j (null in dot mode)
-  const __nv_bfloat16* dot_with;  // dot mode: [T, H]
-  float* dot_out;              // dot mode: [T, K] = <dot_with[t], row_j>
-  // Optional, with out: *loss = loss_scale * sum((residual + out)^2), the sum rounded to bf16 first.
+  __nv_bfloat16* out;          // [T, H] sum_j w * row_j
+  // Optional: *loss = loss_scale * sum((residual + out)^2), the sum rounded to bf16 first.
   const __nv_bfloat16* residual;   // [T, H]
   float* loss_partials;        // [kMaxLossPartials] scratch
   unsigned int* ticket;        // one zeroed word; zero again afterwards
@@ -356,11 +354,8 @@ cudaError_t launch_sumsq_add(const __nv_bfloat16* a, const __nv_bfloat16* b, lon
 // out = bf16(a + b) * (*gscale) * factor (gradient of the above).
 cudaError_t launch_scaled_sum(const __nv_bfloat16* a, const __nv_bfloat16* b, long long n, const float* gscale, float factor, __nv_bfloat16* out,
                               cudaStream_t stream);
-// Table gradient of an embedding lookup from ids sorted ascending (with their positions); rows of grad_table not named by any id are left as they are.
-cudaError_t launch_embedding_bwd(const long long* sorted_ids, const long long* perm, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, long long T,
-                                 int H, cudaStream_t stream);
-// Groups token positions by id with a counting sort (stable: positions ascending inside an id): sorted_ids / perm [T] as
-// launch_embedding_bwd takes them; entries past start[V] (ids outside [0, V)) are left as they were. Scratch: hist
+// Groups token positions by id with a counting sort (stable: positions ascending inside an id): sorted_ids / perm [T], the run of
+// id v from start[v] on; past start[V] (ids outside [0, V)) sorted_ids is -1 and perm is left as it was. Scratch: hist
 // [ceil(T / embedding_index_block())][V] ints (cleared here), rank_in_block [T], total [V], start [V + 1].
 cudaError_t launch_embedding_index(const long long* ids, long long T, int V, int* hist, int* rank_in_block, int* total, int* start, long long* sorted_ids,
                                    long long* perm, cudaStream_t stream);

@@ -186,39 +186,13 @@ __global__ void scaled_sum_kernel(const uint4* __restrict__ a, const uint4* __re
   }
 }
 
-// Embedding gradient: ids sorted ascending with their original positions; the warp that sits on the
-// first entry of a run of equal ids sums the run's rows in fp32 (in position order) and writes one
-// bf16 row of the table gradient.
-__global__ void embedding_bwd_kernel(const long long* __restrict__ sorted_ids, const long long* __restrict__ perm, const uint4* __restrict__ grad_out,
-                                     uint4* __restrict__ grad_table, long long T, int H) {
-  const long long i = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= T) return;
-  const long long id = sorted_ids[i];
-  if (id < 0) return;  // slots no valid id was sorted into
-  if (i > 0 && sorted_ids[i - 1] == id) return;
-  long long end = i + 1;
-  while (end < T && sorted_ids[end] == id) ++end;
-  const int chunks = H / 8;
-  for (int c = lane; c < chunks; c += 32) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long j = i; j < end; ++j) {
-      float f[8];
-      unpack8(grad_out[perm[j] * chunks + c], f);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += f[k];
-    }
-    grad_table[id * chunks + c] = pack8(acc);
-  }
-}
-
 // ---- ids grouped by value, positions in order: a counting sort the embedding gradient is fed from -----------
-// Work is independent of the data (heavy duplicates cost the same as none). Blocks of kIdxBlock tokens:
+// The sort's work is independent of the data (heavy duplicates cost the same as none). Blocks of kIdxBlock tokens:
 //   1. per-block histogram of the ids (counts) and, per token, its rank among the block's earlier tokens with
 //      the same id (position order, so the grouping is stable and the later summation order is fixed);
 //   2. per id, the running sum over blocks (where a block's tokens of that id start inside the id's run);
 //   3. exclusive scan over the ids (where each id's run starts);
-//   4. scatter: sorted_ids / perm, the arrays embedding_bwd_kernel consumes.
+//   4. scatter: sorted_ids / perm; embedding_rows_kernel reads start and perm.
 constexpr int kIdxBlock = 256;
 
 __global__ void __launch_bounds__(kIdxBlock) emb_block_hist_kernel(const long long* __restrict__ ids, long long T, int V, int* __restrict__ hist,
@@ -310,7 +284,8 @@ __global__ void emb_scatter_kernel(const long long* __restrict__ ids, const int*
 
 // ---- the whole gradient of an embedding table ------------------------------------------------------------------
 // A warp per table row, after the counting sort: every row is written once, its sum or zeros (cleared beforehand by a kernel of
-// its own, the table cost one more pass of writes: 91 us for 32000 x 4096).
+// its own, the table cost one more pass of writes: 91 us for 32000 x 4096). One warp adds up all rows of its id, one after another
+// in position order: evenly spread ids are bound by HBM, an id that names many positions by its own chain of loads.
 __global__ void embedding_rows_kernel(const int* __restrict__ start, const long long* __restrict__ perm, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int V, int H) {
   const long long v = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, chunks = H / 8;
@@ -446,16 +421,6 @@ cudaError_t launch_scaled_sum(const __nv_bfloat16* a, const __nv_bfloat16* b, lo
   if (n == 0) return cudaSuccess;
   scaled_sum_kernel<<<grid_for(n / 8), 256, 0, stream>>>(reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), n / 8, gscale, factor,
                                                        reinterpret_cast<uint4*>(out));
-  note_launch();
-  return cudaGetLastError();
-}
-cudaError_t launch_embedding_bwd(const long long* sorted_ids, const long long* perm, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, long long T,
-                                 int H, cudaStream_t stream) {
-  if (H % 8) return cudaErrorInvalidValue;
-  if (T == 0) return cudaSuccess;
-  const long long threads = T * 32;
-  embedding_bwd_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(sorted_ids, perm, reinterpret_cast<const uint4*>(grad_out),
-                                                                                      reinterpret_cast<uint4*>(grad_table), T, H);
   note_launch();
   return cudaGetLastError();
 }

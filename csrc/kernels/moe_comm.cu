@@ -4,8 +4,7 @@
 //                   row of the owning expert's receive buffer on the peer; per-expert arrival
 //                   counters are bumped with release semantics once a CTA's rows are out.
 //   combine_pull  : un-permute + top-k weighted reduction: every token pulls its k expert rows
-//                   from the peers and accumulates them in fp32 (fixed slot order => reproducible),
-//                   or, in dot mode, produces <grad_out[t], row_j> for the router gradient.
+//                   from the peers and accumulates them in fp32 (fixed slot order => reproducible).
 // In FAST's terms these are the all-to-all of the forward pass and its transpose
 // (amd/flash.cpp:400-408 `backward` flag) with the permute / reduce fused in; the reference moves
 // opaque bytes with ncclSend/ncclRecv groups or NVSHMEM puts and leaves the packing to the caller.
@@ -454,9 +453,9 @@ __global__ void __launch_bounds__(kCommThreads, KM > 2 ? 2 : LOSS ? 3 : 4) combi
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  const int chunks = a.H / 8, rounds = chunks / 32, segs = a.segments;
+  const int rounds = a.H / 256, segs = a.segments;   // rounds of 32 lanes x 8 elements
   float square = 0.0f;   // my share of sum((residual + out)^2)
-  // A warp takes one of `segs` column ranges of a token's row (1 in dot mode, whose sums span the row).
+  // A warp takes one of `segs` column ranges of a token's row.
   for (long long u = blockIdx.x * wpb + warp; u < static_cast<long long>(a.T) * segs; u += gridDim.x * wpb) {
     const int t = static_cast<int>(u / segs), seg = static_cast<int>(u % segs);
     const int c_end = rounds * (seg + 1) / segs * 32;
@@ -477,69 +476,42 @@ __global__ void __launch_bounds__(kCommThreads, KM > 2 ? 2 : LOSS ? 3 : 4) combi
         w[j] = a.weights ? a.weights[tj] : 1.0f;
       }
     }
-    if (a.dot_out == nullptr) {
-      uint4* out = reinterpret_cast<uint4*>(a.out + static_cast<long long>(t) * a.H);
-      constexpr int U = 2;  // two chunks x K rows of peer loads in flight per lane
-      for (int c0 = rounds * seg / segs * 32 + lane; c0 < c_end; c0 += 32 * U) {
-        uint4 v[U][KM], res[U];
-        if (LOSS) {
-          const uint4* h = reinterpret_cast<const uint4*>(a.residual + static_cast<long long>(t) * a.H);
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (c0 + 32 * u < c_end) res[u] = __ldg(h + c0 + 32 * u);
-        }
+    uint4* out = reinterpret_cast<uint4*>(a.out + static_cast<long long>(t) * a.H);
+    constexpr int U = 2;  // two chunks x K rows of peer loads in flight per lane
+    for (int c0 = rounds * seg / segs * 32 + lane; c0 < c_end; c0 += 32 * U) {
+      uint4 v[U][KM], res[U];
+      if (LOSS) {
+        const uint4* h = reinterpret_cast<const uint4*>(a.residual + static_cast<long long>(t) * a.H);
 #pragma unroll
         for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int j = 0; j < KM; ++j)
-            if (j < a.K && c0 + 32 * u < c_end) v[u][j] = rows[j] ? __ldcg(rows[j] + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int c = c0 + 32 * u;
-          if (c >= c_end) break;
-          float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-          for (int j = 0; j < KM; ++j) {
-            if (j >= a.K) break;
-            float f[8];
-            unpack8(v[u][j], f);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i] = fmaf(w[j], f[i], acc[i]);
-          }
-          const uint4 o = pack8(acc);
-          out[c] = o;
-          if (LOSS) {
-            float q[8];
-            unpack8(add8(o, res[u]), q);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) square = fmaf(q[i], q[i], square);
-          }
-        }
+          if (c0 + 32 * u < c_end) res[u] = __ldg(h + c0 + 32 * u);
       }
-    } else {
-      const uint4* g = reinterpret_cast<const uint4*>(a.dot_with + static_cast<long long>(t) * a.H);
-      float dots[KM];
 #pragma unroll
-      for (int j = 0; j < KM; ++j) dots[j] = 0.0f;
-      for (int c = lane; c < chunks; c += 32) {
-        float gf[8];
-        unpack8(__ldg(g + c), gf);
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < KM; ++j)
+          if (j < a.K && c0 + 32 * u < c_end) v[u][j] = rows[j] ? __ldcg(rows[j] + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c = c0 + 32 * u;
+        if (c >= c_end) break;
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int j = 0; j < KM; ++j) {
           if (j >= a.K) break;
           float f[8];
-          unpack8(rows[j] ? __ldcg(rows[j] + c) : make_uint4(0, 0, 0, 0), f);
+          unpack8(v[u][j], f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) dots[j] = fmaf(gf[i], f[i], dots[j]);
+          for (int i = 0; i < 8; ++i) acc[i] = fmaf(w[j], f[i], acc[i]);
         }
-      }
+        const uint4 o = pack8(acc);
+        out[c] = o;
+        if (LOSS) {
+          float q[8];
+          unpack8(add8(o, res[u]), q);
 #pragma unroll
-      for (int j = 0; j < KM; ++j) {
-        if (j >= a.K) break;
-        float d = dots[j];
-#pragma unroll
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (lane == 0) a.dot_out[static_cast<long long>(t) * a.K + j] = d;
+          for (int i = 0; i < 8; ++i) square = fmaf(q[i], q[i], square);
+        }
       }
     }
   }
@@ -629,7 +601,7 @@ cudaError_t launch_combine_pull(const CombineArgs& a, int ctas, cudaStream_t str
   if (ctas == 0) return cudaSuccess;
   CombineArgs b = a;
   // Few tokens: as many warps per row as fill the grid, down to one round of loads per warp.
-  b.segments = a.dot_out != nullptr ? 1 : static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / std::max(a.T, 1), 1, a.H / 256));
+  b.segments = static_cast<int>(std::clamp<long long>(static_cast<long long>(ctas) * (kCommThreads / 32) / std::max(a.T, 1), 1, a.H / 256));
   cudaError_t e = launch_early(a.K <= 2 ? (a.residual != nullptr ? combine_pull_kernel<true, 2> : combine_pull_kernel<false, 2>)
                                       : (a.residual != nullptr ? combine_pull_kernel<true, kMaxK> : combine_pull_kernel<false, kMaxK>),
                                dim3(ctas), kCommThreads, 0, stream, b);

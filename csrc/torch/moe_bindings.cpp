@@ -370,9 +370,9 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
   cu_check(launch_dispatch_push(a, ctas, stream_now()), "dispatch_push");
 }
 
+// The two arguments after `out` are always None: positions that callers of an earlier form still fill.
 void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, torch::Tensor dest_row, c10::optional<torch::Tensor> weights, int64_t src_off,
-                  int64_t ready_off, uint64_t ready_epoch, c10::optional<torch::Tensor> out, c10::optional<torch::Tensor> dot_with,
-                  c10::optional<torch::Tensor> dot_out, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr, bool signal,
+                  int64_t ready_off, uint64_t ready_epoch, torch::Tensor out, py::none, py::none, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr, bool signal,
                   c10::optional<torch::Tensor> residual, c10::optional<torch::Tensor> loss, double loss_scale, c10::optional<torch::Tensor> ticket) {
   CombineArgs a{};
   torch::Tensor partials;
@@ -390,9 +390,8 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
   a.topk_idx = topk_idx.data_ptr<int>(); a.dest_row = dest_row.data_ptr<int>(); a.weights = ptr_or_null<const float>(weights);
   a.src_heap_off = src_off; a.ready_flags_heap_off = ready_off; a.ready_epoch = ready_epoch;
   a.epoch_dev = reinterpret_cast<const unsigned long long*>(epoch_dev_ptr);
-  a.out = ptr_or_null<__nv_bfloat16>(out); a.dot_with = ptr_or_null<const __nv_bfloat16>(dot_with); a.dot_out = ptr_or_null<float>(dot_out);
-  if (out.has_value()) want16(*out, torch::kBFloat16, "out");
-  TORCH_CHECK(out.has_value() != dot_out.has_value(), "combine_pull: give either out or dot_out");   // no pointers: without tokens both are null
+  want16(out, torch::kBFloat16, "out");
+  a.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
   a.status = st.d; a.timeout_ns = timeout_ns;
   cu_check(launch_combine_pull(a, ctas, stream_now()), "combine_pull");
 }
@@ -500,7 +499,7 @@ void bind_moe(py::module_& m) {
                                   q.data_ptr<uint8_t>(), scales.data_ptr<float>(), ctas, stream_now()), "quantise_rows");
   });
   m.def("combine_pull", &combine_pull, py::arg("heap"), py::arg("num_experts"), py::arg("topk_idx"), py::arg("dest_row"), py::arg("weights"), py::arg("src_off"), py::arg("ready_off"),
-        py::arg("ready_epoch"), py::arg("out"), py::arg("dot_with"), py::arg("dot_out"), py::arg("hidden"), py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"),
+        py::arg("ready_epoch"), py::arg("out"), py::arg("unused1"), py::arg("unused2"), py::arg("hidden"), py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"),
         py::arg("epoch_dev_ptr"), py::arg("signal") = false, py::arg("residual") = py::none(), py::arg("loss") = py::none(), py::arg("loss_scale") = 1.0, py::arg("ticket") = py::none());
   m.def("wait_counters", [](int64_t counter_ptr, torch::Tensor target, const StatusPy& st, uint64_t timeout_ns) {
     cu_check(launch_wait_counters(reinterpret_cast<const unsigned long long*>(counter_ptr), reinterpret_cast<const unsigned long long*>(target.data_ptr()),
@@ -532,13 +531,6 @@ void bind_moe(py::module_& m) {
     want16(a, torch::kBFloat16, "a"); want16(b, torch::kBFloat16, "b"); want(gscale, torch::kFloat32, "gscale"); want16(out, torch::kBFloat16, "out");
     cu_check(launch_scaled_sum(reinterpret_cast<const __nv_bfloat16*>(a.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(b.data_ptr()), a.numel(),
                                gscale.data_ptr<float>(), static_cast<float>(factor), reinterpret_cast<__nv_bfloat16*>(out.data_ptr()), stream_now()), "scaled_sum");
-  });
-  m.def("embedding_bwd", [](torch::Tensor sorted_ids, torch::Tensor perm, torch::Tensor grad_out, torch::Tensor grad_table) {
-    want(sorted_ids, torch::kInt64, "sorted_ids"); want(perm, torch::kInt64, "perm"); want16(grad_out, torch::kBFloat16, "grad_out");
-    want(grad_table, torch::kBFloat16, "grad_table");
-    cu_check(launch_embedding_bwd(reinterpret_cast<const long long*>(sorted_ids.data_ptr()), reinterpret_cast<const long long*>(perm.data_ptr()),
-                                  reinterpret_cast<const __nv_bfloat16*>(grad_out.data_ptr()), reinterpret_cast<__nv_bfloat16*>(grad_table.data_ptr()),
-                                  sorted_ids.numel(), static_cast<int>(grad_out.size(1)), stream_now()), "embedding_bwd");
   });
   // grad_out [T, H] summed by id in position order -> a new table gradient [V, H] (rows that no id names are zero).
   m.def("embedding_grad", [](torch::Tensor ids, int V, torch::Tensor grad_out) {

@@ -17,7 +17,8 @@ class _Embedding(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         (ids,) = ctx.saved_tensors
-        # positions grouped by id by this library's counting sort (stable, cost independent of duplicates)
+        # positions grouped by id by this library's counting sort (stable; its cost does not depend on duplicates), then one warp per
+        # id adds up its rows in position order: an id that names many positions is a serial chain as long as they are
         grad_table = runtime.ext().embedding_grad(ids.reshape(-1).contiguous(), ctx.shape[0], grad_out.reshape(-1, ctx.shape[1]).contiguous())
         return None, grad_table
 
