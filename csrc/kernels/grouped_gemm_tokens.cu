@@ -46,13 +46,12 @@ __host__ __device__ constexpr int stage_bytes(int tile_n) { return kABytes + til
 constexpr int kThreads = 192;
 constexpr int kStepTokens = 32;                   // tokens per epilogue step = rows of a TMA store
 constexpr int kBox = kStepTokens * 128;           // 4 KiB: 32 tokens x 64 features
-constexpr int kPrefix = 256;                      // entries of the tile-count prefix (several groups each when there are more)
 
 struct __align__(8) TokCtl {
   uint64_t full[kMaxStages], empty[kMaxStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load[2];
   uint32_t tmem_base;
   int abort_flag, last_arrived, widest, share_weights;
-  int base[kPrefix + 1];                          // tiles of the groups before entry i
+  int base[kTokPrefix + 1];                         // tiles of the groups before entry i
 };
 __host__ __device__ constexpr int epi_boxes(GemmEpilogue e) { return e == GemmEpilogue::kStore ? 2 : e == GemmEpilogue::kSwiGLU ? 3 : 4; }
 constexpr int kSmemLimit = 227 * 1024;
@@ -67,31 +66,6 @@ constexpr int smem_bytes(GemmEpilogue e, int tile_n) { return stages_for(e, tile
 static_assert(stages_for(GemmEpilogue::kSwiGLUBwd, kTokTileN) == 6 && stages_for(GemmEpilogue::kSwiGLU, 64) == 10, "stages at both ends of the range");
 static_assert(kAccStages * kTokTileN <= kTmemCols, "two accumulators of 256 columns");
 static_assert(kTokPartialFloats == kHalfM * kTokTileN, "a partial is one CTA's accumulator");
-
-// Rows of group q that are worked on: the real ones, up to a multiple of the granule.
-__device__ __forceinline__ int tok_rows(const TokGemmArgs& p, int q) {
-  return p.group_rows ? ceil_to(p.group_rows[q], p.granule) : p.group_off[q + 1] - p.group_off[q];
-}
-
-// Tiles in order, group by group; `locate` wants non-decreasing tile numbers.
-struct TokTiles {
-  const TokGemmArgs& p;
-  const int* base;
-  int per_entry, entry = 0, g = 0, g_base = 0;
-  __device__ __forceinline__ int rows_of(int q) const { return tok_rows(p, q); }
-  struct Tile { int g, m, row0, n; };             // first row of the tile in the grouped matrix, rows = columns of the MMA
-  __device__ __forceinline__ Tile locate(int tile) {
-    if (tile >= base[entry + 1]) {
-      while (tile >= base[entry + 1]) ++entry;
-      g = entry * per_entry; g_base = base[entry];
-    }
-    int rows = rows_of(g);
-    while (tile >= g_base + tok_tiles(rows, p.tile_n) * p.m_tiles) { g_base += tok_tiles(rows, p.tile_n) * p.m_tiles; rows = rows_of(++g); }
-    const TokPlace at = tok_place(tile - g_base, p.m_tiles, tok_tiles(rows, p.tile_n), p.band_tiles);
-    const TokSpan span = tok_span(rows, p.tile_n, at.t);
-    return Tile{g, at.m, p.group_off[g] + span.begin, span.n};
-  }
-};
 
 __device__ __forceinline__ void tma_load_5d_pair(void* smem_dst, const CUtensorMap* map, int x0, int x1, int x2, int x3, int x4, uint32_t bar_cluster_addr) {
   asm volatile(
@@ -154,7 +128,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     if (EPI != GemmEpilogue::kStore) prefetch_tmap(&map_c2);
   }
   if (warp == 1) { tmem_alloc_pair(&ctl->tmem_base, kTmemCols); tmem_relinquish_pair(); }
-  const int per_entry = div_up(p.num_groups, kPrefix);
+  const int per_entry = tok_per_entry(p.num_groups);
   if (warp == 2) {
     // Prefix sums of the tile counts over the groups, the widest tile, and whether any group has several token tiles.
     int run = 0, widest = 0, most = 0;
@@ -163,7 +137,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       int mine = 0;
       for (int q = (e0 + lane) * per_entry; q < min((e0 + lane + 1) * per_entry, p.num_groups); ++q) {
         const int rows = tok_rows(p, q);
-        mine += tok_tiles(rows, p.tile_n) * p.m_tiles;
+        mine += tok_group_tiles(p, q);
         widest = max(widest, tok_tile_size(rows, p.tile_n));
         most = max(most, tok_tiles(rows, p.tile_n));
       }
@@ -187,7 +161,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const TokSplit split = TokSplit::make(ctl->base[div_up(p.num_groups, per_entry)], p.red_blocks, pairs, ctl->widest, ctl->share_weights != 0);
   TokSegments segs(split, pair);
-  TokTiles walk{p, ctl->base, per_entry};
+  TokTiles<TokGemmArgs> walk{p, ctl->base, per_entry};
   TokSegment sg;
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs, each for its own halves) ----------------
@@ -199,7 +173,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       // The first stages' weights do not depend on the kernel before this one: with p.early they are on their way before it has ended.
       bool first = true;
       while (ok && segs.next(sg)) {
-        const TokTiles::Tile tc = walk.locate(sg.tile);
+        const TokTile tc = walk.locate(sg.tile);
         const int half = tc.n >> 1, x_row = tc.row0 + cta * half;
         const uint32_t bytes = 2u * (kABytes + static_cast<uint32_t>(half) * 128u);
         // Where the token panels of a band are a good part of the L2 (p.back_tiles) and a group has several bands, every other
@@ -261,7 +235,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       uint32_t ph = 0, acc_it = 0;
       bool ok = true;
       while (ok && segs.next(sg)) {
-        const TokTiles::Tile tc = walk.locate(sg.tile);
+        const TokTile tc = walk.locate(sg.tile);
         const uint32_t idesc = make_idesc_bf16(kPairM, tc.n, A_MN, false);
         const int a = acc_it % kAccStages;
         const uint32_t aph = (acc_it / kAccStages) & 1;
@@ -298,7 +272,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     uint32_t acc_it = 0, ring_n = 0, load_ph = 0u;   // load_ph: one parity bit per half of the ring
     bool ok = true;
     while (ok && segs.next(sg)) {
-      const TokTiles::Tile tc = walk.locate(sg.tile);
+      const TokTile tc = walk.locate(sg.tile);
       const int a = acc_it % kAccStages;
       const uint32_t aph = (acc_it / kAccStages) & 1;
       ++acc_it;

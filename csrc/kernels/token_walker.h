@@ -1,5 +1,6 @@
 // Work split of the grouped GEMM whose N dimension is the tokens (grouped_gemm_tokens.cu): which tiles there are, in which
-// order, and which part of the reduction of which tile a CTA pair does. Plain arithmetic, usable from host code too.
+// order, and which part of the reduction of which tile a CTA pair does. Plain arithmetic: the native self-check
+// (csrc/sched/selfcheck.cc) walks it on the host over random groups.
 #pragma once
 
 #if defined(__CUDACC__)
@@ -128,6 +129,38 @@ FASTB_HD inline TokPlace tok_place(int local, int m_tiles, int t_tiles, int band
   const int t0 = band * band_tiles, left = t_tiles - t0, cur = left < band_tiles ? left : band_tiles;
   return TokPlace{rem / cur, t0 + rem % cur};
 }
+
+// Rows of group q that are worked on: the real ones, up to a multiple of the granule. Args: TokGemmArgs, or on the host anything with its
+// group_off, group_rows, granule, tile_n, m_tiles and band_tiles.
+template <class Args>
+FASTB_HD inline int tok_rows(const Args& p, int q) { return p.group_rows ? ceil_to(p.group_rows[q], p.granule) : p.group_off[q + 1] - p.group_off[q]; }
+template <class Args>
+FASTB_HD inline int tok_group_tiles(const Args& p, int q) { return tok_tiles(tok_rows(p, q), p.tile_n) * p.m_tiles; }
+
+// Prefix of the tile counts: entry i holds the tiles of the groups before group i * tok_per_entry (several groups an entry
+// when there are more than kTokPrefix).
+constexpr int kTokPrefix = 256;
+FASTB_HD constexpr int tok_per_entry(int groups) { return div_up(groups, kTokPrefix); }
+
+// Tiles in order, group by group; `locate` wants non-decreasing tile numbers.
+struct TokTile { int g, m, row0, n; };            // first row of the tile in the grouped matrix, rows = columns of the MMA
+template <class Args>
+struct TokTiles {
+  const Args& p;
+  const int* base;
+  int per_entry, entry = 0, g = 0, g_base = 0;
+  FASTB_HD TokTile locate(int tile) {
+    if (tile >= base[entry + 1]) {
+      while (tile >= base[entry + 1]) ++entry;
+      g = entry * per_entry; g_base = base[entry];
+    }
+    int rows = tok_rows(p, g);
+    while (tile >= g_base + tok_tiles(rows, p.tile_n) * p.m_tiles) { g_base += tok_tiles(rows, p.tile_n) * p.m_tiles; rows = tok_rows(p, ++g); }
+    const TokPlace at = tok_place(tile - g_base, p.m_tiles, tok_tiles(rows, p.tile_n), p.band_tiles);
+    const TokSpan span = tok_span(rows, p.tile_n, at.t);
+    return TokTile{g, at.m, p.group_off[g] + span.begin, span.n};
+  }
+};
 
 }  // namespace gemm
 }  // namespace fastb

@@ -2,11 +2,13 @@
 // topologies; every plan must validate, deliver the matrix exactly, survive a binary round trip
 // and replay bit-exactly on host buffers. Exit code 0 = all good. Mirrors the role of the
 // reference's DecompositionTester (simulation/test.cpp:15-60) for the whole planner.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <vector>
 
 #include "../kernels/tile_walker.h"
+#include "../kernels/token_walker.h"
 #include "../runtime/range_allocator.h"
 #include "plan.h"
 
@@ -120,10 +122,99 @@ static void walker_check() {
   }
 }
 
+// The work split of the GEMM whose N are the tokens, as its kernel walks it: every pair steps through its own segments. Together
+// they must cover the whole reduction of every tile exactly once, the parts of a cut tile must be where TokSegment says they are, and no
+// partial sum may have to share its place; the tiles must cover the worked-on rows of every group times the features.
+static void token_walker_check() {
+  using namespace fastb::gemm;
+  struct Args { const int *group_off, *group_rows; int granule, tile_n, m_tiles, band_tiles; };
+  struct Part { int kb0, kb1, pair, part, parts, first_pair, pair_step; };
+  uint64_t x = 0x2545f4914f6cdd1dull;
+  auto rnd = [&](int m) { x ^= x << 13; x ^= x >> 7; x ^= x << 17; return static_cast<int>(x % static_cast<uint64_t>(m)); };
+  int cut_stream = 0, cut_parts = 0, long_prefix = 0;
+  for (int trial = 0; trial < 3000; ++trial) {
+    const int G = trial % 50 == 0 ? 257 + rnd(600) : 1 + rnd(trial % 2 ? 9 : 40), pairs = trial % 3 ? 74 : 1 + rnd(74);
+    const int tile_n = 64 << rnd(3), granule = rnd(2) ? 64 : 32, m_tiles = 1 + rnd(trial % 5 ? 6 : 60), kb_tile = 1 + rnd(trial % 4 ? 60 : 460);
+    const bool live = rnd(4) != 0;
+    std::vector<int> off(G + 1, 0), rows(G, 0);
+    for (int g = 0; g < G; ++g) {
+      rows[g] = rnd(5) == 0 ? 0 : 1 + rnd(trial % 7 == 0 ? 3000 : rnd(2) ? 64 : 700);
+      off[g + 1] = off[g] + (rows[g] + 255) / 256 * 256;
+    }
+    const Args p{off.data(), live ? rows.data() : nullptr, granule, tile_n, m_tiles, tok_band_tiles(64 * kb_tile)};
+    CHECK(p.band_tiles >= 1 && p.band_tiles <= kTokBandTiles, "token walker: band");
+    // the prefix as the kernel makes it
+    const int per_entry = tok_per_entry(G), entries = div_up(G, per_entry);
+    CHECK(entries <= kTokPrefix, "token walker: prefix entries");
+    if (per_entry > 1) ++long_prefix;
+    std::vector<int> base(entries + 1, 0);
+    int widest = 0, most = 0;
+    for (int e = 0; e < entries; ++e) {
+      base[e + 1] = base[e];
+      for (int g = e * per_entry; g < std::min(G, (e + 1) * per_entry); ++g) {
+        const int r = tok_rows(p, g), t = tok_tiles(r, tile_n);
+        base[e + 1] += tok_group_tiles(p, g);
+        widest = std::max(widest, tok_tile_size(r, tile_n));
+        most = std::max(most, t);
+        int at = 0, lo = 1 << 30, hi = 0;
+        for (int i = 0; i < t; ++i) {
+          const TokSpan sp = tok_span(r, tile_n, i);
+          CHECK(sp.begin == at && sp.n >= 32 && sp.n % 32 == 0 && sp.n <= tile_n, "token walker: span");
+          at += sp.n; lo = std::min(lo, sp.n); hi = std::max(hi, sp.n);
+        }
+        CHECK(at == r && (t == 0 || (hi - lo <= 32 && hi == tok_tile_size(r, tile_n))), "token walker: spans of a group");
+      }
+    }
+    const int tiles = base[entries];
+    const TokSplit split = TokSplit::make(tiles, kb_tile, pairs, widest, most > 1);
+    CHECK(split.cut_tiles + split.whole_tiles == tiles && split.cut_tiles <= 2 * pairs, "token walker: an arrival counter for every cut tile");
+    if (split.cut_tiles > 0) ++(split.stream ? cut_stream : cut_parts);
+    std::vector<std::vector<Part>> parts(tiles);
+    std::vector<TokTile> where(tiles);
+    for (int pair = 0; pair < pairs; ++pair) {
+      TokSegments segs(split, pair);
+      TokTiles<Args> walk{p, base.data(), per_entry};
+      TokSegment sg;
+      int last = -1, first_slot = 0, later_slot = 0;   // places for partial sums that this pair has used
+      while (segs.next(sg)) {
+        CHECK(sg.tile >= last && sg.tile < tiles && sg.kb0 >= 0 && sg.kb0 < sg.kb1 && sg.kb1 <= kb_tile, "token walker: segment");
+        if (sg.tile < last || sg.tile >= tiles) return;
+        last = sg.tile;
+        if (sg.parts > 1) ++(sg.part == 0 ? first_slot : later_slot);
+        parts[sg.tile].push_back(Part{sg.kb0, sg.kb1, pair, sg.part, sg.parts, sg.first_pair, sg.pair_step});
+        where[sg.tile] = walk.locate(sg.tile);
+      }
+      CHECK(first_slot <= 1 && later_slot <= 1, "token walker: pair %d leaves two partial sums in one place", pair);
+    }
+    std::vector<std::vector<int>> seen(G);   // [feature tile][32 rows]
+    for (int g = 0; g < G; ++g) seen[g].assign(static_cast<size_t>(m_tiles) * (tok_rows(p, g) / 32), 0);
+    for (int t = 0; t < tiles; ++t) {
+      auto& v = parts[t];
+      std::sort(v.begin(), v.end(), [](const Part& a, const Part& b) { return a.kb0 < b.kb0; });
+      int at = 0;
+      for (size_t j = 0; j < v.size(); ++j) {
+        CHECK(v[j].kb0 == at, "token walker: tile %d: reduction covered with a gap or twice", t);
+        CHECK(v[j].parts == static_cast<int>(v.size()) && v[j].part == static_cast<int>(j) && v[j].pair == v[j].first_pair + static_cast<int>(j) * v[j].pair_step,
+              "token walker: tile %d: parts", t);
+        at = v[j].kb1;
+      }
+      CHECK(at == kb_tile, "token walker: tile %d: reduction not covered", t);
+      const TokTile& w = where[t];
+      CHECK(w.g >= 0 && w.g < G && w.m >= 0 && w.m < m_tiles && w.row0 >= off[w.g] && w.row0 + w.n <= off[w.g] + tok_rows(p, w.g), "token walker: place of a tile");
+      if (w.g >= 0 && w.g < G && w.m >= 0 && w.m < m_tiles)
+        for (int r = (w.row0 - off[w.g]) / 32; r < (w.row0 - off[w.g] + w.n) / 32 && r < tok_rows(p, w.g) / 32; ++r) ++seen[w.g][static_cast<size_t>(w.m) * (tok_rows(p, w.g) / 32) + r];
+    }
+    for (auto& v : seen)
+      for (int n : v) CHECK(n == 1, "token walker: rows covered %d times", n);
+  }
+  CHECK(cut_stream > 100 && cut_parts > 100 && long_prefix > 20, "token walker: the trials reach every way of cutting");
+}
+
 int main() {
   allocator_check();
   walker_check<128>();
   walker_check<256>();
+  token_walker_check();
   const int topo[][2] = {{1, 1}, {1, 4}, {4, 1}, {2, 2}, {2, 4}, {3, 3}, {8, 1}, {4, 2}};
   const PlanKind kinds[] = {PlanKind::kStaged, PlanKind::kSingleBurst, PlanKind::kFanout, PlanKind::kSpreadOut};
   int plans = 0;

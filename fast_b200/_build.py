@@ -96,7 +96,7 @@ def build_selfcheck(force=False):
     out = ROOT / "build" / "fastb-selfcheck"
     out.parent.mkdir(exist_ok=True)
     srcs = [CSRC / "sched" / "selfcheck.cc"] + [CSRC / "sched" / f"{s}.cc" for s in SCHED_SRCS]
-    if force or _stale(out, srcs + _headers("sched") + _headers("runtime") + [CSRC / "kernels" / "tile_walker.h"]):
+    if force or _stale(out, srcs + _headers("sched") + _headers("runtime") + [CSRC / "kernels" / "tile_walker.h", CSRC / "kernels" / "token_walker.h"]):
         _run(["g++", "-std=c++17", "-O2", "-Wall", "-pthread", *srcs, "-o", out])
     return out
 
