@@ -79,6 +79,12 @@ def test_graft_entry_has_build_and_smoke():
     assert any(f.startswith("_C.") and f.endswith(".so") for f in os.listdir(os.path.dirname(fast_b200.__file__)))
 
 
+def test_cmake_kernel_library_names_every_kernel_source():
+    text = open(os.path.join(ROOT, "CMakeLists.txt")).read()
+    missing = [f for f in os.listdir(os.path.join(ROOT, "csrc", "kernels")) if f.endswith(".cu") and f"/{f}" not in text]
+    assert not missing, missing
+
+
 def test_bench_clock_sampler_parses_samples_inside_the_window():
     import importlib.util
     import time
