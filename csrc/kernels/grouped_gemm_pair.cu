@@ -136,9 +136,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             gated = slot;
           }
         }
-        // Weight gradients over many tokens (a band's 16 panels fill a good part of the L2): every other wave walks the
-        // reduction backwards, from the panel ends that the wave before left there. 19.3 -> 19.0 ms at 8 x 8192 tokens.
-        const bool back = MODE == GemmMode::kWgrad && tc.red_blocks > 64 && ((tile / pairs) & 1);
+        const bool back = MODE == GemmMode::kWgrad && wgrad_back(tc.red_blocks, p.band_rows) && ((tile / pairs) & 1);
         for (int kbi = 0; kbi < tc.red_blocks; ++kbi, ++it) {
           const int kb = back ? tc.red_blocks - 1 - kbi : kbi;
           const int s = it % NS;

@@ -25,7 +25,18 @@ struct TileCoord {
 // operand bytes a wave pulls from DRAM (a wave of p x q tiles reads p A-panels and q B-panels).
 // TILE_M is 128 (one CTA) or 256 (CTA pair). `locate` must be called with non-decreasing tile
 // indices (each role of a CTA steps its own walker by the grid stride).
+// For weight gradients that is 16 tiles: 8 experts of 8192 rows of a training step, seconds at the power cap, TFLOP/s at bands of 4, 8
+// and 16 tiles, down projection 1193, 1284, 1292, gate|up 1258, 1269, 1265; at 4096 rows 1208, 1290, 1316 and 1320, 1292, 1299.
 constexpr int kDefaultBandRows = 4096;
+// Weight gradients: whether every other wave walks the reduction (the group's rows) backwards, from the panel ends that the wave before
+// left in L2. It pays where a band's panels are more than a quarter of the 126 MB L2, i.e. above 4096 rows in the default
+// band. 8 experts of 8192 rows of a training step, seconds at the power cap, always forwards -> this: 1240 -> 1292 TFLOP/s (down
+// projection), 1198 -> 1262 (gate|up). On normal random rows, forwards against every other wave backwards: 6144 rows 1309, 1326 and
+// 1252, 1256; 5120 rows 1331, 1336 and 1271, 1270; 4096 rows 1350, 1337 and 1291, 1285; 3072 rows 1344, 1333 and 1318, 1305.
+constexpr long long kBackBandBytes = 32ll << 20;
+FASTB_HD inline bool wgrad_back(int red_blocks, int band_rows) {
+  return 2ll * red_blocks * kWalkBK * (band_rows > 0 ? band_rows : kDefaultBandRows) > kBackBandBytes;
+}
 template <int TILE_M>
 struct TileWalker {
   const int* off; int G, tiles_n, fixed_m, red_len; bool wgrad; int band_rows;

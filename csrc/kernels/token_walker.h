@@ -112,8 +112,10 @@ struct TokSegments {
 // tiles that run together cover a squarish patch and share their operand panels in L2.
 // How many: as the reduction grows, fewer, so that the token panels of a band take at most half of the L2 while the weights
 // stream past them; at most 8, where a wave of 74 tiles is square. What this saves is the power that moving operands costs,
-// and with it clock: 8 experts of 8192 tokens, seconds at the power cap, TFLOP/s at
-// bands of 16, 8, 4 tiles: reduction of 4096 1312, 1396, 1340; of 14336 1115, 1353, 1356; of 28672 1050, 1267, 1315.
+// and with it clock. 8 experts of 8192, 4096 and 2048 rows of a training step, seconds at the power cap, TFLOP/s at bands of 16, 8, 4
+// tiles: reduction of 4096 1280, 1262, 1152; 1265, 1254, 1163; 1276, 1235, 1146; of 14336 1103, 1134, 1073; 1155, 1137, 1123; 1189,
+// 1182, 1124; of 28672 981, 1010, 1007; 1052, 1040, 1073; 1098, 1100, 1063. On normal random rows 16 tiles are ahead by 3-5 % at 8192 rows;
+// inside the step (32768 tokens) 16 and this rule are equal: 58.6 and 58.8 ms of GEMMs, single runs 58.0-59.6.
 constexpr int kTokBandBytes = 60 << 20, kTokBandTiles = 8;
 FASTB_HD inline int tok_band_tiles(int red_len) {
   const long long fit = kTokBandBytes / (2ll * red_len * kTokTileN);

@@ -214,6 +214,7 @@ int main() {
   allocator_check();
   walker_check<128>();
   walker_check<256>();
+  CHECK(!fastb::gemm::wgrad_back(64, 0) && fastb::gemm::wgrad_back(65, 0) && fastb::gemm::wgrad_back(33, 8192), "walker: reductions walked backwards from 4096 rows on");
   token_walker_check();
   const int topo[][2] = {{1, 1}, {1, 4}, {4, 1}, {2, 2}, {2, 4}, {3, 3}, {8, 1}, {4, 2}};
   const PlanKind kinds[] = {PlanKind::kStaged, PlanKind::kSingleBurst, PlanKind::kFanout, PlanKind::kSpreadOut};
