@@ -76,13 +76,14 @@ struct A2AProgramPy {
 
   static bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
 
-  // Called before a launch on `stream` (the current one): the launch comes after the upload, and the list's memory is not given
-  // to anybody else before the launch has ended, also when the schedule is dropped earlier.
-  void ready_on(c10::cuda::CUDAStream stream) const {
-    if (!uploaded) {
+  // Called before a launch on `stream` (the current one; `captured`: it is being captured): the launch comes after the upload, and
+  // the list's memory is not given to anybody else before the launch has ended, also when the schedule is dropped earlier. On the
+  // stream of the upload itself both hold as they are.
+  void ready_on(c10::cuda::CUDAStream stream, bool captured) const {
+    if (!uploaded && (captured || stream != home)) {
       c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);   // a capture elsewhere does not mind the query
       if (upload.query()) uploaded = true;
-      else if (capturing()) { upload.synchronize(); uploaded = true; }   // a captured launch cannot wait for an event from outside of its graph
+      else if (captured) { upload.synchronize(); uploaded = true; }   // a captured launch cannot wait for an event from outside of its graph
       else upload.block(stream);
     }
     if (stream != home) c10::cuda::CUDACachingAllocator::recordStream(program_dev.storage().data_ptr(), stream);
@@ -111,7 +112,7 @@ void a2a_launch(const A2AProgramPy& p, const HeapPy& heap, std::array<int64_t, 4
   TORCH_CHECK(heap.h->world() <= kSigMaxWorld, "world larger than the signal block supports");
   A2ARankArgs a = p.args(heap, src_ptrs, dst_offs, sig_off, epoch, st, timeout_ns, stamps_ptr);
   a.bulk = bulk ? 1 : 0;
-  p.ready_on(c10::cuda::getCurrentCUDAStream());
+  p.ready_on(c10::cuda::getCurrentCUDAStream(), !p.uploaded && A2AProgramPy::capturing());
   cuda_check(launch_a2a_push(a, ctas, threads, cur_stream(), p.has_waits), "a2a_push launch");
 }
 
@@ -142,7 +143,8 @@ bool a2a_launch_group(const std::vector<const A2AProgramPy*>& progs, const std::
     host[r] = progs[r]->args(*heaps[r], {reinterpret_cast<int64_t>(ins[r].data_ptr()), 0, base + dst[2], base + dst[3]}, dst, sig_off, epoch, *sts[r], timeout_ns);
   }
   const auto stream = c10::cuda::getCurrentCUDAStream();
-  for (const A2AProgramPy* p : progs) p->ready_on(stream);
+  const bool captured = std::any_of(progs.begin(), progs.end(), [](const A2AProgramPy* p) { return !p->uploaded; }) && A2AProgramPy::capturing();
+  for (const A2AProgramPy* p : progs) p->ready_on(stream, captured);
   // A rank with a handful of work items needs a handful of CTAs (every launched CTA takes a turn at the exit counter).
   cuda_check(launch_a2a_push_group(host.data(), static_cast<int>(n), std::min(ctas, most), threads, cur_stream()), "a2a_push group launch");
   return true;
