@@ -36,6 +36,11 @@ class FusedAdamW:
                 p.grad.zero_()
 
     def _update(self, params, grads, grad_scale: float) -> None:
+        if len(set(params)) < len(params):
+            # One launch updates its tensors side by side: a parameter that is listed twice is updated twice, one after the other.
+            for p, g in zip(params, grads):
+                self._update([p], [g], grad_scale)
+            return
         state = [self.state[p] for p in params]
         for p in params:
             self.steps[p] += 1
