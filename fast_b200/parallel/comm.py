@@ -423,7 +423,7 @@ class LocalGroup:
         self.comms = [Communicator(heap_bytes=heap_bytes, topo=topo, device=device, timeout_s=timeout_s, ctas=ctas, threads=threads,
                                    _heap=h, _rank=r, _world=world) for r, h in enumerate(heaps)]
         self.world, self.ctas, self.threads = world, ctas, threads
-        self._heaps, self._statuses = heaps, [c.status for c in self.comms]
+        self._statuses = [c.status for c in self.comms]
 
     def schedule(self, matrix, **kw) -> List[Schedule]:
         return [c.schedule(matrix, **kw) for c in self.comms]
@@ -437,14 +437,15 @@ class LocalGroup:
             c.epoch += 1
         c0 = comms[0]
         progs, ins = [s.program for s in scheds], list(inputs)
+        heaps = [c.heap for c in comms]   # not kept: a closed communicator lets go of its slab
         args = ((bal, rail), c0.sig_off, c0.epoch, self._statuses, c0.timeout_ns, self.ctas, self.threads)
-        if self._C.a2a_launch_group(progs, self._heaps, list(outputs), ins, *args):
+        if self._C.a2a_launch_group(progs, heaps, list(outputs), ins, *args):
             return
         recv = [c.heap.tensor(c._stage("recv", need["output"]), [need["output"]], torch.uint8) for c in comms]  # library-owned, copied out afterwards
         for o, s in zip(outputs, scheds):
             if o.numel() * o.element_size() < s.output_bytes:
                 raise ValueError("output smaller than the schedule needs")
-        self._C.a2a_launch_group(progs, self._heaps, recv, ins, *args)
+        self._C.a2a_launch_group(progs, heaps, recv, ins, *args)
         for o, t, s in zip(outputs, recv, scheds):
             o.view(torch.uint8).reshape(-1)[: s.output_bytes].copy_(t[: s.output_bytes])
 

@@ -277,6 +277,21 @@ def test_close_refuses_further_launches_and_keeps_live_tensors_valid():
     comm.close()                     # idempotent
 
 
+def test_closed_group_gives_its_slabs_back():
+    """Closing every communicator of an in-process group frees the slabs, also while the group object lives on."""
+    from fast_b200.parallel import LocalGroup
+
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    grp = LocalGroup(2, heap_bytes=512 << 20, topo=Topology.flat(2), ctas=2, threads=64)
+    assert before - torch.cuda.mem_get_info()[0] > 900 << 20
+    for c in grp.comms:
+        c.close()
+    assert before - torch.cuda.mem_get_info()[0] < 200 << 20
+    with pytest.raises(RuntimeError, match="closed"):
+        grp.all_to_all_v([], [], [type("S", (), {"max_bytes": {"balance": 0, "rail": 0}})()])
+
+
 @pytest.mark.parametrize("servers,gpus", [(2, 2), (2, 4)])
 @pytest.mark.parametrize("kind", [PlanKind.STAGED, PlanKind.SINGLE_BURST])
 def test_rail_segments_bit_exact(servers, gpus, kind):
