@@ -115,7 +115,7 @@ def measure(comm, tokens=4096, hidden=7168, inter=2048, experts_per_gpu=32, top_
             # phase boundary for timing only: all rows of this rank's experts have landed
             C.wait_counters(eng._arrive_ptr(0), eng.tile_target[0] if eng.tile_rows else eng.arrive_target[0], eng.status, eng.timeout_ns)
         ev[2].record()
-        eng.experts_forward(w13, w2, rs)
+        eng.experts_forward(w13, w2, rs, settled=True)
         ev[3].record()
         out = eng.combine(rs, rs.topk_w)
         ev[4].record()

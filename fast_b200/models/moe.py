@@ -32,7 +32,7 @@ class _MoEFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weights, w13, w2, engine, rs):
         engine.dispatch(x, rs)
-        engine.experts_forward(w13, w2, rs)
+        engine.experts_forward(w13, w2, rs, settled=True)
         out = engine.combine(rs, weights.detach().float().contiguous())
         ctx.engine, ctx.rs, ctx.w2_param = engine, rs, w2
         ctx.save_for_backward(weights, w13, w2)
@@ -85,7 +85,7 @@ class _NormRouteMoEFunction(torch.autograd.Function):
         rs, hn, rstd, _ = engine.route_fused(h, norm_w, gate, eps, layer.router_bias)
         layer.last_route = rs
         engine.dispatch(hn, rs)
-        engine.experts_forward(w13, w2, rs)
+        engine.experts_forward(w13, w2, rs, settled=True)
         out = engine.combine(rs, rs.topk_w)
         ctx.engine, ctx.rs, ctx.w2_param = engine, rs, w2
         ctx.save_for_backward(h, norm_w, gate, rstd, w13, w2)
@@ -111,7 +111,7 @@ class _NormRouteMoELossFunction(torch.autograd.Function):
         rs, hn, rstd, _ = engine.route_fused(h, norm_w, gate, eps, layer.router_bias)
         layer.last_route = rs
         engine.dispatch(hn, rs)
-        engine.experts_forward(w13, w2, rs)
+        engine.experts_forward(w13, w2, rs, settled=True)
         loss = torch.empty(1, dtype=torch.float32, device=h.device)
         out = engine.combine(rs, rs.topk_w, residual=h, loss=loss)
         ctx.engine, ctx.rs, ctx.w2_param = engine, rs, w2
@@ -179,7 +179,7 @@ class MoELayer(nn.Module):
         rs = self.engine.route_gate(x, self.gate, self.router_bias)
         self.last_route = rs
         self.engine.dispatch(x, rs)
-        self.engine.experts_forward(self.w13, self.w2, rs)
+        self.engine.experts_forward(self.w13, self.w2, rs, settled=True)
         return self.engine.combine(rs, rs.topk_w)
 
     def forward_from_residual(self, h: torch.Tensor, norm_w: torch.Tensor, eps: float) -> torch.Tensor:

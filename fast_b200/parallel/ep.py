@@ -192,10 +192,10 @@ class ExpertParallel:
         """Whether rows past an expert's real ones are computed with: by the one-CTA GEMM always, else by weight gradients only."""
         return self.training or not gemm.USE_PAIR
 
-    def _live(self, rs: RouteState) -> dict:
+    def _live(self, rs: RouteState, settled: bool = True) -> dict:
         if self.scratch is None:
             return {}
-        self.scratch.early = rs.topk_idx.shape[0] > 0   # without tokens there is no dispatch kernel between routing and GEMM
+        self.scratch.early = settled and rs.topk_idx.shape[0] > 0   # without tokens there is no dispatch kernel between routing and GEMM
         # a token picks an expert at most once; other ranks may have up to max_tokens of them
         most = rs.topk_idx.shape[0] if self.comm.world == 1 else self.T * self.comm.world
         return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch, most_rows=most)
@@ -307,7 +307,9 @@ class ExpertParallel:
             torch.cuda.current_stream().wait_event(self._dispatch_done)
             self._dispatch_done = None
 
-    def experts_forward(self, w13: torch.Tensor, w2: torch.Tensor, rs: RouteState) -> None:
+    def experts_forward(self, w13: torch.Tensor, w2: torch.Tensor, rs: RouteState, settled: bool = False) -> None:
+        """The two expert GEMMs on the rows that ``dispatch`` has sent. ``settled``: nothing queued since ``dispatch`` writes ``w13``;
+        the first GEMM may then read it before the kernel ahead of it has ended."""
         C = self._C
         if self.comm.world == 1 and not self.overlap:   # alone, every row is in once the dispatch kernel is over
             gate, gate_tile = None, 0
@@ -330,7 +332,7 @@ class ExpertParallel:
                 gate = None
             # A gated GEMM leaves SMs to the dispatch it waits for; an ungated one (every row is in) takes them all.
             gemm.grouped_gemm_fwd(self.x_recv, w13, rs.group_off, self.act, swiglu=True, gate_up_out=self.gu if self.training else None, gate=gate,
-                                  gate_tile_rows=gate_tile, ctas=self.gemm1_ctas if gate is not None else None, **self._live(rs))
+                                  gate_tile_rows=gate_tile, ctas=self.gemm1_ctas if gate is not None else None, **self._live(rs, settled))
         gemm.grouped_gemm_fwd(self.act, w2, rs.group_off, self.y, **self._live(rs))
         self._join_dispatch()
 
@@ -353,7 +355,7 @@ class ExpertParallel:
         with nvtx_range("dispatch"):
             self.dispatch(x, rs)
         with nvtx_range("experts"):
-            self.experts_forward(w13, w2, rs)
+            self.experts_forward(w13, w2, rs, settled=True)
         with nvtx_range("combine"):
             out = self.combine(rs, rs.topk_w if weights is None else weights)
         return out, rs

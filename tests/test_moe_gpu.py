@@ -504,6 +504,34 @@ def test_views_that_start_between_16_byte_words():
     comm.check()
 
 
+def test_weights_written_after_dispatch_are_waited_for(monkeypatch):
+    """The expert GEMM may read its weights before the kernel ahead of it has ended only where its caller says that this kernel does
+    not write them: the layer does, a caller of the engine's own steps does not by default."""
+    from fast_b200.models import MoELayer
+    from fast_b200.ops import gemm
+    from fast_b200.parallel import Communicator
+
+    if not gemm.USE_PAIR:
+        pytest.skip("one-CTA kernels are not launched early")
+    comm = Communicator(heap_bytes=128 << 20, device=0)
+    layer = MoELayer(comm, 256, 256, 8, 2, max_tokens=512, training=False).eval()
+    eng, early, fwd = layer.engine, [], gemm.grouped_gemm_fwd
+    monkeypatch.setattr(gemm, "grouped_gemm_fwd", lambda *a, **k: (early.append(k["scratch"].early), fwd(*a, **k))[1])
+    x = torch.randn(300, 256, device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        want = layer(x)
+        assert early == [True, True]
+        early.clear()
+        w13 = torch.zeros_like(layer.w13)
+        rs = eng.route_gate(x, layer.gate)
+        eng.dispatch(x, rs)
+        w13.copy_(layer.w13)
+        eng.experts_forward(w13, layer.w2, rs)
+        assert early == [False, True]
+        assert torch.equal(eng.combine(rs, rs.topk_w), want)
+    comm.check()
+
+
 def test_forward_layer_in_cuda_graph():
     """The forward-only layer captured in a CUDA graph replays correctly on new inputs (the step's
     epoch lives in device memory, so a replay is a new step)."""
