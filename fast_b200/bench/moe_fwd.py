@@ -140,7 +140,7 @@ def measure(comm, tokens=4096, hidden=7168, inter=2048, experts_per_gpu=32, top_
     route_us, dispatch_us, experts_us, combine_us, layer_us = _max_over_ranks(acc, world)
     tm = eng.traffic_matrix().cpu().numpy()
     res = {"bench": "moe_forward", "world": world, "overlap_dispatch": overlap, "overlap_reserve_sms": eng.overlap_reserve_sms, "tokens_per_rank": T, "hidden": H, "inter": I, "experts": E, "top_k": K,
-           "dispatch_dtype": "fp8_e4m3_1x128" if fp8 else "bf16", "expert_feed": "e4m3 rows converted inside the GEMM" if eng.fp8_direct else ("dequantised to bf16 first" if fp8 else "bf16"), "route_us": round(route_us, 1), "dispatch_us": round(dispatch_us, 1),
+           "dispatch_dtype": "fp8_e4m3_1x128" if fp8 else "bf16", "expert_feed": "e4m3 rows converted inside the GEMM" if eng.fp8_direct else "bf16 values of the e4m3 rows, stored by the dispatch" if eng.local_bf16 else "dequantised to bf16 first" if fp8 else "bf16", "route_us": round(route_us, 1), "dispatch_us": round(dispatch_us, 1),
            "experts_us": round(experts_us, 1), "combine_us": round(combine_us, 1), "combine_alone_us": round(combine_alone_us, 1),
            "dispatch_plus_combine_us": round(dispatch_us + combine_alone_us, 1),
            "layer_us": round(layer_us, 1),  # whole layer per iteration, max over ranks (phase maxima above fall on different ranks)
