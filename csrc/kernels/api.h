@@ -108,6 +108,7 @@ struct GemmArgs {
                            // over them up to a multiple of 64
   int gate_tile_rows;      // 0: gate_counter / gate_target are indexed by group; > 0: by (row of the grouped matrix) / gate_tile_rows
   int gate_slots;          // entries of gate_counter / gate_target (indices are clamped to the last one)
+  int wide;                // CTA-pair weight gradients: tiles of 512 columns (tiles_n counts those) instead of 256
 };
 
 int grouped_gemm_smem_bytes();
@@ -125,9 +126,9 @@ cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUte
 
 // Weights as operand A, tokens as operand B (grouped_gemm_tokens.cu): forward and dgrad on CTA pairs, tiles of 256 features by
 // up to 256 tokens, the last wave cut into shares of the reduction.
-constexpr int kTokPartialFloats = 128 * 256;   // fp32 sums of one CTA's part of a tile
+constexpr int kTokPartialFloats = 128 * 256;   // fp32 sums of one CTA's part of an accumulator
 constexpr int tok_counters(int ctas) { return 2 * ctas; }                                  // arrival counters a launch needs
-constexpr long long tok_partial_floats(int ctas) { return 2ll * ctas * kTokPartialFloats; }  // two partial tiles per CTA
+constexpr long long tok_partial_floats(int ctas, int tile_n) { return (tile_n > 256 ? 4ll : 2ll) * ctas * kTokPartialFloats; }  // two partial tiles per CTA
 // Maps of the tokens: entry j loads boxes of {64, 16 << j}. Half a tile's tokens (a multiple of 16 up to 128) are at most three.
 constexpr int kTokBoxes = 4;
 struct TokMapsX { CUtensorMap box[kTokBoxes]; };
@@ -144,14 +145,14 @@ struct TokGemmArgs {
   int m_tiles;               // 256-feature tiles of the output's columns (SwiGLU forward: of gate|up)
   int red_blocks;            // 64-wide blocks of the reduction
   int w_rows_per_group;      // rows of a group's slice in w's matrix (forward: features, dgrad: reduction)
-  int tile_n;                // most tokens of a tile: 64, 128 or 256
+  int tile_n;                // most tokens of a tile: 64, 128, 256 or 512
   int stages;                // set by the launcher
   int band_tiles;            // token tiles of a raster band
   int back_tiles;            // groups of more token tiles than this alternate the direction of the reduction from wave to wave
   int granule;               // tile widths are multiples of this (32 or 64); rows up to a multiple of it are written
   int keep_gate_up;
   int early;                 // 1: weights, group_off and group_rows were written by no kernel later than the last but one of the stream
-  float* partials;           // tok_partial_floats(ctas)
+  float* partials;           // tok_partial_floats(ctas, tile_n)
   unsigned int* counters;    // num_counters >= tok_counters(ctas), zero before the launch and after it
   unsigned int* counters_next;   // num_counters; cleared by the launch
   int num_counters;

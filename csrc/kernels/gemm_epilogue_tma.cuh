@@ -22,6 +22,9 @@ constexpr int kEpiThreads = 128;
 // Named barrier 1: the four epilogue warps only (barrier 0 is __syncthreads of the whole CTA).
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
+// Named barriers 1 and 2: the four warps of one of two epilogue groups.
+__device__ __forceinline__ void group_bar(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(ptx::smem_u32(smem_src)), "r"(x), "r"(y)

@@ -49,6 +49,21 @@ constexpr int kQBytes = PM * BK;      // 8 KiB of e4m3
 constexpr int kCvtWarps = 4;
 constexpr int kThreadsFp8 = kThreads + 32 * kCvtWarps;
 
+// Weight gradients in tiles of 512 columns (WIDE): two accumulators that share operand A, which the tensor core reads from shared
+// memory once for both; four stages of 48 KiB; two groups of four epilogue warps, which take the columns in turn and hold
+// what they have read from tensor memory in registers that the first four warps have given up.
+// Bound by the power cap, and what it saves is operand traffic: 96 KiB from L2 per block of 64 rows instead of 2 x 64, and a shared-memory
+// reading of operand A for every second product. Seconds at the cap, TFLOP/s, 256 -> 512 columns: 8 experts x 8192 rows, W2 (4096 x 14336)
+// 1306 -> 1432, W13 1240 -> 1413. With few rows the output is the work, and half as many tiles pass through the kernel: us at 256, 512,
+// 1024, 2048, 4096 rows for W2 380 -> 311, 484 -> 446, 743 -> 742, 1399 -> 1367, 2743 -> 2726; for W13 696 -> 610, 944 -> 854, 1471 -> 1458,
+// 2830 -> 2767, 5741 -> 5480. So they are taken wherever the columns are a multiple of 512.
+constexpr int kWideStages = 4;
+constexpr int kWideStageBytes = kABytes + 2 * kBBytes;
+constexpr int kWideFirstEpiWarp = 4;
+constexpr int kWideThreads = 32 * kWideFirstEpiWarp + 2 * 32 * kEpiWarps;
+constexpr int kLaunchRegs = 168, kOtherRegs = 72, kEpilogueRegs = 216;   // a thread
+static_assert(kOtherRegs + 2 * kEpilogueRegs <= 3 * kLaunchRegs && kWideThreads * kLaunchRegs <= 65536, "what the epilogue takes, the others have given");
+
 struct __align__(8) SmemCtl {
   uint64_t full[kStages], empty[kStages], acc_full[kAccStages], acc_empty[kAccStages], q_full[kQStages], q_empty[kQStages];
   uint32_t tmem_base;
@@ -56,6 +71,8 @@ struct __align__(8) SmemCtl {
 };
 constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024 + sizeof(SmemCtl);
 constexpr int kSmemBytesFp8 = kStagesFp8 * kStageBytes + kQStages * kQBytes + kEpiBytes + 1024 + sizeof(SmemCtl);
+constexpr int kSmemBytesWide = kWideStages * kWideStageBytes + kEpiBytes + 1024 + sizeof(SmemCtl);
+static_assert(kSmemBytesWide <= 227 * 1024 && kWideStages <= kStages, "wide tiles: shared memory and barriers");
 static_assert(kSmemBytes <= 227 * 1024 && kSmemBytesFp8 <= 227 * 1024, "dynamic shared memory of one CTA on sm_100a");
 static_assert(kStagesFp8 <= kStages, "barrier arrays are sized for the larger stage count");
 static_assert(kABytes % 1024 == 0 && kBBytes % 1024 == 0, "operand tiles start on 1024-byte boundaries (128-byte swizzle atoms)");
@@ -78,15 +95,19 @@ __device__ __forceinline__ uint32_t bf16_pair_of(float x) {  // x is bf16-repres
 // thread writes its own row in global memory.
 // A_FP8 (forward only): map_a describes e4m3 bytes (boxes of 64 bytes x 128 rows, no swizzle) and
 // p.a_scales their 1x128 scales; see kStagesFp8 above.
-template <GemmMode MODE, GemmEpilogue EPI, bool TMA_EPI, bool A_FP8>
-__global__ void __launch_bounds__(A_FP8 ? kThreadsFp8 : kThreads, 1)
+template <GemmMode MODE, GemmEpilogue EPI, bool TMA_EPI, bool A_FP8, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kWideThreads : A_FP8 ? kThreadsFp8 : kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                          const __grid_constant__ CUtensorMap map_c2, const GemmArgs p) {
   static_assert(A_FP8 ? MODE == GemmMode::kForward && TMA_EPI : MODE == GemmMode::kWgrad && EPI == GemmEpilogue::kStore, "e4m3 forward or bf16 weight gradient");
-  constexpr int NS = A_FP8 ? kStagesFp8 : kStages;  // operand stages in use
+  static_assert(!WIDE || (TMA_EPI && !A_FP8), "wide tiles: weight gradients through TMA stores");
+  constexpr int NS = WIDE ? kWideStages : A_FP8 ? kStagesFp8 : kStages;  // operand stages in use
+  constexpr int STAGE = WIDE ? kWideStageBytes : kStageBytes;
+  constexpr int ACCS = WIDE ? 2 : 1;                 // accumulators of a tile
+  constexpr int FIRST_EPI_WARP = WIDE ? kWideFirstEpiWarp : 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* q_ring = tiles + NS * kStageBytes;                                 // A_FP8 only: kQStages x 8 KiB of e4m3
+  uint8_t* q_ring = tiles + NS * STAGE;                                 // A_FP8 only: kQStages x 8 KiB of e4m3
   uint8_t* epi_stage = q_ring + (A_FP8 ? kQStages * kQBytes : 0);            // two 16 KiB buffers, 1024-byte aligned like the operand tiles
   SmemCtl* ctl = reinterpret_cast<SmemCtl*>(epi_stage + kEpiBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -99,7 +120,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     // full[s] (leader's copy is the one in use): the producer's expect_tx arrival, plus one arrival from
     // each CTA's converter warp when the A tile is written by them instead of by TMA.
     for (int s = 0; s < NS; ++s) { mbar_init(&ctl->full[s], A_FP8 ? 1 + 2 : 1); mbar_init(&ctl->empty[s], 1); }
-    for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * kEpiWarps); }
+    for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * ACCS * kEpiWarps); }
     for (int q = 0; q < kQStages; ++q) { mbar_init(&ctl->q_full[q], 1); mbar_init(&ctl->q_empty[q], 1); }
     ctl->abort_flag = 0;
     mbar_fence_init();
@@ -119,8 +140,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   TileWalker<TILE_M> walk{p.group_off, p.num_groups, p.tiles_n, p.fixed_m_tiles, p.red_len, MODE == GemmMode::kWgrad, p.band_rows, MODE == GemmMode::kWgrad ? p.group_rows : nullptr};
   TileCoord tc;
+  auto give_registers = [] {
+    if constexpr (WIDE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+  };
 
   if (warp == 0) {
+    give_registers();
     // ---------------- TMA producer (both CTAs, each for its own halves) ----------------
     if (elect_one()) {
       uint32_t it = 0;
@@ -142,11 +167,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const int s = it % NS;
           const uint32_t ph = (it / NS) & 1;
           if (!(ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1, abort_flag, p.status, 100 + s, p.timeout_ns))) break;
-          uint8_t* sa = tiles + s * kStageBytes;
+          uint8_t* sa = tiles + s * STAGE;
           uint8_t* sb = sa + kABytes;
           const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
           const int m0 = tc.m_idx * TILE_M + static_cast<int>(cta) * PM;  // first row of my A half inside the group / fixed dim
-          const int n0 = tc.n_idx * BN + static_cast<int>(cta) * PN;      // first column of my B half
+          const int n0 = tc.n_idx * (ACCS * BN) + static_cast<int>(cta) * PN;   // first column of my B half (of the first accumulator)
           if (A_FP8) {  // e4m3 block into the ring (its converter warp writes the A half of the stage), B by TMA as usual
             const int q = it % kQStages;
             const uint32_t qph = (it / kQStages) & 1;
@@ -157,14 +182,68 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             tma_load_2d_pair(sb, &map_b, kb * BK, tc.g * p.b_rows_per_group + n0, full_leader);
             continue;
           }
-          if (leader) mbar_arrive_expect_tx(&ctl->full[s], 2 * kStageBytes);
+          if (leader) mbar_arrive_expect_tx(&ctl->full[s], 2 * STAGE);
 #pragma unroll
           for (int j = 0; j < PM / 64; ++j)
             tma_load_2d_pair(sa + j * (BK * 128), &map_a, m0 + j * 64, tc.row0 + kb * BK, full_leader);
 #pragma unroll
-          for (int j = 0; j < PN / 64; ++j)
-            tma_load_2d_pair(sb + j * (BK * 128), &map_b, n0 + j * 64, tc.row0 + kb * BK, full_leader);
+          for (int j = 0; j < ACCS * (PN / 64); ++j)
+            tma_load_2d_pair(sb + j * (BK * 128), &map_b, n0 + j / 2 * BN + j % 2 * 64, tc.row0 + kb * BK, full_leader);
         }
+      }
+    }
+  } else if (WIDE && warp == 1) {
+    give_registers();
+    // ---------------- MMA issuer of wide tiles (leader CTA only) ----------------
+    if (leader && elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(TILE_M, BN, A_MN, B_MN);
+      uint32_t ph = 0, done = 0;
+      int s = 0;
+      bool ok = true;
+      enum { kFirst, kSecond, kBoth };
+      auto multiply = [&](int which, bool fresh) {
+        const uint32_t sa = smem_u32(tiles + s * STAGE), sb = sa + kABytes;
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) {
+          const uint64_t da = make_smem_desc(sa + k * 2048, BK * 128, 1024);
+          const uint64_t db0 = make_smem_desc(sb + k * 2048, BK * 128, 1024), db1 = make_smem_desc(sb + kBBytes + k * 2048, BK * 128, 1024);
+          const uint32_t add = (!fresh || k != 0) ? 1u : 0u;
+          if (which == kBoth) {
+            mma_bf16_ss_pair_fill_a(tmem_base, da, db0, idesc, add);
+            mma_bf16_ss_pair_last_a(tmem_base + BN, da, db1, idesc, add);
+          } else if (which == kFirst) {
+            mma_bf16_ss_pair(tmem_base, da, db0, idesc, add);
+          } else {
+            mma_bf16_ss_pair(tmem_base + BN, da, db1, idesc, add);
+          }
+        }
+      };
+      auto claim = [&](int a) {
+        ok = mbar_wait_bounded(&ctl->acc_empty[a], (done & 1) ^ 1, abort_flag, p.status, 200 + a, p.timeout_ns);
+        tc_fence_after_sync();
+        return ok;
+      };
+      for (int tile = pair; ok && walk.locate(tile, tc); tile += pairs) {
+        if (tc.red_blocks == 0) continue;
+        if (!claim(0)) break;
+        for (int kb = 0; kb < tc.red_blocks; ++kb) {
+          if (!(ok = mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.status, 300 + s, p.timeout_ns))) break;
+          tc_fence_after_sync();
+          const bool head = kb == 0, tail = kb + 1 == tc.red_blocks;
+          if (!head && !tail) {
+            multiply(kBoth, false);
+          } else {   // one accumulator after the other, so that the first is full, and needed again, a little earlier than the second
+            multiply(kFirst, head);
+            if (tail) mma_commit_pair(&ctl->acc_full[0], 0x3);
+            if (head && !claim(1)) break;
+            multiply(kSecond, head);
+          }
+          mma_commit_pair(&ctl->empty[s], 0x3);
+          if (++s == NS) { s = 0; ph ^= 1; }
+        }
+        if (!ok) break;
+        mma_commit_pair(&ctl->acc_full[1], 0x3);
+        ++done;
       }
     }
   } else if (warp == 1) {
@@ -186,7 +265,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const uint32_t ph = (it / NS) & 1;
           if (!(ok = mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.status, 300 + s, p.timeout_ns))) break;
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(tiles + s * kStageBytes), sb = sa + kABytes;
+          const uint32_t sa = smem_u32(tiles + s * STAGE), sb = sa + kABytes;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t da = A_MN ? make_smem_desc(sa + k * 2048, BK * 128, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
@@ -231,7 +310,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
         if (!(ok = mbar_wait_bounded(&ctl->q_full[cw], (it / kQStages) & 1, abort_flag, p.status, 700 + cw, p.timeout_ns))) break;
         const uint8_t* qb = q_ring + cw * kQBytes;
-        uint8_t* sa = tiles + s * kStageBytes;
+        uint8_t* sa = tiles + s * STAGE;
         // No conversion instruction is used. An e4m3 byte (sign s, magnitude g = eeeemmm) read as the bf16 bit
         // pattern (s << 15) | (g << 4) is exactly the value x 2^-120, subnormals included (both formats then sit at
         // exponent field 0). Two exact multiplications of the bf16 pair bring it back: by 2^60, then by scale x 2^60;
@@ -262,6 +341,68 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
       }
     }
+  } else if (WIDE && warp < kWideFirstEpiWarp) {
+    give_registers();
+  } else if constexpr (WIDE) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
+    // ---------------- epilogue of wide tiles: group g of four warps has the 64-column chunks 2 i + g of each accumulator ----------------
+    const int group = (warp - kWideFirstEpiWarp) >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+    const bool issuer = (threadIdx.x & 127) == 0;
+    uint8_t* buf = epi_stage + group * kEpiBufBytes;
+    constexpr int kMine = BN / kEpiChunkCols / 2;    // chunks of an accumulator that a group has
+    uint32_t done = 0;
+    bool ok = true;
+    for (int tile = pair; ok && walk.locate(tile, tc); tile += pairs) {
+      const bool empty_reduction = tc.red_blocks == 0;
+      const int c_row0 = tc.g * p.c_rows_per_group + tc.m_idx * TILE_M + static_cast<int>(cta) * PM;
+      uint32_t keep[ACCS][kMine][kEpiChunkCols / 2];   // bf16 pairs: tensor memory is free again before anything is stored
+#pragma unroll
+      for (int a = 0; a < ACCS; ++a) {
+        if (!empty_reduction) {
+          if (!(ok = mbar_wait_bounded(&ctl->acc_full[a], done & 1, abort_flag, p.status, 400 + a, p.timeout_ns))) break;
+          tc_fence_after_sync();
+        }
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+          uint32_t lo[32], hi[32];
+          if (!empty_reduction) {
+            const uint32_t t = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * BN + (2 * i + group) * kEpiChunkCols;
+            tmem_ld_32x32(t, lo);
+            tmem_ld_32x32(t + 32, hi);
+            tmem_wait_ld();
+          }
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            keep[a][i][q] = empty_reduction ? 0u : pack_bf16(__uint_as_float(lo[2 * q]), __uint_as_float(lo[2 * q + 1]));
+            keep[a][i][16 + q] = empty_reduction ? 0u : pack_bf16(__uint_as_float(hi[2 * q]), __uint_as_float(hi[2 * q + 1]));
+          }
+        }
+        if (!empty_reduction) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->acc_empty[a]), 0));
+        }
+      }
+      if (!ok) break;
+      if (!empty_reduction) ++done;
+#pragma unroll
+      for (int a = 0; a < ACCS; ++a)
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+          if (issuer) bulk_wait_read<0>();
+          group_bar(group);
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            *chunk_ptr(buf, r, q) = make_uint4(keep[a][i][4 * q], keep[a][i][4 * q + 1], keep[a][i][4 * q + 2], keep[a][i][4 * q + 3]);
+          fence_proxy_async_smem();
+          group_bar(group);
+          if (issuer) {
+            tma_store_2d(&map_c, buf, tc.n_idx * (ACCS * BN) + a * BN + (2 * i + group) * kEpiChunkCols, c_row0);
+            bulk_commit();
+          }
+        }
+    }
+    if (issuer) bulk_wait_all();   // every bulk store of this CTA has landed before anything is torn down
   } else {
     // ---------------- epilogue (both CTAs, each for its 128 rows) ----------------
     const int quarter = warp & 3;
@@ -334,13 +475,17 @@ cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUte
     // e4m3 rows with 1x128 scales as operand A: forward contractions, TMA-store epilogues only.
     if (mode != GemmMode::kForward || args.direct_epilogue || args.red_len % 128 != 0 || epi == GemmEpilogue::kSwiGLUBwd) return cudaErrorInvalidValue;
     if (epi == GemmEpilogue::kSwiGLU)
-      return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kForward, GemmEpilogue::kSwiGLU, true, true>, kThreadsFp8, kSmemBytesFp8, map_a, map_b, map_c, c2, args, ctas, stream);
-    return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kForward, GemmEpilogue::kStore, true, true>, kThreadsFp8, kSmemBytesFp8, map_a, map_b, map_c, c2, args, ctas, stream);
+      return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kForward, GemmEpilogue::kSwiGLU, true, true, false>, kThreadsFp8, kSmemBytesFp8, map_a, map_b, map_c, c2, args, ctas, stream);
+    return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kForward, GemmEpilogue::kStore, true, true, false>, kThreadsFp8, kSmemBytesFp8, map_a, map_b, map_c, c2, args, ctas, stream);
   }
   if (mode != GemmMode::kWgrad || epi != GemmEpilogue::kStore) return cudaErrorInvalidValue;
+  if (args.wide) {
+    if (args.direct_epilogue) return cudaErrorInvalidValue;
+    return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, true, false, true>, kWideThreads, kSmemBytesWide, map_a, map_b, map_c, c2, args, ctas, stream);
+  }
   if (args.direct_epilogue)
-    return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, false, false>, kThreads, kSmemBytes, map_a, map_b, map_c, c2, args, ctas, stream);
-  return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, true, false>, kThreads, kSmemBytes, map_a, map_b, map_c, c2, args, ctas, stream);
+    return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, false, false, false>, kThreads, kSmemBytes, map_a, map_b, map_c, c2, args, ctas, stream);
+  return launch_kernel(grouped_gemm_pair_kernel<GemmMode::kWgrad, GemmEpilogue::kStore, true, false, false>, kThreads, kSmemBytes, map_a, map_b, map_c, c2, args, ctas, stream);
 }
 
 }  // namespace fastb

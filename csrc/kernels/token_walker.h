@@ -12,7 +12,7 @@
 namespace fastb {
 namespace gemm {
 
-constexpr int kTokTileN = 256;      // most tokens of one tile
+constexpr int kTokAccN = 256;       // most tokens of one accumulator: a tile has one, or two with one read of the weights (tile_n 512)
 
 FASTB_HD constexpr int ceil_to(int x, int q) { return (x + q - 1) / q * q; }
 FASTB_HD constexpr int div_up(int a, int b) { return (a + b - 1) / b; }
@@ -50,7 +50,7 @@ struct TokSplit {
   bool stream;
   FASTB_HD static TokSplit make(int tiles, int kb_tile, int pairs, int widest_n, bool share_weights) {
     TokSplit s{pairs, kb_tile, tiles, 0, 1, !share_weights};
-    const int rest = tiles % pairs, cost = 2 + widest_n / 16;
+    const int rest = tiles % pairs, cost = 2 + (widest_n < kTokAccN ? widest_n : kTokAccN) / 16;
     if (rest == 0 || kb_tile < 2) return s;
     if (share_weights) {
       int n = pairs / rest < kb_tile / 4 ? pairs / rest : kb_tile / 4;
@@ -111,20 +111,23 @@ struct TokSegments {
 // Place of tile `local` inside its group: bands of `band` token tiles, token tiles fastest inside a band, so that the
 // tiles that run together cover a squarish patch and share their operand panels in L2.
 // How many: as the reduction grows, fewer, so that the token panels of a band take at most half of the L2 while the weights
-// stream past them; at most 8, where a wave of 74 tiles is square. What this saves is the power that moving operands costs,
+// stream past them; at most 16: every further one saves a reading of the weights. What this saves is the power that moving operands costs,
 // and with it clock. 8 experts of 8192, 4096 and 2048 rows of a training step, seconds at the power cap, TFLOP/s at bands of 16, 8, 4
 // tiles: reduction of 4096 1280, 1262, 1152; 1265, 1254, 1163; 1276, 1235, 1146; of 14336 1103, 1134, 1073; 1155, 1137, 1123; 1189,
 // 1182, 1124; of 28672 981, 1010, 1007; 1052, 1040, 1073; 1098, 1100, 1063. On normal random rows 16 tiles are ahead by 3-5 % at 8192 rows;
-// inside the step (32768 tokens) 16 and this rule are equal: 58.6 and 58.8 ms of GEMMs, single runs 58.0-59.6.
-constexpr int kTokBandBytes = 60 << 20, kTokBandTiles = 8;
+// DRAM reads of a reduction of 4096 over 8192 rows at bands of 4, 8, 16, 32 tiles: 2.2, 1.1, 0.7, 1.7 GB an expert.
+constexpr int kTokBandBytes = 60 << 20, kTokBandTiles = 16;
 FASTB_HD inline int tok_band_tiles(int red_len) {
-  const long long fit = kTokBandBytes / (2ll * red_len * kTokTileN);
+  const long long fit = kTokBandBytes / (2ll * red_len * kTokAccN);
   return fit < 1 ? 1 : fit > kTokBandTiles ? kTokBandTiles : static_cast<int>(fit);
 }
 // From how many token tiles of a group on alternating the direction of the reduction pays (grouped_gemm_tokens.cu).
-FASTB_HD inline int tok_back_tiles(int red_len, int band_tiles) {
-  return 2ll * red_len * kTokTileN * band_tiles > kTokBandBytes / 2 ? band_tiles : 1 << 30;
+FASTB_HD inline int tok_back_tiles(int red_len, int band_tiles, int tile_n = kTokAccN) {
+  return 2ll * red_len * tile_n * band_tiles > kTokBandBytes / 2 ? band_tiles : 1 << 30;
 }
+// Token tiles of a band of wide tiles (512 tokens). Same operands, 8192 rows, TFLOP/s at 2, 4, 8 and 16 tiles: reduction of 4096 (SwiGLU
+// backward) 1151, 1180, 1176, 1117; of 14336 1320, 1342, 1333, 1275; of 28672 1313, 1330, 1305, 1172.
+constexpr int kTokWideBandTiles = 4;
 struct TokPlace { int m, t; };
 FASTB_HD inline TokPlace tok_place(int local, int m_tiles, int t_tiles, int band_tiles) {
   const int per_band = band_tiles * m_tiles, band = local / per_band, rem = local - band * per_band;

@@ -101,11 +101,12 @@ struct TokGemmPlan {
   bool has_c2;
   int device;
   int64_t groups;
+  int band_rows_;
   TokGemmArgs a{};
 
   // weights [G, N, K]; forward: tokens [R, K] -> out [R, N] (SwiGLU [R, N / 2]); dgrad: tokens [R, N] -> out [R, K] (SwiGLU backward [R, 2 K]).
   TokGemmPlan(int mode_, int epi_, torch::Tensor weights, torch::Tensor tokens, torch::Tensor out, c10::optional<torch::Tensor> gate_up, int granule, int band_rows)
-      : mode(static_cast<GemmMode>(mode_)), epi(static_cast<GemmEpilogue>(epi_)), has_c2(gate_up.has_value()) {
+      : mode(static_cast<GemmMode>(mode_)), epi(static_cast<GemmEpilogue>(epi_)), has_c2(gate_up.has_value()), band_rows_(band_rows) {
     TORCH_CHECK(weights.is_cuda() && weights.scalar_type() == torch::kBFloat16 && weights.dim() == 3 && weights.is_contiguous(), "weights: contiguous CUDA bf16 [G, N, K]");
     const int64_t G = weights.size(0), N = weights.size(1), K = weights.size(2);
     const bool fwd = mode == GemmMode::kForward;
@@ -140,6 +141,10 @@ struct TokGemmPlan {
     TORCH_CHECK(group_off.is_cuda() && group_off.dtype() == torch::kInt32 && group_off.is_contiguous() && group_off.numel() == groups + 1, "group_off: cuda int32[G+1]");
     TokGemmArgs g = a;
     g.tile_n = tile_n;
+    if (tile_n > gemm::kTokAccN) {
+      g.band_tiles = band_rows_ > 0 ? g.band_tiles : gemm::kTokWideBandTiles;
+      g.back_tiles = gemm::tok_back_tiles(64 * g.red_blocks, g.band_tiles, tile_n);
+    }
     g.early = early ? 1 : 0;
     g.group_off = group_off.data_ptr<int>();
     if (group_rows.has_value()) {
@@ -159,7 +164,7 @@ struct TokGemmPlan {
     }
     ctas &= ~1;
     const auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, device);
-    auto partials = torch::empty({tok_partial_floats(ctas)}, i32.dtype(torch::kFloat32));  // stream-ordered, as the launch is
+    auto partials = torch::empty({tok_partial_floats(ctas, tile_n)}, i32.dtype(torch::kFloat32));  // stream-ordered, as the launch is
     torch::Tensor cnt = counters.has_value() ? *counters : torch::zeros({2, tok_counters(ctas)}, i32);
     TORCH_CHECK(cnt.dim() == 2 && cnt.size(0) == 2 && cnt.is_contiguous() && cnt.scalar_type() == torch::kInt32, "counters: int32 [2, n]");
     unsigned int* base = reinterpret_cast<unsigned int*>(cnt.data_ptr<int>());
@@ -176,7 +181,7 @@ void grouped_gemm(int mode, int epilogue, const TensorMap2D& a, const TensorMap2
                   int red_len, int b_rows_per_group, int c_rows_per_group, torch::Tensor c, c10::optional<torch::Tensor> c2, int64_t status_ptr,
                   uint64_t timeout_ns, int ctas, int64_t gate_counter_ptr, c10::optional<torch::Tensor> gate_target, bool pair, int band_rows,
                   const TensorMap2D* map_c, const TensorMap2D* map_c2, bool direct_epilogue, c10::optional<torch::Tensor> a_scales,
-                  c10::optional<torch::Tensor> group_rows, int gate_tile_rows) {
+                  c10::optional<torch::Tensor> group_rows, int gate_tile_rows, bool wide) {
   TORCH_CHECK(group_off.is_cuda() && group_off.dtype() == torch::kInt32 && group_off.is_contiguous() && group_off.numel() >= 2, "group_off: cuda int32[G+1]");
   TORCH_CHECK(c.is_cuda() && c.dtype() == torch::kBFloat16 && c.dim() == 2 && c.stride(1) == 1, "c: cuda bf16 [rows, cols]");
   TORCH_CHECK(red_len % 64 == 0 && tiles_n >= 1, "reduction length must be a multiple of 64");
@@ -195,6 +200,8 @@ void grouped_gemm(int mode, int epilogue, const TensorMap2D& a, const TensorMap2
   g.band_rows = band_rows;
   g.direct_epilogue = direct_epilogue ? 1 : 0;
   g.gate_tile_rows = gate_tile_rows;
+  TORCH_CHECK(!wide || (pair && mode == static_cast<int>(GemmMode::kWgrad) && c.size(1) == 512ll * tiles_n), "grouped_gemm: tiles of 512 columns are for CTA-pair weight gradients of a multiple of 512 columns");
+  g.wide = wide ? 1 : 0;
   if (a_scales.has_value()) {
     want(*a_scales, torch::kFloat32, "a_scales");
     TORCH_CHECK(pair && red_len % 128 == 0 && a_scales->dim() == 2 && a_scales->size(1) == red_len / 128, "a_scales: float [rows, red_len / 128], CTA-pair kernel");
@@ -409,7 +416,7 @@ void bind_moe(py::module_& m) {
         py::arg("fixed_m_tiles"), py::arg("red_len"), py::arg("b_rows_per_group"), py::arg("c_rows_per_group"), py::arg("c"), py::arg("c2"),
         py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"), py::arg("gate_counter_ptr"), py::arg("gate_target"), py::arg("pair"),
         py::arg("band_rows"), py::arg("map_c") = nullptr, py::arg("map_c2") = nullptr, py::arg("direct_epilogue") = false, py::arg("a_scales") = py::none(),
-        py::arg("group_rows") = py::none(), py::arg("gate_tile_rows") = 0);
+        py::arg("group_rows") = py::none(), py::arg("gate_tile_rows") = 0, py::arg("wide") = false);
   m.def("grouped_gemm_smem_bytes", &grouped_gemm_smem_bytes);
   m.attr("ROUTE_TOKENS_PER_BLOCK") = kRouteTokensPerBlock;
   m.def("route_topk", &route_topk);

@@ -105,6 +105,21 @@ class TokScratch:
 _plans: dict = {}
 
 
+def wide_tiles(epi: int, reduction: int, mean_rows: int) -> bool:
+    """Whether tiles of 512 tokens are faster than tiles of 256 for groups of about ``mean_rows`` rows (grouped_gemm_tokens.cu says why).
+
+    SwiGLU forward: where a group fits one wide tile but not one of 256; up to 448, so that most groups still do if the mean does. us, 256 ->
+    512 tokens: 8 experts of 4096 x 14336 with 288, 384, 448, 480, 576 rows 617 -> 533, 651 -> 618, 697 -> 671, 823 -> 747, 902 -> 948; 32 of
+    7168 x 2048 with 288, 400, 448, 512 rows 620 -> 510, 785 -> 634, 670 -> 663, 743 -> 747.
+    Others: where tiles are long (the reduction) and many (the rows), so that neither their ends nor the last wave weigh. Reduction of 28672 with
+    768, 1024, 2048, 4096 rows 1082 -> 1081, 1387 -> 1368, 2755 -> 2645, 5838 -> 5323; of 14336 with 512, 1024, 2048 385 -> 503, 694 -> 690,
+    1385 -> 1310; SwiGLU backward, 4096 with 2048 and 4096 rows 1518 -> 1552, 3056 -> 3013, 7168 with 1024 and 2048 771 -> 762, 1536 -> 1482.
+    Shorter reductions lose at any size (3584 with 4096 rows 178 -> 189)."""
+    if epi == SWIGLU:
+        return 256 < mean_rows <= 448
+    return reduction >= 4096 and mean_rows * reduction >= 12 << 20
+
+
 def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor]) -> tuple:
     """Everything that a ``TokGemmPlan`` is made from or refuses by: another view, shape, type or device at the same address is
     another plan (or none)."""
@@ -114,7 +129,8 @@ def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tenso
 
 
 def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
-             granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch], most_rows: int = 0) -> None:
+             granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch], most_rows: int = 0,
+             mean_rows: int = 0) -> None:
     key = _plan_key(mode, epi, granule, w, x, out, gu)
     plan = _plans.get(key)
     if plan is None:
@@ -129,13 +145,16 @@ def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.T
         counters, parity, early = scratch.counters, scratch.parity, scratch.early
     # Where no group can have more tokens than a narrow tile holds, narrow tiles leave shared memory to the weights in flight.
     tile_n = 64 if 0 < most_rows <= 64 else 128 if 0 < most_rows <= 128 else 256
+    if tile_n == 256 and wide_tiles(epi, x.shape[1], mean_rows or x.shape[0] // w.shape[0]):
+        tile_n = 512
     plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, counters, parity, tile_n, early)
 
 
 def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, swiglu: bool = False,
                      gate_up_out: Optional[torch.Tensor] = None, timeout_s: float = 5.0, gate=None, a_scales: Optional[torch.Tensor] = None,
                      group_rows: Optional[torch.Tensor] = None, gate_tile_rows: int = 0, ctas: Optional[int] = None,
-                     live_rows: Optional[torch.Tensor] = None, granule: int = 32, scratch: Optional[TokScratch] = None, most_rows: int = 0) -> torch.Tensor:
+                     live_rows: Optional[torch.Tensor] = None, granule: int = 32, scratch: Optional[TokScratch] = None, most_rows: int = 0,
+                     mean_rows: int = 0) -> torch.Tensor:
     """out[rows of g] = a[rows of g] @ w[g].T  (a [R, K], w [G, N, K], out [R, N]).
 
     With ``swiglu`` the N columns of every 256-wide tile are [128 gate | 128 up] of the same 128
@@ -152,14 +171,15 @@ def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, 
 
     ``live_rows`` (int32[G], real rows per group; CTA-pair kernels, bf16 ``a``): only these rows, up to a multiple of
     ``granule`` (32 or 64), are computed and written. ``scratch``: see ``TokScratch``. ``most_rows`` > 0: no group has more real
-    rows than this (a hint that sizes the tiles; the result does not depend on it).
+    rows than this; ``mean_rows`` > 0: about how many they have (hints that size the tiles; the result does not depend on them but for
+    the rounding of sums that are cut into parts).
     """
     G, N, K = w.shape
     assert a.shape[1] == K and K % _BK == 0 and N % _BN == 0 and a.shape[0] % _BM == 0
     assert out.shape[0] == a.shape[0] and out.shape[1] == (N // 2 if swiglu else N)
     if USE_PAIR and a.dtype == torch.bfloat16:
         assert a_scales is None
-        _tok_run(FORWARD, SWIGLU if swiglu else STORE, w, a, out, gate_up_out, group_off, live_rows, granule, timeout_s, ctas, gate, gate_tile_rows, scratch, most_rows)
+        _tok_run(FORWARD, SWIGLU if swiglu else STORE, w, a, out, gate_up_out, group_off, live_rows, granule, timeout_s, ctas, gate, gate_tile_rows, scratch, most_rows, mean_rows)
         return out
     C = runtime.ext()
     map_b = _tmap(w.view(G * N, K), 128 if USE_PAIR else _BN)
@@ -177,19 +197,19 @@ def grouped_gemm_fwd(a: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, 
 
 def grouped_gemm_dgrad(dy: torch.Tensor, w: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, timeout_s: float = 5.0, gate=None,
                        swiglu_bwd_of: Optional[torch.Tensor] = None, live_rows: Optional[torch.Tensor] = None, granule: int = 64,
-                       scratch: Optional[TokScratch] = None, most_rows: int = 0) -> torch.Tensor:
+                       scratch: Optional[TokScratch] = None, most_rows: int = 0, mean_rows: int = 0) -> torch.Tensor:
     """out[rows of g] = dy[rows of g] @ w[g]  (dy [R, N], w [G, N, K], out [R, K]).
 
     With ``swiglu_bwd_of`` (the saved gate|up tiles [R, 2K]) the product is taken as d(act) and the
     epilogue writes d(gate|up) [R, 2K] into ``out`` instead (CTA-pair kernel only): the SwiGLU
-    backward costs no extra pass over memory. ``live_rows``, ``granule``, ``scratch``, ``most_rows``: as in ``grouped_gemm_fwd``.
+    backward costs no extra pass over memory. ``live_rows``, ``granule``, ``scratch``, ``most_rows``, ``mean_rows``: as in ``grouped_gemm_fwd``.
     """
     G, N, K = w.shape
     assert dy.shape[1] == N and N % _BK == 0 and K % _BN == 0 and dy.shape[0] % _BM == 0
     if swiglu_bwd_of is not None:
         assert USE_PAIR and out.shape[1] == 2 * K and swiglu_bwd_of.shape == out.shape
     if USE_PAIR:
-        _tok_run(DGRAD, SWIGLU_BWD if swiglu_bwd_of is not None else STORE, w, dy, out, swiglu_bwd_of, group_off, live_rows, granule, timeout_s, None, gate, 0, scratch, most_rows)
+        _tok_run(DGRAD, SWIGLU_BWD if swiglu_bwd_of is not None else STORE, w, dy, out, swiglu_bwd_of, group_off, live_rows, granule, timeout_s, None, gate, 0, scratch, most_rows, mean_rows)
         return out
     C = runtime.ext()
     C.grouped_gemm(DGRAD, STORE, _tmap(dy, _BM), _tmap(w.view(G * N, K), _BK), group_off, K // _BN, 0, N, N, 0, out, None, _st().ptr(),
@@ -206,6 +226,7 @@ def grouped_gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, group_off: torch.Tenso
     bm = 256 if USE_PAIR else _BM
     assert dy.shape[1] == N and x.shape[1] == K and N % bm == 0 and K % _BN == 0
     C = runtime.ext()
-    C.grouped_gemm(WGRAD, STORE, _tmap(dy, _BK), _tmap(x, _BK), group_off, K // _BN, N // bm, 0, 0, N, out.view(G * N, K), None, _st().ptr(),
-                   int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *_out_maps(out.view(G * N, K), None), DIRECT_EPILOGUE, None, live_rows)
+    wide = USE_PAIR and not DIRECT_EPILOGUE and K % 512 == 0   # never slower: see the kernel
+    C.grouped_gemm(WGRAD, STORE, _tmap(dy, _BK), _tmap(x, _BK), group_off, K // (512 if wide else _BN), N // bm, 0, 0, N, out.view(G * N, K), None, _st().ptr(),
+                   int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *_out_maps(out.view(G * N, K), None), DIRECT_EPILOGUE, None, live_rows, 0, wide)
     return out

@@ -198,7 +198,8 @@ class ExpertParallel:
         self.scratch.early = settled and rs.topk_idx.shape[0] > 0   # without tokens there is no dispatch kernel between routing and GEMM
         # a token picks an expert at most once; other ranks may have up to max_tokens of them
         most = rs.topk_idx.shape[0] if self.comm.world == 1 else self.T * self.comm.world
-        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch, most_rows=most)
+        mean = rs.topk_idx.shape[0] * self.K // self.El   # about as many come from the other ranks as go to them
+        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch, most_rows=most, mean_rows=mean)
 
     def traffic_matrix(self) -> torch.Tensor:
         """Token traffic matrix [src, dst] of the last routed step (device tensor)."""

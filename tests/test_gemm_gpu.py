@@ -216,6 +216,27 @@ def test_live_rows_and_cut_reductions(counts, N, K, granule, keep_counters, kern
             _close(got[:, :, 1].reshape(n, K), ut.grad)
 
 
+@pytest.mark.parametrize("counts,N,K,granule,keep_counters", [
+    ([1, 32, 255, 256, 257, 288, 289, 511, 512, 513, 545], 512, 1024, 32, True),   # one and two accumulators, every remainder at the edges
+    ([300], 1024, 14336, 32, True),                                                 # cut as a stream: parts of both accumulators
+    ([1030, 2100, 64], 768, 2048, 64, True),                                        # several wide tiles per group: cut in equal parts
+    ([(13 * i) % 600 for i in range(260)], 256, 256, 64, False),                    # more groups than prefix entries, tiles of one and of two
+    ([700], 256, 64, 32, False),                                                    # a single block: nothing between the two ends of a tile
+])
+def test_wide_tiles(counts, N, K, granule, keep_counters, kernel_variant, monkeypatch):
+    """The same on tiles of up to 512 tokens in two accumulators, whichever sizes the rule would take them for."""
+    from fast_b200.ops import gemm
+
+    monkeypatch.setattr(gemm, "wide_tiles", lambda *a: True)
+    test_live_rows_and_cut_reductions(counts, N, K, granule, keep_counters, kernel_variant)
+
+
+@pytest.mark.parametrize("counts,N,K", [([0, 1, 64, 65, 128, 129, 192, 193], 256, 512), ([700, 0, 5000], 512, 1536), ([300, 200], 256, 768)])
+def test_wgrad_of_few_and_many_blocks(counts, N, K, kernel_variant):
+    """Weight gradients in tiles of 512 columns (of 256 for 768 columns), with none, one, two ... blocks of 64 rows to reduce over."""
+    test_wgrad(len(counts), N, K, counts)
+
+
 def test_wgrad_stops_at_the_live_rows(kernel_variant):
     """Rows past the next multiple of 64 are not read: what lies there (here NaN) does not reach the gradient."""
     from fast_b200.ops import gemm
