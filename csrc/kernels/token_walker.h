@@ -40,8 +40,17 @@ FASTB_HD inline TokSpan tok_span(int rows, int tile_n, int i) {
 //   parts  (tiles share weights): the rest is cut into as many equal parts as there are pairs for it, part by part: pairs that
 //       run side by side stay at the same depth of the reduction and share operand panels in L2. Cut as a stream, a
 //       reduction of 28672 over 4096 tokens fell from 1.5 to 1.2 PFLOP/s: each pair fetched panels of its own.
-// A cut pays when the blocks that the last wave would leave idle exceed what the exchange costs: about 2 blocks plus one per 16
-// tokens of the tile, i.e. its fp32 sums written and read once at an SM's share of L2.
+// When a cut pays, in cycles of an SM. A block of n tokens takes 256 + n (its products read 128 rows of operand A and n / 2 of B from shared
+// memory); where no tiles share weights, the tiles that are under way also share HBM, which gives one of them a block about every 8 (rest
+// tiles: 8 * rest). So the last wave costs kb_tile blocks of max(256 + n, 8 * rest) as it is, and of max((256 + n) * rest / pairs, 8 * rest)
+// when cut. The exchange costs, per step of 32 tokens, 800 to leave the sums, 600 to store and 550 per part to read (L2 to an SM: 64 bytes a
+// cycle), and 2000 to meet. Counting only idle blocks against 2 + n / 16 blocks, as before, cut weight-bound
+// waves for nothing: us before -> after, forward W2 / data gradient of W13 of 8 experts of 4096 x 14336 at 200 tokens 174 -> 159 / 351 -> 289, 512
+// tokens 221 -> 188 / 459 -> 347; forward W13 / W2 of 1024 x 3584 at 16 tokens 35 -> 29 / 24 -> 21, 512 tokens 47 -> 37 / 35 -> 29.
+FASTB_HD inline int tok_block_cycles(int n) { return kTokAccN + (n < kTokAccN ? n : kTokAccN) + (n > kTokAccN ? 2 * (n - kTokAccN) : 0); }
+FASTB_HD inline int tok_exchange_cycles(int n, int parts) {
+  return 2000 + div_up(n, n > kTokAccN ? 64 : 32) * (1400 + 550 * parts);   // wide tiles: two groups of warps share the steps
+}
 struct TokSplit {
   int pairs, kb_tile;
   int whole_tiles;     // tiles done whole: the i-th of them, tile cut_tiles + i, by pair i % pairs
@@ -50,18 +59,22 @@ struct TokSplit {
   bool stream;
   FASTB_HD static TokSplit make(int tiles, int kb_tile, int pairs, int widest_n, bool share_weights) {
     TokSplit s{pairs, kb_tile, tiles, 0, 1, !share_weights};
-    const int rest = tiles % pairs, cost = 2 + (widest_n < kTokAccN ? widest_n : kTokAccN) / 16;
+    const int rest = tiles % pairs, block = tok_block_cycles(widest_n);
     if (rest == 0 || kb_tile < 2) return s;
     if (share_weights) {
-      int n = pairs / rest < kb_tile / 4 ? pairs / rest : kb_tile / 4;
-      n = n < 8 ? n : 8;
-      if (n < 2 || kb_tile - div_up(kb_tile, n) <= cost) return s;
-      s.whole_tiles = tiles - rest; s.cut_tiles = rest; s.shares = n;
+      int most = pairs / rest < kb_tile / 4 ? pairs / rest : kb_tile / 4;
+      most = most < 8 ? most : 8;
+      int best = 1, best_cycles = kb_tile * block;
+      for (int n = 2; n <= most; ++n) {
+        const int c = div_up(kb_tile, n) * block + tok_exchange_cycles(widest_n, n);
+        if (c < best_cycles) { best = n; best_cycles = c; }
+      }
+      if (best > 1) { s.whole_tiles = tiles - rest; s.cut_tiles = rest; s.shares = best; }
       return s;
     }
-    const long long idle = static_cast<long long>(pairs - rest) * kb_tile / pairs;   // blocks per pair that a last wave leaves idle
-    if (idle <= cost) return s;
-    const int full = tiles / pairs;
+    const int full = tiles / pairs, hbm = 8 * rest, even = div_up(block * rest, pairs);
+    const int alone = block > hbm ? block : hbm, cut = even > hbm ? even : hbm;
+    if (static_cast<long long>(kb_tile) * (alone - cut) <= tok_exchange_cycles(widest_n, pairs / (full > 0 ? rest + pairs : rest) + 1)) return s;
     s.whole_tiles = full > 1 ? (full - 1) * pairs : 0;
     s.cut_tiles = tiles - s.whole_tiles;
     const long long units = static_cast<long long>(s.cut_tiles) * kb_tile;

@@ -134,7 +134,7 @@ static void token_walker_check() {
   int cut_stream = 0, cut_parts = 0, long_prefix = 0;
   for (int trial = 0; trial < 3000; ++trial) {
     const int G = trial % 50 == 0 ? 257 + rnd(600) : 1 + rnd(trial % 2 ? 9 : 40), pairs = trial % 3 ? 74 : 1 + rnd(74);
-    const int tile_n = 64 << rnd(4), granule = rnd(2) ? 64 : 32, m_tiles = 1 + rnd(trial % 5 ? 6 : 60), kb_tile = 1 + rnd(trial % 4 ? 60 : 460);
+    const int tile_n = 64 << rnd(4), granule = rnd(2) ? 64 : 32, m_tiles = 1 + rnd(trial % 5 ? 6 : 60), kb_tile = 1 + rnd(trial % 4 ? 460 : 60);
     const bool live = rnd(4) != 0;
     std::vector<int> off(G + 1, 0), rows(G, 0);
     for (int g = 0; g < G; ++g) {

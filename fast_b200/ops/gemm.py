@@ -114,10 +114,10 @@ def wide_tiles(epi: int, reduction: int, mean_rows: int) -> bool:
     Others: where tiles are long (the reduction) and many (the rows), so that neither their ends nor the last wave weigh. Reduction of 28672 with
     768, 1024, 2048, 4096 rows 1082 -> 1081, 1387 -> 1368, 2755 -> 2645, 5838 -> 5323; of 14336 with 512, 1024, 2048 385 -> 503, 694 -> 690,
     1385 -> 1310; SwiGLU backward, 4096 with 2048 and 4096 rows 1518 -> 1552, 3056 -> 3013, 7168 with 1024 and 2048 771 -> 762, 1536 -> 1482.
-    Shorter reductions lose at any size (3584 with 4096 rows 178 -> 189)."""
-    if epi == SWIGLU:
-        return 256 < mean_rows <= 448
-    return reduction >= 4096 and mean_rows * reduction >= 12 << 20
+    Shorter reductions lose at any size (plain, 3584 with 4096 rows 178 -> 189; a whole SwiGLU layer, 1024 with 444 rows 115 -> 122)."""
+    if reduction < 4096:
+        return False
+    return 256 < mean_rows <= 448 if epi == SWIGLU else mean_rows * reduction >= 12 << 20
 
 
 def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor]) -> tuple:
