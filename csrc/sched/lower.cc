@@ -102,8 +102,12 @@ RankProgram lower_for_rank(const Plan& p, int rank, const LowerOptions& lo) {
 
   // slot 0: balance | slot 1: rail 0, intrinsic, un-staged direct ops | slot k+1: rail k (+ staged
   // direct ops of round k) and redistribution of stage k-1 | last slot: final redistribution.
-  std::vector<std::vector<Piece>> push_slot(K + 3), fwd_slot(K + 3);
-  std::vector<Piece> tmp;
+  // One list for all pieces, filed by (slot, push before forward) afterwards: a vector per slot allocates 2 (K + 3) times, mostly for one piece.
+  std::vector<Piece> pieces, tmp;
+  std::vector<int> cell_of;
+  pieces.reserve(p.ops.size() / static_cast<size_t>(n) + static_cast<size_t>(K) + 16);
+  cell_of.reserve(pieces.capacity());
+  const int cells = 2 * (K + 3);
   for (const Op& o : p.ops) {
     if (o.dst_rank == rank) {
       const int64_t bytes = o.len * ub;
@@ -116,14 +120,24 @@ RankProgram lower_for_rank(const Plan& p, int rank, const LowerOptions& lo) {
       }
     }
     if (o.src_rank != rank) continue;
-    std::vector<Piece>* dst = nullptr;
+    int cell = 0;
     switch (o.phase) {
-      case Phase::kBalance: dst = &push_slot[0]; break;
-      case Phase::kIntrinsic: dst = &push_slot[o.stage < 0 ? 1 : 1 + o.stage]; break;
-      case Phase::kRail: dst = &push_slot[1 + o.stage]; break;
-      case Phase::kRedistribute: dst = &fwd_slot[2 + o.stage]; break;
+      case Phase::kBalance: cell = 0; break;
+      case Phase::kIntrinsic: cell = 2 * (o.stage < 0 ? 1 : 1 + o.stage); break;
+      case Phase::kRail: cell = 2 * (1 + o.stage); break;
+      case Phase::kRedistribute: cell = 2 * (2 + o.stage) + 1; break;
     }
-    pieces_of(o, *dst);
+    pieces_of(o, pieces);
+    cell_of.resize(pieces.size(), cell);
+  }
+  std::vector<size_t> cell_start(static_cast<size_t>(cells) + 1, 0);
+  for (int c : cell_of) ++cell_start[static_cast<size_t>(c) + 1];
+  for (int c = 0; c < cells; ++c) cell_start[static_cast<size_t>(c) + 1] += cell_start[static_cast<size_t>(c)];
+  if (!std::is_sorted(cell_of.begin(), cell_of.end())) {
+    std::vector<Piece> filed(pieces.size());
+    std::vector<size_t> at(cell_start.begin(), cell_start.end() - 1);
+    for (size_t k = 0; k < pieces.size(); ++k) filed[at[static_cast<size_t>(cell_of[k])]++] = pieces[k];
+    pieces.swap(filed);
   }
   auto chunk_of = [&](int64_t bytes) {
     int64_t c = lo.chunk_bytes;
@@ -131,14 +145,13 @@ RankProgram lower_for_rank(const Plan& p, int rank, const LowerOptions& lo) {
     c = (c + 15) / 16 * 16;
     return c;
   };
-  struct Slice { double key; size_t pc; int64_t begin, bytes; };
-  std::vector<Slice> slices;
-  auto emit = [&](const Piece& pc, int64_t begin, int64_t bytes) {
+  // The item of a whole piece; its chunks differ in offsets and bytes only.
+  auto whole = [&](const Piece& pc) {
     const Op& o = *pc.op;
     WorkItem w{};
-    w.src_off = o.src_off * ub + pc.begin + begin;
-    w.dst_off = o.dst_off * ub + pc.begin + begin;
-    w.bytes = bytes;
+    w.src_off = o.src_off * ub + pc.begin;
+    w.dst_off = o.dst_off * ub + pc.begin;
+    w.bytes = pc.bytes;
     w.dst_rank = o.dst_rank;
     w.src_buf = static_cast<uint8_t>(o.src_buf);
     w.dst_buf = static_cast<uint8_t>(o.dst_buf);
@@ -146,41 +159,62 @@ RankProgram lower_for_rank(const Plan& p, int rank, const LowerOptions& lo) {
     w.signal_kind = o.dst_buf == Buf::kBalance ? 1 : o.dst_buf == Buf::kRail ? 2 : 3;
     w.stage = pc.signal_slot;
     w.wait_stage = pc.wait_slot;
-    prog.items.push_back(w);
+    return w;
   };
-  auto emit_interleaved = [&](const std::vector<Piece>& pcs) {
-    if (pcs.empty()) return;
-    if (pcs.size() == 1) {  // a stage of a flat plan: one transfer, its chunks in order
+  struct Slice { double key; uint32_t pc; uint32_t chunk; };
+  std::vector<Slice> slices, filed;
+  std::vector<uint32_t> bucket;
+  std::vector<WorkItem> model;
+  std::vector<int64_t> size;
+  auto emit_interleaved = [&](const Piece* pcs, size_t n_pcs) {
+    if (n_pcs == 0) return;
+    if (n_pcs == 1) {  // a stage of a flat plan: one transfer, its chunks in order
+      WorkItem w = whole(pcs[0]);
       const int64_t total = pcs[0].bytes, c = chunk_of(total);
-      for (int64_t at = 0; at < total; at += c) emit(pcs[0], at, std::min(c, total - at));
+      for (int64_t left = total; left > 0; left -= c, w.src_off += c, w.dst_off += c) { w.bytes = std::min(c, left); prog.items.push_back(w); }
       return;
     }
     // Proportional interleave: chunk j of a piece with c chunks gets key (j + 1/2) / c and chunks are
     // issued in key order, so every transfer of the slot advances at a rate proportional to its size
     // and all of them finish together (equal ones degenerate to plain round-robin). A heavy pair
     // is then in flight from the first chunk on instead of trailing alone at the end.
-    slices.clear();
-    for (size_t k = 0; k < pcs.size(); ++k) {
-      const int64_t total = pcs[k].bytes;
-      const int64_t c = chunk_of(total);
-      const int64_t pieces = (total + c - 1) / c;
-      for (int64_t j = 0; j < pieces; ++j)
-        slices.push_back(Slice{(static_cast<double>(j) + 0.5) / static_cast<double>(pieces), k, j * c, std::min(c, total - j * c)});
+    slices.clear(); model.clear(); size.clear();
+    for (size_t k = 0; k < n_pcs; ++k) {
+      const int64_t c = chunk_of(pcs[k].bytes), count = (pcs[k].bytes + c - 1) / c;
+      model.push_back(whole(pcs[k]));
+      size.push_back(c);
+      for (int64_t j = 0; j < count; ++j) slices.push_back(Slice{(static_cast<double>(j) + 0.5) / static_cast<double>(count), static_cast<uint32_t>(k), static_cast<uint32_t>(j)});
     }
-    std::stable_sort(slices.begin(), slices.end(), [](const Slice& x, const Slice& y) { return x.key < y.key; });
-    for (const Slice& sl : slices) emit(pcs[sl.pc], sl.begin, sl.bytes);
+    // In key order, equal keys in list order. The keys lie in (0, 1), about evenly: filed into as many buckets as there are chunks, what is left to
+    // do is an insertion here and there. Lowering the 1026 chunks of a fan-out of eight ranks: 22.7 us with a stable sort, 15.6 so.
+    const size_t m = slices.size();
+    const double buckets = static_cast<double>(m);
+    bucket.assign(m + 1, 0);
+    for (const Slice& s : slices) ++bucket[static_cast<size_t>(s.key * buckets) + 1];
+    for (size_t q = 1; q <= m; ++q) bucket[q] += bucket[q - 1];
+    filed.resize(m);
+    for (const Slice& s : slices) filed[bucket[static_cast<size_t>(s.key * buckets)]++] = s;
+    for (size_t q = 1; q < m; ++q) {
+      const Slice s = filed[q];
+      size_t at = q;
+      for (; at > 0 && filed[at - 1].key > s.key; --at) filed[at] = filed[at - 1];
+      filed[at] = s;
+    }
+    for (const Slice& s : filed) {
+      WorkItem w = model[s.pc];
+      const int64_t begin = static_cast<int64_t>(s.chunk) * size[s.pc];
+      w.src_off += begin;
+      w.dst_off += begin;
+      w.bytes = std::min(size[s.pc], w.bytes - begin);
+      prog.items.push_back(w);
+    }
   };
   {  // one allocation for the whole list
     size_t items = 0;
-    for (const auto* slots_of : {&push_slot, &fwd_slot})
-      for (const auto& pcs : *slots_of)
-        for (const Piece& pc : pcs) { const int64_t c = chunk_of(pc.bytes); items += static_cast<size_t>((pc.bytes + c - 1) / c); }
+    for (const Piece& pc : pieces) { const int64_t c = chunk_of(pc.bytes); items += static_cast<size_t>((pc.bytes + c - 1) / c); }
     prog.items.reserve(items);
   }
-  for (int s = 0; s < K + 3; ++s) {
-    emit_interleaved(push_slot[s]);
-    emit_interleaved(fwd_slot[s]);
-  }
+  for (int c = 0; c < cells; ++c) emit_interleaved(pieces.data() + cell_start[static_cast<size_t>(c)], cell_start[static_cast<size_t>(c) + 1] - cell_start[static_cast<size_t>(c)]);
   return prog;
 }
 

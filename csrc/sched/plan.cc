@@ -253,10 +253,15 @@ Plan build_plan(const Matrix& traffic, Topology topo, const PlanOptions& opt) {
   std::vector<size_t> at(static_cast<size_t>(K) * 2 + 1, 0);
   for (const Op& o : later) ++at[slot_of(o) + 1];
   for (size_t q = 1; q < at.size(); ++q) at[q] += at[q - 1];
+  p.num_stages = K;
+  if (std::is_sorted(later.begin(), later.end(), [&](const Op& x, const Op& y) { return slot_of(x) < slot_of(y); })) {   // one GPU per server
+    if (p.ops.empty()) p.ops.swap(later);
+    else p.ops.insert(p.ops.end(), later.begin(), later.end());
+    return p;
+  }
   const size_t first = p.ops.size();
   p.ops.resize(first + later.size());
   for (const Op& o : later) p.ops[first + at[slot_of(o)]++] = o;
-  p.num_stages = K;
   return p;
 }
 

@@ -3,6 +3,7 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstring>
 
@@ -96,6 +97,8 @@ PYBIND11_MODULE(_sched, m) {
   m.def("choose_scale", [](const I64Array& a, int gpus, ScalePolicy sp, LinkModel inter, LinkModel intra, double mbpu) {
     return choose_scale(to_matrix(a), gpus, sp, inter, intra, mbpu);
   });
+  m.def("matrix_digest", [](const I64Array& a) { const Matrix mm = to_matrix(a); return py::make_tuple(mm.hash(), mm.max_line_sum()); },
+        "hash and largest line sum in one call");
   m.def("matrix_hash", [](const I64Array& a) { return to_matrix(a).hash(); });
   m.def("max_line_sum", [](const I64Array& a) { return to_matrix(a).max_line_sum(); });
 
@@ -122,6 +125,14 @@ PYBIND11_MODULE(_sched, m) {
         int64_t* q = a.mutable_data();
         for (const RankBuffers& b : p.buffers) { *q++ = b.input_units; *q++ = b.output_units; *q++ = b.balance_units; *q++ = b.rail_units; }
         return a; })
+      .def_property_readonly("max_buffers", [](const Plan& p) {
+        // largest input, output, balance and rail units of any rank
+        RankBuffers m;
+        for (const RankBuffers& b : p.buffers) {
+          m.input_units = std::max(m.input_units, b.input_units); m.output_units = std::max(m.output_units, b.output_units);
+          m.balance_units = std::max(m.balance_units, b.balance_units); m.rail_units = std::max(m.rail_units, b.rail_units);
+        }
+        return py::make_tuple(m.input_units, m.output_units, m.balance_units, m.rail_units); })
       .def_property_readonly("ops", [](const Plan& p) {
         // int64[k, 12]: phase, stage, src_rank, dst_rank, src_buf, dst_buf, src_off, dst_off, len, origin, final, pair_off
         I64Array a({static_cast<py::ssize_t>(p.ops.size()), static_cast<py::ssize_t>(12)});

@@ -2,6 +2,7 @@
 // launchers of every sm_100a kernel. Takes the place of the reference's TORCH_LIBRARY class
 // flash_comm_t (nvidia/alltoall_nvshmem.cpp:390-662) and pybind module flash_t
 // (amd/flash.cpp:650-666); the user-facing API built on top lives in fast_b200/parallel.
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -50,7 +51,7 @@ struct A2AProgramPy {
     // Work list and expected rail bytes go up in one copy from pinned memory, in stream order: nothing here waits for the GPU.
     const int64_t list_bytes = std::max<int64_t>(n_items, 1) * static_cast<int64_t>(sizeof(A2AWork)), all_bytes = list_bytes + std::max(num_stages, 1) * 8;
     const auto u8 = torch::TensorOptions().dtype(torch::kUInt8);
-    auto host = torch::empty({all_bytes}, u8.pinned_memory(true));
+    auto host = torch::empty({all_bytes}, u8.pinned_memory(true));   // given back once the copy is done, see below
     A2AWork* w = reinterpret_cast<A2AWork*>(host.data_ptr());
     auto it = items.contiguous();
     const int64_t* q = it.data_ptr<int64_t>();
@@ -69,7 +70,9 @@ struct A2AProgramPy {
     total_bytes = total; largest_item = largest; has_waits = waits != 0;
     std::copy(expect_rail.begin(), expect_rail.end(), reinterpret_cast<int64_t*>(host.data_ptr<uint8_t>() + list_bytes));
     program_dev = torch::empty({all_bytes}, u8.device(torch::kCUDA, device));
-    program_dev.copy_(host, /*non_blocking=*/true);
+    // The copy itself, and the note that the host block is in use until it is done: what Tensor::copy_ does, without its dispatch.
+    cuda_check(cudaMemcpyAsync(program_dev.data_ptr(), host.data_ptr(), static_cast<size_t>(all_bytes), cudaMemcpyHostToDevice, home.stream()), "work list upload");
+    at::getHostAllocator(at::kCUDA)->record_event(host.data_ptr(), host.storage().data_ptr().get_context(), home.unwrap());
     upload.record(home);
     rail_off = list_bytes;
   }

@@ -66,8 +66,8 @@ class Schedule:
         into several ``all_to_all_v`` calls over slices of the matrix, which reuse the same staging."""
         mb = self.__dict__.get("_max_bytes")
         if mb is None:  # computed once: this sits on the launch path of every collective
-            b = self.plan.buffers.max(axis=0) * self.unit_bytes
-            mb = self.__dict__["_max_bytes"] = {"input": int(b[0]), "output": int(b[1]), "balance": int(b[2]), "rail": int(b[3])}
+            u, b = self.unit_bytes, self.plan.max_buffers
+            mb = self.__dict__["_max_bytes"] = {"input": b[0] * u, "output": b[1] * u, "balance": b[2] * u, "rail": b[3] * u}
         return mb
 
     def buffer_sizes(self) -> dict:
@@ -195,16 +195,16 @@ class Communicator:
             from .host_executor import check_same_plan_inputs
 
             check_same_plan_inputs(m, self.group)
+        digest, busiest = sched.matrix_digest(m)   # a matrix that was never seen costs its hash once
         if chunk_bytes is None:
             # Work items: about 8 per CTA for the busiest rank (an uneven last round of 1 MiB items costs
             # up to half the bandwidth at 148 CTAs), between 64 KiB and 1 MiB, a power of two.
-            busiest = sched.max_line_sum(m) * unit_bytes
             chunk_bytes = 1 << 16
-            while chunk_bytes < (1 << 20) and chunk_bytes * 2 * self.ctas * 8 <= busiest:
+            while chunk_bytes < (1 << 20) and chunk_bytes * 2 * self.ctas * 8 <= busiest * unit_bytes:
                 chunk_bytes *= 2
         if "split_align" not in plan_opts:
             plan_opts["split_align"] = 16 // math.gcd(16, unit_bytes)
-        key = (sched.matrix_hash(m), unit_bytes, transpose, sched.option_text(kind), chunk_bytes, rail_segment_bytes, tuple(sorted((k, sched.option_text(v)) for k, v in plan_opts.items())))
+        key = (digest, unit_bytes, transpose, sched.option_text(kind), chunk_bytes, rail_segment_bytes, tuple(sorted([(k, sched.option_text(v)) for k, v in plan_opts.items()])))
         s = self._sched_cache.get(key)
         if s is None:
             if kind == "auto":
@@ -213,7 +213,7 @@ class Communicator:
                 # Large jobs: keep only this rank's ops (same sizes, offsets and work list); the op list
                 # of a full plan grows with the cube of the server count.
                 plan_opts.setdefault("only_rank", self.rank)
-            plan = self.plan_cache.get(m, self.topo, kind=kind, transpose=transpose, **plan_opts)
+            plan = self.plan_cache.get_hashed(m, digest, self.topo, {"kind": kind, "transpose": transpose, **plan_opts})
             err = plan.validate()
             if err:
                 raise RuntimeError(f"scheduler produced an invalid plan: {err}")

@@ -75,6 +75,11 @@ def inter_link(name: str) -> "LinkModel":
     return LinkModel(a, b)
 
 
+def matrix_digest(matrix):
+    """``(matrix_hash, max_line_sum)`` in one call."""
+    return _S.matrix_digest(matrix)
+
+
 def max_line_sum(matrix) -> int:
     """Largest row or column sum: the units through the busiest port."""
     return _S.max_line_sum(matrix)
@@ -151,7 +156,11 @@ class PlanCache:
 
     def get(self, matrix, topo: Topology, **opts) -> Plan:
         m = np.ascontiguousarray(matrix, dtype=np.int64)
-        key = (matrix_hash(m), topo.servers, topo.gpus, tuple(sorted((k, option_text(v)) for k, v in opts.items())))
+        return self.get_hashed(m, matrix_hash(m), topo, opts)
+
+    def get_hashed(self, m: np.ndarray, digest: int, topo: Topology, opts: dict) -> Plan:
+        """``get`` for an int64 matrix whose ``matrix_hash`` is known already."""
+        key = (digest, topo.servers, topo.gpus, tuple(sorted([(k, option_text(v)) for k, v in opts.items()])))
         p = self._d.get(key)
         if p is None:
             self.misses += 1

@@ -606,3 +606,20 @@ def test_cost_model_reproduces_the_reference_published_large_message_logs():
             got[kind] = per_gpu / (t_us * 1e-6) / 1e9
             assert abs(got[kind] / want - 1.0) < 0.06, (nodes, kind, got[kind], want)
         assert got[PlanKind.STAGED] > got[PlanKind.SINGLE_BURST] > got[PlanKind.SPREAD_OUT]
+
+
+@pytest.mark.parametrize("n,row,chunk,seed", [(2, 4096, 64, 0), (8, 1 << 20, 4096, 1), (8, 1 << 20, 1 << 20, 2), (40, 1 << 16, 256, 3), (5, 7 * 1000, 16, 4)])
+def test_chunks_of_a_slot_are_issued_in_key_order(n, row, chunk, seed):
+    """Chunk j of a transfer with c chunks has the key (j + 1/2) / c; the work list has them in key order, equal keys in the order of
+    the transfers: what a stable sort gives."""
+    m = sched.workload_zipf_rows(n, 1.2, row, seed, 1) if seed % 2 else sched.workload_balanced(n, row // n)
+    p = sched.build_plan(m, sched.Topology.flat(n), kind=sched.PlanKind.FANOUT)
+    for rank in (0, n - 1):
+        want = []
+        for op in (o for o in p.ops if o[2] == rank):
+            size = (chunk + 15) // 16 * 16
+            count = -(-int(op[8]) // size)
+            want += [((j + 0.5) / count, int(op[6]) + j * size, int(op[7]) + j * size, min(size, int(op[8]) - j * size), int(op[3])) for j in range(count)]
+        want.sort(key=lambda w: w[0])
+        got = p.lower(rank, 1, chunk)["items"][:, :4]
+        assert np.array_equal(got, np.array([w[1:] for w in want], dtype=np.int64))
