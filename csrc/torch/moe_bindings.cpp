@@ -103,6 +103,22 @@ struct TokGemmPlan {
   int64_t groups;
   int band_rows_;
   TokGemmArgs a{};
+  // What the plan was made from.
+  struct View {
+    const void* ptr = nullptr;
+    c10::ScalarType type = c10::ScalarType::Undefined;
+    int64_t device = -1;
+    c10::SmallVector<int64_t, 3> sizes, strides;
+    View() = default;
+    explicit View(const torch::Tensor& t) : ptr(t.data_ptr()), type(t.scalar_type()), device(t.get_device()), sizes(t.sizes().begin(), t.sizes().end()), strides(t.strides().begin(), t.strides().end()) {}
+    bool is(const torch::Tensor& t) const {
+      return t.data_ptr() == ptr && t.scalar_type() == type && t.get_device() == device && t.sizes() == at::IntArrayRef(sizes) && t.strides() == at::IntArrayRef(strides);
+    }
+  };
+  View of_w, of_x, of_out, of_gu;
+  bool matches(const torch::Tensor& weights, const torch::Tensor& tokens, const torch::Tensor& out, const c10::optional<torch::Tensor>& gate_up, int granule, int band_rows) const {
+    return granule == a.granule && band_rows == band_rows_ && of_w.is(weights) && of_x.is(tokens) && of_out.is(out) && gate_up.has_value() == has_c2 && (!has_c2 || of_gu.is(*gate_up));
+  }
 
   // weights [G, N, K]; forward: tokens [R, K] -> out [R, N] (SwiGLU [R, N / 2]); dgrad: tokens [R, N] -> out [R, K] (SwiGLU backward [R, 2 K]).
   TokGemmPlan(int mode_, int epi_, torch::Tensor weights, torch::Tensor tokens, torch::Tensor out, c10::optional<torch::Tensor> gate_up, int granule, int band_rows)
@@ -116,6 +132,8 @@ struct TokGemmPlan {
     TORCH_CHECK(!has_c2 || (gate_up->size(0) == tokens.size(0) && gate_up->size(1) == (fwd ? N : 2 * K)), "grouped_gemm_tokens: gate|up shape");
     device = weights.get_device();
     groups = G;
+    of_w = View(weights); of_x = View(tokens); of_out = View(out);
+    if (has_c2) of_gu = View(*gate_up);
     const int64_t wp = reinterpret_cast<int64_t>(weights.data_ptr());
     if (fwd && epi == GemmEpilogue::kSwiGLU) {
       // [G * N / 256 tiles][8 groups of 16 features][gate, up][16][K], fetched as four groups with both halves
@@ -403,12 +421,53 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
   cu_check(launch_combine_pull(a, ctas, stream_now()), "combine_pull");
 }
 
+// Routing, dispatch and combine of an engine that is alone (one rank, forward only, eager): the launches of the functions above with what
+// the engine's buffers fix bound once, so that a pass with few tokens, whose kernels take 45 us, is not paid for in interpreter time (the five
+// launches of a layer took 54-71 us of the host, now 43-45). Heap, rows and gate come with every call.
+struct LocalTransport {
+  torch::Tensor slot_in_block, block_base, send_base, x_recv;
+  bool fp8;
+  int64_t recv_off, scale_off, y_off, ready_off;
+  int K, tile_rows, num_tiles, comm_ctas;
+  uint64_t timeout_ns;
+
+  // Returns (topk_idx, topk_w, dest_row).
+  py::tuple route_and_send(const HeapPy& heap, const SplitsPlan& splits, const StatusPy& st, torch::Tensor x, torch::Tensor gate, c10::optional<torch::Tensor> bias, uint64_t epoch,
+                           bool gate_in_kernel) const {
+    const int64_t T = x.size(0);
+    const auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(x.device());
+    auto topk_idx = torch::empty({T, K}, i32), dest_row = torch::empty({T, K}, i32), topk_w = torch::empty({T, K}, i32.dtype(torch::kFloat32));
+    if (gate_in_kernel) gate_route(splits, x, gate, bias, K, topk_idx, topk_w, slot_in_block, epoch);
+    else route_splits(splits, at::matmul(x, gate.t()).to(torch::kFloat32), bias, K, topk_idx, topk_w, slot_in_block, epoch);
+    c10::optional<torch::Tensor> none;
+    dispatch_push(heap, x, topk_idx, none, slot_in_block, block_base, send_base, dest_row, true, fp8, recv_off, scale_off, -1, 0, 0, st, timeout_ns, comm_ctas, none, tile_rows, num_tiles,
+                  none, none, fp8 ? c10::optional<torch::Tensor>(x_recv) : none, none, 0, none, none, none, 0.0);
+    return py::make_tuple(topk_idx, topk_w, dest_row);
+  }
+  torch::Tensor combine(const HeapPy& heap, const StatusPy& st, torch::Tensor topk_idx, torch::Tensor dest_row, torch::Tensor weights, uint64_t epoch) const {
+    auto out = torch::empty({topk_idx.size(0), x_recv.size(1)}, x_recv.options());
+    combine_pull(heap, static_cast<int>(send_base.numel()), topk_idx, dest_row, weights, y_off, ready_off, epoch, out, py::none(), py::none(), static_cast<int>(x_recv.size(1)), st, timeout_ns,
+                 comm_ctas, 0, true, c10::nullopt, c10::nullopt, 1.0, c10::nullopt);
+    return out;
+  }
+};
+
 }  // namespace
 
 void bind_moe(py::module_& m) {
+  py::class_<LocalTransport>(m, "LocalTransport")
+      .def(py::init([](torch::Tensor slot_in_block, torch::Tensor block_base, torch::Tensor send_base, torch::Tensor x_recv, bool fp8, int64_t recv_off, int64_t scale_off, int64_t y_off,
+                       int64_t ready_off, int K, int tile_rows, int num_tiles, int comm_ctas, uint64_t timeout_ns) {
+        want(slot_in_block, torch::kInt32, "slot_in_block"); want(block_base, torch::kInt32, "block_base"); want(send_base, torch::kInt32, "send_base");
+        want16(x_recv, torch::kBFloat16, "x_recv");
+        return LocalTransport{slot_in_block, block_base, send_base, x_recv, fp8, recv_off, scale_off, y_off, ready_off, K, tile_rows, num_tiles, comm_ctas, timeout_ns};
+      }))
+      .def("route_and_send", &LocalTransport::route_and_send)
+      .def("combine", &LocalTransport::combine);
   py::class_<TensorMap2D>(m, "TensorMap2D").def(py::init<int64_t, int64_t, int64_t, int64_t, int, int>()).def_static("bytes", &TensorMap2D::bytes);
   py::class_<TokGemmPlan>(m, "TokGemmPlan")
       .def(py::init<int, int, torch::Tensor, torch::Tensor, torch::Tensor, c10::optional<torch::Tensor>, int, int>())
+      .def("matches", &TokGemmPlan::matches)
       .def("run", &TokGemmPlan::run, py::arg("group_off"), py::arg("group_rows"), py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"),
            py::arg("gate_counter_ptr") = 0, py::arg("gate_target") = py::none(), py::arg("gate_tile_rows") = 0, py::arg("counters") = py::none(), py::arg("parity") = 0, py::arg("tile_n") = 256, py::arg("early") = false);
   m.attr("TOK_COUNTERS_PER_CTA") = tok_counters(1);

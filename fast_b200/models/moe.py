@@ -176,9 +176,8 @@ class MoELayer(nn.Module):
         return self._gout
 
     def _infer(self, x: torch.Tensor) -> torch.Tensor:
-        rs = self.engine.route_gate(x, self.gate, self.router_bias)
+        rs = self.engine.route_and_send(x, self.gate, self.router_bias)
         self.last_route = rs
-        self.engine.dispatch(x, rs)
         self.engine.experts_forward(self.w13, self.w2, rs, settled=True)
         return self.engine.combine(rs, rs.topk_w)
 

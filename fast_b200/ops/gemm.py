@@ -100,6 +100,7 @@ class TokScratch:
         # True while weights and group tables are older than the kernel that a launch follows in the stream (an engine whose routing
         # lies behind its dispatch): the launch may then start on them before that kernel has ended.
         self.early = False
+        self.plans: dict = {}   # (mode, epilogue) -> the plan of the last launch; asked whether it fits before every other
 
 
 _plans: dict = {}
@@ -128,25 +129,33 @@ def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tenso
             None if gu is None else (gu.data_ptr(), gu.dtype, gu.shape, gu.stride(), gu.get_device()))
 
 
+def token_tile(epi: int, reduction: int, most_rows: int, mean_rows: int) -> int:
+    """Most tokens of a tile. Where no group can have more than a narrow tile holds, narrow tiles leave shared memory to the weights in flight."""
+    if 0 < most_rows <= 128:
+        return 64 if most_rows <= 64 else 128
+    return 512 if wide_tiles(epi, reduction, mean_rows) else 256
+
+
 def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
              granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch], most_rows: int = 0,
              mean_rows: int = 0) -> None:
-    key = _plan_key(mode, epi, granule, w, x, out, gu)
-    plan = _plans.get(key)
-    if plan is None:
-        if len(_plans) > 1024:
-            _plans.clear()
-        plan = _plans[key] = runtime.ext().TokGemmPlan(mode, epi, w, x, out, gu, granule, BAND_ROWS)
+    plan = scratch.plans.get((mode, epi)) if scratch is not None else None
+    if plan is None or not plan.matches(w, x, out, gu, granule, BAND_ROWS):
+        key = _plan_key(mode, epi, granule, w, x, out, gu)
+        plan = _plans.get(key)
+        if plan is None:
+            if len(_plans) > 1024:
+                _plans.clear()
+            plan = _plans[key] = runtime.ext().TokGemmPlan(mode, epi, w, x, out, gu, granule, BAND_ROWS)
+        if scratch is not None:
+            scratch.plans[mode, epi] = plan
     n = scratch.ctas if scratch is not None else _ctas()
     counter_ptr, target = gate or (0, None)
     counters, parity, early = None, 0, False
     if scratch is not None:
         scratch.parity ^= 1
         counters, parity, early = scratch.counters, scratch.parity, scratch.early
-    # Where no group can have more tokens than a narrow tile holds, narrow tiles leave shared memory to the weights in flight.
-    tile_n = 64 if 0 < most_rows <= 64 else 128 if 0 < most_rows <= 128 else 256
-    if tile_n == 256 and wide_tiles(epi, x.shape[1], mean_rows or x.shape[0] // w.shape[0]):
-        tile_n = 512
+    tile_n = token_tile(epi, x.shape[1], most_rows, mean_rows or x.shape[0] // w.shape[0])
     plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, counters, parity, tile_n, early)
 
 

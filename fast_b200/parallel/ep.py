@@ -158,6 +158,12 @@ class ExpertParallel:
         self.scratch = gemm.TokScratch(dev) if gemm.USE_PAIR else None
         self.status = comm.status
         self.timeout_ns = comm.timeout_ns
+        # Alone, forward only and eager: what the transport kernels' launches have in common is bound once.
+        self._local = None
+        if W == 1 and not (training or graph_mode or overlap_dispatch or self.fp8_direct) and gemm.USE_PAIR:
+            self._local = C.LocalTransport(self.slot_in_block, self.block_base, self.send_base, self.x_recv, fp8_dispatch, self._off(self.xq_recv if fp8_dispatch else self.x_recv),
+                                           self._off(self.xs_recv) if fp8_dispatch else 0, self._off(self.y), self._flag_off(1), top_k, self.tile_rows, self.ntiles, self.comm_ctas,
+                                           self.timeout_ns)
         torch.cuda.synchronize(dev)
         if W > 1:
             import torch.distributed as dist
@@ -167,6 +173,7 @@ class ExpertParallel:
     def close(self) -> None:
         """Return this engine's symmetric allocations to the heap (collective: every rank, same order)."""
         torch.cuda.synchronize(self.comm.device)
+        self._local = None
         for name in ("dx_recv", "dy_recv", "y", "x_recv", "xs_recv", "xq_recv", "arrive", "flags", "counts"):
             t = getattr(self, name, None)
             if t is not None and hasattr(t, "_symm_off"):
@@ -230,13 +237,26 @@ class ExpertParallel:
         64 MiB of such reads; beyond that a GEMM reads the gate less often than it costs a launch. The kernel reads 16-byte words;
         a gate that is a view at another address goes through the GEMM too."""
         T = x.shape[0]
-        if (1 <= T <= self._C.ROUTE_TOKENS_PER_BLOCK and 2 * T * self.E * self.H <= 64 << 20 and self.E <= 256 and x.dtype == gate.dtype == torch.bfloat16
-                and x.is_contiguous() and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and T <= self.T):
+        if self._gate_in_kernel(x, gate):
             topk_idx, topk_w, dest_row = self._route_outputs(T, x.device)
             self.epoch += 1
             self._C.gate_route(self.splits, x, gate, bias, self.K, topk_idx, topk_w, self.slot_in_block, self.epoch)
             return self._route_state(topk_idx, topk_w, dest_row)
         return self.route((x @ gate.t()).float(), bias)
+
+    def _gate_in_kernel(self, x: torch.Tensor, gate: torch.Tensor) -> bool:
+        T = x.shape[0]
+        return (1 <= T <= self._C.ROUTE_TOKENS_PER_BLOCK and 2 * T * self.E * self.H <= 64 << 20 and self.E <= 256 and x.dtype == gate.dtype == torch.bfloat16
+                and x.is_contiguous() and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and T <= self.T)
+
+    def route_and_send(self, x: torch.Tensor, gate: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
+        """``route_gate`` and ``dispatch``; of a rank that is alone as one call."""
+        if self._local is None or not gemm.USE_PAIR or not 0 < x.shape[0] <= self.T:
+            rs = self.route_gate(x, gate, bias)
+            self.dispatch(x, rs)
+            return rs
+        self.epoch += 1
+        return self._route_state(*self._local.route_and_send(self.comm.heap, self.splits, self.status, x, gate, bias, self.epoch, self._gate_in_kernel(x, gate)))
 
     def can_fuse_gate(self) -> bool:
         """Whether ``route_fused`` (RMSNorm + router logits + top-k in one kernel) covers this layer."""
@@ -341,6 +361,8 @@ class ExpertParallel:
                 loss: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out[t] = sum_j weights[t, j] * y_row(t, j)``. With ``residual`` ([T, H] bf16), ``loss`` (float [1]) receives
         mean((residual + out)^2), the sum rounded to bf16."""
+        if self._local is not None and out is None and residual is None:
+            return self._local.combine(self.comm.heap, self.status, rs.topk_idx, rs.dest_row, weights, rs.epoch)
         T = rs.topk_idx.shape[0]
         if out is None:
             out = torch.empty(T, self.H, dtype=torch.bfloat16, device=rs.topk_idx.device)
