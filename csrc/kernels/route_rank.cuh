@@ -17,9 +17,11 @@ __host__ __device__ constexpr size_t rank_smem_bytes(int E, int K) {
 // block after the ids are in place. A warp takes 32 entries at a time and finds equal ids with match_any; counts per
 // 32 entries are then summed up by one thread per expert. One thread per expert walking all n entries took
 // 60 us at top-8 of 32 experts (1024 dependent steps); this takes about 2 us.
-__device__ __forceinline__ void block_stable_ranks(const int* s_eid, unsigned short* s_hist, int E, int K, int* __restrict__ slot_in_block, int* __restrict__ block_cnt) {
+// used: how many groups of 32 entries there are (the others hold -1); s_cnt: the counts in shared memory too.
+__device__ __forceinline__ void block_stable_ranks(const int* s_eid, unsigned short* s_hist, int E, int K, int* __restrict__ slot_in_block, int* __restrict__ block_cnt,
+                                                   int used = 1 << 30, int* s_cnt = nullptr) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int groups = kTokensPerBlock * K / 32, pitch = (E + 1) & ~1;
+  const int groups = min(kTokensPerBlock * K / 32, used), pitch = (E + 1) & ~1;
   for (int i = threadIdx.x; i < groups * pitch / 2; i += blockDim.x) reinterpret_cast<unsigned int*>(s_hist)[i] = 0u;
   __syncthreads();
   for (int g = warp; g < groups; g += nwarps) {
@@ -36,6 +38,7 @@ __device__ __forceinline__ void block_stable_ranks(const int* s_eid, unsigned sh
       run += c;
     }
     block_cnt[e] = run;
+    if (s_cnt != nullptr) s_cnt[e] = run;
   }
   __syncthreads();
   for (int g = warp; g < groups; g += nwarps) {

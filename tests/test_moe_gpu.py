@@ -652,3 +652,49 @@ def test_moe_multi_process():
                         "--master-port", "29543", os.path.join(os.path.dirname(__file__), "mp_moe_worker.py")], capture_output=True, text=True, env=env, timeout=900)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
     assert "MOE_MP_OK" in r.stdout
+
+
+@pytest.mark.parametrize("T,E,K,H", [(1, 8, 2, 256), (1, 64, 8, 512), (2, 8, 8, 1024), (17, 5, 3, 256), (33, 33, 4, 512), (128, 32, 8, 768), (127, 256, 2, 256)])
+@pytest.mark.parametrize("capacity", [None, 256])
+def test_routing_of_few_tokens_alone(T, E, K, H, capacity):
+    """The kernel that makes logits, choice, ranks and the split scan of few tokens: choice and weights against torch, ranks, rows and
+    groups against a count in token order; a step whose padded rows exceed the capacity is refused, with empty groups."""
+    from fast_b200.parallel import Communicator
+    from fast_b200.parallel.ep import ExpertParallel
+    from fast_b200.ops import gemm
+
+    comm = Communicator(heap_bytes=256 << 20, device=0)
+    eng = ExpertParallel(comm, E, H, 256, K, max_tokens=128, training=False, capacity_rows=capacity)
+    g = torch.Generator(device="cuda").manual_seed(T * 131 + E)
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    gate = (torch.randn(E, H, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    assert eng._gate_in_kernel(x, gate)
+    before = eng.arrive_target.clone()
+    rs = eng.route_gate(x, gate)
+    torch.cuda.synchronize()
+    logits = (x.float() @ gate.float().t()).to(torch.bfloat16).float()
+    idx = rs.topk_idx.long()
+    chosen = logits.gather(1, idx)
+    # a choice is right if nothing that was left out is larger by more than a rounding of a bf16 logit
+    left = logits.scatter(1, idx, float("-inf")).max(1).values if K < E else torch.full((T,), float("-inf"), device="cuda")
+    assert bool((chosen.min(1).values >= left - logits.abs().max() * 2 ** -7).all()) and bool((idx.sort(1).values.diff(dim=1) > 0).all())
+    assert torch.allclose(rs.topk_w, torch.softmax(chosen, 1), atol=2e-2)   # two bf16 logits off by one rounding: exp(2 * 2^-8) - 1
+    counts = torch.bincount(idx.flatten(), minlength=E)
+    align = gemm.row_align()
+    padded = (counts + align - 1) // align * align
+    if int(padded.sum()) > eng.cap:
+        with pytest.raises(Exception):
+            comm.check()
+        comm.status.clear()
+        assert int(rs.group_rows.abs().sum()) == 0 and int(rs.group_off.abs().sum()) == 0
+        return
+    comm.check()
+    assert torch.equal(rs.group_rows.long(), counts) and torch.equal(rs.group_off.long(), torch.cat([padded.new_zeros(1), padded.cumsum(0)]))
+    assert torch.equal((eng.arrive_target - before)[0], counts) and int(eng.traffic[0, 0]) == T * K
+    assert torch.equal(rs.send_base.long(), rs.group_off[:E].long())
+    seen = [0] * E
+    slots = rs.slot_in_block[:T].tolist()
+    for t, row in enumerate(idx.tolist()):
+        for j, e in enumerate(row):
+            assert slots[t][j] == seen[e]
+            seen[e] += 1
