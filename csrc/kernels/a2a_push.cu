@@ -176,6 +176,18 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
   __shared__ __align__(8) uint64_t s_bulk_full[kBulkBufs];
   extern __shared__ __align__(128) unsigned char s_bulk_ring[];  // kBulkSmemBytes when a.bulk, else nothing
   const int tid = threadIdx.x;
+  // A small collective is a chain of dependent steps, 14 thousand cycles for 1 KiB per rank: what peers wait for leaves first, the first work item
+  // is on its way while the block sets itself up, a counter's release is the only fence in front of it, and what a later launch of this
+  // stream reads is ordered by the end of the kernel. us a pass, before -> after: 2 x 4 ranks staged, 1 KiB 16.8 -> 12.9, 1 MiB 20.9 -> 17.0, 16 MiB of odd
+  // elements 101.8 -> 95.1; 8 ranks staged, 64 KiB 14.3 -> 12.6, 1 MiB 15.9 -> 14.0.
+  // Tell every peer that this rank's buffers may be written for this epoch.
+  if (blockIdx.x == 0 && tid < a.world) {
+    unsigned long long* peer_sig = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[tid]) + a.sig_heap_off);
+    st_release_sys(peer_sig + kSigReadyOff + a.rank, a.epoch);
+  }
+  const int n_slices = a.n_items * a.split;
+  A2AWork next{};
+  if (static_cast<int>(blockIdx.x) < n_slices) next = a.items[blockIdx.x / a.split];
   for (int i = tid; i < kSigMaxWorld; i += blockDim.x) { s_pending[i] = 0ull; s_peer_ready[i] = 0; }
   if (tid == 0) {
     s_ok = 1;
@@ -198,20 +210,14 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
   unsigned long long* stamps = a.phase_stamps;
   if (stamps && tid == 0) atomicMin(stamps + 0, global_timer_ns());
 
-  // Tell every peer that this rank's buffers may be written for this epoch.
-  if (blockIdx.x == 0 && tid < a.world) {
-    unsigned long long* peer_sig = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[tid]) + a.sig_heap_off);
-    st_release_sys(peer_sig + kSigReadyOff + a.rank, a.epoch);
-  }
   bool alive = true;
   // Items whose bytes are only announced at the end are walked in slices, so that the last round of the CTAs is a small
   // one: 15 rounds of 1 MiB items for 14.2 rounds of work cost 5 %. (8 x 256 MiB on one GPU: 742 us whole, 687 us in
   // 128 KiB slices, 707 us in 64 KiB ones, whose item reads are no longer hidden.) Staged data keeps whole items: one
   // barrier and one release each.
-  const int n_slices = a.n_items * a.split;
   for (int slice = blockIdx.x; slice < n_slices && alive; slice += gridDim.x) {
     const int it = slice / a.split, part = slice % a.split;
-    A2AWork w = a.items[it];
+    A2AWork w = slice == static_cast<int>(blockIdx.x) ? next : a.items[it];
     if (a.split > 1) {
       const long long step = w.signal_kind == 3 ? a.slice_bytes : w.bytes;
       const long long begin = part * step;
@@ -258,7 +264,6 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
       if (tid == 0 && bulk_ok) {
         unsigned long long* dst_cnt = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[w.dst_rank]) + a.sig_heap_off) + kSigCounterOff;
         const int slot = w.signal_kind == 1 ? 0 : 2 + w.stage;
-        fence_sys();
         red_add_release_sys(dst_cnt + slot, static_cast<unsigned long long>(w.bytes));
       }
     }
@@ -272,7 +277,6 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
   __syncthreads();  // all copies of this CTA are issued; announce the output bytes, one peer per thread
   if (tid < a.world && s_pending[tid] != 0ull) {
     unsigned long long* dst_cnt = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a.peer_table[tid]) + a.sig_heap_off) + kSigCounterOff;
-    fence_sys();
     red_add_release_sys(dst_cnt + 1, s_pending[tid]);
   }
   // The collective is over for this rank once everything addressed to its output has landed. Only
@@ -290,7 +294,6 @@ __device__ __forceinline__ void run_rank(const A2ARankArgs& a) {
         for (int k = 0; k < a.num_stages; ++k) my_cnt[2 + k] = 0;
       }
       my_sig[kSigTicketOff] = 0;
-      __threadfence_system();
       if (stamps) atomicMax(stamps + 9, global_timer_ns());
     }
   }
