@@ -423,7 +423,7 @@ class LocalGroup:
         self.comms = [Communicator(heap_bytes=heap_bytes, topo=topo, device=device, timeout_s=timeout_s, ctas=ctas, threads=threads,
                                    _heap=h, _rank=r, _world=world) for r, h in enumerate(heaps)]
         self.world, self.ctas, self.threads = world, ctas, threads
-        self._statuses = [c.status for c in self.comms]
+        self._native = C.A2AGroup(heaps, [c.status for c in self.comms])
 
     def schedule(self, matrix, **kw) -> List[Schedule]:
         return [c.schedule(matrix, **kw) for c in self.comms]
@@ -431,21 +431,25 @@ class LocalGroup:
     def all_to_all_v(self, outputs, inputs, scheds) -> None:
         comms = self.comms
         need = scheds[0].max_bytes
+        balance, relay = need["balance"], need["rail"]
         for c in comms:
-            c._require_usable()
-            bal, rail = c._stage("balance", need["balance"]), c._stage("rail", need["rail"])  # the same offsets on every rank
+            if c.heap is None or c.broken or c.liveness is not None:
+                c._require_usable()
+            b, r = c._staging.get("balance"), c._staging.get("rail")   # the same offsets on every rank
+            if b is None or r is None or b[1] < balance or r[1] < relay:
+                c._stage("balance", balance), c._stage("rail", relay)
+                b, r = c._staging["balance"], c._staging["rail"]
             c.epoch += 1
         c0 = comms[0]
         progs, ins = [s.program for s in scheds], list(inputs)
-        heaps = [c.heap for c in comms]   # not kept: a closed communicator lets go of its slab
-        args = ((bal, rail), c0.sig_off, c0.epoch, self._statuses, c0.timeout_ns, self.ctas, self.threads)
-        if self._C.a2a_launch_group(progs, heaps, list(outputs), ins, *args):
+        args = ((b[0], r[0]), c0.sig_off, c0.epoch, c0.timeout_ns, self.ctas, self.threads)
+        if self._C.a2a_launch_group(self._native, progs, list(outputs), ins, *args):
             return
         recv = [c.heap.tensor(c._stage("recv", need["output"]), [need["output"]], torch.uint8) for c in comms]  # library-owned, copied out afterwards
         for o, s in zip(outputs, scheds):
             if o.numel() * o.element_size() < s.output_bytes:
                 raise ValueError("output smaller than the schedule needs")
-        self._C.a2a_launch_group(progs, heaps, recv, ins, *args)
+        self._C.a2a_launch_group(self._native, progs, recv, ins, *args)
         for o, t, s in zip(outputs, recv, scheds):
             o.view(torch.uint8).reshape(-1)[: s.output_bytes].copy_(t[: s.output_bytes])
 
