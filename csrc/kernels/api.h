@@ -108,7 +108,7 @@ struct GemmArgs {
                            // over them up to a multiple of 64
   int gate_tile_rows;      // 0: gate_counter / gate_target are indexed by group; > 0: by (row of the grouped matrix) / gate_tile_rows
   int gate_slots;          // entries of gate_counter / gate_target (indices are clamped to the last one)
-  int wide;                // CTA-pair weight gradients: tiles of 512 columns (tiles_n counts those) instead of 256
+  int wide;                // CTA-pair weight gradients: tiles of 512 columns (tiles_n counts those) instead of 256; map_c has boxes {64,32}
 };
 
 int grouped_gemm_smem_bytes();

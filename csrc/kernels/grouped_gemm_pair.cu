@@ -50,13 +50,13 @@ constexpr int kCvtWarps = 4;
 constexpr int kThreadsFp8 = kThreads + 32 * kCvtWarps;
 
 // Weight gradients in tiles of 512 columns (WIDE): two accumulators that share operand A, which the tensor core reads from shared
-// memory once for both; four stages of 48 KiB; two groups of four epilogue warps, which take the columns in turn and hold
+// memory once for both; four stages of 48 KiB; two groups of four epilogue warps, one per accumulator, which hold
 // what they have read from tensor memory in registers that the first four warps have given up.
 // Bound by the power cap, and what it saves is operand traffic: 96 KiB from L2 per block of 64 rows instead of 2 x 64, and a shared-memory
 // reading of operand A for every second product. Seconds at the cap, TFLOP/s, 256 -> 512 columns: 8 experts x 8192 rows, W2 (4096 x 14336)
-// 1306 -> 1432, W13 1240 -> 1413. With few rows the output is the work, and half as many tiles pass through the kernel: us at 256, 512,
-// 1024, 2048, 4096 rows for W2 380 -> 311, 484 -> 446, 743 -> 742, 1399 -> 1367, 2743 -> 2726; for W13 696 -> 610, 944 -> 854, 1471 -> 1458,
-// 2830 -> 2767, 5741 -> 5480. So they are taken wherever the columns are a multiple of 512.
+// 1306 -> 1432, W13 1240 -> 1413. With few rows the output is the work: us at 16, 64, 256, 512, 1024 rows for W2 273 -> 198, 273 -> 202, 385 -> 306,
+// 470 -> 430, 752 -> 745; for W13 530 -> 378, 530 -> 392, 712 -> 590, 955 -> 867, 1500 -> 1480. Where the last wave would lose more than that:
+// wide_columns in ops/gemm.py.
 constexpr int kWideStages = 4;
 constexpr int kWideStageBytes = kABytes + 2 * kBBytes;
 constexpr int kWideFirstEpiWarp = 4;
@@ -120,7 +120,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     // full[s] (leader's copy is the one in use): the producer's expect_tx arrival, plus one arrival from
     // each CTA's converter warp when the A tile is written by them instead of by TMA.
     for (int s = 0; s < NS; ++s) { mbar_init(&ctl->full[s], A_FP8 ? 1 + 2 : 1); mbar_init(&ctl->empty[s], 1); }
-    for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * ACCS * kEpiWarps); }
+    for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * kEpiWarps); }
     for (int q = 0; q < kQStages; ++q) { mbar_init(&ctl->q_full[q], 1); mbar_init(&ctl->q_empty[q], 1); }
     ctl->abort_flag = 0;
     mbar_fence_init();
@@ -345,64 +345,60 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     give_registers();
   } else if constexpr (WIDE) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
-    // ---------------- epilogue of wide tiles: group g of four warps has the 64-column chunks 2 i + g of each accumulator ----------------
-    const int group = (warp - kWideFirstEpiWarp) >> 2, quarter = warp & 3, r = quarter * 32 + lane;
-    const bool issuer = (threadIdx.x & 127) == 0;
-    uint8_t* buf = epi_stage + group * kEpiBufBytes;
-    constexpr int kMine = BN / kEpiChunkCols / 2;    // chunks of an accumulator that a group has
+    // ---------------- epilogue of wide tiles: group a of four warps has accumulator a ----------------
+    // Tensor memory gives an SM about 64 bytes a cycle: 4000 cycles for the two accumulators, which the products of four blocks last. One group's reading
+    // therefore runs beside the other's stores (both groups on both accumulators, one after the other, took 4100 + 3100 cycles a tile). A warp stores its
+    // own 32 rows through 4 KiB of its own: no warp waits for another.
+    const int a = (warp - kWideFirstEpiWarp) >> 2, quarter = warp & 3;
+    constexpr int kWarpRows = 32, kChunks = BN / kEpiChunkCols;
+    uint8_t* buf = epi_stage + (warp - kWideFirstEpiWarp) * (kWarpRows * 128);
     uint32_t done = 0;
     bool ok = true;
     for (int tile = pair; ok && walk.locate(tile, tc); tile += pairs) {
       const bool empty_reduction = tc.red_blocks == 0;
-      const int c_row0 = tc.g * p.c_rows_per_group + tc.m_idx * TILE_M + static_cast<int>(cta) * PM;
-      uint32_t keep[ACCS][kMine][kEpiChunkCols / 2];   // bf16 pairs: tensor memory is free again before anything is stored
+      uint32_t keep[kChunks][kEpiChunkCols / 2];     // bf16 pairs: tensor memory is free again before anything is stored
+      if (!empty_reduction) {
+        if (!(ok = mbar_wait_bounded(&ctl->acc_full[a], done & 1, abort_flag, p.status, 400 + a, p.timeout_ns))) break;
+        ++done;
+        tc_fence_after_sync();
+      }
 #pragma unroll
-      for (int a = 0; a < ACCS; ++a) {
+      for (int i = 0; i < kChunks; ++i) {
+        uint32_t lo[32], hi[32];
         if (!empty_reduction) {
-          if (!(ok = mbar_wait_bounded(&ctl->acc_full[a], done & 1, abort_flag, p.status, 400 + a, p.timeout_ns))) break;
-          tc_fence_after_sync();
+          const uint32_t t = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * BN + i * kEpiChunkCols;
+          tmem_ld_32x32(t, lo);
+          tmem_ld_32x32(t + 32, hi);
+          tmem_wait_ld();
         }
 #pragma unroll
-        for (int i = 0; i < kMine; ++i) {
-          uint32_t lo[32], hi[32];
-          if (!empty_reduction) {
-            const uint32_t t = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * BN + (2 * i + group) * kEpiChunkCols;
-            tmem_ld_32x32(t, lo);
-            tmem_ld_32x32(t + 32, hi);
-            tmem_wait_ld();
-          }
-#pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            keep[a][i][q] = empty_reduction ? 0u : pack_bf16(__uint_as_float(lo[2 * q]), __uint_as_float(lo[2 * q + 1]));
-            keep[a][i][16 + q] = empty_reduction ? 0u : pack_bf16(__uint_as_float(hi[2 * q]), __uint_as_float(hi[2 * q + 1]));
-          }
-        }
-        if (!empty_reduction) {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->acc_empty[a]), 0));
+        for (int q = 0; q < 16; ++q) {
+          keep[i][q] = empty_reduction ? 0u : pack_bf16(__uint_as_float(lo[2 * q]), __uint_as_float(lo[2 * q + 1]));
+          keep[i][16 + q] = empty_reduction ? 0u : pack_bf16(__uint_as_float(hi[2 * q]), __uint_as_float(hi[2 * q + 1]));
         }
       }
-      if (!ok) break;
-      if (!empty_reduction) ++done;
+      if (!empty_reduction) {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->acc_empty[a]), 0));
+      }
+      const int row0 = tc.g * p.c_rows_per_group + tc.m_idx * TILE_M + static_cast<int>(cta) * PM + quarter * kWarpRows;
 #pragma unroll
-      for (int a = 0; a < ACCS; ++a)
+      for (int i = 0; i < kChunks; ++i) {
+        if (lane == 0) bulk_wait_read<0>();
+        __syncwarp();
 #pragma unroll
-        for (int i = 0; i < kMine; ++i) {
-          if (issuer) bulk_wait_read<0>();
-          group_bar(group);
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            *chunk_ptr(buf, r, q) = make_uint4(keep[a][i][4 * q], keep[a][i][4 * q + 1], keep[a][i][4 * q + 2], keep[a][i][4 * q + 3]);
-          fence_proxy_async_smem();
-          group_bar(group);
-          if (issuer) {
-            tma_store_2d(&map_c, buf, tc.n_idx * (ACCS * BN) + a * BN + (2 * i + group) * kEpiChunkCols, c_row0);
-            bulk_commit();
-          }
+        for (int q = 0; q < 8; ++q)
+          *chunk_ptr(buf, lane, q) = make_uint4(keep[i][4 * q], keep[i][4 * q + 1], keep[i][4 * q + 2], keep[i][4 * q + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&map_c, buf, tc.n_idx * (ACCS * BN) + a * BN + i * kEpiChunkCols, row0);
+          bulk_commit();
         }
+      }
     }
-    if (issuer) bulk_wait_all();   // every bulk store of this CTA has landed before anything is torn down
+    if (lane == 0) bulk_wait_all();   // every bulk store of this CTA has landed before anything is torn down
   } else {
     // ---------------- epilogue (both CTAs, each for its 128 rows) ----------------
     const int quarter = warp & 3;

@@ -129,6 +129,16 @@ def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tenso
             None if gu is None else (gu.data_ptr(), gu.dtype, gu.shape, gu.stride(), gu.get_device()))
 
 
+def wide_columns(row_tiles: int, columns: int, pairs: int, mean_rows: int) -> bool:
+    """Whether weight gradients take tiles of 512 columns instead of 256 (grouped_gemm_pair.cu: faster at any number of rows). Tiles twice as
+    large can leave more of the last wave idle, which counts once there is more to multiply than to store: 8 experts of 3584 x 1024, 4 waves
+    instead of 3.5 (W2) and 7 instead of 6.5 (W13), 256 rows 28.6 -> 26.3 and 53 -> 45, 1024 rows 57.5 -> 62.7 and 101.6 -> 109.7 us."""
+    if columns % 512:
+        return False
+    waves = lambda tiles: -(-tiles // pairs)
+    return mean_rows < 512 or 50 * waves(row_tiles * (columns // 512)) <= 26 * waves(row_tiles * (columns // 256))
+
+
 def token_tile(epi: int, reduction: int, most_rows: int, mean_rows: int) -> int:
     """Most tokens of a tile. Where no group can have more than a narrow tile holds, narrow tiles leave shared memory to the weights in flight."""
     if 0 < most_rows <= 128:
@@ -227,15 +237,15 @@ def grouped_gemm_dgrad(dy: torch.Tensor, w: torch.Tensor, group_off: torch.Tenso
 
 
 def grouped_gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, group_off: torch.Tensor, out: torch.Tensor, timeout_s: float = 5.0,
-                       live_rows: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out[g] = dy[rows of g].T @ x[rows of g]  (dy [R, N], x [R, K], out [G, N, K]). Rows between a
+                       live_rows: Optional[torch.Tensor] = None, mean_rows: int = 0) -> torch.Tensor:
+    """out[g] = dy[rows of g].T @ x[rows of g]  (dy [R, N], x [R, K], out [G, N, K]). ``mean_rows`` as in ``grouped_gemm_fwd``. Rows between a
     group's real end and its padded end must be zero in at least one operand and finite in both; with ``live_rows``
     (int32[G], real rows per group) that holds for the rows up to the next multiple of 64, the others are not read."""
     G, N, K = out.shape
     bm = 256 if USE_PAIR else _BM
     assert dy.shape[1] == N and x.shape[1] == K and N % bm == 0 and K % _BN == 0
     C = runtime.ext()
-    wide = USE_PAIR and not DIRECT_EPILOGUE and K % 512 == 0   # never slower: see the kernel
+    wide = USE_PAIR and not DIRECT_EPILOGUE and wide_columns(G * (N // bm), K, _ctas() // 2, mean_rows or x.shape[0] // G)
     C.grouped_gemm(WGRAD, STORE, _tmap(dy, _BK), _tmap(x, _BK), group_off, K // (512 if wide else _BN), N // bm, 0, 0, N, out.view(G * N, K), None, _st().ptr(),
-                   int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *_out_maps(out.view(G * N, K), None), DIRECT_EPILOGUE, None, live_rows, 0, wide)
+                   int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *((_tmap(out.view(G * N, K), 32), None) if wide else _out_maps(out.view(G * N, K), None)), DIRECT_EPILOGUE, None, live_rows, 0, wide)
     return out

@@ -422,14 +422,14 @@ class ExpertParallel:
             gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dgu, gate=gate, swiglu_bwd_of=self.gu, **self._live(rs))
         else:
             gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dact, gate=gate, **self._live(rs))
-        live = rs.group_rows if self.scratch is not None else None
-        gemm.grouped_gemm_wgrad(self.dy_recv, self.act, rs.group_off, dw2, live_rows=live)
+        live = dict(live_rows=rs.group_rows if self.scratch is not None else None, mean_rows=T * self.K // self.El)
+        gemm.grouped_gemm_wgrad(self.dy_recv, self.act, rs.group_off, dw2, **live)
         if after_dw2 is not None:
             after_dw2()
         if not gemm.USE_PAIR:
             C.swiglu_bwd(self.gu, self.dact, self.dgu, rs.group_off.data_ptr() + 4 * self.El)
         gemm.grouped_gemm_dgrad(self.dgu, w13, rs.group_off, self.dx_recv, **self._live(rs))
-        gemm.grouped_gemm_wgrad(self.dgu, self.x_recv, rs.group_off, dw13, live_rows=live)
+        gemm.grouped_gemm_wgrad(self.dgu, self.x_recv, rs.group_off, dw13, **live)
         grad_x = torch.empty(T, self.H, dtype=torch.bfloat16, device=dev)
         # Transposed dispatch: every token pulls and sums the gradients of its k rows.
         C.combine_pull(self.comm.heap, self.E, rs.topk_idx, rs.dest_row, None, self._off(self.dx_recv), self._flag_off(3), rs.epoch, grad_x, None, None,
