@@ -130,10 +130,14 @@ def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tenso
 
 
 def wide_columns(row_tiles: int, columns: int, pairs: int, mean_rows: int) -> bool:
-    """Whether weight gradients take tiles of 512 columns instead of 256 (grouped_gemm_pair.cu: faster at any number of rows). Tiles twice as
-    large can leave more of the last wave idle, which counts once there is more to multiply than to store: 8 experts of 3584 x 1024, 4 waves
-    instead of 3.5 (W2) and 7 instead of 6.5 (W13), 256 rows 28.6 -> 26.3 and 53 -> 45, 1024 rows 57.5 -> 62.7 and 101.6 -> 109.7 us."""
-    if columns % 512:
+    """Whether weight gradients take tiles of 512 columns instead of 256 (grouped_gemm_pair.cu). Few rows: the tile's way out is the time, and half
+    as many pass through. Many: the power cap is, and operand traffic saved is clock won. Between them neither, and two tiles of 256 in turn
+    keep the tensor cores busier: us between other work, as in a step, W2 / W13 of 8 experts of 4096 x 14336 at 640, 768, 1024, 1280, 1536, 2048 rows
+    452 / 888 -> 438 / 867, 496 / 984 -> 504 / 1003, 620 / 1263 -> 642 / 1283, 767 / 1562 -> 780 / 1566, 906 / 1826 -> 916 / 1824, 1201 / 2454 ->
+    1201 / 2419. And tiles twice as large can leave more of the last wave idle, which counts once there is more to multiply than to store: 8
+    experts of 3584 x 1024, 4 waves instead of 3.5 (W2) and 7 instead of 6.5 (W13), 256 rows 28.6 -> 26.3 and 53 -> 45, 1024 rows 57.5 -> 62.7 and
+    101.6 -> 109.7 us."""
+    if columns % 512 or 704 <= mean_rows < 1536:
         return False
     waves = lambda tiles: -(-tiles // pairs)
     return mean_rows < 512 or 50 * waves(row_tiles * (columns // 512)) <= 26 * waves(row_tiles * (columns // 256))

@@ -232,8 +232,11 @@ def test_wide_tiles(counts, N, K, granule, keep_counters, kernel_variant, monkey
 
 
 @pytest.mark.parametrize("counts,N,K", [([0, 1, 64, 65, 128, 129, 192, 193], 256, 512), ([700, 0, 5000], 512, 1536), ([300, 200], 256, 768)])
-def test_wgrad_of_few_and_many_blocks(counts, N, K, kernel_variant):
+def test_wgrad_of_few_and_many_blocks(counts, N, K, kernel_variant, monkeypatch):
     """Weight gradients in tiles of 512 columns (of 256 for 768 columns), with none, one, two ... blocks of 64 rows to reduce over."""
+    from fast_b200.ops import gemm
+
+    monkeypatch.setattr(gemm, "wide_columns", lambda row_tiles, columns, pairs, mean_rows: columns % 512 == 0)
     test_wgrad(len(counts), N, K, counts)
 
 
