@@ -361,10 +361,10 @@ cudaError_t launch_scaled_sum(const __nv_bfloat16* a, const __nv_bfloat16* b, lo
 cudaError_t launch_embedding_index(const long long* ids, long long T, int V, int* hist, int* rank_in_block, int* total, int* start, long long* sorted_ids,
                                    long long* perm, cudaStream_t stream);
 int embedding_index_block();
-// The whole table gradient [V, H]: from the sort's start [V + 1] and perm (every row is written), or straight from the ids (few
-// tokens: about T * T / 32 comparisons per warp).
+// The whole table gradient [V, H]: from the sort's start [V + 1] and perm (every row is written), or straight from at most 4096
+// ids.
 cudaError_t launch_embedding_rows(const int* start, const long long* perm, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int V, int H, cudaStream_t stream);
-cudaError_t launch_embedding_leaders(const long long* ids, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int T, int V, int H, cudaStream_t stream);
+cudaError_t launch_embedding_few(const long long* ids, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int T, int V, int H, cudaStream_t stream);
 // AdamW on bf16 parameters with fp32 master weights and moments, several tensors per launch.
 struct AdamWTensor {
   __nv_bfloat16* param;

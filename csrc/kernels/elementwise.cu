@@ -318,71 +318,102 @@ __global__ void embedding_rows_kernel(const int* __restrict__ start, const long 
   }
 }
 
-// Few tokens, on a table that is zero already: a warp per position looks for its id among the earlier ones; the first of an id sums
-// all of its rows, in position order. T * T / 32 comparisons a warp's width replace the sort's six launches. The ids are
-// compared in shared memory (read from global memory every 32 of them were a trip to L2: 69 us at 4096 tokens).
-constexpr int kLeaderTokens = 4096;
-__global__ void __launch_bounds__(256) embedding_leaders_kernel(const long long* __restrict__ ids, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int T, int V, int H) {
-  __shared__ int s_id[kLeaderTokens];   // ids outside [0, V) take no part: each gets a value of its own
-  for (int i = threadIdx.x; i < T; i += blockDim.x) {
-    const long long x = __ldg(ids + i);
-    s_id[i] = x >= 0 && x < V ? static_cast<int>(x) : -1 - i;
+// Few tokens: the whole table gradient in one pass, every row written once. Of each 2^bits rows a block has one, and another one in
+// the next 2^bits (frequent ids, neighbours or a power of two apart, fall to different blocks). A block files the positions that
+// name its rows, in position order; its warps clear the rows that none names and share the others' columns, 512 at a time, four
+// positions' loads ahead. Bound by the writes, and where one id has hundreds of positions by the reads that a warp has in flight.
+// Against a memset and a warp per position that searched all others for its id (T * T / 32 comparisons) and summed them
+// alone, on a table of 32000 x 4096: 4096 ids spread evenly 91 -> 62 us, skewed (one of them 27 %) 8411 -> 363, all the same 30590 ->
+// 1200, 64 ids 48 -> 46. In blocks: 512, 1024, 2048 took 71, 68, 62 us there and 25, 22.5, 25 on 32000 x 1024 (the ids are read by
+// each block): 2048 from 128 MB of table on.
+constexpr int kEmbTokens = 4096, kEmbWarps = 8;
+__device__ __forceinline__ int emb_mix(int low, int local, int bits) { return (low ^ local ^ local >> bits) & ((1 << bits) - 1); }   // its own inverse in low
+__global__ void __launch_bounds__(32 * kEmbWarps, 4) embedding_few_kernel(const long long* __restrict__ ids, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int T, int V, int H, int bits) {
+  constexpr int R = kEmbTokens / (32 * kEmbWarps), U = 2;
+  __shared__ int s_row[kEmbTokens];              // of the block's own rows: which one, and the position that names it
+  __shared__ unsigned short s_pos[kEmbTokens];
+  __shared__ unsigned s_named[32];                  // a bit per own row (modulo 1024): clear means that no position names it
+  __shared__ int s_count[kEmbWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = H / 8, own = static_cast<int>(blockIdx.x);
+  if (threadIdx.x < 32) s_named[threadIdx.x] = 0;
+  const int part = (T + 32 * kEmbWarps - 1) / (32 * kEmbWarps) * 32, first = warp * part;
+  int row[R], n = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int p = first + 32 * r + lane;
+    const long long id = 32 * r < part && p < T ? __ldg(ids + p) : -1;   // ids outside [0, V) take no part
+    row[r] = id >= 0 && id < V && emb_mix(static_cast<int>(id), static_cast<int>(id) >> bits, bits) == own ? static_cast<int>(id) >> bits : -1;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) n += __popc(__ballot_sync(0xffffffffu, row[r] >= 0));
+  if (lane == 0) s_count[warp] = n;
+  __syncthreads();
+  int at = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kEmbWarps; ++w) {
+    at += w < warp ? s_count[w] : 0;
+    total += s_count[w];
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const unsigned m = __ballot_sync(0xffffffffu, row[r] >= 0);
+    if (row[r] >= 0) {
+      const int k = at + __popc(m & ((1u << lane) - 1));
+      s_row[k] = row[r];
+      s_pos[k] = static_cast<unsigned short>(first + 32 * r + lane);
+      atomicOr(&s_named[row[r] >> 5 & 31], 1u << (row[r] & 31));
+    }
+    at += __popc(m);
   }
   __syncthreads();
-  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, chunks = H / 8;
-  if (p >= T) return;
-  const int id = s_id[p];
-  if (id < 0) return;
-  bool earlier = false;
+  const int rows = ((V - 1) >> bits) + 1;
+  const auto named = [&](int local) { return (s_named[local >> 5 & 31] >> (local & 31) & 1) != 0; };
+  const auto row_of = [&](int local) { return (static_cast<long long>(local) << bits) + emb_mix(own, local, bits); };
+  for (int local = warp; local < rows; local += kEmbWarps)
+    if (row_of(local) < V && !named(local)) {
+      uint4* out = grad_table + row_of(local) * chunks;
 #pragma unroll 4
-  for (int q = lane; q < p; q += 32) earlier |= s_id[q] == id;
-  if (__any_sync(0xffffffffu, earlier)) return;
-  // My id's later positions: kept one per lane where there are at most 32 of them, else looked up again for every chunk.
-  int mine = -1, found = 0;
-  for (int q0 = p / 32 * 32; q0 < T; q0 += 32) {
-    unsigned m = __ballot_sync(0xffffffffu, q0 + lane > p && q0 + lane < T && s_id[min(q0 + lane, T - 1)] == id);
-    while (m) {
-      const int q = q0 + __ffs(m) - 1;
-      m &= m - 1;
-      if (found == lane) mine = q;
-      ++found;
+      for (int c = lane; c < chunks; c += 32) out[c] = make_uint4(0, 0, 0, 0);
     }
-  }
-  uint4* out = grad_table + static_cast<long long>(id) * chunks;
-  constexpr int U = 4;
-  for (int c0 = 0; c0 < chunks; c0 += 32 * U) {
-    float acc[U][8];
+  int turn = 0;
+  for (int local = 0; total && local < rows; ++local) {
+    if (!named(local) || row_of(local) >= V) continue;
+    uint4* out = grad_table + row_of(local) * chunks;
+    for (int first_c = 0; first_c < chunks; first_c += 32 * U) {
+      if (turn++ % kEmbWarps != warp) continue;
+      int c[U];   // past the end: the last one again, not written
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+      for (int u = 0; u < U; ++u) c[u] = min(first_c + 32 * u + lane, chunks - 1);
+      float acc[U][8] = {};
+      for (int q0 = 0; q0 < total; q0 += 32) {
+        unsigned m = __ballot_sync(0xffffffffu, q0 + lane < total && s_row[min(q0 + lane, total - 1)] == local);
+        const auto add = [&](auto depth) {   // `depth` positions' loads ahead, added one after the other
+          constexpr int J = decltype(depth)::value;
+          uint4 v[J][U];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[u][k] = 0.0f;
-    auto add = [&](int q) {
-      uint4 v[U];
+          for (int j = 0; j < J; ++j) {
+            const uint4* from = grad_out + static_cast<long long>(s_pos[q0 + __ffs(m) - 1]) * chunks;
+            m &= m - 1;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c = c0 + 32 * u + lane;
-        v[u] = c < chunks ? __ldg(grad_out + static_cast<long long>(q) * chunks + c) : make_uint4(0, 0, 0, 0);
+            for (int u = 0; u < U; ++u) v[j][u] = __ldg(from + c[u]);
+          }
+#pragma unroll
+          for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              float f[8];
+              unpack8(v[j][u], f);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+            }
+        };
+        while (__popc(m) >= 4) add(std::integral_constant<int, 4>());
+        while (m) add(std::integral_constant<int, 1>());
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        float f[8];
-        unpack8(v[u], f);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
-      }
-    };
-    add(p);
-    if (found <= 32) {
-      for (int j = 0; j < found; ++j) add(__shfl_sync(0xffffffffu, mine, j));
-    } else {
-      for (int q0 = p / 32 * 32; q0 < T; q0 += 32) {
-        unsigned m = __ballot_sync(0xffffffffu, q0 + lane > p && q0 + lane < T && s_id[min(q0 + lane, T - 1)] == id);
-        while (m) { add(q0 + __ffs(m) - 1); m &= m - 1; }
-      }
+      for (int u = 0; u < U; ++u)
+        if (first_c + 32 * u + lane < chunks) out[c[u]] = pack8(acc[u]);
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (c0 + 32 * u + lane < chunks) out[c0 + 32 * u + lane] = pack8(acc[u]);
   }
 }
 
@@ -446,11 +477,11 @@ cudaError_t launch_embedding_rows(const int* start, const long long* perm, const
   note_launch();
   return cudaGetLastError();
 }
-cudaError_t launch_embedding_leaders(const long long* ids, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int T, int V, int H, cudaStream_t stream) {
-  if (H % 8 || T > kLeaderTokens) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(grad_table, 0, static_cast<size_t>(V) * H * 2, stream);
-  if (e != cudaSuccess || T == 0) return e;
-  embedding_leaders_kernel<<<static_cast<unsigned>((T * 32ll + 255) / 256), 256, 0, stream>>>(ids, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), T, V, H);
+cudaError_t launch_embedding_few(const long long* ids, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int T, int V, int H, cudaStream_t stream) {
+  if (H % 8 || T > kEmbTokens) return cudaErrorInvalidValue;
+  if (V == 0 || H == 0) return cudaSuccess;
+  const int bits = static_cast<long long>(V) * H >= 1ll << 26 ? 11 : 10;
+  embedding_few_kernel<<<1 << bits, 32 * kEmbWarps, 0, stream>>>(ids, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), T, V, H, bits);
   note_launch();
   return cudaGetLastError();
 }

@@ -607,9 +607,9 @@ void bind_moe(py::module_& m) {
     const long long* idp = reinterpret_cast<const long long*>(ids.data_ptr());
     const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(grad_out.data_ptr());
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(table.data_ptr());
-    // Up to here comparing all pairs of positions (5 us at 4096) is cheaper than the sort's six launches.
+    // What a block can file in shared memory; above, the sort's six launches.
     if (T <= 4096) {
-      cu_check(launch_embedding_leaders(idp, g, out, static_cast<int>(T), V, static_cast<int>(H), stream_now()), "embedding_grad");
+      cu_check(launch_embedding_few(idp, g, out, static_cast<int>(T), V, static_cast<int>(H), stream_now()), "embedding_grad");
       return table;
     }
     const int64_t blocks = (T + embedding_index_block() - 1) / embedding_index_block();

@@ -290,6 +290,26 @@ def test_embedding_gradient_of_any_length(T, V, H, spread):
     assert bool((table.grad[torch.bincount(ids, minlength=V) == 0] == 0).all())
 
 
+@pytest.mark.parametrize("T,V,H,step", [(0, 40, 64, 1), (4096, 513, 520, 512), (4096, 2200000, 8, 2097152), (300, 32769, 2048, 1024), (4095, 9000, 1032, 512), (257, 32000, 4096, 31999)])
+def test_embedding_gradient_of_few_positions_in_one_block(T, V, H, step):
+    """Ids that all fall to one block's rows, rows that share a bit of its filter (2097152 apart), ids outside the table, ragged
+    widths. n fp32 additions of bf16 values, one rounding to bf16: an error of at most 2^-8 of the sum plus n 2^-24 of the terms."""
+    from fast_b200 import _C
+
+    g = torch.Generator(device="cuda").manual_seed(T + V)
+    ids = torch.randint(0, (V - 1) // step + 1, (T,), generator=g, device="cuda") * step
+    if T:
+        ids[::5], ids[3::7] = V, -1
+    go = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    got = _C.embedding_grad(ids, V, go)
+    used = (ids >= 0) & (ids < V)
+    want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids[used], go[used].double())
+    terms = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids[used], go[used].double().abs())
+    n = torch.bincount(ids[used], minlength=V).double()[:, None]
+    assert bool(((got.double() - want).abs() <= 2.0**-8 * want.abs() + n * 2.0**-24 * terms + 1e-30).all())
+    assert bool((got[n[:, 0] == 0] == 0).all())
+
+
 @pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 256, 4, 2), (127, 512, 256, 8, 2), (130, 1024, 256, 12, 3), (700, 2048, 256, 8, 2)])
 def test_loss_inside_the_layer_matches_the_separate_ops(T, H, I, E, K):
     """mean((h + MoE(RMSNorm(h)))^2) with loss and gradients made inside combine, the backward dispatch and the norm's backward,
