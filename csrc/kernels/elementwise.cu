@@ -284,37 +284,63 @@ __global__ void emb_scatter_kernel(const long long* __restrict__ ids, const int*
 
 // ---- the whole gradient of an embedding table ------------------------------------------------------------------
 // A warp per table row, after the counting sort: every row is written once, its sum or zeros (cleared beforehand by a kernel of
-// its own, the table cost one more pass of writes: 91 us for 32000 x 4096). One warp adds up all rows of its id, one after another
-// in position order: evenly spread ids are bound by HBM, an id that names many positions by its own chain of loads.
-__global__ void embedding_rows_kernel(const int* __restrict__ start, const long long* __restrict__ perm, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int V, int H) {
-  const long long v = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31, chunks = H / 8;
-  if (v >= V) return;
-  const int begin = __ldg(start + v), end = __ldg(start + v + 1);
-  uint4* out = grad_table + v * chunks;
-  constexpr int U = 4;   // chunks in flight per row
-  for (int c0 = lane; c0 < chunks; c0 += 32 * U) {
-    float acc[U][8];
+// its own, the table cost one more pass of writes: 91 us for 32000 x 4096), in position order: evenly spread ids are bound by HBM.
+// A row with more than kEmbAlone positions is summed by its block's eight warps, 256 columns each and eight positions' loads
+// ahead; by one warp, one load ahead, it was a chain: 32768 skewed ids (one of them 27 %) on 32000 x 4096 took 67.3 ms with the sort,
+// 3.8 now; spread evenly 194 and 198 us, 8192 of them 114 and 114.
+constexpr int kEmbAlone = 16;
+__global__ void __launch_bounds__(256) embedding_rows_kernel(const int* __restrict__ start, const long long* __restrict__ perm, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int V, int H) {
+  const long long v0 = blockIdx.x * 8ll;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = H / 8;
+  const int bound = v0 + lane <= V && lane <= 8 ? __ldg(start + v0 + lane) : 0;   // lane i: where row v0 + i starts
+  const int next = __shfl_down_sync(0xffffffffu, bound, 1);
+  const unsigned shared = __ballot_sync(0xffffffffu, lane < 8 && v0 + lane < V && next - bound > kEmbAlone);
+  const int begin = __shfl_sync(0xffffffffu, bound, warp), end = __shfl_sync(0xffffffffu, next, warp);
+  if (v0 + warp < V && !(shared >> warp & 1)) {
+    uint4* out = grad_table + (v0 + warp) * chunks;
+    constexpr int U = 4;   // chunks in flight per row
+    for (int c0 = lane; c0 < chunks; c0 += 32 * U) {
+      float acc[U][8] = {};
+      for (int j = begin; j < end; ++j) {
+        const uint4* row = grad_out + __ldg(perm + j) * chunks;
+        uint4 x[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u) x[u] = c0 + 32 * u < chunks ? __ldg(row + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[u][k] = 0.0f;
-    for (int j = begin; j < end; ++j) {
-      const uint4* row = grad_out + __ldg(perm + j) * chunks;
-      uint4 x[U];
+        for (int u = 0; u < U; ++u) {
+          float f[8];
+          unpack8(x[u], f);
 #pragma unroll
-      for (int u = 0; u < U; ++u) x[u] = c0 + 32 * u < chunks ? __ldg(row + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        float f[8];
-        unpack8(x[u], f);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+          for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+        }
       }
-    }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (c0 + 32 * u < chunks) __stcs(out + c0 + 32 * u, pack8(acc[u]));
+      for (int u = 0; u < U; ++u)
+        if (c0 + 32 * u < chunks) __stcs(out + c0 + 32 * u, pack8(acc[u]));
+    }
+  }
+  for (unsigned left = shared; left; left &= left - 1) {
+    const int i = __ffs(left) - 1, first = __shfl_sync(0xffffffffu, bound, i), last = __shfl_sync(0xffffffffu, next, i);
+    for (int c = threadIdx.x; c < chunks; c += 256) {
+      float acc[8] = {};
+      const auto add = [&](int j, auto depth) {
+        constexpr int J = decltype(depth)::value;
+        uint4 x[J];
+#pragma unroll
+        for (int d = 0; d < J; ++d) x[d] = __ldg(grad_out + __ldg(perm + j + d) * chunks + c);
+#pragma unroll
+        for (int d = 0; d < J; ++d) {
+          float f[8];
+          unpack8(x[d], f);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[k] += f[k];
+        }
+      };
+      int j = first;
+      for (; j + 8 <= last; j += 8) add(j, std::integral_constant<int, 8>());
+      for (; j < last; ++j) add(j, std::integral_constant<int, 1>());
+      __stcs(grad_table + (v0 + i) * chunks + c, pack8(acc));
+    }
   }
 }
 
@@ -473,7 +499,7 @@ cudaError_t launch_embedding_index(const long long* ids, long long T, int V, int
 int embedding_index_block() { return kIdxBlock; }
 cudaError_t launch_embedding_rows(const int* start, const long long* perm, const __nv_bfloat16* grad_out, __nv_bfloat16* grad_table, int V, int H, cudaStream_t stream) {
   if (H % 8) return cudaErrorInvalidValue;
-  embedding_rows_kernel<<<static_cast<unsigned>((V * 32ll + 255) / 256), 256, 0, stream>>>(start, perm, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), V, H);
+  embedding_rows_kernel<<<static_cast<unsigned>((V + 7ll) / 8), 256, 0, stream>>>(start, perm, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), V, H);
   note_launch();
   return cudaGetLastError();
 }

@@ -310,6 +310,24 @@ def test_embedding_gradient_of_few_positions_in_one_block(T, V, H, step):
     assert bool((got[n[:, 0] == 0] == 0).all())
 
 
+@pytest.mark.parametrize("V,H", [(9, 264), (16, 2056), (8193, 8)])
+def test_embedding_gradient_of_many_positions_with_frequent_ids(V, H):
+    """Rows of 0, 1, 16 (one warp), 17, 24 and thousands of positions (the block's warps together), the last row of a table that is
+    no multiple of eight rows among them. n fp32 additions of bf16 values, one rounding to bf16."""
+    from fast_b200 import _C
+
+    rows = [(0, 1), (1, 16), (2, 17), (4, 24), (5, 1700), (V - 1, 3000)]
+    ids = torch.cat([torch.full((n,), v) for v, n in rows])
+    g = torch.Generator().manual_seed(V)
+    ids = ids[torch.randperm(ids.numel(), generator=g)].cuda()
+    go = torch.randn(ids.numel(), H, generator=g).to(torch.bfloat16).cuda()
+    got = _C.embedding_grad(ids, V, go)
+    want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids, go.double())
+    terms = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids, go.double().abs())
+    n = torch.bincount(ids, minlength=V).double()[:, None]
+    assert ids.numel() > 4096 and bool(((got.double() - want).abs() <= 2.0**-8 * want.abs() + n * 2.0**-24 * terms).all())
+
+
 @pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 256, 4, 2), (127, 512, 256, 8, 2), (130, 1024, 256, 12, 3), (700, 2048, 256, 8, 2)])
 def test_loss_inside_the_layer_matches_the_separate_ops(T, H, I, E, K):
     """mean((h + MoE(RMSNorm(h)))^2) with loss and gradients made inside combine, the backward dispatch and the norm's backward,
