@@ -1,9 +1,11 @@
-// Programmatic dependent launch: a kernel of the forward chain may be set up (blocks placed, barriers and tensor memory made)
+// Programmatic dependent launch: a kernel of the layer or of its training step may be set up (blocks placed, barriers and tensor memory made)
 // while the kernel before it in the stream still runs. Rules that keep it safe:
 //   * grid_dependency_wait() comes before the first access to anything an earlier kernel reads or writes. The one exception, where its
 //     caller vouches for it (TokGemmArgs::early), is the expert GEMM's weights and group table: at least one kernel lies
 //     between their writers and the GEMM, and that kernel gives leave after its own wait or not at all.
 //   * launch_dependents() comes after the wait, so leave is given only by kernels whose own predecessors are complete.
+// Measured: a training step of 1022 tokens (small shape) went from 847 to 841 us, 836 to 820 under a trace, when weight gradients, the
+// zeroing of pad rows, the norm's and gate's two kernels and the optimizer joined the chain; each hand-over was 2 us before.
 // A kernel that gives no leave lets its successor start when it ends, as always.
 #pragma once
 #include <cuda_runtime.h>

@@ -2,6 +2,7 @@
 #include <cuda_fp8.h>
 
 #include "api.h"
+#include "early_start.cuh"
 
 namespace fastb {
 
@@ -93,6 +94,8 @@ constexpr int kAdamThreads = 256, kAdamPerThread = 2, kAdamChunk = 4 * kAdamThre
 __global__ void __launch_bounds__(kAdamThreads) adamw_kernel(const __grid_constant__ AdamWArgs a) {
   int k = 0;
   unsigned int block = blockIdx.x;
+  grid_dependency_wait();
+  launch_dependents();
   while (block >= a.t[k].blocks) block -= a.t[k++].blocks;
   const AdamWTensor& t = a.t[k];
   const long long n4 = t.n / 4, base = static_cast<long long>(block) * (kAdamChunk / 4) + threadIdx.x;
@@ -362,6 +365,8 @@ __global__ void __launch_bounds__(32 * kEmbWarps, 4) embedding_few_kernel(const 
   __shared__ int s_count[kEmbWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = H / 8, own = static_cast<int>(blockIdx.x);
   if (threadIdx.x < 32) s_named[threadIdx.x] = 0;
+  grid_dependency_wait();
+  launch_dependents();
   const int part = (T + 32 * kEmbWarps - 1) / (32 * kEmbWarps) * 32, first = warp * part;
   int row[R], n = 0;
 #pragma unroll
@@ -507,9 +512,9 @@ cudaError_t launch_embedding_few(const long long* ids, const __nv_bfloat16* grad
   if (H % 8 || T > kEmbTokens) return cudaErrorInvalidValue;
   if (V == 0 || H == 0) return cudaSuccess;
   const int bits = static_cast<long long>(V) * H >= 1ll << 26 ? 11 : 10;
-  embedding_few_kernel<<<1 << bits, 32 * kEmbWarps, 0, stream>>>(ids, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), T, V, H, bits);
+  const cudaError_t e = launch_early(embedding_few_kernel, dim3(1 << bits), 32 * kEmbWarps, 0, stream, ids, reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<uint4*>(grad_table), T, V, H, bits);
   note_launch();
-  return cudaGetLastError();
+  return e;
 }
 cudaError_t launch_dequant_fp8(const unsigned char* q, const float* scales, __nv_bfloat16* out, long long rows, int H, const int* rows_dev,
                                cudaStream_t stream) {
@@ -530,9 +535,9 @@ cudaError_t launch_adamw(AdamWArgs args, cudaStream_t stream) {
   }
   if (blocks == 0) return cudaSuccess;
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
-  adamw_kernel<<<static_cast<unsigned>(blocks), kAdamThreads, 0, stream>>>(args);
+  const cudaError_t e = launch_early(adamw_kernel, dim3(static_cast<unsigned>(blocks)), kAdamThreads, 0, stream, args);
   note_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace fastb

@@ -19,6 +19,7 @@
 // (gemm_epilogue_tma.cuh): output matrices are described by tensor maps of 64 x 128 boxes.
 #include <cuda_fp8.h>
 
+#include "early_start.cuh"
 #include "gemm_epilogue_tma.cuh"
 
 namespace fastb {
@@ -134,6 +135,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after_sync();
+  grid_dependency_wait();   // up to here nothing that an earlier kernel reads or writes
+  launch_dependents();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abort_flag = &ctl->abort_flag;
 
@@ -450,11 +453,12 @@ cudaError_t launch_kernel(Kernel kern, int threads, int smem, const CUtensorMap&
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1] = early_start_attribute();
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   e = cudaLaunchKernelEx(&cfg, kern, a, b, c, c2, args);
   if (e == cudaSuccess) note_launch();
   return e;

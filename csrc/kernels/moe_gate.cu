@@ -12,6 +12,7 @@
 // or the gate matrix plus the fp32 gradient accumulators (backward) must fit in shared memory.
 #include <algorithm>
 
+#include "early_start.cuh"
 #include "route_rank.cuh"
 #include "route_splits.cuh"
 
@@ -58,6 +59,8 @@ __global__ void __launch_bounds__(kGateThreads) norm_gate_route_kernel(const Nor
   uint4* s_nw = s_gate + static_cast<size_t>(E) * (H / 8);                  // [H / 8]
   int* s_eid = reinterpret_cast<int*>(s_nw + H / 8);                        // [kTokensPerBlock * K]
   const int chunks = H / 8;
+  grid_dependency_wait();
+  launch_dependents();
   for (int i = threadIdx.x; i < E * chunks; i += blockDim.x) s_gate[i] = __ldg(reinterpret_cast<const uint4*>(a.gate) + i);
   for (int i = threadIdx.x; i < chunks; i += blockDim.x) s_nw[i] = __ldg(reinterpret_cast<const uint4*>(a.norm_w) + i);
   __syncthreads();
@@ -198,6 +201,8 @@ __global__ void __launch_bounds__(kGateBwdThreads) norm_gate_bwd_kernel(const No
   uint4* s_nw = s_gate + static_cast<size_t>(E) * chunks;
   float* s_dgate = reinterpret_cast<float*>(s_nw + chunks);  // [E][H]
   float* s_dnw = s_dgate + static_cast<size_t>(E) * H;       // [H]
+  grid_dependency_wait();
+  launch_dependents();
   for (int i = threadIdx.x; i < E * chunks; i += nt) s_gate[i] = __ldg(reinterpret_cast<const uint4*>(a.gate) + i);
   for (int i = threadIdx.x; i < chunks; i += nt) s_nw[i] = __ldg(reinterpret_cast<const uint4*>(a.norm_w) + i);
   for (int i = threadIdx.x; i < (E + 1) * H; i += nt) s_dgate[i] = 0.0f;  // d_gate and d_nw are contiguous
@@ -342,6 +347,8 @@ __global__ void __launch_bounds__(1024) fold_gate_grads_kernel(const float* __re
   __shared__ float4 s[8][128];
   const int x = threadIdx.x & 127, y = threadIdx.x >> 7, n4 = (E + 1) * H / 4, i = blockIdx.x * 128 + x;
   float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  grid_dependency_wait();
+  launch_dependents();
   if (i < n4)
     for (int b = y; b < blocks; b += 8) {
       const float4 p = __ldcs(reinterpret_cast<const float4*>(partials) + static_cast<size_t>(b) * n4 + i);
@@ -390,9 +397,9 @@ cudaError_t launch_norm_gate_route(const NormGateArgs& a, const SplitsArgs* sp, 
     if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGateThreads, smem);
     if (err != cudaSuccess) return err;
     const int blocks = std::min((a.T + tokens_per_group - 1) / tokens_per_group, sms * std::max(per_sm, 1));
-    kern<<<blocks, kGateThreads, smem, stream>>>(a, sp ? *sp : SplitsArgs{}, sp ? 1 : 0, tickets);
+    err = launch_early(kern, dim3(blocks), kGateThreads, smem, stream, a, sp ? *sp : SplitsArgs{}, sp ? 1 : 0, tickets);
     note_launch();
-    return cudaGetLastError();
+    return err;
   };
   // Two tokens a warp save a quarter of the arithmetic; below two groups of 32 per SM the tokens are better spread out.
   const bool two = a.T >= 64 * sms;
@@ -419,10 +426,11 @@ cudaError_t launch_norm_gate_bwd(const NormGateBwdArgs& a, int blocks, cudaStrea
   auto* kern = a.H / 8 > kGateBwdThreads ? norm_gate_bwd_kernel<2> : norm_gate_bwd_kernel<1>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  kern<<<blocks, threads, smem, stream>>>(a);
-  fold_gate_grads_kernel<<<((a.num_experts + 1) * a.H / 4 + 127) / 128, 1024, 0, stream>>>(a.partials, blocks, a.num_experts, a.H, a.d_gate_bf16, a.d_norm_w_bf16, a.d_gate, a.d_norm_w);
+  e = launch_early(kern, dim3(blocks), threads, smem, stream, a);
+  if (e != cudaSuccess) return e;
+  e = launch_early(fold_gate_grads_kernel, dim3(((a.num_experts + 1) * a.H / 4 + 127) / 128), 1024, 0, stream, a.partials, blocks, a.num_experts, a.H, a.d_gate_bf16, a.d_norm_w_bf16, a.d_gate, a.d_norm_w);
   note_launch(2);
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace fastb

@@ -195,6 +195,8 @@ __global__ void build_send_list_kernel(const int* __restrict__ topk_idx, const i
 // Zeroes the rows between each group's real end and its padded end, or the next multiple of `align` rows.
 __global__ void zero_pad_rows_kernel(unsigned char* buf, long long row_bytes, const int* __restrict__ group_off, const int* __restrict__ group_rows, int groups, int align) {
   const int g = blockIdx.y;
+  grid_dependency_wait();
+  launch_dependents();
   if (g >= groups) return;
   const long long begin = (static_cast<long long>(group_off[g]) + group_rows[g]) * row_bytes;
   const long long last = align > 0 ? static_cast<long long>(group_off[g]) + (group_rows[g] + align - 1) / align * align : group_off[g + 1];
@@ -285,9 +287,9 @@ cudaError_t launch_build_send_list(const int* topk_idx, const int* slot_in_block
 cudaError_t launch_zero_pad_rows(void* buf, long long row_bytes, const int* group_off, const int* group_rows, int groups, int align, cudaStream_t stream) {
   if (row_bytes % 16 || align < 0) return cudaErrorInvalidValue;
   if (groups == 0) return cudaSuccess;
-  zero_pad_rows_kernel<<<dim3(8, groups), 256, 0, stream>>>(static_cast<unsigned char*>(buf), row_bytes, group_off, group_rows, groups, align);
+  const cudaError_t e = launch_early(zero_pad_rows_kernel, dim3(8, groups), 256, 0, stream, static_cast<unsigned char*>(buf), row_bytes, group_off, group_rows, groups, align);
   note_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace fastb
