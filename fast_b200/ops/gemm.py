@@ -106,8 +106,9 @@ class TokScratch:
 _plans: dict = {}
 
 
-def wide_tiles(epi: int, reduction: int, mean_rows: int) -> bool:
-    """Whether tiles of 512 tokens are faster than tiles of 256 for groups of about ``mean_rows`` rows (grouped_gemm_tokens.cu says why).
+def wide_tiles(epi: int, reduction: int, mean_rows: int, waves: float) -> bool:
+    """Whether tiles of 512 tokens are faster than tiles of 256 for groups of about ``mean_rows`` rows (grouped_gemm_tokens.cu says why);
+    ``waves`` is how many rounds of the GPU they make.
 
     SwiGLU forward: where a group fits one wide tile but not one of 256; up to 448, so that most groups still do if the mean does. us, 256 ->
     512 tokens: 8 experts of 4096 x 14336 with 288, 384, 448, 480, 576 rows 617 -> 533, 651 -> 618, 697 -> 671, 823 -> 747, 902 -> 948; 32 of
@@ -115,10 +116,11 @@ def wide_tiles(epi: int, reduction: int, mean_rows: int) -> bool:
     Others: where tiles are long (the reduction) and many (the rows), so that neither their ends nor the last wave weigh. Reduction of 28672 with
     768, 1024, 2048, 4096 rows 1082 -> 1081, 1387 -> 1368, 2755 -> 2645, 5838 -> 5323; of 14336 with 512, 1024, 2048 385 -> 503, 694 -> 690,
     1385 -> 1310; SwiGLU backward, 4096 with 2048 and 4096 rows 1518 -> 1552, 3056 -> 3013, 7168 with 1024 and 2048 771 -> 762, 1536 -> 1482.
+    Cutting the last wave pays for long reductions only: 4096 with 8192 rows in 3.5 waves 176 -> 190 (2 experts, 2048 columns, plain).
     Shorter reductions lose at any size (plain, 3584 with 4096 rows 178 -> 189; a whole SwiGLU layer, 1024 with 444 rows 115 -> 122)."""
     if reduction < 4096:
         return False
-    return 256 < mean_rows <= 448 if epi == SWIGLU else mean_rows * reduction >= 12 << 20
+    return 256 < mean_rows <= 448 if epi == SWIGLU else mean_rows * reduction >= 12 << 20 and (reduction >= 8192 or waves >= 6)
 
 
 def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor]) -> tuple:
@@ -143,11 +145,12 @@ def wide_columns(row_tiles: int, columns: int, pairs: int, mean_rows: int) -> bo
     return mean_rows < 512 or 50 * waves(row_tiles * (columns // 512)) <= 26 * waves(row_tiles * (columns // 256))
 
 
-def token_tile(epi: int, reduction: int, most_rows: int, mean_rows: int) -> int:
+def token_tile(epi: int, reduction: int, most_rows: int, mean_rows: int, groups: int, features: int, pairs: int) -> int:
     """Most tokens of a tile. Where no group can have more than a narrow tile holds, narrow tiles leave shared memory to the weights in flight."""
     if 0 < most_rows <= 128:
         return 64 if most_rows <= 64 else 128
-    return 512 if wide_tiles(epi, reduction, mean_rows) else 256
+    waves = groups * -(-mean_rows // 512) * (features / 256) / pairs
+    return 512 if wide_tiles(epi, reduction, mean_rows, waves) else 256
 
 
 def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
@@ -169,7 +172,7 @@ def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.T
     if scratch is not None:
         scratch.parity ^= 1
         counters, parity, early = scratch.counters, scratch.parity, scratch.early
-    tile_n = token_tile(epi, x.shape[1], most_rows, mean_rows or x.shape[0] // w.shape[0])
+    tile_n = token_tile(epi, x.shape[1], most_rows, mean_rows or x.shape[0] // w.shape[0], w.shape[0], w.shape[1 + mode], n // 2)
     plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, counters, parity, tile_n, early)
 
 
