@@ -129,10 +129,13 @@ struct TokSegments {
 // tiles: reduction of 4096 1280, 1262, 1152; 1265, 1254, 1163; 1276, 1235, 1146; of 14336 1103, 1134, 1073; 1155, 1137, 1123; 1189,
 // 1182, 1124; of 28672 981, 1010, 1007; 1052, 1040, 1073; 1098, 1100, 1063. On normal random rows 16 tiles are ahead by 3-5 % at 8192 rows;
 // DRAM reads of a reduction of 4096 over 8192 rows at bands of 4, 8, 16, 32 tiles: 2.2, 1.1, 0.7, 1.7 GB an expert.
+// Where the weights of a group stay in L2 from band to band nothing is saved by more than 8: 2 experts of 2048 x 4096 and 8192 rows,
+// bands of 16 and 8, us: forward 184 -> 182.5, its SwiGLU 191 -> 189.5, data gradient of 4096 186 -> 183.
 constexpr int kTokBandBytes = 60 << 20, kTokBandTiles = 16;
-FASTB_HD inline int tok_band_tiles(int red_len) {
+FASTB_HD inline int tok_band_tiles(int red_len, int m_tiles) {
   const long long fit = kTokBandBytes / (2ll * red_len * kTokAccN);
-  return fit < 1 ? 1 : fit > kTokBandTiles ? kTokBandTiles : static_cast<int>(fit);
+  const int most = 512ll * red_len * m_tiles <= kTokBandBytes / 2 ? kTokBandTiles / 2 : kTokBandTiles;
+  return fit < 1 ? 1 : fit > most ? most : static_cast<int>(fit);
 }
 // From how many token tiles of a group on alternating the direction of the reduction pays (grouped_gemm_tokens.cu).
 FASTB_HD inline int tok_back_tiles(int red_len, int band_tiles, int tile_n = kTokAccN) {

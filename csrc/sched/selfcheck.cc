@@ -141,7 +141,7 @@ static void token_walker_check() {
       rows[g] = rnd(5) == 0 ? 0 : 1 + rnd(trial % 7 == 0 ? 3000 : rnd(2) ? 64 : 700);
       off[g + 1] = off[g] + (rows[g] + 255) / 256 * 256;
     }
-    const Args p{off.data(), live ? rows.data() : nullptr, granule, tile_n, m_tiles, tok_band_tiles(64 * kb_tile)};
+    const Args p{off.data(), live ? rows.data() : nullptr, granule, tile_n, m_tiles, tok_band_tiles(64 * kb_tile, m_tiles)};
     CHECK(p.band_tiles >= 1 && p.band_tiles <= kTokBandTiles, "token walker: band");
     // the prefix as the kernel makes it
     const int per_entry = tok_per_entry(G), entries = div_up(G, per_entry);

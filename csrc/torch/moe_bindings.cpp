@@ -148,7 +148,7 @@ struct TokGemmPlan {
     if (has_c2) c2 = bf16_map_2d(*gate_up, 32);
     a.num_groups = static_cast<int>(G);
     a.m_tiles = static_cast<int>(feats / 256); a.red_blocks = static_cast<int>(red / 64); a.w_rows_per_group = static_cast<int>(N);
-    a.band_tiles = band_rows > 0 ? std::max(1, band_rows / 256) : gemm::tok_band_tiles(static_cast<int>(red));
+    a.band_tiles = band_rows > 0 ? std::max(1, band_rows / 256) : gemm::tok_band_tiles(static_cast<int>(red), a.m_tiles);
     a.back_tiles = gemm::tok_back_tiles(static_cast<int>(red), a.band_tiles);
     a.granule = granule; a.keep_gate_up = fwd && has_c2 ? 1 : 0;
   }
