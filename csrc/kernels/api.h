@@ -215,6 +215,7 @@ struct GateRouteArgs {
   int* slot_in_block;
   int* block_cnt;               // [E], the same as SplitsArgs::block_cnt
 };
+bool gate_route_fits(int world, int E, int K, int H);   // the token's row (4 H bytes) and the tables in a block's shared memory
 cudaError_t launch_gate_route(const GateRouteArgs& g, const SplitsArgs& sp, unsigned int* ticket, cudaStream_t stream);
 // list[send_pos[e] + rank of (t, j) among my entries for e] = t*K + j  (see SplitsArgs::send_pos).
 // Entries whose expert id is outside [0, E) are skipped and reported in `status` (kSiteExpertId).

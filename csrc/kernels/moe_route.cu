@@ -250,10 +250,16 @@ cudaError_t launch_route_splits(const float* logits, const float* bias, int T, i
   return route_topk_any<true>(logits, bias, T, sp.num_experts, K, topk_idx, topk_w, slot_in_block, const_cast<int*>(sp.block_cnt), sp, ticket, stream);
 }
 
+static size_t gate_route_smem_bytes(int world, int E, int K, int H) {
+  return std::max({route::rank_smem_bytes(E, K), route::splits_smem_bytes(world, E), sizeof(int) * gate_route_parts_ints(E) + sizeof(float) * static_cast<size_t>(H)});
+}
+bool gate_route_fits(int world, int E, int K, int H) { return gate_route_smem_bytes(world, E, K, H) <= 225 * 1024; }   // of 227 KiB; the rest is static
+
 cudaError_t launch_gate_route(const GateRouteArgs& g, const SplitsArgs& sp, unsigned int* ticket, cudaStream_t stream) {
   const int E = sp.num_experts;
   if (g.T < 1 || g.T > kTokensPerBlock || E > 256 || g.K < 1 || g.K > 32 || g.K > E || g.H % 8 || ticket == nullptr || !splits_args_ok(sp) || sp.num_blocks != 1) return cudaErrorInvalidValue;
-  const size_t smem = std::max({route::rank_smem_bytes(E, g.K), route::splits_smem_bytes(sp.world, E), sizeof(int) * gate_route_parts_ints(E) + sizeof(float) * static_cast<size_t>(g.H)});
+  if (!gate_route_fits(sp.world, E, g.K, g.H)) return cudaErrorInvalidValue;
+  const size_t smem = gate_route_smem_bytes(sp.world, E, g.K, g.H);
   auto go = [&](auto kern) {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

@@ -487,6 +487,7 @@ void bind_moe(py::module_& m) {
            py::arg("status"), py::arg("timeout_ns"), py::arg("send_pos"), py::arg("epoch_dev_ptr"), py::arg("tile_target"), py::arg("tile_rows"), py::arg("ticket"));
   m.def("route_splits", &route_splits);
   m.def("gate_route", &gate_route);
+  m.def("gate_route_fits", &gate_route_fits, py::arg("world"), py::arg("experts"), py::arg("k"), py::arg("hidden"));
   m.def("zero_pad_rows", &zero_pad_rows, py::arg("buf"), py::arg("group_off"), py::arg("group_rows"), py::arg("align") = 0);
   m.def("build_send_list", [](torch::Tensor topk_idx, torch::Tensor slot_in_block, torch::Tensor block_base, torch::Tensor send_pos, torch::Tensor list, const StatusPy& st) {
     want(topk_idx, torch::kInt32, "topk_idx"); want(send_pos, torch::kInt32, "send_pos"); want(list, torch::kInt32, "list");

@@ -146,6 +146,7 @@ class ExpertParallel:
                                    self.send_pos if overlap_dispatch else None, self.epoch_dev.data_ptr() if graph_mode else 0, self.tile_target, self.tile_rows,
                                    torch.zeros(1 + blocks, **i32))
         self.ticket = torch.zeros(1, **i32)
+        self._gate_fits = C.gate_route_fits(W, num_experts, top_k, hidden)
         # One rank alone: nothing crosses a wire, so the fp8 dispatch stores the bf16 values that a receiver would make of its rows.
         self.local_bf16 = fp8_dispatch and W == 1 and not self.fp8_direct and not overlap_dispatch
         if graph_mode:
@@ -234,8 +235,9 @@ class ExpertParallel:
     def route_gate(self, x: torch.Tensor, gate: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
         """Route on the router logits ``x @ gate.T`` (bf16, as a GEMM returns them). For a few tokens the logits are made in the
         routing kernel itself: one block per token, each reading the whole gate, so up to a block's worth of tokens and
-        64 MiB of such reads; beyond that a GEMM reads the gate less often than it costs a launch. The kernel reads 16-byte words;
-        a gate that is a view at another address goes through the GEMM too."""
+        64 MiB of such reads; beyond that a GEMM reads the gate less often than it costs a launch. The kernel reads 16-byte words and
+        keeps the token's row in shared memory as fp32; a gate that is a view at another address, and a hidden size above some 57
+        thousand, go through the GEMM too."""
         T = x.shape[0]
         if self._gate_in_kernel(x, gate):
             topk_idx, topk_w, dest_row = self._route_outputs(T, x.device)
@@ -246,7 +248,7 @@ class ExpertParallel:
 
     def _gate_in_kernel(self, x: torch.Tensor, gate: torch.Tensor) -> bool:
         T = x.shape[0]
-        return (1 <= T <= self._C.ROUTE_TOKENS_PER_BLOCK and 2 * T * self.E * self.H <= 64 << 20 and self.E <= 256 and x.dtype == gate.dtype == torch.bfloat16
+        return (self._gate_fits and 1 <= T <= self._C.ROUTE_TOKENS_PER_BLOCK and 2 * T * self.E * self.H <= 64 << 20 and self.E <= 256 and x.dtype == gate.dtype == torch.bfloat16
                 and x.is_contiguous() and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and T <= self.T)
 
     def route_and_send(self, x: torch.Tensor, gate: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:

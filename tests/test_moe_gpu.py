@@ -434,6 +434,24 @@ def test_forward_layer_of_few_tokens(E, K, H, I, T, fp8):
         assert bool(((rows >= off[idx]) & (rows < off[idx] + counts[idx])).all()) and rows.unique().numel() == n * K
 
 
+@pytest.mark.parametrize("H,in_kernel", [(57344, True), (57600, False), (65536, False)])
+def test_few_tokens_of_the_widest_rows(H, in_kernel):
+    """A row that the routing kernel's shared memory cannot hold is routed through the GEMM: a layer of any width takes few tokens."""
+    from fast_b200.models import MoELayer
+    from fast_b200.parallel import Communicator
+
+    comm = Communicator(heap_bytes=512 << 20, device=0)
+    layer = MoELayer(comm, H, 256, 2, 1, max_tokens=4, training=False, init_std=0.01).eval()
+    x = torch.randn(3, H, generator=torch.Generator(device="cuda").manual_seed(H), device="cuda").to(torch.bfloat16)
+    assert layer.engine._gate_in_kernel(x, layer.gate) == in_kernel
+    with torch.no_grad():
+        y = layer(x)
+    comm.check()
+    want, _, _ = _ref_forward(x, layer.gate, layer.w13, layer.w2, 1, idx=layer.last_route.topk_idx.long())
+    assert _rel(y, want) < 2e-2
+    comm.close()
+
+
 @pytest.mark.parametrize("fp8,overlap", [(False, False), (True, False), (False, True), (True, True)])
 def test_forward_layer_without_tokens(fp8, overlap):
     """A step of no tokens returns no rows, and the step after it is as if it had not been."""
