@@ -350,20 +350,36 @@ void zero_pad_rows(torch::Tensor buf, torch::Tensor group_off, torch::Tensor gro
                                 static_cast<int>(group_rows.numel()), align, stream_now()), "zero_pad_rows");
 }
 
+// What every dispatch has: who sends (heap), the rows and the routing tables.
+DispatchArgs dispatch_args(const HeapPy& heap, const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& slot_in_block, const torch::Tensor& block_base,
+                           const torch::Tensor& send_base, const torch::Tensor& dest_row, const StatusPy& st, uint64_t timeout_ns) {
+  want16(x, torch::kBFloat16, "x"); want(topk_idx, torch::kInt32, "topk_idx"); want(dest_row, torch::kInt32, "dest_row");
+  DispatchArgs a{};
+  a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
+  a.num_experts = static_cast<int>(send_base.numel()); a.T = static_cast<int>(x.size(0)); a.H = static_cast<int>(x.size(1));
+  a.K = static_cast<int>(topk_idx.size(1));
+  a.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()); a.topk_idx = topk_idx.data_ptr<int>();
+  a.slot_in_block = slot_in_block.data_ptr<int>(); a.block_base = block_base.data_ptr<int>(); a.send_base = send_base.data_ptr<int>();
+  a.dest_row = dest_row.data_ptr<int>();
+  a.status = st.d; a.timeout_ns = timeout_ns;
+  return a;
+}
+// ... and the receiver's matrix of bf16 rows that a rank alone may fill in place of the e4m3 one.
+__nv_bfloat16* local_bf16_rows(const torch::Tensor& rows, const DispatchArgs& a) {
+  want16(rows, torch::kBFloat16, "local_rows");
+  TORCH_CHECK(a.fp8 && rows.dim() == 2 && rows.size(1) == a.H, "dispatch_push: local_rows belongs to the fp8 rows");
+  return reinterpret_cast<__nv_bfloat16*>(rows.data_ptr());
+}
+
 void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, c10::optional<torch::Tensor> row_scale, torch::Tensor slot_in_block,
                    torch::Tensor block_base, torch::Tensor send_base, torch::Tensor dest_row, bool compute_rows, bool fp8, int64_t recv_off,
                    int64_t scale_off, int64_t arrive_off, int64_t entry_flags_off, uint64_t entry_epoch, const StatusPy& st, uint64_t timeout_ns, int ctas,
                    c10::optional<torch::Tensor> send_list, int tile_rows, int num_tiles, c10::optional<torch::Tensor> xq,
                    c10::optional<torch::Tensor> xq_scales, c10::optional<torch::Tensor> local_rows, c10::optional<torch::Tensor> dot_out, int64_t y_off,
                    c10::optional<torch::Tensor> sum_with, c10::optional<torch::Tensor> grad_out, c10::optional<torch::Tensor> grad_loss, double grad_factor) {
-  want16(x, torch::kBFloat16, "x"); want(topk_idx, torch::kInt32, "topk_idx"); want(dest_row, torch::kInt32, "dest_row");
-  DispatchArgs a{};
-  a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world();
-  a.num_experts = static_cast<int>(send_base.numel()); a.T = static_cast<int>(x.size(0)); a.H = static_cast<int>(x.size(1));
-  a.K = static_cast<int>(topk_idx.size(1));
-  a.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()); a.topk_idx = topk_idx.data_ptr<int>(); a.row_scale = ptr_or_null<const float>(row_scale);
-  a.slot_in_block = slot_in_block.data_ptr<int>(); a.block_base = block_base.data_ptr<int>(); a.send_base = send_base.data_ptr<int>();
-  a.dest_row = dest_row.data_ptr<int>(); a.compute_rows = compute_rows; a.fp8 = fp8;
+  DispatchArgs a = dispatch_args(heap, x, topk_idx, slot_in_block, block_base, send_base, dest_row, st, timeout_ns);
+  a.row_scale = ptr_or_null<const float>(row_scale);
+  a.compute_rows = compute_rows; a.fp8 = fp8;
   a.send_list = ptr_or_null<const int>(send_list);
   a.tile_rows = tile_rows; a.num_tiles = num_tiles;
   if (xq.has_value()) {
@@ -385,21 +401,31 @@ void dispatch_push(const HeapPy& heap, torch::Tensor x, torch::Tensor topk_idx, 
       a.grad_loss = grad_loss->data_ptr<float>(); a.grad_factor = static_cast<float>(grad_factor);
     }
   }
-  if (local_rows.has_value()) {
-    want16(*local_rows, torch::kBFloat16, "local_rows");
-    TORCH_CHECK(fp8 && local_rows->dim() == 2 && local_rows->size(1) == a.H, "dispatch_push: local_rows belongs to the fp8 rows");
-    a.local_rows = reinterpret_cast<__nv_bfloat16*>(local_rows->data_ptr());
-  }
+  if (local_rows.has_value()) a.local_rows = local_bf16_rows(*local_rows, a);
   a.recv_heap_off = recv_off; a.scale_heap_off = scale_off; a.arrive_heap_off = arrive_off;
-  a.entry_flags_heap_off = entry_flags_off; a.entry_epoch = entry_epoch; a.status = st.d; a.timeout_ns = timeout_ns;
+  a.entry_flags_heap_off = entry_flags_off; a.entry_epoch = entry_epoch;
   cu_check(launch_dispatch_push(a, ctas, stream_now()), "dispatch_push");
+}
+
+// What every combine has: who pulls (heap), the routing tables, where the rows and the ready flags lie, and the output.
+CombineArgs combine_args(const HeapPy& heap, int num_experts, const torch::Tensor& topk_idx, const torch::Tensor& dest_row, const c10::optional<torch::Tensor>& weights, int64_t src_off,
+                         int64_t ready_off, uint64_t ready_epoch, const torch::Tensor& out, int H, const StatusPy& st, uint64_t timeout_ns) {
+  CombineArgs a{};
+  a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world(); a.num_experts = num_experts;
+  a.T = static_cast<int>(topk_idx.size(0)); a.K = static_cast<int>(topk_idx.size(1)); a.H = H;
+  a.topk_idx = topk_idx.data_ptr<int>(); a.dest_row = dest_row.data_ptr<int>(); a.weights = ptr_or_null<const float>(weights);
+  a.src_heap_off = src_off; a.ready_flags_heap_off = ready_off; a.ready_epoch = ready_epoch;
+  want16(out, torch::kBFloat16, "out");
+  a.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+  a.status = st.d; a.timeout_ns = timeout_ns;
+  return a;
 }
 
 // The two arguments after `out` are always None: positions that callers of an earlier form still fill.
 void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, torch::Tensor dest_row, c10::optional<torch::Tensor> weights, int64_t src_off,
                   int64_t ready_off, uint64_t ready_epoch, torch::Tensor out, py::none, py::none, int H, const StatusPy& st, uint64_t timeout_ns, int ctas, int64_t epoch_dev_ptr, bool signal,
                   c10::optional<torch::Tensor> residual, c10::optional<torch::Tensor> loss, double loss_scale, c10::optional<torch::Tensor> ticket) {
-  CombineArgs a{};
+  CombineArgs a = combine_args(heap, num_experts, topk_idx, dest_row, weights, src_off, ready_off, ready_epoch, out, H, st, timeout_ns);
   torch::Tensor partials;
   if (residual.has_value()) {
     TORCH_CHECK(loss.has_value() && ticket.has_value(), "combine_pull: residual needs loss and ticket");
@@ -410,44 +436,44 @@ void combine_pull(const HeapPy& heap, int num_experts, torch::Tensor topk_idx, t
     a.loss_partials = partials.data_ptr<float>(); a.ticket = reinterpret_cast<unsigned int*>(ticket->data_ptr<int>());
   }
   a.signal = signal ? 1 : 0;
-  a.peer_table = heap.h->device_peer_table(); a.rank = heap.h->rank(); a.world = heap.h->world(); a.num_experts = num_experts;
-  a.T = static_cast<int>(topk_idx.size(0)); a.K = static_cast<int>(topk_idx.size(1)); a.H = H;
-  a.topk_idx = topk_idx.data_ptr<int>(); a.dest_row = dest_row.data_ptr<int>(); a.weights = ptr_or_null<const float>(weights);
-  a.src_heap_off = src_off; a.ready_flags_heap_off = ready_off; a.ready_epoch = ready_epoch;
   a.epoch_dev = reinterpret_cast<const unsigned long long*>(epoch_dev_ptr);
-  want16(out, torch::kBFloat16, "out");
-  a.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
-  a.status = st.d; a.timeout_ns = timeout_ns;
   cu_check(launch_combine_pull(a, ctas, stream_now()), "combine_pull");
 }
 
-// Routing, dispatch and combine of an engine that is alone (one rank, forward only, eager): the launches of the functions above with what
-// the engine's buffers fix bound once, so that a pass with few tokens, whose kernels take 45 us, is not paid for in interpreter time (the five
-// launches of a layer took 54-71 us of the host, now 43-45). Heap, rows and gate come with every call.
+// Routing of few tokens, dispatch and combine of an engine that is alone (one rank, forward only, eager): the launches of the functions above
+// with the engine's buffers bound once, so that a pass with few tokens, whose kernels take 45 us, is not paid for in interpreter time.
+// What may change between passes (heap, rows, tables, grid, time limit) comes with every call.
 struct LocalTransport {
-  torch::Tensor slot_in_block, block_base, send_base, x_recv;
+  torch::Tensor slot_in_block, x_recv;
   bool fp8;
   int64_t recv_off, scale_off, y_off, ready_off;
-  int K, tile_rows, num_tiles, comm_ctas;
-  uint64_t timeout_ns;
+  int K, tile_rows, num_tiles;
 
   // Returns (topk_idx, topk_w, dest_row).
-  py::tuple route_and_send(const HeapPy& heap, const SplitsPlan& splits, const StatusPy& st, torch::Tensor x, torch::Tensor gate, c10::optional<torch::Tensor> bias, uint64_t epoch,
-                           bool gate_in_kernel) const {
+  py::tuple gate_route(const SplitsPlan& splits, torch::Tensor x, torch::Tensor gate, c10::optional<torch::Tensor> bias, uint64_t epoch) const {
     const int64_t T = x.size(0);
     const auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(x.device());
     auto topk_idx = torch::empty({T, K}, i32), dest_row = torch::empty({T, K}, i32), topk_w = torch::empty({T, K}, i32.dtype(torch::kFloat32));
-    if (gate_in_kernel) gate_route(splits, x, gate, bias, K, topk_idx, topk_w, slot_in_block, epoch);
-    else route_splits(splits, at::matmul(x, gate.t()).to(torch::kFloat32), bias, K, topk_idx, topk_w, slot_in_block, epoch);
-    c10::optional<torch::Tensor> none;
-    dispatch_push(heap, x, topk_idx, none, slot_in_block, block_base, send_base, dest_row, true, fp8, recv_off, scale_off, -1, 0, 0, st, timeout_ns, comm_ctas, none, tile_rows, num_tiles,
-                  none, none, fp8 ? c10::optional<torch::Tensor>(x_recv) : none, none, 0, none, none, none, 0.0);
+    ::gate_route(splits, x, gate, bias, K, topk_idx, topk_w, slot_in_block, epoch);
     return py::make_tuple(topk_idx, topk_w, dest_row);
   }
-  torch::Tensor combine(const HeapPy& heap, const StatusPy& st, torch::Tensor topk_idx, torch::Tensor dest_row, torch::Tensor weights, uint64_t epoch) const {
-    auto out = torch::empty({topk_idx.size(0), x_recv.size(1)}, x_recv.options());
-    combine_pull(heap, static_cast<int>(send_base.numel()), topk_idx, dest_row, weights, y_off, ready_off, epoch, out, py::none(), py::none(), static_cast<int>(x_recv.size(1)), st, timeout_ns,
-                 comm_ctas, 0, true, c10::nullopt, c10::nullopt, 1.0, c10::nullopt);
+  void dispatch(const HeapPy& heap, const StatusPy& st, torch::Tensor x, torch::Tensor topk_idx, torch::Tensor slots, torch::Tensor block_base, torch::Tensor send_base, torch::Tensor dest_row,
+                uint64_t timeout_ns, int ctas) const {
+    DispatchArgs a = dispatch_args(heap, x, topk_idx, slots, block_base, send_base, dest_row, st, timeout_ns);
+    a.compute_rows = true; a.fp8 = fp8;
+    if (fp8) a.local_rows = local_bf16_rows(x_recv, a);
+    a.recv_heap_off = recv_off; a.scale_heap_off = scale_off;
+    a.arrive_heap_off = -1;   // the rows are in when the kernel ends: nobody waits for a count
+    a.tile_rows = tile_rows; a.num_tiles = num_tiles;
+    cu_check(launch_dispatch_push(a, ctas, stream_now()), "dispatch_push");
+  }
+  torch::Tensor combine(const HeapPy& heap, const StatusPy& st, int num_experts, torch::Tensor topk_idx, torch::Tensor dest_row, c10::optional<torch::Tensor> weights,
+                        uint64_t epoch, uint64_t timeout_ns, int ctas) const {
+    const int H = static_cast<int>(x_recv.size(1));
+    auto out = torch::empty({topk_idx.size(0), H}, x_recv.options());
+    CombineArgs a = combine_args(heap, num_experts, topk_idx, dest_row, weights, y_off, ready_off, epoch, out, H, st, timeout_ns);
+    a.signal = 1;
+    cu_check(launch_combine_pull(a, ctas, stream_now()), "combine_pull");
     return out;
   }
 };
@@ -456,13 +482,13 @@ struct LocalTransport {
 
 void bind_moe(py::module_& m) {
   py::class_<LocalTransport>(m, "LocalTransport")
-      .def(py::init([](torch::Tensor slot_in_block, torch::Tensor block_base, torch::Tensor send_base, torch::Tensor x_recv, bool fp8, int64_t recv_off, int64_t scale_off, int64_t y_off,
-                       int64_t ready_off, int K, int tile_rows, int num_tiles, int comm_ctas, uint64_t timeout_ns) {
-        want(slot_in_block, torch::kInt32, "slot_in_block"); want(block_base, torch::kInt32, "block_base"); want(send_base, torch::kInt32, "send_base");
-        want16(x_recv, torch::kBFloat16, "x_recv");
-        return LocalTransport{slot_in_block, block_base, send_base, x_recv, fp8, recv_off, scale_off, y_off, ready_off, K, tile_rows, num_tiles, comm_ctas, timeout_ns};
-      }))
-      .def("route_and_send", &LocalTransport::route_and_send)
+      .def(py::init([](torch::Tensor slot_in_block, torch::Tensor x_recv, bool fp8, int64_t recv_off, int64_t scale_off, int64_t y_off, int64_t ready_off, int k, int tile_rows, int num_tiles) {
+        want(slot_in_block, torch::kInt32, "slot_in_block"); want16(x_recv, torch::kBFloat16, "x_recv");
+        return LocalTransport{slot_in_block, x_recv, fp8, recv_off, scale_off, y_off, ready_off, k, tile_rows, num_tiles};
+      }), py::arg("slot_in_block"), py::arg("x_recv"), py::arg("fp8"), py::arg("recv_off"), py::arg("scale_off"), py::arg("y_off"), py::arg("ready_off"), py::arg("k"), py::arg("tile_rows"),
+           py::arg("num_tiles"))
+      .def("gate_route", &LocalTransport::gate_route)
+      .def("dispatch", &LocalTransport::dispatch)
       .def("combine", &LocalTransport::combine);
   py::class_<TensorMap2D>(m, "TensorMap2D").def(py::init<int64_t, int64_t, int64_t, int64_t, int, int>()).def_static("bytes", &TensorMap2D::bytes);
   py::class_<TokGemmPlan>(m, "TokGemmPlan")

@@ -159,12 +159,12 @@ class ExpertParallel:
         self.scratch = gemm.TokScratch(dev) if gemm.USE_PAIR else None
         self.status = comm.status
         self.timeout_ns = comm.timeout_ns
-        # Alone, forward only and eager: what the transport kernels' launches have in common is bound once.
+        # Alone, forward only and eager: what this engine's buffers fix of the transport kernels' launches is bound once.
         self._local = None
         if W == 1 and not (training or graph_mode or overlap_dispatch or self.fp8_direct) and gemm.USE_PAIR:
-            self._local = C.LocalTransport(self.slot_in_block, self.block_base, self.send_base, self.x_recv, fp8_dispatch, self._off(self.xq_recv if fp8_dispatch else self.x_recv),
-                                           self._off(self.xs_recv) if fp8_dispatch else 0, self._off(self.y), self._flag_off(1), top_k, self.tile_rows, self.ntiles, self.comm_ctas,
-                                           self.timeout_ns)
+            self._local = C.LocalTransport(self.slot_in_block, self.x_recv, fp8_dispatch, recv_off=self._off(self.xq_recv if fp8_dispatch else self.x_recv),
+                                           scale_off=self._off(self.xs_recv) if fp8_dispatch else 0, y_off=self._off(self.y), ready_off=self._flag_off(1), k=top_k,
+                                           tile_rows=self.tile_rows, num_tiles=self.ntiles)
         torch.cuda.synchronize(dev)
         if W > 1:
             import torch.distributed as dist
@@ -240,6 +240,9 @@ class ExpertParallel:
         thousand, go through the GEMM too."""
         T = x.shape[0]
         if self._gate_in_kernel(x, gate):
+            if self._local is not None:
+                self.epoch += 1
+                return self._route_state(*self._local.gate_route(self.splits, x, gate, bias, self.epoch))
             topk_idx, topk_w, dest_row = self._route_outputs(T, x.device)
             self.epoch += 1
             self._C.gate_route(self.splits, x, gate, bias, self.K, topk_idx, topk_w, self.slot_in_block, self.epoch)
@@ -252,13 +255,10 @@ class ExpertParallel:
                 and x.is_contiguous() and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and T <= self.T)
 
     def route_and_send(self, x: torch.Tensor, gate: torch.Tensor, bias: Optional[torch.Tensor] = None) -> RouteState:
-        """``route_gate`` and ``dispatch``; of a rank that is alone as one call."""
-        if self._local is None or not gemm.USE_PAIR or not 0 < x.shape[0] <= self.T:
-            rs = self.route_gate(x, gate, bias)
-            self.dispatch(x, rs)
-            return rs
-        self.epoch += 1
-        return self._route_state(*self._local.route_and_send(self.comm.heap, self.splits, self.status, x, gate, bias, self.epoch, self._gate_in_kernel(x, gate)))
+        """``route_gate`` and ``dispatch``."""
+        rs = self.route_gate(x, gate, bias)
+        self.dispatch(x, rs)
+        return rs
 
     def can_fuse_gate(self) -> bool:
         """Whether ``route_fused`` (RMSNorm + router logits + top-k in one kernel) covers this layer."""
@@ -284,6 +284,9 @@ class ExpertParallel:
         return rs, hn, rstd, logits
 
     def dispatch(self, x: torch.Tensor, rs: RouteState) -> None:
+        if self._local is not None and gemm.USE_PAIR:
+            self._local.dispatch(self.comm.heap, self.status, x, rs.topk_idx, rs.slot_in_block, rs.block_base, rs.send_base, rs.dest_row, self.timeout_ns, self.comm_ctas)
+            return
         C = self._C
         send_list = xq = xs = None
         if not self.fp8 and self._needs_zero_pads():
@@ -364,7 +367,7 @@ class ExpertParallel:
         """``out[t] = sum_j weights[t, j] * y_row(t, j)``. With ``residual`` ([T, H] bf16), ``loss`` (float [1]) receives
         mean((residual + out)^2), the sum rounded to bf16."""
         if self._local is not None and out is None and residual is None:
-            return self._local.combine(self.comm.heap, self.status, rs.topk_idx, rs.dest_row, weights, rs.epoch)
+            return self._local.combine(self.comm.heap, self.status, self.E, rs.topk_idx, rs.dest_row, weights, rs.epoch, self.timeout_ns, self.comm_ctas)
         T = rs.topk_idx.shape[0]
         if out is None:
             out = torch.empty(T, self.H, dtype=torch.bfloat16, device=rs.topk_idx.device)

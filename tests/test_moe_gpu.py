@@ -588,6 +588,43 @@ def test_weights_written_after_dispatch_are_waited_for(monkeypatch):
     comm.check()
 
 
+@pytest.mark.parametrize("T", [5, 300])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_layer_alone_takes_its_engine_s_steps(T, fp8):
+    """A rank that is alone has shorter launch calls of its own. They give the bits of the general ones, they follow a grid that is set
+    after construction, and a step that is replaced is the one that runs."""
+    from fast_b200.models import MoELayer
+    from fast_b200.ops import gemm
+    from fast_b200.parallel import Communicator
+
+    if not gemm.USE_PAIR:
+        pytest.skip("the one-CTA kernels have the general launches only")
+    comm = Communicator(heap_bytes=128 << 20, device=0)
+    layer = MoELayer(comm, 256, 256, 8, 2, max_tokens=512, fp8_dispatch=fp8, training=False, router_bias=True).eval()
+    eng, local = layer.engine, layer.engine._local
+    assert local is not None
+    x = torch.randn(T, 256, generator=torch.Generator(device="cuda").manual_seed(T), device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        want, rows = layer(x), layer.last_route.dest_row.clone()
+        unweighted = eng.combine(layer.last_route, None)
+        eng._local = None
+        assert torch.equal(layer(x), want) and torch.equal(layer.last_route.dest_row, rows)
+        assert torch.equal(eng.combine(layer.last_route, None), unweighted)
+        eng._local = local
+        grid, seen, dispatch = eng.comm_ctas, [], eng.dispatch
+        eng.comm_ctas = 3
+        assert torch.equal(layer(x), want)
+        eng.comm_ctas = 0                                     # refused on the host
+        with pytest.raises(RuntimeError):
+            eng.dispatch(x, layer.last_route)
+        with pytest.raises(RuntimeError):
+            eng.combine(layer.last_route, layer.last_route.topk_w)
+        eng.comm_ctas = grid
+        eng.dispatch = lambda rows_in, rs: (seen.append(rows_in.shape[0]), dispatch(rows_in, rs))[1]
+        assert torch.equal(layer(x), want) and seen == [T]
+    comm.check()
+
+
 def test_forward_layer_in_cuda_graph():
     """The forward-only layer captured in a CUDA graph replays correctly on new inputs (the step's
     epoch lives in device memory, so a replay is a new step)."""
