@@ -15,14 +15,19 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// 1 / (1 + exp(-x)) in two operations of the special-function unit. Written as a division it takes more: the approximate division
-// guards divisors above 2^126, for which the reciprocal is zero anyway.
+// 1 / (1 + exp(-x)) and x times that. Built with --use_fast_math (FASTB_FAST_MATH): two operations of the special-function unit; a division, approximate
+// too, takes more of them, for divisors above 2^126, whose reciprocal is zero anyway. Built without: the rounded division.
+#ifdef FASTB_FAST_MATH
 __device__ __forceinline__ float sigmoid(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-x)));
   return r;
 }
 __device__ __forceinline__ float silu(float x) { return x * sigmoid(x); }
+#else
+__device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + __expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x)); }
+#endif
 __device__ __forceinline__ uint4 pack8(const uint32_t* r) {
   return make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
                     pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));

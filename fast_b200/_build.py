@@ -122,7 +122,7 @@ def build_cuda(force=False, verbose=False):
     def nvcc(src):
         o = OBJ / (src.stem + ".o")
         if force or _stale(o, [src] + hdrs):
-            log.append(_run([f"{cuda_home}/bin/nvcc", *NVCC_ARCH, "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
+            log.append(_run([f"{cuda_home}/bin/nvcc", *NVCC_ARCH, "-lineinfo", "-O3", "-std=c++17", "--use_fast_math", "-DFASTB_FAST_MATH",
                              "-Xcompiler", "-fPIC", "-Xptxas", "-v", f"-I{CSRC}", f"-I{cuda_home}/include", "-c", src, "-o", o]))
         return o
 

@@ -5,6 +5,8 @@ import re
 import subprocess
 import sys
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC_DIRS = ("csrc", "fast_b200", "tests", "baseline")
 SRC_EXT = (".cu", ".cuh", ".cc", ".cpp", ".h", ".py", ".sh")
@@ -83,6 +85,21 @@ def test_cmake_kernel_library_names_every_kernel_source():
     text = open(os.path.join(ROOT, "CMakeLists.txt")).read()
     missing = [f for f in os.listdir(os.path.join(ROOT, "csrc", "kernels")) if f.endswith(".cu") and f"/{f}" not in text]
     assert not missing, missing
+
+
+@pytest.mark.parametrize("fast", [False, True])
+def test_sigmoid_is_approximate_only_where_the_build_asks_for_it(fast):
+    """The kernel library that is built without --use_fast_math divides with rounding, as the rest of it does."""
+    nvcc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    header = os.path.join(ROOT, "csrc", "kernels", "gemm_common.cuh")
+    text = subprocess.run([nvcc, "-E", "-x", "cu", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", *(["--use_fast_math", "-DFASTB_FAST_MATH"] if fast else []), header],
+                          capture_output=True, text=True, check=True).stdout
+    body = text[text.index("float sigmoid(float x)"):text.index("uint4 pack8")]
+    assert ("rcp.approx" in body) == fast and ("x / (1.0f" in body) == (not fast)
+    flags = open(os.path.join(ROOT, "fast_b200", "_build.py")).read()
+    assert ("--use_fast_math" in flags) == ("-DFASTB_FAST_MATH" in flags)
 
 
 def test_bench_clock_sampler_parses_samples_inside_the_window():
