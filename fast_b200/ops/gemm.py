@@ -153,6 +153,12 @@ def token_tile(epi: int, reduction: int, most_rows: int, mean_rows: int, groups:
     return 512 if wide_tiles(epi, reduction, mean_rows, waves) else 256
 
 
+def group_rows_hint(mean_rows: int, rows: int, groups: int, live_rows) -> int:
+    """About how many rows a group has: the caller's ``mean_rows``, else those that the matrix holds, unless ``live_rows`` says that these
+    are a capacity: then 0, unknown, and tiles are those that suit any number."""
+    return mean_rows or (rows // groups if live_rows is None else 0)
+
+
 def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor], group_off: torch.Tensor, live_rows,
              granule: int, timeout_s: float, ctas: Optional[int], gate, gate_tile_rows: int, scratch: Optional[TokScratch], most_rows: int = 0,
              mean_rows: int = 0) -> None:
@@ -172,7 +178,7 @@ def _tok_run(mode: int, epi: int, w: torch.Tensor, x: torch.Tensor, out: torch.T
     if scratch is not None:
         scratch.parity ^= 1
         counters, parity, early = scratch.counters, scratch.parity, scratch.early
-    tile_n = token_tile(epi, x.shape[1], most_rows, mean_rows or x.shape[0] // w.shape[0], w.shape[0], w.shape[1 + mode], n // 2)
+    tile_n = token_tile(epi, x.shape[1], most_rows, group_rows_hint(mean_rows, x.shape[0], w.shape[0], live_rows), w.shape[0], w.shape[1 + mode], n // 2)
     plan.run(group_off, live_rows, _st().ptr(), int(timeout_s * 1e9), min(ctas or n, n), counter_ptr, target, gate_tile_rows, counters, parity, tile_n, early)
 
 
@@ -252,7 +258,8 @@ def grouped_gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, group_off: torch.Tenso
     bm = 256 if USE_PAIR else _BM
     assert dy.shape[1] == N and x.shape[1] == K and N % bm == 0 and K % _BN == 0
     C = runtime.ext()
-    wide = USE_PAIR and not DIRECT_EPILOGUE and wide_columns(G * (N // bm), K, _ctas() // 2, mean_rows or x.shape[0] // G)
+    mean = group_rows_hint(mean_rows, x.shape[0], G, live_rows)
+    wide = USE_PAIR and not DIRECT_EPILOGUE and (mean > 0 or live_rows is None) and wide_columns(G * (N // bm), K, _ctas() // 2, mean)
     C.grouped_gemm(WGRAD, STORE, _tmap(dy, _BK), _tmap(x, _BK), group_off, K // (512 if wide else _BN), N // bm, 0, 0, N, out.view(G * N, K), None, _st().ptr(),
                    int(timeout_s * 1e9), _ctas(), 0, None, USE_PAIR, BAND_ROWS, *((_tmap(out.view(G * N, K), 32), None) if wide else _out_maps(out.view(G * N, K), None)), DIRECT_EPILOGUE, None, live_rows, 0, wide)
     return out

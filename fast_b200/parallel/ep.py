@@ -206,8 +206,12 @@ class ExpertParallel:
         self.scratch.early = settled and rs.topk_idx.shape[0] > 0   # without tokens there is no dispatch kernel between routing and GEMM
         # a token picks an expert at most once; other ranks may have up to max_tokens of them
         most = rs.topk_idx.shape[0] if self.comm.world == 1 else self.T * self.comm.world
-        mean = rs.topk_idx.shape[0] * self.K // self.El   # about as many come from the other ranks as go to them
-        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch, most_rows=most, mean_rows=mean)
+        return dict(live_rows=rs.group_rows, granule=self.granule, scratch=self.scratch, most_rows=most, mean_rows=self._mean_rows(rs.topk_idx.shape[0]))
+
+    def _mean_rows(self, T: int) -> int:
+        """About how many rows an expert has: as many come from the other ranks as go to them. At least 1 (0 means "unknown" to a GEMM, which then
+        goes by the capacity)."""
+        return max(1, T * self.K // self.El)
 
     def traffic_matrix(self) -> torch.Tensor:
         """Token traffic matrix [src, dst] of the last routed step (device tensor)."""
@@ -427,7 +431,7 @@ class ExpertParallel:
             gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dgu, gate=gate, swiglu_bwd_of=self.gu, **self._live(rs))
         else:
             gemm.grouped_gemm_dgrad(self.dy_recv, w2, rs.group_off, self.dact, gate=gate, **self._live(rs))
-        live = dict(live_rows=rs.group_rows if self.scratch is not None else None, mean_rows=T * self.K // self.El)
+        live = dict(live_rows=rs.group_rows if self.scratch is not None else None, mean_rows=self._mean_rows(T))
         gemm.grouped_gemm_wgrad(self.dy_recv, self.act, rs.group_off, dw2, **live)
         if after_dw2 is not None:
             after_dw2()

@@ -1,6 +1,7 @@
 """What tells one cached launch plan of the expert GEMMs from another (no GPU)."""
 import torch
 
+from fast_b200.ops import gemm
 from fast_b200.ops.gemm import _plan_key
 
 
@@ -22,3 +23,23 @@ def test_a_plan_belongs_to_one_geometry_type_and_device():
         _plan_key(0, 1, 64, w, x, out, gu),
     ]
     assert all(k != base for k in others) and len(set(others)) == len(others)
+
+
+def test_tiles_are_not_sized_by_a_capacity():
+    """A step of fewer entries than experts counts as one row per expert, not as unknown; and where the number of rows is unknown and the matrix
+    is a receive buffer, its capacity does not stand in for it."""
+    from types import SimpleNamespace
+
+    from fast_b200.parallel.ep import ExpertParallel
+
+    engine = SimpleNamespace(scratch=SimpleNamespace(early=False), comm=SimpleNamespace(world=4), T=4096, K=2, El=32, granule=32)
+    engine._mean_rows = lambda T: ExpertParallel._mean_rows(engine, T)
+    for T in (0, 1, 3, 15, 16, 4096):
+        rs = SimpleNamespace(topk_idx=torch.empty(T, 2), group_rows=torch.empty(32))
+        live = ExpertParallel._live(engine, rs)
+        assert live["mean_rows"] == max(1, T * 2 // 32)
+        mean = gemm.group_rows_hint(live["mean_rows"], 32 * 1024, 32, live["live_rows"])
+        tile = gemm.token_tile(gemm.STORE, 28672, live["most_rows"], mean, 32, 4096, 74)
+        assert T == 4096 or tile == 256
+    assert gemm.group_rows_hint(0, 8192, 8, None) == 1024 and gemm.group_rows_hint(0, 8192, 8, torch.empty(8)) == 0
+    assert gemm.token_tile(gemm.STORE, 28672, 0, 0, 8, 4096, 74) == gemm.token_tile(gemm.SWIGLU, 4096, 0, 0, 8, 28672, 74) == 256
