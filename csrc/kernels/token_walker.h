@@ -144,6 +144,12 @@ FASTB_HD inline int tok_back_tiles(int red_len, int band_tiles, int tile_n = kTo
 // Token tiles of a band of wide tiles (512 tokens). Same operands, 8192 rows, TFLOP/s at 2, 4, 8 and 16 tiles: reduction of 4096 (SwiGLU
 // backward) 1151, 1180, 1176, 1117; of 14336 1320, 1342, 1333, 1275; of 28672 1313, 1330, 1305, 1172.
 constexpr int kTokWideBandTiles = 4;
+// The band of a launch: by the rules above, or of the rows that its caller wants.
+FASTB_HD inline int tok_band(int band_rows, int red_len, int m_tiles, int tile_n) {
+  const int tile = tile_n > kTokAccN ? tile_n : kTokAccN;
+  if (band_rows > 0) return band_rows < tile ? 1 : band_rows / tile;
+  return tile_n > kTokAccN ? kTokWideBandTiles : tok_band_tiles(red_len, m_tiles);
+}
 struct TokPlace { int m, t; };
 FASTB_HD inline TokPlace tok_place(int local, int m_tiles, int t_tiles, int band_tiles) {
   const int per_band = band_tiles * m_tiles, band = local / per_band, rem = local - band * per_band;

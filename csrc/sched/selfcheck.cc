@@ -141,8 +141,10 @@ static void token_walker_check() {
       rows[g] = rnd(5) == 0 ? 0 : 1 + rnd(trial % 7 == 0 ? 3000 : rnd(2) ? 64 : 700);
       off[g + 1] = off[g] + (rows[g] + 255) / 256 * 256;
     }
-    const Args p{off.data(), live ? rows.data() : nullptr, granule, tile_n, m_tiles, tok_band_tiles(64 * kb_tile, m_tiles)};
+    const Args p{off.data(), live ? rows.data() : nullptr, granule, tile_n, m_tiles, tok_band(0, 64 * kb_tile, m_tiles, tile_n)};
     CHECK(p.band_tiles >= 1 && p.band_tiles <= kTokBandTiles, "token walker: band");
+    const int asked = 1 + rnd(9000), bands = tok_band(asked, 64 * kb_tile, m_tiles, tile_n), rows_of = bands * std::max(tile_n, kTokAccN);
+    CHECK(bands >= 1 && (bands == 1 || rows_of <= asked) && asked < rows_of + std::max(tile_n, kTokAccN), "token walker: a band of %d rows where %d were asked for", rows_of, asked);
     // the prefix as the kernel makes it
     const int per_entry = tok_per_entry(G), entries = div_up(G, per_entry);
     CHECK(entries <= kTokPrefix, "token walker: prefix entries");

@@ -148,8 +148,6 @@ struct TokGemmPlan {
     if (has_c2) c2 = bf16_map_2d(*gate_up, 32);
     a.num_groups = static_cast<int>(G);
     a.m_tiles = static_cast<int>(feats / 256); a.red_blocks = static_cast<int>(red / 64); a.w_rows_per_group = static_cast<int>(N);
-    a.band_tiles = band_rows > 0 ? std::max(1, band_rows / 256) : gemm::tok_band_tiles(static_cast<int>(red), a.m_tiles);
-    a.back_tiles = gemm::tok_back_tiles(static_cast<int>(red), a.band_tiles);
     a.granule = granule; a.keep_gate_up = fwd && has_c2 ? 1 : 0;
   }
 
@@ -159,10 +157,8 @@ struct TokGemmPlan {
     TORCH_CHECK(group_off.is_cuda() && group_off.dtype() == torch::kInt32 && group_off.is_contiguous() && group_off.numel() == groups + 1, "group_off: cuda int32[G+1]");
     TokGemmArgs g = a;
     g.tile_n = tile_n;
-    if (tile_n > gemm::kTokAccN) {
-      g.band_tiles = band_rows_ > 0 ? g.band_tiles : gemm::kTokWideBandTiles;
-      g.back_tiles = gemm::tok_back_tiles(64 * g.red_blocks, g.band_tiles, tile_n);
-    }
+    g.band_tiles = gemm::tok_band(band_rows_, 64 * g.red_blocks, g.m_tiles, tile_n);
+    g.back_tiles = gemm::tok_back_tiles(64 * g.red_blocks, g.band_tiles, std::max(tile_n, gemm::kTokAccN));
     g.early = early ? 1 : 0;
     g.group_off = group_off.data_ptr<int>();
     if (group_rows.has_value()) {
