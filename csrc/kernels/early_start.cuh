@@ -24,6 +24,13 @@ inline cudaLaunchAttribute early_start_attribute() {
   return a;
 }
 
+// Dynamic shared memory that the kernel has not been allowed yet makes its launch fail, and the 48 KiB that need no leave include its static
+// tables: asked for from 40 KiB on (no kernel here has 8 KiB of them).
+template <class Kern>
+cudaError_t allow_smem(Kern kern, size_t smem) {
+  return smem > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) : cudaSuccess;
+}
+
 // kern<<<grid, block, smem, stream>>>(args...), allowed to start early. The kernel calls grid_dependency_wait().
 template <class... P, class... A>
 cudaError_t launch_early(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A&&... args) {

@@ -566,11 +566,8 @@ cudaError_t launch_dispatch_push(const DispatchArgs& a, int ctas, cudaStream_t s
   const size_t smem = sizeof(int) * (a.tile_rows > 0 ? static_cast<size_t>(a.world) * a.num_tiles : static_cast<size_t>(a.num_experts));
   if (smem > 200 * 1024) return cudaErrorInvalidValue;  // per-CTA histogram of destination tiles must fit in shared memory
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return e;
-    }
-    cudaError_t e = launch_early(kern, dim3(ctas), kCommThreads, smem, stream, b);
+    cudaError_t e = allow_smem(kern, smem);
+    if (e == cudaSuccess) e = launch_early(kern, dim3(ctas), kCommThreads, smem, stream, b);
     if (e == cudaSuccess) note_launch();
     return e;
   };

@@ -223,11 +223,8 @@ cudaError_t route_topk_any(const float* logits, const float* bias, int T, int E,
   if (blocks == 0) return cudaSuccess;
   const size_t smem = std::max(route::rank_smem_bytes(E, K), SPLITS ? route::splits_smem_bytes(sp.world, E) : size_t{0});
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return e;
-    }
-    cudaError_t e = launch_early(kern, dim3(blocks), kRouteThreads, smem, stream, logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt, sp, ticket);
+    cudaError_t e = allow_smem(kern, smem);
+    if (e == cudaSuccess) e = launch_early(kern, dim3(blocks), kRouteThreads, smem, stream, logits, bias, T, E, K, topk_idx, topk_w, slot_in_block, block_cnt, sp, ticket);
     if (e == cudaSuccess) note_launch();
     return e;
   };
@@ -261,11 +258,8 @@ cudaError_t launch_gate_route(const GateRouteArgs& g, const SplitsArgs& sp, unsi
   if (!gate_route_fits(sp.world, E, g.K, g.H)) return cudaErrorInvalidValue;
   const size_t smem = gate_route_smem_bytes(sp.world, E, g.K, g.H);
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return e;
-    }
-    cudaError_t e = launch_early(kern, dim3(g.T), kGateSmallThreads, smem, stream, g, sp, ticket);
+    cudaError_t e = allow_smem(kern, smem);
+    if (e == cudaSuccess) e = launch_early(kern, dim3(g.T), kGateSmallThreads, smem, stream, g, sp, ticket);
     if (e == cudaSuccess) note_launch();
     return e;
   };

@@ -791,3 +791,9 @@ def test_routing_of_few_tokens_alone(T, E, K, H, capacity):
         for j, e in enumerate(row):
             assert slots[t][j] == seen[e]
             seen[e] += 1
+
+
+@pytest.mark.parametrize("T,E,H", [(1, 8, 12032), (2, 8, 12032), (2, 8, 12288), (1, 256, 11776), (2, 256, 12032)])
+def test_routing_of_few_tokens_in_rows_that_nearly_fill_the_unasked_shared_memory(T, E, H):
+    """4 H bytes for a token's row, 32 words or one per expert, and a kilobyte of static tables: just below and above the 48 KiB that a launch may use unasked."""
+    test_routing_of_few_tokens_alone(T, E, 2, H, 1024)
