@@ -122,11 +122,12 @@ void a2a_launch(const A2AProgramPy& p, const HeapPy& heap, std::array<int64_t, 4
 // One cooperative launch that runs every virtual rank of an in-process group. Outputs lie in the ranks' heaps at one common
 // offset (else nothing is launched and the answer is false: the caller stages them); the checks of sizes are made here, so
 // that a small collective is not paid for in interpreter time. stage_offs: heap offsets of the balance and rail areas.
-// The ranks' heaps and status blocks are handed over once; the heaps are not kept alive (a closed communicator lets go of its slab).
+// The ranks' heaps and status blocks are handed over once; the status blocks, which kernels write to, live as long as the group, the heaps
+// are not kept alive (a closed communicator lets go of its slab).
 struct A2AGroupPy {
   std::vector<std::weak_ptr<SymmHeap>> heaps;
-  std::vector<const StatusPy*> statuses;   // owned by the communicators that the Python group holds
-  A2AGroupPy(const std::vector<const HeapPy*>& hs, std::vector<const StatusPy*> sts) : statuses(std::move(sts)) {
+  std::vector<std::shared_ptr<StatusPy>> statuses;
+  A2AGroupPy(const std::vector<const HeapPy*>& hs, std::vector<std::shared_ptr<StatusPy>> sts) : statuses(std::move(sts)) {
     TORCH_CHECK(hs.size() == statuses.size(), "one heap and one status block per virtual rank");
     for (const HeapPy* h : hs) heaps.push_back(h->h);
   }
@@ -134,7 +135,7 @@ struct A2AGroupPy {
 bool a2a_launch_group(const A2AGroupPy& group, const std::vector<const A2AProgramPy*>& progs, const std::vector<torch::Tensor>& outs, const std::vector<torch::Tensor>& ins,
                       std::array<int64_t, 2> stage_offs, int64_t sig_off, uint64_t epoch, uint64_t timeout_ns, int ctas, int threads) {
   const size_t n = progs.size();
-  const std::vector<const StatusPy*>& sts = group.statuses;
+  const std::vector<std::shared_ptr<StatusPy>>& sts = group.statuses;
   std::array<HeapPy, kSigMaxWorld> locked{};
   std::array<const HeapPy*, kSigMaxWorld> heaps{};
   TORCH_CHECK(n <= group.heaps.size() && n <= static_cast<size_t>(kSigMaxWorld), "one entry per virtual rank");
@@ -208,7 +209,7 @@ PYBIND11_MODULE(_C, m) {
       .def_property_readonly("bytes", [](const HeapPy& h) { return static_cast<int64_t>(h.h->bytes()); })
       .def_property_readonly("in_use", [](const HeapPy& h) { return static_cast<int64_t>(h.h->in_use()); });
 
-  py::class_<StatusPy>(m, "StatusBlock")
+  py::class_<StatusPy, std::shared_ptr<StatusPy>>(m, "StatusBlock")
       .def(py::init<>())
       .def("read", &StatusPy::read)
       .def("clear", &StatusPy::clear)
@@ -227,7 +228,7 @@ PYBIND11_MODULE(_C, m) {
         py::arg("status"), py::arg("timeout_ns"), py::arg("ctas"), py::arg("threads"), py::arg("stamps_ptr") = 0, py::arg("bulk") = false);
   m.attr("PHASE_STAMP_WORDS") = kPhaseStampWords;
   m.attr("SIG_MAX_WORLD") = kSigMaxWorld;
-  py::class_<A2AGroupPy>(m, "A2AGroup").def(py::init<const std::vector<const HeapPy*>&, std::vector<const StatusPy*>>());
+  py::class_<A2AGroupPy>(m, "A2AGroup").def(py::init<const std::vector<const HeapPy*>&, std::vector<std::shared_ptr<StatusPy>>>());
   m.def("a2a_launch_group", &a2a_launch_group);
   m.def("wait_probe", [](int64_t flag_ptr, uint64_t want, const StatusPy& st, uint64_t timeout_ns) {
     cuda_check(launch_wait_probe(reinterpret_cast<const unsigned long long*>(flag_ptr), want, st.d, timeout_ns, cur_stream()), "wait_probe");

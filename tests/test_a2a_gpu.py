@@ -128,6 +128,29 @@ def test_schedule_is_not_made_under_capture():
     assert grp.schedule(np.full((2, 2), 5, np.int64), unit_bytes=16)[0].output_bytes == 160
 
 
+def test_group_outlives_its_communicators_status_blocks():
+    """The group's launches go on with the status blocks that they were made with, whatever becomes of the communicators' own references."""
+    import gc
+
+    from fast_b200 import _C
+    from fast_b200.parallel import LocalGroup
+
+    n = 4
+    grp = LocalGroup(n, heap_bytes=16 << 20, topo=Topology(2, 2), ctas=4, threads=128)
+    for c in grp.comms:
+        c.status = _C.StatusBlock()
+    gc.collect()
+    other = [_C.StatusBlock() for _ in range(64)]   # what was given back would be handed out again
+    m = sched.workload_uniform(n, 300, 3, zero_diag=False)
+    ss = grp.schedule(m, unit_bytes=16, kind=PlanKind.STAGED, chunk_bytes=1024)
+    ins = _pattern_inputs(m, 4)
+    d_out = [c.alloc(max(s.max_bytes["output"] for s in ss) // 4, torch.int32) for c in grp.comms]
+    grp.all_to_all_v(d_out, [torch.from_numpy(x).cuda() for x in ins], ss)
+    for r, want in enumerate(_expected_outputs(m, ins, 4)):
+        assert np.array_equal(d_out[r][: want.size].cpu().numpy(), want)
+    assert all(st.read()[0] == 0 for st in other)
+
+
 def test_unaligned_byte_units():
     from fast_b200.parallel import LocalGroup
 
