@@ -64,7 +64,7 @@ constexpr int kStepTokens = 32;                   // tokens per epilogue step = 
 constexpr int kBox = kStepTokens * 128;           // 4 KiB: 32 tokens x 64 features
 
 struct __align__(8) TokCtl {
-  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load[2];
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[kAccStages], acc_empty[kAccStages], epi_load[2], meet;
   uint32_t tmem_base;
   int abort_flag, last_arrived, widest, share_weights;
   int base[kTokPrefix + 1];                         // tiles of the groups before entry i
@@ -117,10 +117,6 @@ __device__ __forceinline__ uint32_t box_row(uint32_t box, int lane, int jj, int 
 }
 __device__ __forceinline__ float as_f(uint32_t x) { return __uint_as_float(x); }
 
-// Named barrier of all epilogue groups.
-template <int SUB>
-__device__ __forceinline__ void groups_bar() { asm volatile("bar.sync 3, %0;" ::"n"(128 * SUB) : "memory"); }
-
 // Tokens of a tile of n that accumulator `sub` holds.
 __device__ __forceinline__ int acc_n(int n, int sub) { return sub == 0 ? min(n, kTokAccN) : max(n - kTokAccN, 0); }
 
@@ -144,6 +140,7 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
     for (int a = 0; a < kAccStages; ++a) { mbar_init(&ctl->acc_full[a], 1); mbar_init(&ctl->acc_empty[a], 2 * 4 * SUB); mbar_init(&ctl->epi_load[a], 1); }
+    mbar_init(&ctl->meet, 4 * SUB);
     ctl->abort_flag = 0;
     mbar_fence_init();
     prefetch_tmap(&map_w);
@@ -343,6 +340,14 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       for (int i = et; i < p.num_counters; i += 128) p.counters_next[i] = 0u;
     uint32_t acc_it = 0, ring_n = 0, load_ph = 0u;   // load_ph: one parity bit per half of the ring
     bool ok = true;
+    // All epilogue warps, twice per part of a tile (phases 0 and 1 of the barrier). Two groups wait with a limit: one of them may have given up.
+    auto meet = [&](uint32_t phase) {
+      if (SUB == 1) { epi_bar(); return; }
+      __syncwarp();
+      if (!ok) return;
+      if (lane == 0) mbar_arrive(&ctl->meet);
+      ok = mbar_wait_bounded(&ctl->meet, phase, abort_flag, p.status, 600 + phase, p.timeout_ns);
+    };
     while (ok && segs.next(sg)) {
       const TokTile tc = walk.locate(sg.tile);
       const int accs = SUB == 2 && tc.n > kTokAccN ? 2 : 1;    // accumulators that the tile fills
@@ -381,9 +386,9 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
           release_acc(sub);
         }
         __threadfence();
-        groups_bar<SUB>();
-        if (issuer && group == 0) ctl->last_arrived = atomicInc(p.counters + sg.tile * 2 + cta, static_cast<unsigned>(sg.parts - 1)) == static_cast<unsigned>(sg.parts - 1);
-        groups_bar<SUB>();
+        meet(0);
+        if (ok && issuer && group == 0) ctl->last_arrived = atomicInc(p.counters + sg.tile * 2 + cta, static_cast<unsigned>(sg.parts - 1)) == static_cast<unsigned>(sg.parts - 1);
+        meet(1);
         if (!ok) break;
         if (!ctl->last_arrived) continue;
         __threadfence();

@@ -283,6 +283,46 @@ def test_reductions_walked_backwards(counts, N, K, kernel_variant):
         _close(dw[i], dy[s:s + n].float().T @ a[s:s + n].float())
 
 
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("counts,N,K", [([700, 0, 1030], 512, 512), ([1030, 300], 1024, 8192)])
+def test_wide_tiles_wait_for_every_arrival_counter_that_they_touch(counts, N, K, swiglu, kernel_variant, monkeypatch):
+    """A tile of up to 512 tokens takes two or three counters of 256 rows. With all rows in, the product is right; with one counter short of one row
+    the launch gives up (whole tiles, and tiles whose reduction is cut), and the next one is as if it had not been."""
+    if kernel_variant != "cta_pair":
+        pytest.skip("belongs to the CTA-pair kernels")
+    from fast_b200 import runtime
+    from fast_b200.ops import gemm
+
+    monkeypatch.setattr(gemm, "wide_tiles", lambda *a: True)
+    counts_t, off, R, a, w = _setup(len(counts), N, K, counts, seed=37)
+    live, o = counts_t.to(torch.int32), off.tolist()
+    target = torch.zeros(R // 256, dtype=torch.int64)
+    for i, n in enumerate(counts):
+        for r in range(0, n, 256):
+            target[(o[i] + r) // 256] = min(256, n - r)
+    target = target.cuda()
+    out = torch.zeros(R, N // 2 if swiglu else N, device="cuda", dtype=torch.bfloat16)
+    want = []
+    for i, n in enumerate(counts):
+        full = a[o[i]:o[i] + n].float() @ w[i].float().T
+        t = full.view(n, N // 256, 2, 128)
+        want.append((torch.nn.functional.silu(t[:, :, 0]) * t[:, :, 1]).reshape(n, N // 2) if swiglu else full)
+    for slot in [None, *range(R // 256), None]:
+        counter = target.clone()
+        if slot is not None:
+            counter[slot] -= 1
+        gemm.grouped_gemm_fwd(a, w, off, out.zero_(), swiglu=swiglu, live_rows=live, gate=(counter.data_ptr(), target), gate_tile_rows=256,
+                              timeout_s=5.0 if slot is None else 0.02)
+        if slot is None:
+            gemm.check()
+            for i, n in enumerate(counts):
+                _close(out[o[i]:o[i] + n], want[i])
+        else:
+            with pytest.raises(runtime.CollectiveTimeout):
+                gemm.check()
+            gemm._st().clear()
+
+
 def test_custom_operators_run_the_same_kernels():
     """torch.ops.fast_b200.* (schemas, mutation annotations) give the same bits as the direct calls."""
     from fast_b200.ops import gemm, registry  # noqa: F401
