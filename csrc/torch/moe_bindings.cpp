@@ -493,6 +493,23 @@ void bind_moe(py::module_& m) {
       .def("run", &TokGemmPlan::run, py::arg("group_off"), py::arg("group_rows"), py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"),
            py::arg("gate_counter_ptr") = 0, py::arg("gate_target") = py::none(), py::arg("gate_tile_rows") = 0, py::arg("counters") = py::none(), py::arg("parity") = 0, py::arg("tile_n") = 256, py::arg("early") = false);
   m.attr("TOK_COUNTERS_PER_CTA") = tok_counters(1);
+  // How a launch with these rows per group splits its work: what a test names the sizes of a path by.
+  m.def("token_split", [](const std::vector<int>& rows, int m_tiles, int red_len, int tile_n, int granule, int pairs) {
+    using namespace gemm;
+    struct Groups { const int *group_off, *group_rows; int granule, tile_n, m_tiles; };
+    const Groups q{nullptr, rows.data(), granule, tile_n, m_tiles};
+    int tiles = 0, widest = 0, most = 0;
+    for (int g = 0; g < static_cast<int>(rows.size()); ++g) {
+      tiles += tok_group_tiles(q, g);
+      widest = std::max(widest, tok_tile_size(tok_rows(q, g), tile_n));
+      most = std::max(most, tok_tiles(tok_rows(q, g), tile_n));
+    }
+    const TokSplit s = TokSplit::make(tiles, red_len / 64, pairs, widest, most > 1);
+    py::dict d;
+    d["token_tiles"] = most; d["cut_tiles"] = s.cut_tiles; d["whole_tiles"] = s.whole_tiles; d["shares"] = s.shares; d["stream"] = s.stream;
+    d["back_tiles"] = tok_back_tiles(red_len, tok_band(0, red_len, m_tiles, tile_n), std::max(tile_n, kTokAccN));
+    return d;
+  }, py::arg("rows"), py::arg("m_tiles"), py::arg("red_len"), py::arg("tile_n"), py::arg("granule"), py::arg("pairs"));
   m.def("grouped_gemm", &grouped_gemm, py::arg("mode"), py::arg("epilogue"), py::arg("a"), py::arg("b"), py::arg("group_off"), py::arg("tiles_n"),
         py::arg("fixed_m_tiles"), py::arg("red_len"), py::arg("b_rows_per_group"), py::arg("c_rows_per_group"), py::arg("c"), py::arg("c2"),
         py::arg("status_ptr"), py::arg("timeout_ns"), py::arg("ctas"), py::arg("gate_counter_ptr"), py::arg("gate_target"), py::arg("pair"),

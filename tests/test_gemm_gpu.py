@@ -165,7 +165,9 @@ def test_dgrad_with_fused_swiglu_backward(kernel_variant):
     ([1], 256, 64, 32, False),                                       # one tile of the narrowest width, one block
     ([1, 0, 2], 1024, 14336, 32, True),                              # few tiles: the reduction is cut as a stream, several parts per tile
     ([31, 32, 33, 255, 256, 257, 513], 512, 1024, 32, True),         # widths around the 32-row steps and the 256-token tile
-    ([63, 64, 65, 1000, 2100], 768, 2048, 64, True),                 # several token tiles per group: cut in equal parts
+    ([63, 64, 65, 1000, 2100], 768, 2048, 64, True),                 # several token tiles per group, of unequal width
+    ([1030, 300], 1024, 8192, 64, True),                             # the same, forward reductions cut in equal parts
+    ([1030, 300], 8192, 1024, 64, True),                             # ... and those of the data gradients
     ([(7 * i) % 70 for i in range(300)], 256, 256, 64, False),       # more groups than prefix entries
 ])
 def test_live_rows_and_cut_reductions(counts, N, K, granule, keep_counters, kernel_variant):
@@ -219,7 +221,9 @@ def test_live_rows_and_cut_reductions(counts, N, K, granule, keep_counters, kern
 @pytest.mark.parametrize("counts,N,K,granule,keep_counters", [
     ([1, 32, 255, 256, 257, 288, 289, 511, 512, 513, 545], 512, 1024, 32, True),   # one and two accumulators, every remainder at the edges
     ([300], 1024, 14336, 32, True),                                                 # cut as a stream: parts of both accumulators
-    ([1030, 2100, 64], 768, 2048, 64, True),                                        # several wide tiles per group: cut in equal parts
+    ([1030, 2100, 64], 768, 2048, 64, True),                                        # several wide tiles per group
+    ([1030, 300], 1024, 8192, 64, True),                                            # the same, forward reductions cut in equal parts
+    ([1030, 300], 8192, 1024, 64, True),                                            # ... and those of the data gradients
     ([(13 * i) % 600 for i in range(260)], 256, 256, 64, False),                    # more groups than prefix entries, tiles of one and of two
     ([700], 256, 64, 32, False),                                                    # a single block: nothing between the two ends of a tile
 ])
@@ -229,6 +233,21 @@ def test_wide_tiles(counts, N, K, granule, keep_counters, kernel_variant, monkey
 
     monkeypatch.setattr(gemm, "wide_tiles", lambda *a: True)
     test_live_rows_and_cut_reductions(counts, N, K, granule, keep_counters, kernel_variant)
+
+
+def test_the_sizes_above_take_the_paths_that_they_name():
+    """What the work split makes of them on this GPU: streams, equal parts, and which passes they are in."""
+    from fast_b200 import _C
+
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    split = lambda rows, feats, red, tile_n, granule: _C.token_split(rows, feats // 256, red, tile_n, granule, pairs)
+    for tile_n in (256, 512):
+        for rows, N, K in (([1030, 300], 1024, 8192), ([1030, 300], 8192, 1024)):
+            cut, whole = split(rows, min(N, K), max(N, K), tile_n, 64), split(rows, max(N, K), min(N, K), tile_n, 64)
+            assert cut["shares"] > 1 and cut["cut_tiles"] > 0 and not cut["stream"] and whole["cut_tiles"] == 0
+    for rows, tile_n in (([1, 0, 2], 256), ([300], 512)):
+        stream = split(rows, 1024, 14336, tile_n, 32)
+        assert stream["stream"] and stream["cut_tiles"] > 0 and stream["shares"] > stream["cut_tiles"]
 
 
 @pytest.mark.parametrize("counts,N,K", [([0, 1, 64, 65, 128, 129, 192, 193], 256, 512), ([700, 0, 5000], 512, 1536), ([300, 200], 256, 768)])
@@ -259,11 +278,11 @@ def test_wgrad_stops_at_the_live_rows(kernel_variant):
 
 
 @pytest.mark.parametrize("counts,N,K", [
-    ([2049, 33], 4608, 8192),   # forward: 9 token tiles in bands of at most 8, more than two waves, 2049 tokens in tiles of unequal width
+    ([2049, 33], 4608, 8192),   # 2049 tokens in tiles of unequal width
     ([4097, 4096, 65], 2560, 2048),   # weight gradient: 65, 64 and 2 reduction blocks, 80 tiles each
 ])
 def test_reductions_walked_backwards(counts, N, K, kernel_variant):
-    """Sizes at which every other wave walks the reduction from its end: forward and weight gradient equal the fp32 product."""
+    """Sizes at which every other wave of the weight gradient walks the reduction from its end: forward and weight gradient equal the fp32 product."""
     if kernel_variant != "cta_pair":
         pytest.skip("belongs to the CTA-pair kernels")
     from fast_b200.ops import gemm
@@ -281,6 +300,34 @@ def test_reductions_walked_backwards(counts, N, K, kernel_variant):
         s = o[i]
         _close(out[s:s + n], a[s:s + n].float() @ w[i].float().T)
         _close(dw[i], dy[s:s + n].float().T @ a[s:s + n].float())
+
+
+@pytest.mark.parametrize("wide,counts,N,K,backwards", [(False, [1800, 33], 4608, 16384, [True, False]), (False, [1800, 33], 16384, 4608, [False, True]),
+                                                      (True, [2100, 33], 9216, 8192, [True, True])])
+def test_token_tiles_walked_backwards(wide, counts, N, K, backwards, kernel_variant, monkeypatch):
+    """Sizes at which every other wave of the forward pass and of the data gradient walks the reduction from its end, with tiles of up to 256 and of
+    up to 512 tokens: more token tiles than a band has, and whole tiles for more than one wave."""
+    if kernel_variant != "cta_pair":
+        pytest.skip("belongs to the CTA-pair kernels")
+    from fast_b200 import _C
+    from fast_b200.ops import gemm
+
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    for (feats, red), back in zip(((N, K), (K, N)), backwards):
+        s = _C.token_split(counts, feats // 256, red, 512 if wide else 256, 32, pairs)
+        assert (s["token_tiles"] > s["back_tiles"] and s["token_tiles"] * (feats // 256) > s["cut_tiles"] + pairs) == back, s
+    monkeypatch.setattr(gemm, "wide_tiles", lambda *a: wide)
+    counts_t, off, R, a, w = _setup(len(counts), N, K, counts, seed=33)
+    live = counts_t.to(torch.int32)
+    dy = torch.randn(R, N, generator=torch.Generator(device="cuda").manual_seed(35), device="cuda").to(torch.bfloat16)
+    out, dx = torch.zeros(R, N, device="cuda", dtype=torch.bfloat16), torch.zeros(R, K, device="cuda", dtype=torch.bfloat16)
+    gemm.grouped_gemm_fwd(a, w, off, out, live_rows=live, granule=32)
+    gemm.grouped_gemm_dgrad(dy, w, off, dx, live_rows=live, granule=32)
+    gemm.check()
+    for i, n in enumerate(counts):
+        s = int(off[i])
+        _close(out[s:s + n], a[s:s + n].float() @ w[i].float().T)
+        _close(dx[s:s + n], dy[s:s + n].float() @ w[i].float())
 
 
 @pytest.mark.parametrize("swiglu", [False, True])
