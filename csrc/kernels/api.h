@@ -125,11 +125,11 @@ cudaError_t launch_grouped_gemm_pair(GemmMode mode, GemmEpilogue epi, const CUte
                                      const CUtensorMap* map_c2, const GemmArgs& args, int ctas, cudaStream_t stream);
 
 // Weights as operand A, tokens as operand B (grouped_gemm_tokens.cu): forward and dgrad on CTA pairs, tiles of 256 features by
-// up to 256 tokens, the last wave cut into shares of the reduction.
+// up to 256 or 512 tokens, the last wave cut into shares of the reduction.
 constexpr int kTokPartialFloats = 128 * 256;   // fp32 sums of one CTA's part of an accumulator
 constexpr int tok_counters(int ctas) { return 2 * ctas; }                                  // arrival counters a launch needs
 constexpr long long tok_partial_floats(int ctas, int tile_n) { return (tile_n > 256 ? 4ll : 2ll) * ctas * kTokPartialFloats; }  // two partial tiles per CTA
-// Maps of the tokens: entry j loads boxes of {64, 16 << j}. Half a tile's tokens (a multiple of 16 up to 128) are at most three.
+// Maps of the tokens: entry j loads boxes of {64, 16 << j}. Half an accumulator's tokens (a multiple of 16 up to 128) are at most three.
 constexpr int kTokBoxes = 4;
 struct TokMapsX { CUtensorMap box[kTokBoxes]; };
 struct TokGemmMaps {   // bf16, 128-byte swizzle; boxes {inner, outer}

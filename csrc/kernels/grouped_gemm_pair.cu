@@ -55,9 +55,9 @@ constexpr int kThreadsFp8 = kThreads + 32 * kCvtWarps;
 // what they have read from tensor memory in registers that the first four warps have given up.
 // Bound by the power cap, and what it saves is operand traffic: 96 KiB from L2 per block of 64 rows instead of 2 x 64, and a shared-memory
 // reading of operand A for every second product. Seconds at the cap, TFLOP/s, 256 -> 512 columns: 8 experts x 8192 rows, W2 (4096 x 14336)
-// 1306 -> 1432, W13 1240 -> 1413. With few rows the output is the work: us at 16, 64, 256, 512, 1024 rows for W2 273 -> 198, 273 -> 202, 385 -> 306,
-// 470 -> 430, 752 -> 745; for W13 530 -> 378, 530 -> 392, 712 -> 590, 955 -> 867, 1500 -> 1480. Where the last wave would lose more than that:
-// wide_columns in ops/gemm.py.
+// 1306 -> 1432, W13 1240 -> 1413. With few rows the output is the work: us at 16, 64, 256, 512 rows for W2 273 -> 198, 273 -> 202, 385 -> 306,
+// 470 -> 430; for W13 530 -> 378, 530 -> 392, 712 -> 590, 955 -> 867. In between, and where the last wave loses more than that, tiles of 256
+// columns are ahead: wide_columns in ops/gemm.py.
 constexpr int kWideStages = 4;
 constexpr int kWideStageBytes = kABytes + 2 * kBBytes;
 constexpr int kWideFirstEpiWarp = 4;
@@ -105,7 +105,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   constexpr int NS = WIDE ? kWideStages : A_FP8 ? kStagesFp8 : kStages;  // operand stages in use
   constexpr int STAGE = WIDE ? kWideStageBytes : kStageBytes;
   constexpr int ACCS = WIDE ? 2 : 1;                 // accumulators of a tile
-  constexpr int FIRST_EPI_WARP = WIDE ? kWideFirstEpiWarp : 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* q_ring = tiles + NS * STAGE;                                 // A_FP8 only: kQStages x 8 KiB of e4m3

@@ -32,7 +32,8 @@
 // traffic -25 %, active cycles 4 % above the products'. 8 experts x 8192 rows, seconds at the cap, TFLOP/s, 256 -> 512: reduction of 14336
 // 1255 -> 1335; of 28672 1182 -> 1330; 4096 with the SwiGLU backward 1145 -> 1180. The price is that no accumulator is free while a tile
 // is multiplied: what the epilogue needs of tensor memory stands still. So it reads both accumulators into registers (eight warps, with the
-// registers of the others), one a little earlier than the other, and stores from there. The SwiGLU forward, 4 to 6 thousand
+// registers of the others; 104 to 156 bytes a thread of them are spilled, 128 values beside a step of 32), one a little earlier than the
+// other, and stores from there. The SwiGLU forward, 4 to 6 thousand
 // cycles of special-function work before its second accumulator is free, gains nothing (reduction of 4096: 1390 -> 1365) but for groups that
 // one wide tile holds and one of 256 does not. Which calls take wide tiles: ops/gemm.py.
 //
@@ -548,8 +549,9 @@ grouped_gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         if (!ok) break;
         if (sg.parts == 1) release_acc(0);
       } else {
-        // The next tile's first accumulator can be multiplied kLead blocks ahead of the second, so what the tensor pipe waits for is the
-        // reading of the second: values move to registers first and leave from there while the next tile is on its way.
+        // The next tile's first accumulator can be multiplied one block ahead of the second (the first and the last block of a tile, see the MMA
+        // issuer), so what the tensor pipe waits for is the reading of the second: values move to registers first and leave from there while
+        // the next tile is on its way.
         constexpr int kMine = kTokAccN / kStepTokens / SUB;      // steps of a group
         if constexpr (EPI == GemmEpilogue::kSwiGLU) {
           uint32_t keep[kMine][32];                              // the first accumulator; a second leaves straight from tensor memory

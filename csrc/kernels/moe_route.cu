@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(1024) splits_scan_kernel(const SplitsArgs a) {
 // Bound by latency, a chain of dependent steps: the block's read of the gate from L2 (eight 16-byte words of it in flight per lane, the token's
 // row in shared memory), the choice, the meeting of the blocks, the ranks, the scan. A single token meets nobody, and the one routing
 // block's counts go to the scan through shared memory. Thousands of cycles inside, before -> after: 1 token and 8 experts of 1024 14.5 -> 9.7, of 4096
-// 16.5 -> 12, 100 tokens 19 -> 15.5; 8 and 128 tokens and 32 experts of 7168 34 -> 30, 36 -> 33.
+// 16.5 -> 12, 100 tokens 19 -> 15.5; 8 and 128 tokens and 32 experts of 7168 34 -> 30, 36 -> 33. (1024 threads have 64 registers each: 16 bytes are spilled.)
 constexpr int kGateSmallThreads = 1024;
 template <int PER_LANE>
 __global__ void __launch_bounds__(kGateSmallThreads) gate_route_kernel(const GateRouteArgs g, const SplitsArgs sp, unsigned int* ticket) {
