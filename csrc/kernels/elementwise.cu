@@ -288,9 +288,11 @@ __global__ void emb_scatter_kernel(const long long* __restrict__ ids, const int*
 // ---- the whole gradient of an embedding table ------------------------------------------------------------------
 // A warp per table row, after the counting sort: every row is written once, its sum or zeros (cleared beforehand by a kernel of
 // its own, the table cost one more pass of writes: 91 us for 32000 x 4096), in position order: evenly spread ids are bound by HBM.
-// A row with more than kEmbAlone positions is summed by its block's eight warps, 256 columns each and eight positions' loads
-// ahead; by one warp, one load ahead, it was a chain: 32768 skewed ids (one of them 27 %) on 32000 x 4096 took 67.3 ms with the sort,
-// 3.8 now; spread evenly 194 and 198 us, 8192 of them 114 and 114.
+// A warp reads its row's positions once and takes two of them at a time, 512 columns at once. A row with more than kEmbAlone positions is summed
+// by its block's eight warps, 256 columns each and sixteen positions' loads ahead; by one warp, one load ahead, it was a chain. us with the
+// sort, spread evenly, one warp per row with one load ahead -> eight loads ahead in shared rows -> this: 32768 ids on 32000 x 4096
+// 189 -> 197 -> 169, 65536 on 32000 x 2048 174 -> 183 -> 159, 8192 on 32000 x 4096 113 -> 114 -> 107; 32768 skewed (one of them 27 %) on
+// 32000 x 4096 67200 -> 3800 -> 3200.
 constexpr int kEmbAlone = 16;
 __global__ void __launch_bounds__(256) embedding_rows_kernel(const int* __restrict__ start, const long long* __restrict__ perm, const uint4* __restrict__ grad_out, uint4* __restrict__ grad_table, int V, int H) {
   const long long v0 = blockIdx.x * 8ll;
@@ -301,22 +303,34 @@ __global__ void __launch_bounds__(256) embedding_rows_kernel(const int* __restri
   const int begin = __shfl_sync(0xffffffffu, bound, warp), end = __shfl_sync(0xffffffffu, next, warp);
   if (v0 + warp < V && !(shared >> warp & 1)) {
     uint4* out = grad_table + (v0 + warp) * chunks;
-    constexpr int U = 4;   // chunks in flight per row
-    for (int c0 = lane; c0 < chunks; c0 += 32 * U) {
+    const int n = end - begin;
+    const long long pos = lane < n ? __ldg(perm + begin + lane) : 0;
+    constexpr int U = 2;   // chunks in flight per row
+    for (int first_c = 0; first_c < chunks; first_c += 32 * U) {
+      const int c0 = first_c + lane;
       float acc[U][8] = {};
-      for (int j = begin; j < end; ++j) {
-        const uint4* row = grad_out + __ldg(perm + j) * chunks;
-        uint4 x[U];
+      const auto add = [&](int j, auto depth) {   // `depth` positions' loads ahead, added one after the other
+        constexpr int J = decltype(depth)::value;
+        uint4 x[J][U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) x[u] = c0 + 32 * u < chunks ? __ldg(row + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
+        for (int d = 0; d < J; ++d) {
+          const uint4* row = grad_out + static_cast<long long>(__shfl_sync(0xffffffffu, pos, j + d)) * chunks;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          float f[8];
-          unpack8(x[u], f);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+          for (int u = 0; u < U; ++u) x[d][u] = c0 + 32 * u < chunks ? __ldg(row + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
         }
-      }
+#pragma unroll
+        for (int d = 0; d < J; ++d)
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            float f[8];
+            unpack8(x[d][u], f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[u][k] += f[k];
+          }
+      };
+      int j = 0;
+      for (; j + 2 <= n; j += 2) add(j, std::integral_constant<int, 2>());
+      if (j < n) add(j, std::integral_constant<int, 1>());
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (c0 + 32 * u < chunks) __stcs(out + c0 + 32 * u, pack8(acc[u]));
@@ -340,7 +354,8 @@ __global__ void __launch_bounds__(256) embedding_rows_kernel(const int* __restri
         }
       };
       int j = first;
-      for (; j + 8 <= last; j += 8) add(j, std::integral_constant<int, 8>());
+      for (; j + 16 <= last; j += 16) add(j, std::integral_constant<int, 16>());
+      for (; j + 4 <= last; j += 4) add(j, std::integral_constant<int, 4>());
       for (; j < last; ++j) add(j, std::integral_constant<int, 1>());
       __stcs(grad_table + (v0 + i) * chunks + c, pack8(acc));
     }
