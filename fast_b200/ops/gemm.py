@@ -107,20 +107,25 @@ _plans: dict = {}
 
 
 def wide_tiles(epi: int, reduction: int, mean_rows: int, waves: float) -> bool:
-    """Whether tiles of 512 tokens are faster than tiles of 256 for groups of about ``mean_rows`` rows (grouped_gemm_tokens.cu says why);
-    ``waves`` is how many rounds of the GPU they make.
+    """Whether tiles of 512 tokens are taken instead of 256 for groups of about ``mean_rows`` rows (grouped_gemm_tokens.cu says what they
+    save); ``waves`` is how many rounds of the GPU they make. What they save is power, so they are ahead in a stream of GEMMs and behind, or even,
+    in a launch that follows other work; the lines lie where the first is several per cent and the second about nothing. us, 256 -> 512 tokens.
 
-    SwiGLU forward: where a group fits one wide tile but not one of 256; up to 448, so that most groups still do if the mean does. us, 256 ->
-    512 tokens: 8 experts of 4096 x 14336 with 288, 384, 448, 480, 576 rows 617 -> 533, 651 -> 618, 697 -> 671, 823 -> 747, 902 -> 948; 32 of
-    7168 x 2048 with 288, 400, 448, 512 rows 620 -> 510, 785 -> 634, 670 -> 663, 743 -> 747.
-    Others: where tiles are long (the reduction) and many (the rows), so that neither their ends nor the last wave weigh. Reduction of 28672 with
-    768, 1024, 2048, 4096 rows 1082 -> 1081, 1387 -> 1368, 2755 -> 2645, 5838 -> 5323; of 14336 with 512, 1024, 2048 385 -> 503, 694 -> 690,
-    1385 -> 1310; SwiGLU backward, 4096 with 2048 and 4096 rows 1518 -> 1552, 3056 -> 3013, 7168 with 1024 and 2048 771 -> 762, 1536 -> 1482.
-    Cutting the last wave pays for long reductions only: 4096 with 8192 rows in 3.5 waves 176 -> 190 (2 experts, 2048 columns, plain).
-    Shorter reductions lose at any size (plain, 3584 with 4096 rows 178 -> 189; a whole SwiGLU layer, 1024 with 444 rows 115 -> 122)."""
+    SwiGLU forward: where a group fits one wide tile but not one of 256, and tiles are many. In a stream / after other work, 264, 320, 400, 440 rows:
+    32 experts of 7168 x 2048 505 -> 477, 568 -> 534, 635 -> 603, 689 -> 663 / 497 -> 491, 562 -> 552, 640 -> 662, 695 -> 734; 10 of 4096 x 5632 (6
+    waves) 265 -> 250, 290 -> 271, 327 -> 315 / 251 -> 251, 279 -> 271, 292 -> 302. Few tiles: 2 experts of 4096 x 2048 24 -> 48, 16 of them (3.5 waves)
+    173 -> 183, 2 of 4096 x 14336 (3 waves) 157 -> 158 / 164 -> 166.
+    Others: where tiles are long (the reduction) and many (the rows). 8 experts, reduction of 28672 with 440, 560, 750, 832, 2048 rows 682 -> 874, 870 -> 840,
+    1182 -> 1060, 1246 -> 1145, 2966 -> 2778 / 560 rows 867 -> 926, 750 and 832 1151 -> 1139, 1285 -> 1215; of 14336 with 640, 1024, 1536, 4096 rows
+    470 -> 450, 718 -> 718, 1111 -> 1053, 2796 -> 2460 / 454 -> 476, 741 -> 773, 1128 -> 1154; of 4096 with the SwiGLU backward and 4096, 8192 rows 2973 ->
+    2794, 5912 -> 5426 / 3130 -> 3134, 6623 -> 6656. Below three waves (2 experts, 14336, 1536 and 3000 rows) 263 -> 279, 501 -> 494 / 310 -> 370,
+    494 -> 554. Whole training steps of 1800 tokens (450 rows) with the data gradient of W13 wide 9920 -> 10190, of 4096, 16384, 32768 tokens against
+    no wide tiles at all 13735 -> 13440, 35400 -> 33900, 66100 -> 61200. Shorter reductions lose at any size (plain, 3584 with 4096 rows 178 -> 189; a whole SwiGLU layer, 1024 with 444 rows 115 -> 122)."""
     if reduction < 4096:
         return False
-    return 256 < mean_rows <= 448 if epi == SWIGLU else mean_rows * reduction >= 12 << 20 and (reduction >= 8192 or waves >= 6)
+    if epi == SWIGLU:
+        return 272 <= mean_rows <= 368 and waves >= 5.5
+    return mean_rows * reduction >= 16 << 20 and waves >= (3 if reduction >= 8192 else 6)
 
 
 def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, gu: Optional[torch.Tensor]) -> tuple:

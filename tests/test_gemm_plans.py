@@ -43,3 +43,15 @@ def test_tiles_are_not_sized_by_a_capacity():
         assert T == 4096 or tile == 256
     assert gemm.group_rows_hint(0, 8192, 8, None) == 1024 and gemm.group_rows_hint(0, 8192, 8, torch.empty(8)) == 0
     assert gemm.token_tile(gemm.STORE, 28672, 0, 0, 8, 4096, 74) == gemm.token_tile(gemm.SWIGLU, 4096, 0, 0, 8, 28672, 74) == 256
+
+
+def test_wide_tiles_only_where_they_are_not_slower():
+    """Sizes at which tiles of 512 tokens or columns were measured slower get tiles of 256, and those that they are for get them."""
+    def tokens(epi, groups, features, reduction, rows):
+        return gemm.token_tile(epi, reduction, 0, rows, groups, features, 74)
+
+    assert tokens(gemm.SWIGLU, 2, 4096, 4096, 320) == tokens(gemm.SWIGLU, 16, 4096, 4096, 320) == 256      # 24 -> 48, 166 -> 174 us
+    assert tokens(gemm.SWIGLU, 8, 28672, 4096, 440) == 256 and tokens(gemm.SWIGLU, 32, 4096, 7168, 320) == 512
+    assert tokens(gemm.STORE, 8, 4096, 28672, 450) == tokens(gemm.STORE, 8, 4096, 28672, 560) == 256      # a training step of 1800 tokens 9944 -> 10307
+    assert tokens(gemm.STORE, 8, 4096, 14336, 1024) == tokens(gemm.STORE, 2, 4096, 14336, 3000) == 256
+    assert tokens(gemm.STORE, 8, 4096, 28672, 8192) == tokens(gemm.STORE, 8, 4096, 14336, 4096) == tokens(gemm.SWIGLU_BWD, 8, 14336, 4096, 8192) == 512
