@@ -138,16 +138,19 @@ def _plan_key(mode: int, epi: int, granule: int, w: torch.Tensor, x: torch.Tenso
 
 def wide_columns(row_tiles: int, columns: int, pairs: int, mean_rows: int) -> bool:
     """Whether weight gradients take tiles of 512 columns instead of 256 (grouped_gemm_pair.cu). Few rows: the tile's way out is the time, and half
-    as many pass through. Many: the power cap is, and operand traffic saved is clock won. Between them neither, and two tiles of 256 in turn
-    keep the tensor cores busier: us between other work, as in a step, W2 / W13 of 8 experts of 4096 x 14336 at 640, 768, 1024, 1280, 1536, 2048 rows
-    452 / 888 -> 438 / 867, 496 / 984 -> 504 / 1003, 620 / 1263 -> 642 / 1283, 767 / 1562 -> 780 / 1566, 906 / 1826 -> 916 / 1824, 1201 / 2454 ->
-    1201 / 2419. And tiles twice as large can leave more of the last wave idle, which counts once there is more to multiply than to store: 8
-    experts of 3584 x 1024, 4 waves instead of 3.5 (W2) and 7 instead of 6.5 (W13), 256 rows 28.6 -> 26.3 and 53 -> 45, 1024 rows 57.5 -> 62.7 and
-    101.6 -> 109.7 us."""
-    if columns % 512 or 704 <= mean_rows < 1536:
+    as many pass through; but tiles twice as large can leave more of the last wave idle, or of the only one. Many: the power cap is, and operand
+    traffic saved is clock won. Between them neither, and two tiles of 256 in turn keep the tensor cores busier. us after other work, 256 -> 512 columns,
+    16, 256, 500, 600, 660, 1600 rows: 8 experts of 4096 x 14336 277 -> 201, 368 -> 263, 460 -> 416, 508 -> 495, 532 -> 529, 1058 -> 1123; 32 of 1024 x 2048 (14 waves
+    to 7) 54 -> 42, 61 -> 49, 76 -> 66, 78 -> 76, 80 -> 80, 177 -> 185; 8 of 2048 x 2048 (7 to 4) 28.7 -> 24.6, 32.8 -> 30.8, 41 -> 41, 43 -> 45, 45 -> 49, 74 -> 84; 4 of
+    them (4 to 2) 20.5 -> 18.5, 22.6 -> 20.5, 26.6 -> 26.6, 28.7 -> 28.7, 28.7 -> 30.7, 47 -> 49; 8 of 1024 x 1024 (2 to 1) 14.3 -> 14.3, 16.4 -> 16.4, 18.4 -> 20.5;
+    2 of them (1 to 1) 12.3 -> 14.3, 12.3 -> 16.3, 14.3 -> 18.4. In a stream, W13 of 8 of 4096 x 14336 with 1536, 2048, 4096, 8192 rows 1920 -> 1892, 2486 -> 2447,
+    4897 -> 4850, 12177 -> 11402; whole training steps of 8192 tokens (2048 rows) 20200 -> 20120."""
+    if columns % 512:
         return False
-    waves = lambda tiles: -(-tiles // pairs)
-    return mean_rows < 512 or 50 * waves(row_tiles * (columns // 512)) <= 26 * waves(row_tiles * (columns // 256))
+    narrow, wide = (-(-row_tiles * (columns // n) // pairs) for n in (256, 512))
+    if mean_rows < 512:
+        return narrow >= 4 and 14 * wide <= 8 * narrow
+    return (narrow >= 14 if mean_rows <= 640 else mean_rows >= 1536) and 50 * wide <= 26 * narrow
 
 
 def token_tile(epi: int, reduction: int, most_rows: int, mean_rows: int, groups: int, features: int, pairs: int) -> int:

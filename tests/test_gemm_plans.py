@@ -55,3 +55,8 @@ def test_wide_tiles_only_where_they_are_not_slower():
     assert tokens(gemm.STORE, 8, 4096, 28672, 450) == tokens(gemm.STORE, 8, 4096, 28672, 560) == 256      # a training step of 1800 tokens 9944 -> 10307
     assert tokens(gemm.STORE, 8, 4096, 14336, 1024) == tokens(gemm.STORE, 2, 4096, 14336, 3000) == 256
     assert tokens(gemm.STORE, 8, 4096, 28672, 8192) == tokens(gemm.STORE, 8, 4096, 14336, 4096) == tokens(gemm.SWIGLU_BWD, 8, 14336, 4096, 8192) == 512
+    columns = lambda groups, n, k, rows: gemm.wide_columns(groups * (n // 256), k, 74, rows)
+    assert not any(columns(2, 1024, 1024, r) or columns(8, 1024, 1024, r) for r in (1, 16, 256, 400, 500, 600))   # 12 -> 16 us
+    assert not any(columns(8, 4096, 14336, r) for r in (660, 1024, 1500)) and not columns(4, 2048, 2048, 600)
+    assert all(columns(8, 4096, 14336, r) for r in (1, 256, 500, 600, 2048, 8192)) and columns(4, 2048, 2048, 256) and columns(8, 2048, 2048, 400)
+    assert not columns(8, 2048, 768, 16)
