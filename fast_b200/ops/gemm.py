@@ -119,8 +119,8 @@ def wide_tiles(epi: int, reduction: int, mean_rows: int, waves: float) -> bool:
     1182 -> 1060, 1246 -> 1145, 2966 -> 2778 / 560 rows 867 -> 926, 750 and 832 1151 -> 1139, 1285 -> 1215; of 14336 with 640, 1024, 1536, 4096 rows
     470 -> 450, 718 -> 718, 1111 -> 1053, 2796 -> 2460 / 454 -> 476, 741 -> 773, 1128 -> 1154; of 4096 with the SwiGLU backward and 4096, 8192 rows 2973 ->
     2794, 5912 -> 5426 / 3130 -> 3134, 6623 -> 6656. Below three waves (2 experts, 14336, 1536 and 3000 rows) 263 -> 279, 501 -> 494 / 310 -> 370,
-    494 -> 554. Whole training steps of 1800 tokens (450 rows) with the data gradient of W13 wide 9920 -> 10190, of 4096, 16384, 32768 tokens against
-    no wide tiles at all 13735 -> 13440, 35400 -> 33900, 66100 -> 61200. Shorter reductions lose at any size (plain, 3584 with 4096 rows 178 -> 189; a whole SwiGLU layer, 1024 with 444 rows 115 -> 122)."""
+    494 -> 554. Whole training steps of 1800 tokens (450 rows) with the data gradient of W13 wide 9920 -> 10190, of 12000, 16384, 32768 tokens
+    against no wide tiles at all 26740 -> 25920, 34750 -> 33330, 66200 -> 61230. Shorter reductions lose at any size (plain, 3584 with 4096 rows 178 -> 189; a whole SwiGLU layer, 1024 with 444 rows 115 -> 122)."""
     if reduction < 4096:
         return False
     if epi == SWIGLU:
@@ -144,7 +144,7 @@ def wide_columns(row_tiles: int, columns: int, pairs: int, mean_rows: int) -> bo
     to 7) 54 -> 42, 61 -> 49, 76 -> 66, 78 -> 76, 80 -> 80, 177 -> 185; 8 of 2048 x 2048 (7 to 4) 28.7 -> 24.6, 32.8 -> 30.8, 41 -> 41, 43 -> 45, 45 -> 49, 74 -> 84; 4 of
     them (4 to 2) 20.5 -> 18.5, 22.6 -> 20.5, 26.6 -> 26.6, 28.7 -> 28.7, 28.7 -> 30.7, 47 -> 49; 8 of 1024 x 1024 (2 to 1) 14.3 -> 14.3, 16.4 -> 16.4, 18.4 -> 20.5;
     2 of them (1 to 1) 12.3 -> 14.3, 12.3 -> 16.3, 14.3 -> 18.4. In a stream, W13 of 8 of 4096 x 14336 with 1536, 2048, 4096, 8192 rows 1920 -> 1892, 2486 -> 2447,
-    4897 -> 4850, 12177 -> 11402; whole training steps of 8192 tokens (2048 rows) 20200 -> 20120."""
+    4897 -> 4850, 12177 -> 11402; whole training steps of 8192 tokens (2048 rows) 20050 -> 20065."""
     if columns % 512:
         return False
     narrow, wide = (-(-row_tiles * (columns // n) // pairs) for n in (256, 512))
